@@ -67,15 +67,22 @@ void* ws_get(scrust_context* ctx, Slot slot, size_t bytes, cudaError_t* err) {
 }
 
 cudaError_t set_smem_limit(scrust_context* ctx, const void* func, int bytes) {
-    for (auto& pr : ctx->smem_limits)
-        if (pr.first == func) {
+    // The attribute belongs to the function on the device, not to a context:
+    // one record for all contexts, so that none lowers a limit another one
+    // has set and launches with.
+    static std::mutex mu;
+    static std::vector<std::pair<std::pair<int, const void*>, int>> limits;
+    const std::pair<int, const void*> key(ctx->device, func);
+    std::lock_guard<std::mutex> lock(mu);
+    for (auto& pr : limits)
+        if (pr.first == key) {
             if (pr.second >= bytes) return cudaSuccess;
             const cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
             if (e == cudaSuccess) pr.second = bytes;
             return e;
         }
     const cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) ctx->smem_limits.emplace_back(func, bytes);
+    if (e == cudaSuccess) limits.emplace_back(key, bytes);
     return e;
 }
 

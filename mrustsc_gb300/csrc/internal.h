@@ -138,8 +138,7 @@ struct scrust_context {
     bool timing = false;
     cudaEvent_t ev[9] = {};             // phase boundaries: prep | candidates | rerank | connectivities, and
     bool ev_recorded[9] = {};           // inside candidates: sweep pass 1 | tile lists | pass 2 | collect 1
-    std::vector<std::pair<const void*, int>> smem_limits;  // dynamic shared memory limits already set
-    std::vector<const void*> carveouts;                      // kernels whose shared-memory carveout is set
+    std::vector<const void*> carveouts;  // kernels whose shared-memory carveout is set
 };
 
 struct scrust_csr {
@@ -179,8 +178,9 @@ int32_t fail(scrust_status* st, int32_t code, const char* fmt, ...);
 int32_t ok(scrust_status* st);
 int32_t cuda_fail(scrust_status* st, cudaError_t e, const char* what);
 
-// Raises a kernel's dynamic shared memory limit once per context (so that
-// launches can be captured into a CUDA graph afterwards).
+// Raises a kernel's dynamic shared memory limit on the context's device, once
+// (so that launches can be captured into a CUDA graph afterwards); never
+// lowers it.
 cudaError_t set_smem_limit(scrust_context* ctx, const void* func, int bytes);
 // Preferred shared-memory carveout (percent of the unified L1/shared memory),
 // set once per context and kernel.

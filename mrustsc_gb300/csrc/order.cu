@@ -975,6 +975,8 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
         ctx->launches += 2;
     }
     anchor_chain_kernel<<<1, kChainThreads, chain_smem, ctx->copy_stream>>>(anchor_nb, (int)m, rank);
+    // The relabelling indexes by rank: never launched without the walk.
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: anchor walk");
     relabel_neighbours_kernel<<<(unsigned)((m * kAnchorNeighbours + 255) / 256), 256, 0, ctx->copy_stream>>>(
         anchor_nb, rank, (int)m, cell_nb);
     if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaEventRecord(ctx->copy_ev, ctx->copy_stream)) != cudaSuccess)
