@@ -150,103 +150,283 @@ __global__ void umap_rescale_kernel(int64_t n, int dim, const uint32_t* __restri
 
 // One epoch, the cells' own edges: attraction of every firing edge (its
 // tail's move kept in tmove) and the negative samples, summed per cell in
-// row order into own.
-__global__ void umap_rows_kernel(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
-                                 int64_t n, int dim, double now, float alpha, float a, float b, int neg_rate,
-                                 const float* __restrict__ y, const double* __restrict__ eps,
-                                 const double* __restrict__ eps_neg, double* __restrict__ next,
-                                 double* __restrict__ next_neg, Tau* __restrict__ rng, float* __restrict__ tmove,
-                                 float* __restrict__ own) {
-    const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= n) return;
-    float yh[kUmapMaxDim], acc[kUmapMaxDim];
+// row order into own -- the bits of one thread walking each row.
+//
+// A block takes kRows consecutive cells, whose edges are one run of the CSR,
+// and goes through them in chunks of kEdges: (1) one thread per edge tests
+// the schedule and computes the attraction, the firing ones compacted in
+// order; (2) one lane per cell steps its stream of draws; (3) one thread per
+// draw computes a repulsion; (4) one thread per cell and component adds the
+// cell's moves in order, attraction then samples, edge by edge.  Draws beyond
+// kDraws go through in windows, the streams and sums carrying on.  What bounds
+// it is issue: two or three powf and divisions per move.  A thread per cell
+// left it to the latency of ~60 moves in a row (613 us an epoch for 30,000
+// cells of 23 edges, 2 components); eight lanes a cell took 131 us, a sixth of
+// its instructions stepping streams in lockstep and its last fifth waiting
+// for cells of five times the mean degree.  DIM: components (0: `dim`, up to
+// kUmapMaxDim).
+template <int DIM>
+struct UmapShape {
+    static constexpr int kDim = DIM ? DIM : kUmapMaxDim;
+    static constexpr int kRows = DIM ? 32 : 16;
+    static constexpr int kEdges = DIM ? 1024 : 256;   // a multiple of the block's threads
+    static constexpr int kDraws = DIM ? 2048 : 256;
+};
+constexpr int kUmapRowThreads = 256;
+
+// The i in [0, count) with at[i] <= x < at[i + 1] (at ascending, count a
+// power of two, x in [at[0], at[count])).
+template <int COUNT>
+__device__ __forceinline__ int umap_owner(const uint32_t* at, uint32_t x) {
+    int i = 0;
 #pragma unroll
-    for (int d = 0; d < kUmapMaxDim; ++d) {
-        yh[d] = d < dim ? y[h * dim + d] : 0.f;
-        acc[d] = 0.f;
-    }
-    Tau t = rng[h];
-    const float two_ab = __fmul_rn(__fmul_rn(-2.0f, a), b);
-    const float two_b = __fmul_rn(2.0f, b);  // 2 * REPULSION_STRENGTH(1) * b
-    for (uint32_t e = indptr[h], e1 = indptr[h + 1]; e < e1; ++e) {
-        if (next[e] > now) {
-            for (int d = 0; d < dim; ++d) tmove[(int64_t)e * dim + d] = 0.f;
-            continue;
-        }
-        const int64_t tail = indices[e];
-        float dist = 0.f;
-#pragma unroll
-        for (int d = 0; d < kUmapMaxDim; ++d) {
-            if (d < dim) {
-                const float diff = __fsub_rn(yh[d], y[tail * dim + d]);
-                dist = __fadd_rn(dist, __fmul_rn(diff, diff));
-            }
-        }
-        float coef = 0.f;
-        if (dist > 0.f)
-            coef = __fdiv_rn(__fmul_rn(two_ab, powf(dist, __fsub_rn(b, 1.0f))),
-                             __fadd_rn(__fmul_rn(a, powf(dist, b)), 1.0f));
-#pragma unroll
-        for (int d = 0; d < kUmapMaxDim; ++d) {
-            if (d < dim) {
-                const float g = clip4(__fmul_rn(coef, __fsub_rn(yh[d], y[tail * dim + d])));
-                const float step = __fmul_rn(g, alpha);
-                acc[d] = __fadd_rn(acc[d], step);
-                tmove[(int64_t)e * dim + d] = step;
-            }
-        }
-        next[e] += eps[e];
-        if (neg_rate == 0) continue;
-        double q = (now - next_neg[e]) / eps_neg[e];
-        const int64_t n_neg = q > 0.0 ? (int64_t)q : 0;
-        for (int64_t s = 0; s < n_neg; ++s) {
-            const int64_t j = (int64_t)(tau_next(t) % (uint32_t)n);
-            if (j == h) continue;
-            float dj = 0.f;
-#pragma unroll
-            for (int d = 0; d < kUmapMaxDim; ++d) {
-                if (d < dim) {
-                    const float diff = __fsub_rn(yh[d], y[j * dim + d]);
-                    dj = __fadd_rn(dj, __fmul_rn(diff, diff));
-                }
-            }
-            if (dj <= 0.f) continue;
-            const float cr = __fdiv_rn(two_b, __fmul_rn(__fadd_rn(kRepulsionEps, dj),
-                                                          __fadd_rn(__fmul_rn(a, powf(dj, b)), 1.0f)));
-#pragma unroll
-            for (int d = 0; d < kUmapMaxDim; ++d)
-                if (d < dim)
-                    acc[d] = __fadd_rn(acc[d], __fmul_rn(clip4(__fmul_rn(cr, __fsub_rn(yh[d], y[j * dim + d]))),
-                                                         alpha));
-        }
-        next_neg[e] += (double)n_neg * eps_neg[e];
-    }
-    rng[h] = t;
-#pragma unroll
-    for (int d = 0; d < kUmapMaxDim; ++d)
-        if (d < dim) own[h * dim + d] = acc[d];
+    for (int o = COUNT / 2; o > 0; o >>= 1)
+        if (at[i + o] <= x) i += o;
+    return i;
 }
 
-// One epoch, the moves a cell receives as the tail of its incoming edges, in
-// edge order, then the cell's next position.
-__global__ void umap_apply_kernel(int64_t n, int dim, const uint32_t* __restrict__ tstart,
-                                  const unsigned long long* __restrict__ tedge, const float* __restrict__ tmove,
-                                  const float* __restrict__ own, const float* __restrict__ y,
-                                  float* __restrict__ y_next) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    float acc[kUmapMaxDim];
+template <int DIM>
+__global__ void __launch_bounds__(kUmapRowThreads)
+    umap_rows_kernel(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices, int64_t n, int dim_,
+                     double now, float alpha, float a, float b, int neg_rate, const float* __restrict__ y,
+                     const double* __restrict__ eps, const double* __restrict__ eps_neg, double* __restrict__ next,
+                     double* __restrict__ next_neg, Tau* __restrict__ rng, float* __restrict__ tmove,
+                     float* __restrict__ own) {
+    using S = UmapShape<DIM>;
+    constexpr int MAXD = S::kDim, R = S::kRows, E = S::kEdges, D = S::kDraws, T = kUmapRowThreads;
+    static_assert(R <= 32 && R * MAXD <= T && E % T == 0, "one warp of streams, one thread per sum");
+    const int dim = DIM ? DIM : dim_;
+    __shared__ uint32_t ip[R + 1];              // the cells' first edges
+    __shared__ float yrow[R][MAXD];
+    __shared__ float fstep[E][MAXD];            // the chunk's firing edges in order: attraction,
+    __shared__ uint32_t fneg[E];                // and samples
+    __shared__ uint32_t fstart[R + 1];          // the cells' first firing edges
+    __shared__ uint32_t fcount[R];
+    __shared__ unsigned long long dcount[R];
+    __shared__ uint32_t dstart[R + 1];          // the cells' first draws in the window
+    __shared__ unsigned long long dtotal;
+    __shared__ float rep[D][MAXD];              // the window's draws (in [.][0] as bits), then their moves
+    __shared__ uint32_t warp_fires[T / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t h0 = (int64_t)blockIdx.x * R;
+    const int rows = (int)min((int64_t)R, n - h0);
+    for (int i = tid; i <= R; i += T) ip[i] = indptr[h0 + min(i, rows)];
+    for (int i = tid; i < rows * dim; i += T) yrow[i / dim][i % dim] = y[h0 * dim + i];
+    const float two_ab = __fmul_rn(__fmul_rn(-2.0f, a), b);
+    const float two_b = __fmul_rn(2.0f, b);  // 2 * REPULSION_STRENGTH(1) * b
+    Tau t{0u, 0u, 0u};                       // warp 0: lane r's stream
+    if (tid < rows) t = rng[h0 + tid];
+    const int sr = tid / MAXD, sd = tid % MAXD;  // the sum this thread keeps
+    const bool sums = sr < rows && sd < dim;
+    float acc = 0.f;
+    __syncthreads();
+    const uint32_t e_end = ip[R];
+    for (uint32_t c0 = ip[0]; c0 < e_end; c0 += E) {
+        if (tid < R) {
+            fcount[tid] = 0;
+            dcount[tid] = 0;
+        }
+        __syncthreads();
+        uint32_t fired = 0;  // of the chunk, before this pass
+        for (uint32_t p = c0; p < min(c0 + (uint32_t)E, e_end); p += T) {
+            const uint32_t e = p + tid;
+            const bool in = e < e_end;
+            const double nx = in ? next[e] : 0.0;
+            const bool fires = in && !(nx > now);
+            uint32_t n32 = 0;
+            float step[MAXD];
+            if (in && !fires)
+                for (int d = 0; d < dim; ++d) tmove[(int64_t)e * dim + d] = 0.f;
+            if (fires) {
+                const int r = umap_owner<R>(ip, e);
+                const int64_t tail = indices[e];
+                float yt[MAXD];
+                float dist = 0.f;
 #pragma unroll
-    for (int d = 0; d < kUmapMaxDim; ++d) acc[d] = d < dim ? own[v * dim + d] : 0.f;
-    for (uint32_t p = tstart[v], p1 = tstart[v + 1]; p < p1; ++p) {
-        const int64_t e = (int64_t)(tedge[p] & 0xffffffffull);
+                for (int d = 0; d < MAXD; ++d) {
+                    if (d < dim) {
+                        yt[d] = y[tail * dim + d];
+                        const float diff = __fsub_rn(yrow[r][d], yt[d]);
+                        dist = __fadd_rn(dist, __fmul_rn(diff, diff));
+                    }
+                }
+                float coef = 0.f;
+                if (dist > 0.f)
+                    coef = __fdiv_rn(__fmul_rn(two_ab, powf(dist, __fsub_rn(b, 1.0f))),
+                                     __fadd_rn(__fmul_rn(a, powf(dist, b)), 1.0f));
 #pragma unroll
-        for (int d = 0; d < kUmapMaxDim; ++d)
-            if (d < dim) acc[d] = __fsub_rn(acc[d], tmove[e * dim + d]);
+                for (int d = 0; d < MAXD; ++d) {
+                    if (d < dim) {
+                        step[d] = __fmul_rn(clip4(__fmul_rn(coef, __fsub_rn(yrow[r][d], yt[d]))), alpha);
+                        tmove[(int64_t)e * dim + d] = step[d];
+                    }
+                }
+                next[e] = nx + eps[e];
+                if (neg_rate != 0) {
+                    const double en = eps_neg[e], nn = next_neg[e];
+                    const double q = (now - nn) / en;
+                    const int64_t n_neg = q > 0.0 ? (int64_t)q : 0;
+                    next_neg[e] = nn + (double)n_neg * en;
+                    n32 = (uint32_t)min(n_neg, (int64_t)0xffffffff);
+                }
+                atomicAdd(&fcount[r], 1u);
+                atomicAdd(&dcount[r], (unsigned long long)n32);
+            }
+            // The firing edges keep their order in the compacted list.
+            const uint32_t ballot = __ballot_sync(0xffffffffu, fires);
+            if (lane == 0) warp_fires[warp] = __popc(ballot);
+            __syncthreads();
+            uint32_t before = fired;
+#pragma unroll
+            for (int i = 0; i < T / 32; ++i) {
+                const uint32_t f = warp_fires[i];
+                if (i < warp) before += f;
+                fired += f;
+            }
+            if (fires) {
+                const uint32_t at = before + __popc(ballot & ((1u << lane) - 1u));
+#pragma unroll
+                for (int d = 0; d < MAXD; ++d)
+                    if (d < dim) fstep[at][d] = step[d];
+                fneg[at] = n32;
+            }
+            __syncthreads();
+        }
+        // Where each cell's firing edges and draws begin (warp 0, lane r).
+        unsigned long long d_end = 0, d_begin = 0;
+        if (warp == 0) {
+            uint32_t f_end = lane < R ? fcount[lane] : 0u;
+            d_end = lane < R ? dcount[lane] : 0ull;
+            d_begin = d_end;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t fu = __shfl_up_sync(0xffffffffu, f_end, o);
+                const unsigned long long du = __shfl_up_sync(0xffffffffu, d_end, o);
+                if (lane >= o) {
+                    f_end += fu;
+                    d_end += du;
+                }
+            }
+            d_begin = d_end - d_begin;
+            if (lane < R) fstart[lane + 1] = f_end;
+            if (lane == 0) fstart[0] = 0;
+            if (lane == 31) dtotal = d_end;
+        }
+        __syncthreads();
+        uint32_t fcur = sums ? fstart[sr] : 0u, f_last = sums ? fstart[sr + 1] : 0u;
+        uint32_t left = 0;  // samples of the current edge not yet added
+        unsigned long long w0 = 0;
+        do {
+            if (warp == 0) {
+                // This window's draws of each cell, from its stream.
+                const unsigned long long w1 = w0 + D;
+                const uint32_t lo = (uint32_t)(min(max(d_begin, w0), w1) - w0);
+                const uint32_t hi = (uint32_t)(min(max(d_end, w0), w1) - w0);
+                if (lane < R) dstart[lane + 1] = hi;
+                if (lane == 0) dstart[0] = 0;
+                for (uint32_t i = lo; i < hi; ++i) rep[i][0] = __uint_as_float(tau_next(t));
+            }
+            __syncthreads();
+            const uint32_t draws = dstart[R];
+            for (uint32_t i = tid; i < draws; i += T) {
+                const int r = umap_owner<R>(dstart, i);
+                const int64_t j = (int64_t)(__float_as_uint(rep[i][0]) % (uint32_t)n);
+                float mv[MAXD];
+#pragma unroll
+                for (int d = 0; d < MAXD; ++d) mv[d] = 0.f;
+                if (j != h0 + r) {
+                    float diff[MAXD];
+                    float dj = 0.f;
+#pragma unroll
+                    for (int d = 0; d < MAXD; ++d) {
+                        if (d < dim) {
+                            diff[d] = __fsub_rn(yrow[r][d], y[j * dim + d]);
+                            dj = __fadd_rn(dj, __fmul_rn(diff[d], diff[d]));
+                        }
+                    }
+                    if (!(dj <= 0.f)) {
+                        const float cr = __fdiv_rn(two_b, __fmul_rn(__fadd_rn(kRepulsionEps, dj),
+                                                                    __fadd_rn(__fmul_rn(a, powf(dj, b)), 1.0f)));
+#pragma unroll
+                        for (int d = 0; d < MAXD; ++d)
+                            if (d < dim) mv[d] = __fmul_rn(clip4(__fmul_rn(cr, diff[d])), alpha);
+                    }
+                }
+                // A draw without a move adds +0, which changes no sum that
+                // began at +0.
+#pragma unroll
+                for (int d = 0; d < MAXD; ++d)
+                    if (d < dim) rep[i][d] = mv[d];
+            }
+            __syncthreads();
+            if (sums) {
+                uint32_t at = dstart[sr];
+                const uint32_t end = dstart[sr + 1];
+                for (;;) {
+                    if (left == 0) {
+                        if (fcur == f_last) break;
+                        acc = __fadd_rn(acc, fstep[fcur][sd]);
+                        left = fneg[fcur];
+                        ++fcur;
+                    } else {
+                        const uint32_t m = min(left, end - at);
+                        if (m == 0) break;  // the rest comes in a later window
+                        for (uint32_t i = 0; i < m; ++i) acc = __fadd_rn(acc, rep[at + i][sd]);
+                        at += m;
+                        left -= m;
+                    }
+                }
+            }
+            w0 += D;
+            __syncthreads();
+        } while (w0 < dtotal);
     }
+    if (tid < rows) rng[h0 + tid] = t;
+    if (sums) own[(h0 + sr) * dim + sd] = acc;
+}
+
+// Lanes that share one cell in the apply kernel: its ~23 incoming edges are
+// fetched eight at a time (57 us an epoch for 30,000 cells with one thread per
+// cell, 10 us so).
+constexpr int kUmapLanes = 8;
+constexpr int kUmapThreads = 128;
+
+// One epoch, the moves a cell receives as the tail of its incoming edges, in
+// edge order, then the cell's next position.  kUmapLanes lanes per cell fetch
+// the moves; their sum runs through the lanes in edge order.
+template <int DIM>
+__global__ void __launch_bounds__(kUmapThreads)
+    umap_apply_kernel(int64_t n, int dim_, const uint32_t* __restrict__ tstart, const uint32_t* __restrict__ tedge,
+                      const float* __restrict__ tmove, const float* __restrict__ own, const float* __restrict__ y,
+                      float* __restrict__ y_next) {
+    constexpr int MAXD = DIM ? DIM : kUmapMaxDim;
+    constexpr uint32_t FULL = 0xffffffffu;
+    const int dim = DIM ? DIM : dim_;
+    const int g = threadIdx.x & (kUmapLanes - 1);
+    const int64_t v = ((int64_t)blockIdx.x * kUmapThreads + threadIdx.x) / kUmapLanes;
+    const bool cell = v < n;
+    float acc[MAXD];
 #pragma unroll
-    for (int d = 0; d < kUmapMaxDim; ++d)
-        if (d < dim) y_next[v * dim + d] = __fadd_rn(y[v * dim + d], acc[d]);
+    for (int d = 0; d < MAXD; ++d) acc[d] = cell && d < dim ? own[v * dim + d] : 0.f;
+    const uint32_t p0 = cell ? tstart[v] : 0u, len = cell ? tstart[v + 1] - p0 : 0u;
+    const uint32_t longest = __reduce_max_sync(FULL, len);
+    for (uint32_t c = 0; c < longest; c += kUmapLanes) {
+        float mv[MAXD];
+        const bool in = c + g < len;
+        const int64_t e = in ? (int64_t)tedge[p0 + c + g] : 0;
+#pragma unroll
+        for (int d = 0; d < MAXD; ++d) mv[d] = in && d < dim ? tmove[e * dim + d] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kUmapLanes; ++i)
+#pragma unroll
+            for (int d = 0; d < MAXD; ++d)
+                if (d < dim) acc[d] = __fsub_rn(acc[d], __shfl_sync(FULL, mv[d], i, kUmapLanes));
+    }
+    if (cell && g == 0) {
+#pragma unroll
+        for (int d = 0; d < MAXD; ++d)
+            if (d < dim) y_next[v * dim + d] = __fadd_rn(y[v * dim + d], acc[d]);
+    }
 }
 
 __global__ void umap_keys_kernel(const uint32_t* __restrict__ indices, int64_t nnz, uint32_t* __restrict__ keys,
@@ -257,11 +437,14 @@ __global__ void umap_keys_kernel(const uint32_t* __restrict__ indices, int64_t n
     vals[e] = (unsigned long long)e;
 }
 
-// start[c] = number of sorted keys below c, for c in [0, n].
-__global__ void umap_starts_kernel(const uint32_t* __restrict__ keys, int64_t nnz, int64_t n,
-                                   uint32_t* __restrict__ start) {
+// start[c] = number of sorted keys below c, for c in [0, n]; the sorted edges
+// as 32-bit ids.
+__global__ void umap_starts_kernel(const uint32_t* __restrict__ keys, const unsigned long long* __restrict__ edges,
+                                   int64_t nnz, int64_t n, uint32_t* __restrict__ start,
+                                   uint32_t* __restrict__ tedge) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p > nnz) return;
+    if (p < nnz) tedge[p] = (uint32_t)edges[p];
     const int64_t lo = p == 0 ? 0 : (int64_t)keys[p - 1] + 1;
     const int64_t hi = p == nnz ? n : (int64_t)keys[p];
     for (int64_t c = lo; c <= hi && c <= n; ++c) start[c] = (uint32_t)p;
@@ -418,7 +601,8 @@ int32_t umap_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint
     if ((e = radix_sort_pairs(ctx, kA, vA, kB, vB, nnz, bits, (uint32_t*)(base + o_hist), (uint32_t*)(base + o_scan),
                               scan_elems, &keys, &vals)) != cudaSuccess)
         return cuda_fail(st, e, "umap: transpose");
-    umap_starts_kernel<<<(unsigned)((nnz + 1 + 255) / 256), 256, 0, s>>>(keys, nnz, n, tstart);
+    uint32_t* tedge = keys == kA ? kB : kA;  // the sort's other key buffer
+    umap_starts_kernel<<<(unsigned)((nnz + 1 + 255) / 256), 256, 0, s>>>(keys, vals, nnz, n, tstart, tedge);
     const unsigned vb = (unsigned)((n + 127) / 128);
     umap_init_kernel<<<vb, 128, 0, s>>>(n, dim, p.seed, out, lo, hi, rng);
     umap_rescale_kernel<<<(unsigned)((n * dim + 255) / 256), 256, 0, s>>>(n, dim, lo, hi, out);
@@ -426,11 +610,17 @@ int32_t umap_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint
     float* cur = out;
     float* nxt = y2;
     float alpha = p.learning_rate;
+    const auto rows = dim == 2 ? umap_rows_kernel<2> : dim == 3 ? umap_rows_kernel<3> : umap_rows_kernel<0>;
+    const auto apply = dim == 2 ? umap_apply_kernel<2> : dim == 3 ? umap_apply_kernel<3> : umap_apply_kernel<0>;
+    const int block_rows = dim == 2 || dim == 3 ? UmapShape<2>::kRows : UmapShape<0>::kRows;
+    static_assert(UmapShape<2>::kRows == UmapShape<3>::kRows, "one grid for both");
+    const unsigned rb = (unsigned)((n + block_rows - 1) / block_rows);
+    const unsigned gb = (unsigned)((n * kUmapLanes + kUmapThreads - 1) / kUmapThreads);
     for (uint32_t epoch = 0; epoch < p.n_epochs; ++epoch) {
-        umap_rows_kernel<<<vb, 128, 0, s>>>(indptr, indices, n, dim, (double)epoch, alpha, a, b,
+        rows<<<rb, kUmapRowThreads, 0, s>>>(indptr, indices, n, dim, (double)epoch, alpha, a, b,
                                             (int)p.negative_sample_rate, cur, eps, eps_neg, next, next_neg, rng,
                                             tmove, own);
-        umap_apply_kernel<<<vb, 128, 0, s>>>(n, dim, tstart, vals, tmove, own, cur, nxt);
+        apply<<<gb, kUmapThreads, 0, s>>>(n, dim, tstart, tedge, tmove, own, cur, nxt);
         std::swap(cur, nxt);
         alpha = p.learning_rate * (1.0f - (float)epoch / (float)p.n_epochs);
     }
