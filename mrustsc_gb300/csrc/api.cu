@@ -152,6 +152,9 @@ namespace {
 
 constexpr uint32_t kMaxK = 128;
 constexpr int64_t kOrderMinRows = 1024;  // automatic ordering from this many rows
+constexpr int64_t kWideMinRows = 2048;   // the tensor form's two operand blocks from this many rows
+constexpr uint32_t kWideMaxK = 32;       // and up to this many neighbours
+static_assert(kWideMinRows >= kOrderMinRows, "two operand blocks serve ordered solves");
 
 int32_t check_knn_args(uint64_t n, uint64_t d, uint32_t k, scrust_status* st) {
     if (n == 0 || d == 0)
@@ -243,24 +246,32 @@ int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_
 namespace {
 
 // Whether the tensor form applies: the mode is exact and the row plus the
-// three norm columns fits one 64-wide operand row.
-bool tensor_form_applies(const scrust_knn_options& o, int d) {
-    return o.mode == SCRUST_MODE_EXACT && d + 3 <= 64;
+// three norm columns fits the operand blocks.  Two blocks (62 to 125
+// dimensions) serve ordered solves alone, where they are the faster: at most
+// 32 neighbours, and kWideMinRows rows (k = 15, d = 70, plain against tensor:
+// 655 and 365 us at 2,048 rows, 3.7 and 0.53 ms at 12,000, 13.4 and 0.68 ms at
+// 30,000; smaller inputs stay where the plain form's rules put them).
+bool tensor_form_applies(const scrust_knn_options& o, int64_t n, int d, uint32_t k) {
+    if (o.mode != SCRUST_MODE_EXACT) return false;
+    if (d <= kTensorMaxDim) return true;
+    return d <= kTensorWideMaxDim && k <= kWideMaxK && n >= kWideMinRows && n <= kOrderMaxRows && o.segments <= 1 &&
+           o.ordering != SCRUST_ORDERING_OFF;
 }
 
 // Whether a solve runs the tensor form: asked for (or automatic) and applies.
-bool uses_tensor_form(const scrust_knn_options& o, int d) {
-    return (o.form == SCRUST_FORM_TENSOR || o.form == SCRUST_FORM_AUTO) && tensor_form_applies(o, d);
+bool uses_tensor_form(const scrust_knn_options& o, int64_t n, int d, uint32_t k) {
+    return (o.form == SCRUST_FORM_TENSOR || o.form == SCRUST_FORM_AUTO) && tensor_form_applies(o, n, d, k);
 }
 
 // Success, noting in the message when an explicit tensor-form request ran the
 // plain form instead.
-int32_t ok_form(scrust_status* st, const scrust_knn_options* opt, int d) {
+int32_t ok_form(scrust_status* st, const scrust_knn_options* opt, uint64_t n, int d, uint32_t k) {
     ok(st);
-    if (st && opt && opt->form == SCRUST_FORM_TENSOR && !tensor_form_applies(*opt, d))
+    if (st && opt && opt->form == SCRUST_FORM_TENSOR && !tensor_form_applies(*opt, (int64_t)n, d, k))
         snprintf(st->message, sizeof(st->message),
-                 "ran the plain form: the tensor form needs exact mode and at most 61 dimensions, got %s mode "
-                 "and %d dimensions",
+                 "ran the plain form: the tensor form needs exact mode and at most %d dimensions (%d from %lld cells "
+                 "on, with k at most %u, ordering and one segment), got %s mode and %d dimensions",
+                 kTensorMaxDim, kTensorWideMaxDim, (long long)kWideMinRows, kWideMaxK,
                  opt->mode == SCRUST_MODE_EXACT ? "exact" : "reference_snap", d);
     return SCRUST_OK;
 }
@@ -286,7 +297,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
     const int d = plan.d;
     const bool ref = o.mode == SCRUST_MODE_REFERENCE_SNAP;
     const bool cosine = o.metric == SCRUST_METRIC_COSINE;
-    const bool tensor = uses_tensor_form(o, d);
+    const bool tensor = uses_tensor_form(o, n, d, k);
     const int64_t n_pad = tensor ? (n + 255) / 256 * 256 : (n + 127) / 128 * 128;
     const int dp = d <= 64 ? (d + 3) / 4 * 4 : (d + 63) / 64 * 64;
     cudaStream_t s = ctx->stream;
@@ -330,8 +341,8 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
     bool rerank_ids_only = false;  // the lists were filled by collect passes (ids, no values)
     if (tensor) {
         const bool bf16 = o.precision == SCRUST_PRECISION_BF16;
-        void* A16 = ws_get(ctx, SLOT_A16, (size_t)n_pad * 64 * 2, &e);
-        void* B16 = ws_get(ctx, SLOT_B16, (size_t)n_pad * 64 * 2, &e);
+        void* A16 = ws_get(ctx, SLOT_A16, (size_t)n_pad * operand_row_bytes(d), &e);
+        void* B16 = ws_get(ctx, SLOT_B16, (size_t)n_pad * operand_row_bytes(d), &e);
         float* rb = (float*)ws_get(ctx, SLOT_QERR, sizeof(float) * 4 * (size_t)n_pad, &e);
         if (!A16 || !B16 || !rb) return cuda_fail(st, e, "workspace");
         float *bA = rb, *beps = rb + n_pad, *bdelta = rb + 2 * n_pad, *beps2 = rb + 3 * n_pad;
@@ -364,7 +375,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
                 return cuda_fail(st, e, "tensor operands");
             ctx->launches += 1;
         }
-        if ((e = launch_tensor_bounds(n, bA, beps, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess)
+        if ((e = launch_tensor_bounds(n, d, bA, beps, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess)
             return cuda_fail(st, e, "tensor bounds");
         ctx->launches += 1;
         // Headroom of 128: a tensor-form list is checked once per tile, after
@@ -507,7 +518,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
                            rerank_ids_only)) != cudaSuccess)
         return cuda_fail(st, e, "knn_rerank");
     mark(ctx, PH_RERANK);
-    return ok_form(st, opt, d);
+    return ok_form(st, opt, (uint64_t)n, d, k);
 }
 
 int32_t take_csr_buffers(scrust_context* ctx, uint64_t rows, uint64_t nnz_cap, CsrBuffers* out,
@@ -901,7 +912,7 @@ int32_t scrust_cuda_knn(scrust_context* ctx, const float* x, uint64_t n, uint64_
             cudaSuccess)
         return cuda_fail(st, e, "download");
     if ((rc = collect_device_errors(ctx, st))) return rc;
-    return ok_form(st, opt, (int)d);
+    return ok_form(st, opt, n, (int)d, k);
 }
 
 int32_t scrust_cuda_connectivities_device(scrust_context* ctx, const uint32_t* idx, const float* dist, uint64_t n,
@@ -985,7 +996,7 @@ int32_t scrust_cuda_neighbors_graph_device(scrust_context* ctx, const float* x, 
     DeviceGuard device_guard(ctx->device);
     if ((rc = knn_device_impl(ctx, x, n, d, k, opt, out_idx, out_dist, st))) return rc;
     if ((rc = conn_device_impl(ctx, out_idx, out_dist, n, k, false, conn, st, true))) return rc;
-    return ok_form(st, opt, (int)d);
+    return ok_form(st, opt, n, (int)d, k);
 }
 
 int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_t n, uint64_t d, uint32_t k,
@@ -1035,7 +1046,7 @@ int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_
     }
     if (rc) return rc;
     if ((rc = collect_device_errors(ctx, st))) return rc;
-    return ok_form(st, opt, (int)d);
+    return ok_form(st, opt, n, (int)d, k);
 }
 
 int32_t scrust_cuda_synchronize(scrust_context* ctx, scrust_status* st) {

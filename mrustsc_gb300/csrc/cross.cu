@@ -68,7 +68,7 @@ int32_t cross_knn_enqueue(scrust_context* ctx, const Reference& ref, const float
     uint32_t* scratch_words = (uint32_t*)(rb + 4 * q_pad);
     if ((e = launch_tensor_operands(dq, q, q_pad, d, ref.means, ref.words, false, ref.bf16, nullptr, A16, B16, bA, eps,
                                     scratch_words, scratch_words + 1, s)) != cudaSuccess ||
-        (e = launch_tensor_bounds(q, bA, eps, ref.words + 1, ref.words + 2, bdelta, beps2, s)) != cudaSuccess)
+        (e = launch_tensor_bounds(q, d, bA, eps, ref.words + 1, ref.words + 2, bdelta, beps2, s)) != cudaSuccess)
         return cuda_fail(st, e, "cross: query operands");
     const int items = (int)(q_pad / 256), col_tiles = (int)(ref.n_pad / 256);
     int csegs = std::max(1, std::min((2 * ctx->sm_count + items - 1) / items, std::min(col_tiles, 16)));

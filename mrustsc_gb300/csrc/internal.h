@@ -304,11 +304,17 @@ cudaError_t launch_column_means(const float* x, int64_t n, int d, bool sequentia
                                 double* partial, cudaStream_t s);
 cudaError_t launch_normalise_rows(const float* x, int64_t n, int d, float* xn, double* norm64,
                                   int* d_err, cudaStream_t s);
-// prep.cu: column means that only fix a centre (tensor form, d <= 64): f32
+// Tensor operands: 64-wide (128-byte) blocks per row that hold d coordinates
+// and the three norm columns: one up to 61 dimensions, two up to 125.
+constexpr int kTensorMaxDim = 61, kTensorWideMaxDim = 125;
+inline int operand_blocks(int d) { return d <= kTensorMaxDim ? 1 : 2; }
+inline size_t operand_row_bytes(int d) { return 128 * (size_t)operand_blocks(d); }
+
+// prep.cu: column means that only fix a centre (tensor form, d <= 125): f32
 // block sums; `partial` as for launch_column_means.
 cudaError_t launch_column_means_centre(const float* x, int64_t n, int d, double* means, double* partial,
                                        cudaStream_t s);
-// prep.cu: the largest centred row norm only (tensor form, d <= 64).
+// prep.cu: the largest centred row norm only (tensor form, d <= 125).
 cudaError_t launch_max_centred_norm(const float* x, int64_t n, int d, const double* means, uint32_t* max_norm_bits,
                                     int sm_count, cudaStream_t s);
 cudaError_t launch_centre_transpose(const float* x, int64_t n, int64_t n_pad, int d, int dp,
@@ -326,13 +332,12 @@ cudaError_t launch_plain_candidates(scrust_context* ctx, const KnnPlan& plan, co
                                     const float* r_norm2, const float* margin, const Lists& lists);
 
 // knn_tensor.cu
-size_t tensor_smem_bytes();
 // Row i of the operands is input row perm[i] (i when perm is null).
 cudaError_t launch_tensor_operands(const float* x, int64_t n, int64_t n_pad, int d, const double* means,
                                    const uint32_t* max_norm_bits, bool cosine, bool bf16, const uint32_t* perm,
                                    void* A16, void* B16, float* bA, float* eps, uint32_t* max_eps_bits,
                                    uint32_t* max_bhat_bits, cudaStream_t s);
-cudaError_t launch_tensor_bounds(int64_t n, const float* bA, const float* eps, const uint32_t* max_eps_bits,
+cudaError_t launch_tensor_bounds(int64_t n, int d, const float* bA, const float* eps, const uint32_t* max_eps_bits,
                                  const uint32_t* max_bhat_bits, float* bdelta, float* beps2, cudaStream_t s);
 // Explicit column tiles per row block of the query rows.
 struct TileLists {

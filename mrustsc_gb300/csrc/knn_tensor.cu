@@ -3,7 +3,8 @@
 // selection.  The exact rerank (rerank.cu) then turns the candidates into the
 // same FP64-equal neighbour lists the plain form produces.
 //
-// Operands (K = 64 halves per row, one 128-byte swizzle row):
+// Operands (K = 64 halves per row, one 128-byte swizzle row; two such blocks
+// from 62 dimensions on):
 //   A_i = [ a_hat_i (D), 1, 1, 1, 0 ... ]
 //   B_j = [ -2 b_hat_j (D), n1_j, n2_j, n3_j, 0 ... ]
 // where a_hat = fp16/bf16(scale * (x - mean)) and n1 + n2 + n3 is
@@ -15,9 +16,9 @@
 //
 // Kernel layout (persistent, one CTA per SM, 576 threads):
 //   warp 0      TMA producer: A (256 query rows) per work item, B (256
-//               reference rows) per tile, 4-stage ring
+//               reference rows) per tile, 4-stage ring (2 for two blocks)
 //   warp 1      TMEM owner and MMA issuer: per B tile, two M=128 x N=256 x
-//               K=16 x4 chains into two TMEM accumulators (query halves)
+//               K=16 x4 (x8) chains into two TMEM accumulators (query halves)
 //   warps 2-17  epilogue: 8 warps per half; warp w reads TMEM lanes
 //               32*(w%4).. and one 128-column part of its half's
 //               accumulator.  Each thread owns one query row and one list per
@@ -54,17 +55,26 @@ namespace {
 
 constexpr int TBM = 128;               // rows per accumulator (MMA M)
 constexpr int TBN = 256;               // reference rows per tile (MMA N)
-constexpr int TK = 64;                 // halves per operand row
+constexpr int TK = 64;                 // halves per operand block (one 128-byte swizzle row)
 constexpr int HALVES = 2;              // query halves per work item
 constexpr int ROWS = TBM * HALVES;     // 256 query rows per work item
-constexpr int STAGES = 4;
 constexpr int PARTS = 2;               // column parts of a tile, one epilogue warp each
 constexpr int EPI_WARPS = HALVES * PARTS * 4;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
-constexpr uint32_t A_BYTES = ROWS * TK * 2;
-constexpr uint32_t B_BYTES = TBN * TK * 2;
 constexpr uint32_t TMEM_COLS = 512;
-constexpr size_t SMEM_BYTES = 2 * A_BYTES + STAGES * B_BYTES + 1024;
+// Shared memory by operand blocks per row: one block leaves room for two work
+// items' A and four B tiles on their way; two blocks (62 to 125 dimensions)
+// double every tile, which leaves one A and two B.
+template <int BLOCKS>
+struct SweepShape {
+    static constexpr int A_BUFS = BLOCKS == 1 ? 2 : 1;
+    static constexpr int STAGES = BLOCKS == 1 ? 4 : 2;
+    static constexpr uint32_t A_BLOCK = ROWS * TK * 2;  // bytes of one operand block's tile
+    static constexpr uint32_t B_BLOCK = TBN * TK * 2;
+    static constexpr uint32_t A_BYTES = A_BLOCK * BLOCKS;
+    static constexpr uint32_t B_BYTES = B_BLOCK * BLOCKS;
+    static constexpr size_t SMEM_BYTES = A_BUFS * A_BYTES + STAGES * B_BYTES + 1024;
+};
 constexpr int kPartCols = TBN / PARTS;  // columns one epilogue warp drains per tile
 
 struct TensorArgs {
@@ -610,7 +620,8 @@ __device__ __forceinline__ void prune_lanes(uint32_t need, const TensorArgs& a, 
 
 // TOPK = K (k <= K, K = 1, 16 or 32): thresholds from a register top-K per
 // lane (TopK); TOPK = 0: from warp-cooperative selections over the lists.
-template <int TOPK, int PASS>
+// BLOCKS: operand blocks per row (SweepShape).
+template <int TOPK, int PASS, int BLOCKS = 1>
 __global__ void __launch_bounds__(THREADS, 1)
     tensor_candidates_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
                              TensorArgs a) {
@@ -624,12 +635,15 @@ __global__ void __launch_bounds__(THREADS, 1)
     const bool thr_only = PASS == 1 || (PASS == 0 && TOPK <= 1 && a.thr_only);
     const bool collect = PASS == 2 || PASS == 4 || (PASS == 0 && TOPK <= 1 && a.collect);
     const bool argmin = PASS == 3 || (PASS == 0 && a.argmin_out != nullptr);
+    using Shape = SweepShape<BLOCKS>;
+    constexpr int STAGES = Shape::STAGES, A_BUFS = Shape::A_BUFS;
+    constexpr uint32_t A_BYTES = Shape::A_BYTES, B_BYTES = Shape::B_BYTES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = base;
-    unsigned char* sB = base + 2 * A_BYTES;
+    unsigned char* sB = base + A_BUFS * A_BYTES;
 
-    __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], afull[2], aempty[2], tfull[HALVES],
+    __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], afull[A_BUFS], aempty[A_BUFS], tfull[HALVES],
         tempty[HALVES];
     __shared__ uint32_t tmem_slot;
     __shared__ unsigned long long theta_s[HALVES][PARTS][TBM];
@@ -650,7 +664,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < A_BUFS; b++) {
             mbar_init(&afull[b], 1);
             mbar_init(&aempty[b], 1);
         }
@@ -681,13 +695,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int ct1 = a.item_range ? (int)a.item_range[w].y : min(a.col_tiles, ct0 + a.tiles_per_seg);
                 const TileOrder<PASS == 2 || PASS == 4 || PASS == 0> order(a, w, qt, ct0, ct1);
                 if (order.count == 0) continue;
-                const uint32_t ab = ac & 1, au = ac >> 1;
+                const uint32_t ab = ac % A_BUFS, au = ac / A_BUFS;
                 if (!mbar_wait_bounded(&aempty[ab], (au & 1) ^ 1, a.err)) {
                     ok = false;
                     break;
                 }
                 mbar_arrive_expect_tx(&afull[ab], A_BYTES);
-                tma_load_2d(sA + ab * A_BYTES, &ta, 0, qt * ROWS, &afull[ab]);
+#pragma unroll
+                for (int b = 0; b < BLOCKS; ++b)
+                    tma_load_2d(sA + ab * A_BYTES + b * Shape::A_BLOCK, &ta, b * TK, qt * ROWS, &afull[ab]);
                 ac++;
                 for (int it = 0; it < order.count; ++it) {
                     const int ct = order.next(it);
@@ -699,7 +715,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                     if (a.stats) w_tma += clock64() - t0;
                     mbar_arrive_expect_tx(&full[st], B_BYTES);
-                    tma_load_2d(sB + st * B_BYTES, &tb, 0, ct * TBN, &full[st]);
+#pragma unroll
+                    for (int b = 0; b < BLOCKS; ++b)
+                        tma_load_2d(sB + st * B_BYTES + b * Shape::B_BLOCK, &tb, b * TK, ct * TBN, &full[st]);
                     sc++;
                 }
             }
@@ -709,7 +727,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t idx = sc - 1 - i;
                 mbar_wait_bounded(&full[idx % STAGES], (idx / STAGES) & 1, a.err, 100000000ull);
             }
-            if (ac) mbar_wait_bounded(&afull[(ac - 1) & 1], ((ac - 1) >> 1) & 1, a.err, 100000000ull);
+            if (ac) mbar_wait_bounded(&afull[(ac - 1) % A_BUFS], ((ac - 1) / A_BUFS) & 1, a.err, 100000000ull);
             if (a.stats) atomicAdd(a.stats + TS_TMA_WAIT, (unsigned long long)w_tma);
         }
     } else if (warp == 1) {
@@ -724,7 +742,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int ct1 = a.item_range ? (int)a.item_range[w].y : min(a.col_tiles, ct0 + a.tiles_per_seg);
                 const TileOrder<PASS == 2 || PASS == 4 || PASS == 0> order(a, w, qt, ct0, ct1);
                 if (order.count == 0) continue;
-                const uint32_t ab = ac & 1, au = ac >> 1;
+                const uint32_t ab = ac % A_BUFS, au = ac / A_BUFS;
                 if (!mbar_wait_bounded(&afull[ab], au & 1, a.err)) {
                     ok = false;
                     break;
@@ -751,9 +769,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                         tc_fence_after();
                         const uint32_t d = tmem + (uint32_t)(h * TBN);
 #pragma unroll
-                        for (int kk = 0; kk < TK / 16; ++kk) {
-                            const uint64_t ad = umma_desc_sw128(a_base + (uint32_t)(h * TBM * 128 + kk * 32));
-                            const uint64_t bd = umma_desc_sw128(b_base + (uint32_t)(kk * 32));
+                        for (int kk = 0; kk < BLOCKS * TK / 16; ++kk) {
+                            const uint32_t blk = kk / (TK / 16), off = (kk % (TK / 16)) * 32;
+                            const uint64_t ad = umma_desc_sw128(a_base + blk * Shape::A_BLOCK + (uint32_t)(h * TBM * 128) + off);
+                            const uint64_t bd = umma_desc_sw128(b_base + blk * Shape::B_BLOCK + off);
                             umma_f16(d, ad, bd, a.idesc, kk > 0 ? 1u : 0u);
                         }
                         umma_commit(&tfull[h]);
@@ -1145,7 +1164,7 @@ __device__ __forceinline__ uint32_t bits16(__half v) { return (uint32_t)__half_a
 __device__ __forceinline__ uint32_t bits16(__nv_bfloat16 v) { return (uint32_t)__bfloat16_as_ushort(v); }
 
 // One thread per padded row: writes A_i and B_i of input row perm[i] (a
-// padding row where perm[i] is 0xffffffff or i >= n) (64 16-bit values each), the
+// padding row where perm[i] is 0xffffffff or i >= n) (64 BLOCKS 16-bit values each), the
 // quantised squared norm A = |a_hat|^2, the per-row error radius
 // eps = |a_hat - scale*c| + scale*u*|c| (+ scale*u for normalised rows), and
 // the running maxima of eps and |b_hat|.
@@ -1156,14 +1175,15 @@ __device__ __forceinline__ uint32_t bits16(__nv_bfloat16 v) { return (uint32_t)_
 // unevaluated pair (two-sum), so its three-part split is as close as an f64
 // sum's.  Sums of rounded non-negative terms are scaled up past their
 // rounding and every step of a bound is rounded upwards.
-template <class T>
+template <class T, int BLOCKS>
 __global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __restrict__ x, int64_t n, int64_t n_pad, int d,
                                        const double* __restrict__ means, const uint32_t* __restrict__ max_norm_bits,
                                        int cosine, const uint32_t* __restrict__ perm, T* __restrict__ A16,
                                        T* __restrict__ B16,
                                        float* __restrict__ bA, float* __restrict__ eps,
                                        uint32_t* __restrict__ max_eps_bits, uint32_t* __restrict__ max_bhat_bits) {
-    __shared__ float mean32[TK];
+    constexpr int W = TK * BLOCKS;  // halves per row
+    __shared__ float mean32[W];
     for (int t = threadIdx.x; t < d; t += blockDim.x) mean32[t] = __double2float_rn(means[t]);
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1175,7 +1195,7 @@ __global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __res
     const float scale = ldexpf(1.0f, sexp);
     // Rows are built as packed 16-bit pairs in registers (static indices
     // only): aw[w] holds columns 2w and 2w + 1.
-    uint32_t aw[TK / 2], bw[TK / 2];
+    uint32_t aw[W / 2], bw[W / 2];
     const bool real = i < n && (!perm || perm[i] != 0xffffffffu);
     const uint32_t one = bits16(to16<T>(1.0f));
     if (real) {
@@ -1183,7 +1203,7 @@ __global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __res
         const float* xr = x + src * d;
         float hs = 0.f, hl = 0.f, e2 = 0.f, c2 = 0.f;
 #pragma unroll
-        for (int w = 0; w < TK / 2; w++) {
+        for (int w = 0; w < W / 2; w++) {
             uint32_t pa = 0u, pb = 0u;
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
@@ -1217,7 +1237,7 @@ __global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __res
         const T n3 = to16<T>(r2);
         // Columns d .. d + 2: ones in A, the split norm in B.
 #pragma unroll
-        for (int w = 0; w < TK / 2; w++)
+        for (int w = 0; w < W / 2; w++)
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
                 const int t = 2 * w + hh;
@@ -1243,7 +1263,7 @@ __global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __res
         // ones as a real row, so that no product is 0 * inf).
         const uint32_t inf = bits16(to16<T>(__int_as_float(0x7f800000)));
 #pragma unroll
-        for (int w = 0; w < TK / 2; w++) {
+        for (int w = 0; w < W / 2; w++) {
             uint32_t pa = 0u, pb = 0u;
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
@@ -1257,21 +1277,21 @@ __global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __res
         bA[i] = 0.f;
         eps[i] = 0.f;
     }
-    uint4* ad = reinterpret_cast<uint4*>(A16 + i * TK);
-    uint4* bd = reinterpret_cast<uint4*>(B16 + i * TK);
+    uint4* ad = reinterpret_cast<uint4*>(A16 + i * W);
+    uint4* bd = reinterpret_cast<uint4*>(B16 + i * W);
 #pragma unroll
-    for (int q = 0; q < TK / 8; q++) {
+    for (int q = 0; q < W / 8; q++) {
         ad[q] = make_uint4(aw[4 * q], aw[4 * q + 1], aw[4 * q + 2], aw[4 * q + 3]);
         bd[q] = make_uint4(bw[4 * q], bw[4 * q + 1], bw[4 * q + 2], bw[4 * q + 3]);
     }
 }
 
-// delta: bound on the FP32 accumulation error of the 64-term MMA chain,
-// 8 * 64 * 2^-24 * (2 |a_hat| Mb + Mb^2 + 3), plus the rounding of A to f32
+// delta: bound on the FP32 accumulation error of the MMA chain over a row's
+// `terms` = 64 or 128 halves, 8 * terms * 2^-24 * (2 |a_hat| Mb + Mb^2 + 3), plus the rounding of A to f32
 // and the residual of the three-part 16-bit split of |b_hat|^2 (at most
 // 2^-24 |b_hat|^2 for bf16 parts, far less for fp16); eps2 = 2 (eps_i + E).
 // Every step rounded upwards.
-__global__ void tensor_bounds_kernel(int64_t n, const float* __restrict__ bA, const float* __restrict__ eps,
+__global__ void tensor_bounds_kernel(int64_t n, int terms, const float* __restrict__ bA, const float* __restrict__ eps,
                                      const uint32_t* __restrict__ max_eps_bits,
                                      const uint32_t* __restrict__ max_bhat_bits, float* __restrict__ bdelta,
                                      float* __restrict__ beps2) {
@@ -1283,7 +1303,7 @@ __global__ void tensor_bounds_kernel(int64_t n, const float* __restrict__ bA, co
     const float a = __fsqrt_ru(A);
     const float mb2 = __fmul_ru(Mb, Mb);
     const float chain = __fadd_ru(__fadd_ru(__fmul_ru(__fmul_ru(2.0f, a), Mb), mb2), 3.0f);
-    float delta = __fmul_ru(3.0517578125e-05f, chain);           // 8 * 64 * 2^-24
+    float delta = __fmul_ru(4.76837158203125e-07f * (float)terms, chain);  // 8 * terms * 2^-24, exact
     delta = __fadd_ru(delta, __fmul_ru(1.1920928955078125e-07f, A));  // 2 * 2^-24
     delta = __fadd_ru(delta, __fmul_ru(2.384185791015625e-07f, mb2)); // 4 * 2^-24
     bdelta[i] = __fadd_ru(delta, 1e-7f);
@@ -1292,27 +1312,27 @@ __global__ void tensor_bounds_kernel(int64_t n, const float* __restrict__ bA, co
 
 }  // namespace
 
-size_t tensor_smem_bytes() { return SMEM_BYTES; }
-
 cudaError_t launch_tensor_operands(const float* x, int64_t n, int64_t n_pad, int d, const double* means,
                                    const uint32_t* max_norm_bits, bool cosine, bool bf16, const uint32_t* perm,
                                    void* A16, void* B16, float* bA, float* eps, uint32_t* max_eps_bits,
                                    uint32_t* max_bhat_bits, cudaStream_t s) {
     const unsigned blocks = (unsigned)((n_pad + 127) / 128);
-    if (bf16)
-        tensor_operands_kernel<__nv_bfloat16><<<blocks, 128, 0, s>>>(
-            x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__nv_bfloat16*)A16, (__nv_bfloat16*)B16,
-            bA, eps, max_eps_bits, max_bhat_bits);
-    else
-        tensor_operands_kernel<__half><<<blocks, 128, 0, s>>>(x, n, n_pad, d, means, max_norm_bits,
-                                                              cosine ? 1 : 0, perm, (__half*)A16, (__half*)B16, bA,
-                                                              eps, max_eps_bits, max_bhat_bits);
+    const int one = operand_blocks(d) == 1;
+    if (bf16) {
+        const auto kern = one ? tensor_operands_kernel<__nv_bfloat16, 1> : tensor_operands_kernel<__nv_bfloat16, 2>;
+        kern<<<blocks, 128, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__nv_bfloat16*)A16,
+                                    (__nv_bfloat16*)B16, bA, eps, max_eps_bits, max_bhat_bits);
+    } else {
+        const auto kern = one ? tensor_operands_kernel<__half, 1> : tensor_operands_kernel<__half, 2>;
+        kern<<<blocks, 128, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__half*)A16,
+                                    (__half*)B16, bA, eps, max_eps_bits, max_bhat_bits);
+    }
     return cudaGetLastError();
 }
 
-cudaError_t launch_tensor_bounds(int64_t n, const float* bA, const float* eps, const uint32_t* max_eps_bits,
+cudaError_t launch_tensor_bounds(int64_t n, int d, const float* bA, const float* eps, const uint32_t* max_eps_bits,
                                  const uint32_t* max_bhat_bits, float* bdelta, float* beps2, cudaStream_t s) {
-    tensor_bounds_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, bA, eps, max_eps_bits, max_bhat_bits,
+    tensor_bounds_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, TK * operand_blocks(d), bA, eps, max_eps_bits, max_bhat_bits,
                                                                       bdelta, beps2);
     return cudaGetLastError();
 }
@@ -1325,9 +1345,11 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
     if (nq_pad % ROWS || nr_pad % TBN) return cudaErrorInvalidValue;
     CUtensorMap ta, tb;
     const CUtensorMapDataType dt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    if (!encode_2d(ctx, &ta, dt, (void*)A16, TK, (uint64_t)nq_pad, TK * 2, TK, ROWS, CU_TENSOR_MAP_SWIZZLE_128B))
+    const int blocks = operand_blocks(plan.d);
+    const uint64_t width = (uint64_t)TK * blocks;
+    if (!encode_2d(ctx, &ta, dt, (void*)A16, width, (uint64_t)nq_pad, width * 2, TK, ROWS, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
-    if (!encode_2d(ctx, &tb, dt, (void*)B16, TK, (uint64_t)nr_pad, TK * 2, TK, TBN, CU_TENSOR_MAP_SWIZZLE_128B))
+    if (!encode_2d(ctx, &tb, dt, (void*)B16, width, (uint64_t)nr_pad, width * 2, TK, TBN, CU_TENSOR_MAP_SWIZZLE_128B))
         return cudaErrorInvalidValue;
     TensorArgs a;
     a.lists = lists;
@@ -1399,25 +1421,40 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
     if (resume && !theta_io) return cudaErrorInvalidValue;
     // Register top-k width of a general pass (threshold and collect passes
     // keep the width that holds k).
-    int width = a.k == 1 ? 1 : a.k <= 16 ? 16 : a.k <= 32 ? 32 : 0;
+    int topk = a.k == 1 ? 1 : a.k <= 16 ? 16 : a.k <= 32 ? 32 : 0;
     if (!a.thr_only && !a.collect && a.k > 1) {
-        if (plan.topk_width < 0) width = 0;
-        else if (plan.topk_width == 32 && a.k <= 32) width = 32;
+        if (plan.topk_width < 0) topk = 0;
+        else if (plan.topk_width == 32 && a.k <= 32) topk = 32;
         else if (plan.topk_width != 0 && plan.topk_width != 16 && plan.topk_width != 32) return cudaErrorInvalidValue;
     }
-    auto kern = width == 1    ? (argmin_out ? tensor_candidates_kernel<1, 3> : tensor_candidates_kernel<1, 0>)
-                : width == 16 ? (a.thr_only ? tensor_candidates_kernel<16, 1>
-                                 : a.collect ? (a.self ? tensor_candidates_kernel<16, 2> : tensor_candidates_kernel<16, 4>)
-                                             : tensor_candidates_kernel<16, 0>)
-                : width == 32 ? (a.thr_only ? tensor_candidates_kernel<32, 1>
-                                 : a.collect ? (a.self ? tensor_candidates_kernel<32, 2> : tensor_candidates_kernel<32, 4>)
-                                             : tensor_candidates_kernel<32, 0>)
-                              : tensor_candidates_kernel<0, 0>;
-    cudaError_t e = set_smem_limit(ctx, (const void*)kern, (int)SMEM_BYTES);
+    using Kernel = decltype(&tensor_candidates_kernel<0, 0>);
+    Kernel kern = nullptr;
+    size_t smem = SweepShape<1>::SMEM_BYTES;
+    if (blocks == 1) {
+        kern = topk == 1    ? (argmin_out ? tensor_candidates_kernel<1, 3> : tensor_candidates_kernel<1, 0>)
+               : topk == 16 ? (a.thr_only ? tensor_candidates_kernel<16, 1>
+                               : a.collect ? (a.self ? tensor_candidates_kernel<16, 2> : tensor_candidates_kernel<16, 4>)
+                                           : tensor_candidates_kernel<16, 0>)
+               : topk == 32 ? (a.thr_only ? tensor_candidates_kernel<32, 1>
+                               : a.collect ? (a.self ? tensor_candidates_kernel<32, 2> : tensor_candidates_kernel<32, 4>)
+                                           : tensor_candidates_kernel<32, 0>)
+                            : tensor_candidates_kernel<0, 0>;
+    } else {
+        // Two operand blocks: the passes of an ordered self solve.
+        smem = SweepShape<2>::SMEM_BYTES;
+        kern = topk == 1 ? (argmin_out ? tensor_candidates_kernel<1, 3, 2> : tensor_candidates_kernel<1, 0, 2>)
+               : topk == 0 ? tensor_candidates_kernel<0, 0, 2>
+               : a.thr_only ? (topk == 16 ? tensor_candidates_kernel<16, 1, 2> : tensor_candidates_kernel<32, 1, 2>)
+               : a.collect && a.self
+                   ? (topk == 16 ? tensor_candidates_kernel<16, 2, 2> : tensor_candidates_kernel<32, 2, 2>)
+                   : nullptr;
+        if (!kern) return cudaErrorInvalidValue;
+    }
+    cudaError_t e = set_smem_limit(ctx, (const void*)kern, (int)smem);
     if (e != cudaSuccess) return e;
     const int grid = std::min(a.items, plan.max_ctas > 0 ? std::min(plan.max_ctas, ctx->sm_count) : ctx->sm_count);
     if (grid_out) *grid_out = grid;
-    kern<<<grid, THREADS, SMEM_BYTES, ctx->stream>>>(ta, tb, a);
+    kern<<<grid, THREADS, smem, ctx->stream>>>(ta, tb, a);
     return cudaGetLastError();
 }
 

@@ -232,8 +232,8 @@ __global__ void relabel_neighbours_kernel(const uint32_t* __restrict__ nb, const
 // parts], summed in f32 over the `words` 16-byte words that hold them) and
 // the smallest taken (ties to the lower anchor): an approximately nearest
 // anchor, which is all an ordering needs.  Eight lanes per row, lane l
-// holding word l of the row and of each of the eight anchors, so that every
-// load of an anchor row is one contiguous line for the eight lanes; the
+// holding word l (and word l + 8, of two operand blocks) of the row and of
+// each of the eight anchors, so that every load of an anchor row is one contiguous line for the eight lanes; the
 // partial sums meet by shuffles.  keys[i] receives the anchor
 // (anchor_rank_kernel turns it into the sort key once the walk is done),
 // vals[i] the row.
@@ -257,7 +257,7 @@ __device__ __forceinline__ float dot_word(uint4 x, uint4 y) {
     return acc;
 }
 
-template <class T>
+template <class T, int BLOCKS>
 __global__ void nearest_anchor_kernel(const unsigned long long* __restrict__ best, int64_t n, int64_t m,
                                       const T* __restrict__ A, const T* __restrict__ B, int words,
                                       uint32_t* __restrict__ keys, unsigned long long* __restrict__ vals) {
@@ -268,12 +268,18 @@ __global__ void nearest_anchor_kernel(const unsigned long long* __restrict__ bes
     const uint32_t g = row_ok ? (uint32_t)min(best[2 * i], best[2 * i + 1]) : 0u;
     const int64_t c0 = (int64_t)g * 8;
     float part[8];
-    const bool lane_ok = row_ok && l < words;
-    const uint4 x = lane_ok ? __ldg(reinterpret_cast<const uint4*>(A + i * 64) + l) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-        part[a] = 0.f;
-        if (lane_ok && c0 + a < m) part[a] = dot_word<T>(x, __ldg(reinterpret_cast<const uint4*>(B + (c0 + a) * 64) + l));
+    for (int a = 0; a < 8; ++a) part[a] = 0.f;
+#pragma unroll
+    for (int b = 0; b < BLOCKS; ++b) {
+        const int lw = l + 8 * b;
+        const bool lane_ok = row_ok && lw < words;
+        const uint4 x =
+            lane_ok ? __ldg(reinterpret_cast<const uint4*>(A + i * 64 * BLOCKS) + lw) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int a = 0; a < 8; ++a)
+            if (lane_ok && c0 + a < m)
+                part[a] += dot_word<T>(x, __ldg(reinterpret_cast<const uint4*>(B + (c0 + a) * 64 * BLOCKS) + lw));
     }
 #pragma unroll
     for (int a = 0; a < 8; ++a)
@@ -403,14 +409,15 @@ struct TileBalls {
 // self-kNN): centres (means) and radii of the tile's quantised rows, and the
 // reach U = max over the rows of sqrt(theta + A + delta), theta being the
 // smaller of the row's two list thresholds.
-template <class T>
+template <class T, int BLOCKS>
 __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ ops, int64_t n, int d, int tiles,
                                                          const uint32_t* __restrict__ cell_of_pos,
                                                          const float* __restrict__ theta, const float* __restrict__ bA,
                                                          const float* __restrict__ bdelta, TileBalls b) {
-    __shared__ float part[8][64];
-    __shared__ float centre[64];
-    __shared__ float scentre[kSegMax][64];
+    constexpr int W = 64 * BLOCKS;  // halves per operand row
+    __shared__ float part[8][W];
+    __shared__ float centre[W];
+    __shared__ float scentre[kSegMax][W];
     __shared__ int sstart[kSegMax + 1];
     __shared__ int wheads[8];
     __shared__ uint32_t rmax_all, rmax_seg[kSegMax];
@@ -420,11 +427,11 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
     const int64_t j = (int64_t)tile * 256 + threadIdx.x;
     const bool valid = j < n;
     const int rows = (int)min((int64_t)256, n - (int64_t)tile * 256);
-    const T* row = ops + j * 64;
-    // The row's 64 16-bit values, read once as eight 16-byte words.
-    uint32_t rw[32];
+    const T* row = ops + j * W;
+    // The row's 16-bit values, read once as 16-byte words.
+    uint32_t rw[W / 2];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < W / 8; ++q) {
         const uint4 u = valid ? reinterpret_cast<const uint4*>(row)[q] : make_uint4(0u, 0u, 0u, 0u);
         rw[4 * q] = u.x;
         rw[4 * q + 1] = u.y;
@@ -454,7 +461,7 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
     if (head && seg == before + __popc(hb & lanemask_lt())) sstart[seg] = threadIdx.x;
     if (threadIdx.x == 0) sstart[nseg] = rows;
 #pragma unroll
-    for (int t = 0; t < 64; ++t) {
+    for (int t = 0; t < W; ++t) {
         if (t < d) {
             float v = valid ? op_bits<T>(rw[t >> 1] >> (16 * (t & 1))) : 0.f;
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -471,7 +478,7 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
     for (int p = threadIdx.x; p < nseg * d; p += blockDim.x) {
         const int sg = p / d, t = p % d;
         float sum = 0.f;
-        for (int r = sstart[sg]; r < sstart[sg + 1]; ++r) sum += op_float(ops[((int64_t)tile * 256 + r) * 64 + t]);
+        for (int r = sstart[sg]; r < sstart[sg + 1]; ++r) sum += op_float(ops[((int64_t)tile * 256 + r) * W + t]);
         const float c = sum / (float)(sstart[sg + 1] - sstart[sg]);
         scentre[sg][t] = c;
         b.seg_centre[((int64_t)sg * d + t) * tiles + tile] = c;
@@ -484,7 +491,7 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
         // 1 + (d + 4) 2^-23 (rounded up) bounds it from above.
         float r2 = 0.f, s2 = 0.f;
 #pragma unroll
-        for (int t = 0; t < 64; ++t) {
+        for (int t = 0; t < W; ++t) {
             if (t < d) {
                 const float v = op_bits<T>(rw[t >> 1] >> (16 * (t & 1)));
                 const float df = v - centre[t], ds = v - scentre[seg][t];
@@ -530,17 +537,17 @@ __device__ __forceinline__ bool tile_needed(float dc2, float rI, float rT, float
     return !(lhs >= reach * reach * (1.0f + 1e-6f));
 }
 
-// The cell-segment balls of all tiles, one row each (centres padded to 64
-// dimensions with zeros), in tile order.
-__global__ void flatten_segments_kernel(TileBalls b, int d, int tiles, const uint32_t* __restrict__ seg_off,
+// The cell-segment balls of all tiles, one row each (centres padded to `width`
+// = 64 or 128 dimensions with zeros), in tile order.
+__global__ void flatten_segments_kernel(TileBalls b, int d, int width, int tiles, const uint32_t* __restrict__ seg_off,
                                         float* __restrict__ fc, float* __restrict__ fr, float* __restrict__ fu,
                                         uint32_t* __restrict__ fo) {
     const int T = blockIdx.x;
     const int ns = (int)min(b.nseg[T], (uint32_t)kSegMax);
     const uint32_t o = seg_off[T];
-    for (int p = threadIdx.x; p < ns * 64; p += blockDim.x) {
-        const int sg = p / 64, t = p % 64;
-        fc[(int64_t)(o + sg) * 64 + t] = t < d ? b.seg_centre[((int64_t)sg * d + t) * tiles + T] : 0.f;
+    for (int p = threadIdx.x; p < ns * width; p += blockDim.x) {
+        const int sg = p / width, t = p % width;
+        fc[(int64_t)(o + sg) * width + t] = t < d ? b.seg_centre[((int64_t)sg * d + t) * tiles + T] : 0.f;
     }
     if (threadIdx.x < ns) {
         fr[o + threadIdx.x] = b.seg_radius[(int64_t)threadIdx.x * tiles + T];
@@ -555,6 +562,7 @@ __global__ void flatten_segments_kernel(TileBalls b, int d, int tiles, const uin
 // segment count S is read on the device; blocks stride over the block pairs
 // of the upper triangle, and each centre distance serves both directions.
 constexpr int SP = 64;
+template <int BLOCKS>
 __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restrict__ fc, const float* __restrict__ fr,
                                                             const float* __restrict__ fu,
                                                             const uint32_t* __restrict__ fo,
@@ -571,25 +579,29 @@ __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restr
         const int bi = (int)(bp / nb), bj = (int)(bp % nb);
         if (bi > bj) continue;
         const int i0 = bi * SP, j0 = bj * SP;
-        __syncthreads();
-        for (int p = threadIdx.x; p < SP * 64; p += blockDim.x) {
-            const int r = p / 64, t = p % 64;
-            As[t][r] = i0 + r < S ? fc[(int64_t)(i0 + r) * 64 + t] : 0.f;
-            Bs[t][r] = j0 + r < S ? fc[(int64_t)(j0 + r) * 64 + t] : 0.f;
-        }
-        __syncthreads();
         float acc[4][4] = {};
-        for (int t = 0; t < d; ++t) {
-            const float4 a4 = *reinterpret_cast<const float4*>(&As[t][ty * 4]);
-            const float4 b4 = *reinterpret_cast<const float4*>(&Bs[t][tx * 4]);
-            const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
+        for (int blk = 0; blk < BLOCKS; ++blk) {  // 64 dimensions at a time
+            __syncthreads();
+            for (int p = threadIdx.x; p < SP * 64; p += blockDim.x) {
+                const int r = p / 64, t = p % 64;
+                As[t][r] = i0 + r < S ? fc[((int64_t)(i0 + r) * BLOCKS + blk) * 64 + t] : 0.f;
+                Bs[t][r] = j0 + r < S ? fc[((int64_t)(j0 + r) * BLOCKS + blk) * 64 + t] : 0.f;
+            }
+            __syncthreads();
+            const int dims = min(64, d - 64 * blk);
+            for (int t = 0; t < dims; ++t) {
+                const float4 a4 = *reinterpret_cast<const float4*>(&As[t][ty * 4]);
+                const float4 b4 = *reinterpret_cast<const float4*>(&Bs[t][tx * 4]);
+                const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float df = av[p] - bv[q];
-                    acc[p][q] = fmaf(df, df, acc[p][q]);
-                }
+                for (int p = 0; p < 4; ++p)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float df = av[p] - bv[q];
+                        acc[p][q] = fmaf(df, df, acc[p][q]);
+                    }
+            }
         }
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
@@ -663,31 +675,33 @@ __global__ void __launch_bounds__(256) tile_lists_kernel(const uint32_t* __restr
     if (threadIdx.x == 0) counts[I] = (uint32_t)base;
 }
 
-// Operand rows (128 bytes each) and their per-row terms moved into list
+// Operand rows (128 BLOCKS bytes each) and their per-row terms moved into list
 // order; padding rows are zero like the operand kernel writes them.
-// Eight lanes per row: lane q of a row copies the row's q-th 16-byte word of
-// A and B (a warp writes four whole 128-byte rows at a time).
+// Eight lanes per block of a row: lane q copies the row's q-th 16-byte word of
+// A and B (a warp writes whole 128-byte lines).
+template <int BLOCKS>
 __global__ void gather_operands_kernel(const uint4* __restrict__ A0, const uint4* __restrict__ B0,
                                        const float* __restrict__ bA0, const float* __restrict__ eps0,
                                        const uint32_t* __restrict__ perm, int64_t n, int64_t n_pad,
                                        uint4* __restrict__ A16, uint4* __restrict__ B16, float* __restrict__ bA,
                                        float* __restrict__ eps) {
+    constexpr int WORDS = 8 * BLOCKS;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t s = t >> 3;
-    const int q = (int)(t & 7);
+    const int64_t s = t / WORDS;
+    const int q = (int)(t % WORDS);
     if (s >= n_pad) return;
     if (s < n) {
         const int64_t r = perm[s];
-        A16[s * 8 + q] = A0[r * 8 + q];
-        B16[s * 8 + q] = B0[r * 8 + q];
+        A16[s * WORDS + q] = A0[r * WORDS + q];
+        B16[s * WORDS + q] = B0[r * WORDS + q];
         if (q == 0) {
             bA[s] = bA0[r];
             eps[s] = eps0[r];
         }
     } else {
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-        A16[s * 8 + q] = z;
-        B16[s * 8 + q] = z;
+        A16[s * WORDS + q] = z;
+        B16[s * WORDS + q] = z;
         if (q == 0) {
             bA[s] = 0.f;
             eps[s] = 0.f;
@@ -861,6 +875,31 @@ __global__ void gather_rows_kernel(const float* __restrict__ x, const uint32_t* 
     xs[i] = (r == 0xffffffffu || t >= d) ? 0.f : x[(int64_t)r * d + t];
 }
 
+// The operand type and width pick the instantiation.
+void launch_tile_balls(bool bf16, const void* ops, int64_t n, int d, int tiles, const uint32_t* cell_of_pos,
+                       const float* theta, const float* bA, const float* bdelta, const TileBalls& b, cudaStream_t s) {
+    const bool one = operand_blocks(d) == 1;
+    if (bf16) {
+        const auto kern = one ? tile_balls_kernel<__nv_bfloat16, 1> : tile_balls_kernel<__nv_bfloat16, 2>;
+        kern<<<tiles, 256, 0, s>>>((const __nv_bfloat16*)ops, n, d, tiles, cell_of_pos, theta, bA, bdelta, b);
+    } else {
+        const auto kern = one ? tile_balls_kernel<__half, 1> : tile_balls_kernel<__half, 2>;
+        kern<<<tiles, 256, 0, s>>>((const __half*)ops, n, d, tiles, cell_of_pos, theta, bA, bdelta, b);
+    }
+}
+
+void launch_nearest_anchor(bool bf16, const unsigned long long* best, int64_t n, int64_t m, const void* A, const void* B,
+                           int blocks, int words, uint32_t* keys, unsigned long long* vals, cudaStream_t s) {
+    const unsigned grid = (unsigned)((n * 8 + 255) / 256);
+    if (bf16) {
+        const auto kern = blocks == 1 ? nearest_anchor_kernel<__nv_bfloat16, 1> : nearest_anchor_kernel<__nv_bfloat16, 2>;
+        kern<<<grid, 256, 0, s>>>(best, n, m, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, words, keys, vals);
+    } else {
+        const auto kern = blocks == 1 ? nearest_anchor_kernel<__half, 1> : nearest_anchor_kernel<__half, 2>;
+        kern<<<grid, 256, 0, s>>>(best, n, m, (const __half*)A, (const __half*)B, words, keys, vals);
+    }
+}
+
 }  // namespace
 
 // Row blocks sorted by decreasing count into `order`; scratch holds
@@ -916,6 +955,8 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     const int64_t m = std::min<int64_t>(std::max<int64_t>(n / 256, 2), kMaxAnchors);
     const int64_t m_pad = (m + 255) / 256 * 256;
     const int nblocks = radix_blocks(n);
+    const int blocks = operand_blocks(d);
+    const size_t row_bytes = operand_row_bytes(d);
     const size_t scan_elems = scan_scratch_elems(std::max<int64_t>((int64_t)256 * nblocks, m + 1));
 
     // Carve the ordering slot.
@@ -925,8 +966,8 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
         off = align_up(off + bytes);
         return o;
     };
-    const size_t o_src = take(4 * (size_t)m), o_anc = take(4 * (size_t)m * d), o_aA = take(128 * (size_t)m_pad),
-                 o_aB = take(128 * (size_t)m_pad), o_arb = take(8 * (size_t)m_pad), o_kA = take(4 * (size_t)n),
+    const size_t o_src = take(4 * (size_t)m), o_anc = take(4 * (size_t)m * d), o_aA = take(row_bytes * (size_t)m_pad),
+                 o_aB = take(row_bytes * (size_t)m_pad), o_arb = take(8 * (size_t)m_pad), o_kA = take(4 * (size_t)n),
                  o_kB = take(4 * (size_t)n), o_vA = take(8 * (size_t)n), o_vB = take(8 * (size_t)n),
                  o_perm = take(4 * (size_t)n), o_cell = take(4 * (size_t)n), o_ccnt = take(4 * (size_t)(m + 1)),
                  o_cst = take(4 * (size_t)(m + 1)), o_nb = take(4 * (size_t)m * kAnchorNeighbours),
@@ -934,8 +975,8 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
                  o_adist = take(4 * (size_t)m * (size_t)m),
                  o_prio = take(4 * (size_t)items * kPrioMax), o_pc = take(4 * (size_t)items),
                  o_theta = take(8 * (size_t)n_pad), o_po = take(4 * (size_t)items),
-                 o_best = take(16 * (size_t)n_pad), o_A0 = take(128 * (size_t)n_pad),
-                 o_B0 = take(128 * (size_t)n_pad), o_bA0 = take(4 * (size_t)n_pad), o_eps0 = take(4 * (size_t)n_pad),
+                 o_best = take(16 * (size_t)n_pad), o_A0 = take(row_bytes * (size_t)n_pad),
+                 o_B0 = take(row_bytes * (size_t)n_pad), o_bA0 = take(4 * (size_t)n_pad), o_eps0 = take(4 * (size_t)n_pad),
                  o_ws = take(work_order_scratch(items)),
                  o_hist = take(4 * ((size_t)256 * nblocks + 16)), o_scan = take(4 * scan_elems);
     char* base = (char*)ws_get(ctx, SLOT_ORDER, off, &e);
@@ -989,7 +1030,7 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     float* eps0 = (float*)(base + o_eps0);
     if ((e = launch_tensor_operands(x, n, n_pad, d, means, max_bits, cosine, bf16, nullptr, A0, B0, bA0, eps0,
                                     max_bits + 1, max_bits + 2, s)) != cudaSuccess ||
-        (e = launch_tensor_bounds(n, bA0, eps0, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess ||
+        (e = launch_tensor_bounds(n, d, bA0, eps0, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess ||
         (e = launch_tensor_operands(x, m, m_pad, d, means, max_bits, cosine, bf16, src, base + o_aA, base + o_aB, arb,
                                     arb + m_pad, max_bits + 1, max_bits + 2, s)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: operands");
@@ -1017,12 +1058,7 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
                                       false, nullptr, nullptr, nullptr, best)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: anchor candidates");
     const int op_words = (d + 3 + 7) / 8;  // 16-byte words of an operand row holding values
-    if (bf16)
-        nearest_anchor_kernel<__nv_bfloat16><<<(unsigned)((n * 8 + 255) / 256), 256, 0, s>>>(
-            best, n, m, (const __nv_bfloat16*)A0, (const __nv_bfloat16*)(base + o_aB), op_words, keysA, valsA);
-    else
-        nearest_anchor_kernel<__half><<<(unsigned)((n * 8 + 255) / 256), 256, 0, s>>>(
-            best, n, m, (const __half*)A0, (const __half*)(base + o_aB), op_words, keysA, valsA);
+    launch_nearest_anchor(bf16, best, n, m, A0, base + o_aB, blocks, op_words, keysA, valsA, s);
     // The walk ranks (copy stream) are needed from here on.
     if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamWaitEvent(s, ctx->copy_ev, 0)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: nearest anchor");
@@ -1054,7 +1090,8 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     if ((e = sort_by_work(ctx, prio_cnt, items, base + o_ws, (uint32_t*)(base + o_po))) != cudaSuccess)
         return cuda_fail(st, e, "ordering: work order");
     // The operands in list order (bounds follow in the caller).
-    gather_operands_kernel<<<(unsigned)((n_pad * 8 + 255) / 256), 256, 0, s>>>(
+    const auto gather = blocks == 1 ? gather_operands_kernel<1> : gather_operands_kernel<2>;
+    gather<<<(unsigned)((n_pad * 8 * blocks + 255) / 256), 256, 0, s>>>(
         (const uint4*)A0, (const uint4*)B0, bA0, eps0, perm, n, n_pad, (uint4*)A16, (uint4*)B16, bA, beps);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: operands");
     ctx->launches += 1;
@@ -1085,12 +1122,13 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
         return o;
     };
     const int words = (tiles + 31) / 32;
+    const int blocks = operand_blocks(d);
     const int64_t smax = (int64_t)tiles * kSegMax;
     const size_t scan_elems = scan_scratch_elems((int64_t)tiles + 1);
     const size_t o_c = take(4 * (size_t)d * tiles), o_r = take(4 * (size_t)tiles), o_u = take(4 * (size_t)tiles),
                  o_sc = take(4 * (size_t)kSegMax * d * tiles), o_sr = take(4 * (size_t)kSegMax * tiles),
                  o_su = take(4 * (size_t)kSegMax * tiles), o_ns = take(4 * ((size_t)tiles + 1)),
-                 o_so = take(4 * ((size_t)tiles + 1)), o_fc = take(4 * 64 * (size_t)smax), o_fr = take(4 * (size_t)smax),
+                 o_so = take(4 * ((size_t)tiles + 1)), o_fc = take(4 * 64 * blocks * (size_t)smax), o_fr = take(4 * (size_t)smax),
                  o_fu = take(4 * (size_t)smax), o_fo = take(4 * (size_t)smax), o_scan = take(4 * scan_elems),
                  o_bm = take(4 * (size_t)tiles * words), o_cnt = take(4 * ((size_t)tiles + 1)),
                  o_wo = take(4 * (size_t)tiles), o_ws = take(work_order_scratch(tiles)),
@@ -1116,19 +1154,15 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
     if ((e = cudaMemsetAsync(balls.nseg + tiles, 0, sizeof(uint32_t), s)) != cudaSuccess ||
         (e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)tiles * words, s)) != cudaSuccess)
         return cuda_fail(st, e, "pruning: memset");
-    if (bf16)
-        tile_balls_kernel<__nv_bfloat16><<<tiles, 256, 0, s>>>((const __nv_bfloat16*)A16, n, d, tiles,
-                                                               order.cell_of_pos, order.theta, bA, bdelta, balls);
-    else
-        tile_balls_kernel<__half><<<tiles, 256, 0, s>>>((const __half*)A16, n, d, tiles, order.cell_of_pos,
-                                                        order.theta, bA, bdelta, balls);
+    launch_tile_balls(bf16, A16, n, d, tiles, order.cell_of_pos, order.theta, bA, bdelta, balls, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: tile balls");
     if ((e = device_exclusive_scan(ctx, balls.nseg, seg_off, (int64_t)tiles + 1, (uint32_t*)(base + o_scan),
                                    scan_elems)) != cudaSuccess)
         return cuda_fail(st, e, "pruning: segment scan");
-    flatten_segments_kernel<<<tiles, 64, 0, s>>>(balls, d, tiles, seg_off, fc, fr, fu, fo);
+    flatten_segments_kernel<<<tiles, 64, 0, s>>>(balls, d, 64 * blocks, tiles, seg_off, fc, fr, fu, fo);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: segments");
-    segment_pairs_kernel<<<8 * ctx->sm_count, 256, 0, s>>>(fc, fr, fu, fo, seg_off + tiles, d, words, bitmap);
+    const auto pairs = blocks == 1 ? segment_pairs_kernel<1> : segment_pairs_kernel<2>;
+    pairs<<<8 * ctx->sm_count, 256, 0, s>>>(fc, fr, fu, fo, seg_off + tiles, d, words, bitmap);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: segment pairs");
     const size_t lists_smem = 4 * (size_t)words;
     if ((e = set_smem_limit(ctx, (const void*)tile_lists_kernel, (int)lists_smem)) !=
@@ -1150,16 +1184,6 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
 // ---- query solves against an ordered atlas -------------------------------------
 
 namespace {
-
-void launch_tile_balls(bool bf16, const void* ops, int64_t n, int d, int tiles, const uint32_t* cell_of_pos,
-                       const float* theta, const float* bA, const float* bdelta, const TileBalls& b, cudaStream_t s) {
-    if (bf16)
-        tile_balls_kernel<__nv_bfloat16><<<tiles, 256, 0, s>>>((const __nv_bfloat16*)ops, n, d, tiles, cell_of_pos,
-                                                               theta, bA, bdelta, b);
-    else
-        tile_balls_kernel<__half><<<tiles, 256, 0, s>>>((const __half*)ops, n, d, tiles, cell_of_pos, theta, bA,
-                                                        bdelta, b);
-}
 
 // The per-tile ball arrays of `tiles` tiles, laid out from byte `at` of
 // `base`; returns the end of the layout.
@@ -1256,7 +1280,7 @@ int32_t atlas_order_build(scrust_context* ctx, const float* atlas, int64_t m, in
         (e = cudaMemcpyAsync(o.cell_nb, ord.cell_nb, 4 * na * kAnchorNeighbours, cudaMemcpyDeviceToDevice, s)) !=
             cudaSuccess ||
         (e = launch_gather_rows(atlas, ord.perm, m, d, P, o.rows, s)) != cudaSuccess ||
-        (e = launch_tensor_bounds(m, bA, beps, words + 1, words + 2, bdelta, beps2, s)) != cudaSuccess ||
+        (e = launch_tensor_bounds(m, d, bA, beps, words + 1, words + 2, bdelta, beps2, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(base + o_th, 0, 4 * 2 * (size_t)o.m_pad, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(balls.nseg + tiles, 0, sizeof(uint32_t), s)) != cudaSuccess)
         return bail(cuda_fail(st, e, "atlas ordering"));
@@ -1269,7 +1293,7 @@ int32_t atlas_order_build(scrust_context* ctx, const float* atlas, int64_t m, in
         (e = device_exclusive_scan(ctx, balls.nseg, seg_off, (int64_t)tiles + 1, (uint32_t*)(base + o_scan),
                                    scan_elems)) != cudaSuccess)
         return bail(cuda_fail(st, e, "atlas ordering: tile balls"));
-    flatten_segments_kernel<<<tiles, 64, 0, s>>>(balls, d, tiles, seg_off, fc, (float*)(base + o_fr),
+    flatten_segments_kernel<<<tiles, 64, 0, s>>>(balls, d, 64, tiles, seg_off, fc, (float*)(base + o_fr),
                                                  (float*)(base + o_fu), (uint32_t*)(base + o_fo));
     uint32_t segs = 0;
     if ((e = cudaGetLastError()) != cudaSuccess ||
@@ -1386,14 +1410,8 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
                                       bf16, nullptr, false, nullptr, nullptr, nullptr, best)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: nearest anchor");
     const int op_words = (d + 3 + 7) / 8;  // 16-byte words of an operand row holding values
-    if (bf16)
-        nearest_anchor_kernel<__nv_bfloat16><<<(unsigned)((q * 8 + 255) / 256), 256, 0, s>>>(
-            best, q, at.anchors, (const __nv_bfloat16*)(base + o_A0), (const __nv_bfloat16*)at.anchor_B16, op_words,
-            (uint32_t*)(base + o_kA), (unsigned long long*)(base + o_vA));
-    else
-        nearest_anchor_kernel<__half><<<(unsigned)((q * 8 + 255) / 256), 256, 0, s>>>(
-            best, q, at.anchors, (const __half*)(base + o_A0), (const __half*)at.anchor_B16, op_words,
-            (uint32_t*)(base + o_kA), (unsigned long long*)(base + o_vA));
+    launch_nearest_anchor(bf16, best, q, at.anchors, base + o_A0, at.anchor_B16, 1, op_words, (uint32_t*)(base + o_kA),
+                          (unsigned long long*)(base + o_vA), s);
     anchor_rank_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>((uint32_t*)(base + o_kA), q, at.anchor_rank);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: nearest anchor");
     ctx->launches += 4;
@@ -1411,11 +1429,11 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
         return cuda_fail(st, e, "query routing: sort");
     unpack_perm_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>(skeys, svals, q, qperm, cell_of_pos,
                                                                   (uint32_t*)(base + o_cc));
-    gather_operands_kernel<<<(unsigned)((q_pad * 8 + 255) / 256), 256, 0, s>>>(
+    gather_operands_kernel<1><<<(unsigned)((q_pad * 8 + 255) / 256), 256, 0, s>>>(
         (const uint4*)(base + o_A0), (const uint4*)(base + o_B0), bA0, eps0, qperm, q, q_pad, (uint4*)(base + o_As),
         (uint4*)(base + o_Bs), bA, beps);
     if ((e = cudaGetLastError()) != cudaSuccess ||
-        (e = launch_tensor_bounds(q, bA, beps, words + 1, words + 2, bdelta, beps2, s)) != cudaSuccess ||
+        (e = launch_tensor_bounds(q, d, bA, beps, words + 1, words + 2, bdelta, beps2, s)) != cudaSuccess ||
         (e = launch_gather_rows(dq, qperm, q, d, P, xs, s)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: gather");
     // Priority tiles per row block, dealt over its column segments.
@@ -1475,7 +1493,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
         (e = device_exclusive_scan(ctx, qballs.nseg, seg_off, (int64_t)items + 1, (uint32_t*)(base + o_scan),
                                    scan_elems)) != cudaSuccess)
         return cuda_fail(st, e, "query knn: query balls");
-    flatten_segments_kernel<<<items, 64, 0, s>>>(qballs, d, items, seg_off, (float*)(base + o_fc),
+    flatten_segments_kernel<<<items, 64, 0, s>>>(qballs, d, 64, items, seg_off, (float*)(base + o_fc),
                                                  (float*)(base + o_fr), (float*)(base + o_fu),
                                                  (uint32_t*)(base + o_fo));
     cross_segment_pairs_kernel<<<(unsigned)std::min<int64_t>(smax, 8 * ctx->sm_count), 256, 0, s>>>(
