@@ -85,8 +85,8 @@ typedef enum scrust_form {
     SCRUST_FORM_PLAIN = 0,  /* FP32 tiled expansion on CUDA cores (the drop-in) */
     SCRUST_FORM_TENSOR = 1, /* 16-bit tcgen05/TMEM candidate GEMM, FP32 accumulate */
     /* The tensor form wherever it applies (exact mode, at most 61
-     * dimensions; up to 125 in ordered self solves of 2048 cells or more with
-     * k at most 32), else the plain form.  Both give the same lists; the
+     * dimensions; up to 125 in ordered self solves of 2048 cells or more),
+     * else the plain form.  Both give the same lists; the
      * tensor form is the faster one. */
     SCRUST_FORM_AUTO = 2
 } scrust_form;

@@ -153,7 +153,9 @@ namespace {
 constexpr uint32_t kMaxK = 128;
 constexpr int64_t kOrderMinRows = 1024;  // automatic ordering from this many rows
 constexpr int64_t kWideMinRows = 2048;   // the tensor form's two operand blocks from this many rows
-constexpr uint32_t kWideMaxK = 32;       // and up to this many neighbours
+// Threshold passes of more neighbours than this take two column segments, and
+// of more than this, four.
+constexpr uint32_t kOneSegmentMaxK = 40, kTwoSegmentMaxK = 72;
 static_assert(kWideMinRows >= kOrderMinRows, "two operand blocks serve ordered solves");
 
 int32_t check_knn_args(uint64_t n, uint64_t d, uint32_t k, scrust_status* st) {
@@ -247,31 +249,31 @@ namespace {
 
 // Whether the tensor form applies: the mode is exact and the row plus the
 // three norm columns fits the operand blocks.  Two blocks (62 to 125
-// dimensions) serve ordered solves alone, where they are the faster: at most
-// 32 neighbours, and kWideMinRows rows (k = 15, d = 70, plain against tensor:
-// 655 and 365 us at 2,048 rows, 3.7 and 0.53 ms at 12,000, 13.4 and 0.68 ms at
-// 30,000; smaller inputs stay where the plain form's rules put them).
-bool tensor_form_applies(const scrust_knn_options& o, int64_t n, int d, uint32_t k) {
+// dimensions) serve ordered solves alone, from the size where they are the
+// faster (k = 15, d = 70, plain against tensor: 655 and 365 us at 2,048 rows,
+// 3.7 and 0.53 ms at 12,000, 13.4 and 0.68 ms at 30,000; smaller inputs stay
+// where the plain form's rules put them).
+bool tensor_form_applies(const scrust_knn_options& o, int64_t n, int d) {
     if (o.mode != SCRUST_MODE_EXACT) return false;
     if (d <= kTensorMaxDim) return true;
-    return d <= kTensorWideMaxDim && k <= kWideMaxK && n >= kWideMinRows && n <= kOrderMaxRows && o.segments <= 1 &&
+    return d <= kTensorWideMaxDim && n >= kWideMinRows && n <= kOrderMaxRows && o.segments <= 1 &&
            o.ordering != SCRUST_ORDERING_OFF;
 }
 
 // Whether a solve runs the tensor form: asked for (or automatic) and applies.
-bool uses_tensor_form(const scrust_knn_options& o, int64_t n, int d, uint32_t k) {
-    return (o.form == SCRUST_FORM_TENSOR || o.form == SCRUST_FORM_AUTO) && tensor_form_applies(o, n, d, k);
+bool uses_tensor_form(const scrust_knn_options& o, int64_t n, int d) {
+    return (o.form == SCRUST_FORM_TENSOR || o.form == SCRUST_FORM_AUTO) && tensor_form_applies(o, n, d);
 }
 
 // Success, noting in the message when an explicit tensor-form request ran the
 // plain form instead.
-int32_t ok_form(scrust_status* st, const scrust_knn_options* opt, uint64_t n, int d, uint32_t k) {
+int32_t ok_form(scrust_status* st, const scrust_knn_options* opt, uint64_t n, int d) {
     ok(st);
-    if (st && opt && opt->form == SCRUST_FORM_TENSOR && !tensor_form_applies(*opt, (int64_t)n, d, k))
+    if (st && opt && opt->form == SCRUST_FORM_TENSOR && !tensor_form_applies(*opt, (int64_t)n, d))
         snprintf(st->message, sizeof(st->message),
                  "ran the plain form: the tensor form needs exact mode and at most %d dimensions (%d from %lld cells "
-                 "on, with k at most %u, ordering and one segment), got %s mode and %d dimensions",
-                 kTensorMaxDim, kTensorWideMaxDim, (long long)kWideMinRows, kWideMaxK,
+                 "on, with ordering and one segment), got %s mode and %d dimensions",
+                 kTensorMaxDim, kTensorWideMaxDim, (long long)kWideMinRows,
                  opt->mode == SCRUST_MODE_EXACT ? "exact" : "reference_snap", d);
     return SCRUST_OK;
 }
@@ -297,7 +299,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
     const int d = plan.d;
     const bool ref = o.mode == SCRUST_MODE_REFERENCE_SNAP;
     const bool cosine = o.metric == SCRUST_METRIC_COSINE;
-    const bool tensor = uses_tensor_form(o, n, d, k);
+    const bool tensor = uses_tensor_form(o, n, d);
     const int64_t n_pad = tensor ? (n + 255) / 256 * 256 : (n + 127) / 128 * 128;
     const int dp = d <= 64 ? (d + 3) / 4 * 4 : (d + 63) / 64 * 64;
     cudaStream_t s = ctx->stream;
@@ -382,9 +384,10 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
         // its warp has appended up to 128 columns.
         // Ordered solves keep long lists (256): a row block's first tiles
         // fill its lists before any threshold exists, and every prune is a
-        // latency the row block waits for.
+        // latency the row block waits for (and 384 for many neighbours, whose
+        // rows keep 1.5 k candidates on average).
         int32_t rc = plan_lists(ctx, lo, (int)k, items, (int)(n_pad / 256), 8 * ctx->sm_count, 128,
-                                order_rows ? 256 : 64, &lists, st);
+                                order_rows ? (k > kTwoSegmentMaxK ? 384 : 256) : 64, &lists, st);
         if (rc) return rc;
         lists.segments *= 2;  // one list per (column segment, column part) of a row
         if ((rc = alloc_lists(ctx, n_pad, &lists, st))) return rc;
@@ -400,58 +403,76 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
             first.count = order.prio_cnt;
             first.stride = kPrioMax;
             first.order = order.prio_order;
-            // k <= 32: the first pass only tightens the thresholds, and one
-            // collect pass over both tile lists appends just the ids of the
-            // columns below them.  The thresholds after the priority tiles
-            // already bound every row (a threshold pass over the other tiles
-            // would lower them by a fraction of a percent of the candidates),
-            // so the other tiles are only collected.  Larger k: two passes
-            // that keep lists.
-            const bool split = k <= 32;
-            const int mode = split ? kPassThresholds : kPassFull;
-            rerank_ids_only = split;
+            // The first pass only tightens the thresholds, and one collect
+            // pass over both tile lists appends just the ids of the columns
+            // below them.  The thresholds after the priority tiles already
+            // bound every row (a threshold pass over the other tiles would
+            // lower them by a fraction of a percent of the candidates), so
+            // the other tiles are only collected.
+            //
             // The threshold pass leaves each list's register top-K (a top-16
             // or top-32: k >= 2; k = 1 keeps a single value a lane), and each
-            // row's threshold is then taken from its two column parts'
-            // lists together.
+            // row's threshold is then taken from its lists together: its two
+            // column parts, and for many neighbours the parts of two or four
+            // column segments that its priority tiles are dealt out to in
+            // turn, so that a list's share of the k stays well inside its 32
+            // values.  (Two passes that kept lists
+            // took 2.3 ms for 50,021 x 30 at k = 50, and left 800 candidates a
+            // row on the way that the rerank spent 3.1 ms on.)
             const int width = k <= 16 ? 16 : 32;
-            const bool merge = split && k >= 2;
+            const bool merge = k >= 2;
+            const int thr_parts = k > kTwoSegmentMaxK && items >= 4 ? 4 : k > kOneSegmentMaxK && items >= 2 ? 2 : 1;
+            const int thr_segments = 2 * thr_parts;
+            rerank_ids_only = true;
             float* topk = nullptr;
+            float* thr_theta = order.theta;
+            TileLists thr = first;
             if (merge) {
-                topk = (float*)ws_get(ctx, SLOT_TOPK, sizeof(float) * (size_t)lists.segments * width * n_pad, &e);
+                // The top-K, and for several segments their thresholds
+                // (unused), tile lists, counts and work order.
+                const size_t top_floats = (size_t)thr_segments * width * n_pad;
+                const size_t extra =
+                    thr_parts == 1 ? 0 : thr_segments * (size_t)n_pad + (size_t)items * thr_parts * (kPrioMax + 2);
+                topk = (float*)ws_get(ctx, SLOT_TOPK, sizeof(float) * (top_floats + extra), &e);
                 if (!topk) return cuda_fail(st, e, "workspace");
+                if (thr_parts > 1) {
+                    thr_theta = topk + top_floats;
+                    uint32_t* dealt = (uint32_t*)(thr_theta + thr_segments * (size_t)n_pad);
+                    uint32_t* dealt_cnt = dealt + (size_t)items * thr_parts * kPrioMax;
+                    uint32_t* dealt_order = dealt_cnt + (size_t)items * thr_parts;
+                    if ((e = launch_deal_tiles(first.tiles, first.count, first.order, items, kPrioMax, thr_parts, dealt,
+                                               dealt_cnt, dealt_order, s)) != cudaSuccess)
+                        return cuda_fail(st, e, "knn_candidates_tc");
+                    ctx->launches += 1;
+                    thr.tiles = dealt;
+                    thr.count = dealt_cnt;
+                    thr.order = dealt_order;
+                }
             }
-            if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16,
-                                              &first, false, order.theta, nullptr, sweep_stats(ctx), nullptr, mode,
-                                              topk)) != cudaSuccess ||
-                (merge && (e = launch_merge_part_thresholds(topk, width, n, n_pad, (int)k, bA, bdelta, beps2,
-                                                            order.theta, s)) != cudaSuccess))
+            Lists thr_lists = lists;
+            thr_lists.segments = thr_segments;
+            if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, thr_lists, bf16,
+                                              &thr, false, thr_theta, nullptr, sweep_stats(ctx), nullptr,
+                                              kPassThresholds, topk)) != cudaSuccess ||
+                (merge && (e = launch_merge_part_thresholds(topk, width, n, n_pad, (int)k, thr_segments, thr.count, bA,
+                                                            bdelta, beps2, order.theta, s)) != cudaSuccess))
                 return cuda_fail(st, e, "knn_candidates_tc");
             ctx->launches += merge ? 2 : 1;
             mark(ctx, PH_PASS1);
             TileLists second;
             if ((rc = build_second_pass(ctx, A16, bf16, n, d, order, bA, bdelta, &second, st))) return rc;
             mark(ctx, PH_LISTS);
-            if (split) {
-                mark(ctx, PH_PASS2);
-                TileLists both = first;
-                both.tiles2 = second.tiles;
-                both.count2 = second.count;
-                both.stride2 = second.stride;
-                if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16,
-                                                  &both, false, order.theta, nullptr, sweep_stats(ctx), nullptr,
-                                                  kPassCollect)) != cudaSuccess)
-                    return cuda_fail(st, e, "knn_candidates_tc");
-                mark(ctx, PH_COLLECT1);
-                ctx->launches += 1;
-            } else {
-                if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16,
-                                                  &second, true, order.theta, nullptr, sweep_stats(ctx), nullptr,
-                                                  mode)) != cudaSuccess)
-                    return cuda_fail(st, e, "knn_candidates_tc");
-                mark(ctx, PH_PASS2);
-                ctx->launches += 1;
-            }
+            mark(ctx, PH_PASS2);
+            TileLists both = first;
+            both.tiles2 = second.tiles;
+            both.count2 = second.count;
+            both.stride2 = second.stride;
+            if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16, &both,
+                                              false, order.theta, nullptr, sweep_stats(ctx), nullptr, kPassCollect)) !=
+                cudaSuccess)
+                return cuda_fail(st, e, "knn_candidates_tc");
+            mark(ctx, PH_COLLECT1);
+            ctx->launches += 1;
         } else {
             // Every list keeps its threshold, so the rerank needs no selection.
             float* theta = (float*)ws_get(ctx, SLOT_THETA, sizeof(float) * (size_t)lists.segments * n_pad, &e);
@@ -518,7 +539,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
                            rerank_ids_only)) != cudaSuccess)
         return cuda_fail(st, e, "knn_rerank");
     mark(ctx, PH_RERANK);
-    return ok_form(st, opt, (uint64_t)n, d, k);
+    return ok_form(st, opt, (uint64_t)n, d);
 }
 
 int32_t take_csr_buffers(scrust_context* ctx, uint64_t rows, uint64_t nnz_cap, CsrBuffers* out,
@@ -912,7 +933,7 @@ int32_t scrust_cuda_knn(scrust_context* ctx, const float* x, uint64_t n, uint64_
             cudaSuccess)
         return cuda_fail(st, e, "download");
     if ((rc = collect_device_errors(ctx, st))) return rc;
-    return ok_form(st, opt, n, (int)d, k);
+    return ok_form(st, opt, n, (int)d);
 }
 
 int32_t scrust_cuda_connectivities_device(scrust_context* ctx, const uint32_t* idx, const float* dist, uint64_t n,
@@ -996,7 +1017,7 @@ int32_t scrust_cuda_neighbors_graph_device(scrust_context* ctx, const float* x, 
     DeviceGuard device_guard(ctx->device);
     if ((rc = knn_device_impl(ctx, x, n, d, k, opt, out_idx, out_dist, st))) return rc;
     if ((rc = conn_device_impl(ctx, out_idx, out_dist, n, k, false, conn, st, true))) return rc;
-    return ok_form(st, opt, n, (int)d, k);
+    return ok_form(st, opt, n, (int)d);
 }
 
 int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_t n, uint64_t d, uint32_t k,
@@ -1046,7 +1067,7 @@ int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_
     }
     if (rc) return rc;
     if ((rc = collect_device_errors(ctx, st))) return rc;
-    return ok_form(st, opt, n, (int)d, k);
+    return ok_form(st, opt, n, (int)d);
 }
 
 int32_t scrust_cuda_synchronize(scrust_context* ctx, scrust_status* st) {

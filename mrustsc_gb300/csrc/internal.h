@@ -371,15 +371,22 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
                                      bool resume, float* theta_io, int* grid_out, unsigned long long* stats,
                                      unsigned long long* argmin_out = nullptr, int pass_mode = 0,
                                      float* topk_out = nullptr);
-// After a threshold pass that wrote its register top-K per list (topk_out,
-// one column segment): each row's threshold from the k-th of both column
-// parts' lists together, into both of its theta slots (knn_tensor.cu).
-cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k,
-                                         const float* bA, const float* bdelta, const float* beps2, float* theta,
-                                         cudaStream_t s);
-// Pass modes of launch_tensor_candidates (k <= 32, one column segment):
+// After a threshold pass that wrote its register top-K per list (topk_out;
+// `segments` lists a row: 2, or 4 or 8 above 32 neighbours, with the tile counts
+// of its work items): each row's threshold from the k-th of its lists together,
+// into both of its theta slots (knn_tensor.cu).
+cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
+                                         const uint32_t* counts, const float* bA, const float* bdelta,
+                                         const float* beps2, float* theta, cudaStream_t s);
+// The tiles of `items` explicit lists (`stride` apart, in work order) dealt out
+// in turn to `parts` column segments: segment s of list i at
+// dst + (parts i + s) stride (order.cu).
+cudaError_t launch_deal_tiles(const uint32_t* src, const uint32_t* cnt, const uint32_t* order, int items, int stride,
+                              int parts, uint32_t* dst, uint32_t* dst_cnt, uint32_t* dst_order, cudaStream_t s);
+// Pass modes of launch_tensor_candidates (k <= kSplitMaxK, one column segment):
 // thresholds only (register top-k, theta_io written, lists untouched), then
 // collection at the fixed thresholds (appends only).
+constexpr int kSplitMaxK = 128;  // at least four lists' register top-32
 constexpr int kPassFull = 0, kPassThresholds = 1, kPassCollect = 2;
 // Kernel counters: words per block, and blocks (the first three sweep
 // launches of a solve, then all later ones).

@@ -75,6 +75,7 @@ struct SweepShape {
     static constexpr uint32_t B_BYTES = B_BLOCK * BLOCKS;
     static constexpr size_t SMEM_BYTES = A_BUFS * A_BYTES + STAGES * B_BYTES + 1024;
 };
+constexpr int kGroup16MaxK = 56;       // threshold passes: most neighbours with groups of 16 columns
 constexpr int kPartCols = TBN / PARTS;  // columns one epilogue warp drains per tile
 
 struct TensorArgs {
@@ -969,7 +970,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                         // The same for a top-32: groups of 4 on an item's
                         // first tile (32 minima per lane), of 16 after it; one
                         // chunk in flight (a top-32 leaves no registers for
-                        // two).
+                        // two).  Above k = 32 the row's lists hold its k-th
+                        // between them: none alone bounds the row, so no
+                        // threshold is formed here.
                         const float kth0 = top.kth();
                         if (it == 0) {
 #pragma unroll 1
@@ -985,7 +988,24 @@ __global__ void __launch_bounds__(THREADS, 1)
                                     top.merge_few(q);
                                 }
                             }
-                            th = fminf(th, bnd.theta_f32(top.kth()));
+                            if (a.k <= TOPK) th = fminf(th, bnd.theta_f32(top.kth()));
+                        } else if (a.k > kGroup16MaxK) {
+                            // Many neighbours share 16-column groups: groups
+                            // of 8, merged chunk by chunk (at k = 100 the
+                            // rows keep 133 candidates instead of 198; at
+                            // k = 50 the dearer pass is not made up for).
+#pragma unroll 1
+                            for (int c = 0; c < 4; ++c) {
+                                float q[4];
+                                tmem_ld32(tbase + 32 * c, va);
+                                tmem_ld_wait(va);
+                                quarter_mins(va, col0 + 32 * c, row, a, q);
+                                cm[c] = fminf(fminf(q[0], q[1]), fminf(q[2], q[3]));
+                                if (__any_sync(0xffffffffu, cm[c] < top.kth())) {
+                                    sort4(q);
+                                    top.merge_few(q);
+                                }
+                            }
                         } else {
                             float g[8];
 #pragma unroll
@@ -1363,8 +1383,11 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
     a.self_offset = plan.self_offset;
     a.col_tiles = (int)(nr_pad / TBN);
     const int col_segs = lists.segments / PARTS;
+    // A threshold pass above 32 neighbours keeps its lists apart; its tiles are
+    // explicit, so the segments cover no ranges.
+    const bool lists_apart = pass_mode == kPassThresholds && plan.k > 32 && tiles && tiles->tiles;
     a.tiles_per_seg = (a.col_tiles + col_segs - 1) / col_segs;
-    if ((a.col_tiles + a.tiles_per_seg - 1) / a.tiles_per_seg != col_segs) return cudaErrorInvalidValue;
+    if (!lists_apart && (a.col_tiles + a.tiles_per_seg - 1) / a.tiles_per_seg != col_segs) return cudaErrorInvalidValue;
     if (lists.ctot < lists.cap + kPartCols || lists.ctot > 32 * kListMaxEntriesPerLane) return cudaErrorInvalidValue;
     // The rerank takes the union of a row's lists: up to kRerankUnion keys.
     a.final_cap = std::max(kListFinalMin, kRerankUnion / lists.segments);
@@ -1390,7 +1413,7 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
         // Explicit tile lists are per work item (row block and column
         // segment); several segments of a row block must share its threshold
         // through row_theta.
-        if ((col_segs != 1 && !tiles->row_theta) || !tiles->count) return cudaErrorInvalidValue;
+        if ((col_segs != 1 && !tiles->row_theta && !lists_apart) || !tiles->count) return cudaErrorInvalidValue;
         a.tl = tiles->tiles;
         a.tl_off = tiles->offset;
         a.tl_cnt = tiles->count;
@@ -1408,20 +1431,24 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
     a.thr_only = pass_mode == kPassThresholds ? 1 : 0;
     a.collect = pass_mode == kPassCollect ? 1 : 0;
     // Threshold and collect passes keep one column segment per row, or share
-    // the row's threshold between its segments through row_theta.
-    if ((a.thr_only || a.collect) && (!theta_io || plan.k > 32 || (lists.segments != PARTS && !a.row_theta)))
+    // the row's threshold between its segments through row_theta.  Above 32
+    // neighbours a threshold pass only leaves its top-32 per list, which
+    // launch_merge_part_thresholds turns into thresholds.
+    if ((a.thr_only || a.collect) &&
+        (!theta_io || plan.k > kSplitMaxK || (lists.segments != PARTS && !a.row_theta && !lists_apart)))
         return cudaErrorInvalidValue;
+    if (a.thr_only && plan.k > 32 && (!topk_out || resume || a.row_theta)) return cudaErrorInvalidValue;
     a.argmin_out = argmin_out;
     a.topk_out = topk_out;
     a.topk_stride = nq_pad * lists.segments;
     // (The top-K is written by the top-16 and top-32 threshold passes: k >= 2.)
-    if (topk_out && (!a.thr_only || lists.segments != PARTS || plan.k < 2)) return cudaErrorInvalidValue;
+    if (topk_out && (!a.thr_only || (lists.segments != PARTS && !lists_apart) || plan.k < 2)) return cudaErrorInvalidValue;
     if (argmin_out && (plan.k != 1 || resume)) return cudaErrorInvalidValue;
     if (a.tl2 && !a.collect) return cudaErrorInvalidValue;  // a second list is read by collect passes only
     if (resume && !theta_io) return cudaErrorInvalidValue;
     // Register top-k width of a general pass (threshold and collect passes
     // keep the width that holds k).
-    int topk = a.k == 1 ? 1 : a.k <= 16 ? 16 : a.k <= 32 ? 32 : 0;
+    int topk = a.k == 1 ? 1 : a.k <= 16 ? 16 : a.k <= 32 || a.thr_only || a.collect ? 32 : 0;
     if (!a.thr_only && !a.collect && a.k > 1) {
         if (plan.topk_width < 0) topk = 0;
         else if (plan.topk_width == 32 && a.k <= 32) topk = 32;
@@ -1458,50 +1485,70 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
     return cudaGetLastError();
 }
 
-// The threshold of each row from both column parts' register top-K of a
-// threshold pass (k <= K; each list ascending with its first K - k slots
-// -inf): the k-th smallest of the two lists' union, which lies at or below
-// each part's own k-th (a row's nearest columns fall in both halves of a
-// tile, so each part alone sees only some of them), bounded as the sweep
-// bounds a k-th, and never above either part's threshold.  Both of the
-// row's theta slots receive it.
-template <int K>
+// The threshold of each row from its lists' register top-K of a threshold pass
+// (each list ascending, for k < K with its first K - k slots -inf): the k-th
+// smallest of the lists' union, which lies at or below each list's own k-th (a
+// row's nearest columns fall in both halves of a tile, so each part alone sees
+// only some of them), bounded as the sweep bounds a k-th, and never above a
+// list's threshold.  LISTS: 2, the column parts, or 4 or 8, the parts of two or
+// four column segments, whose tile counts say which lists were written.  For k > K a list
+// may end before its share of the k does; the lists' values are distinct
+// columns all the same, so the k-th of the union is still no smaller than the
+// row's.  Both of the row's theta slots receive the threshold.
+template <int K, int LISTS>
 __global__ void merge_part_thresholds_kernel(const float* __restrict__ topk, int64_t stride, int64_t n, int k,
-                                             const float* __restrict__ bA, const float* __restrict__ bdelta,
-                                             const float* __restrict__ beps2, float* __restrict__ theta) {
+                                             const uint32_t* __restrict__ counts, const float* __restrict__ bA,
+                                             const float* __restrict__ bdelta, const float* __restrict__ beps2,
+                                             float* __restrict__ theta) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float* p0 = topk + (int64_t)(K - k) * stride + i * PARTS;
-    const float* p1 = p0 + 1;
-    int u = 0, v = 0;
+    const int held = min(k, K);
+    const float* p = topk + (int64_t)(K - held) * stride + i * LISTS;
+    int at[LISTS];
+    float head[LISTS];
+#pragma unroll
+    for (int l = 0; l < LISTS; ++l) {
+        const bool written = LISTS == PARTS || counts[i / ROWS * (LISTS / PARTS) + l / PARTS] != 0u;
+        at[l] = written ? 0 : held;
+        head[l] = written ? p[l] : __int_as_float(0x7f800000);
+    }
     float kth = __int_as_float(0x7f800000);
     for (int t = 0; t < k; ++t) {
-        const float x = u < k ? p0[u * stride] : __int_as_float(0x7f800000);
-        const float y = v < k ? p1[v * stride] : __int_as_float(0x7f800000);
-        if (x <= y) {
-            kth = x;
-            ++u;
-        } else {
-            kth = y;
-            ++v;
-        }
+        int best = 0;
+        kth = head[0];
+#pragma unroll
+        for (int l = 1; l < LISTS; ++l)
+            if (head[l] < kth) {
+                kth = head[l];
+                best = l;
+            }
+#pragma unroll
+        for (int l = 0; l < LISTS; ++l)
+            if (l == best) {
+                ++at[l];
+                head[l] = at[l] < held ? p[at[l] * stride + l] : __int_as_float(0x7f800000);
+            }
     }
-    const float t0 = theta[i * PARTS], t1 = theta[i * PARTS + 1];
-    const float th = fminf(fminf(t0, t1), TensorBound{bA[i], bdelta[i], beps2[i]}.theta_f32(kth));
+    float th = TensorBound{bA[i], bdelta[i], beps2[i]}.theta_f32(kth);
+    // (Above K neighbours no list has a threshold of its own.)
+    if (k <= K) th = fminf(th, fminf(theta[i * PARTS], theta[i * PARTS + 1]));
     theta[i * PARTS] = th;
     theta[i * PARTS + 1] = th;
 }
 
-cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k,
-                                         const float* bA, const float* bdelta, const float* beps2, float* theta,
-                                         cudaStream_t s) {
-    if (k < 1 || k > width || (width != 16 && width != 32)) return cudaErrorInvalidValue;
+cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
+                                         const uint32_t* counts, const float* bA, const float* bdelta,
+                                         const float* beps2, float* theta, cudaStream_t s) {
+    if (k < 1 || (width != 16 && width != 32) || k > (width == 32 ? kSplitMaxK : width)) return cudaErrorInvalidValue;
+    if (segments != PARTS && ((segments != 2 * PARTS && segments != 4 * PARTS) || k <= 32 || !counts))
+        return cudaErrorInvalidValue;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    const int64_t stride = n_pad * PARTS;  // one column segment: PARTS lists a row
-    if (width == 16)
-        merge_part_thresholds_kernel<16><<<blocks, 256, 0, s>>>(topk, stride, n, k, bA, bdelta, beps2, theta);
-    else
-        merge_part_thresholds_kernel<32><<<blocks, 256, 0, s>>>(topk, stride, n, k, bA, bdelta, beps2, theta);
+    const int64_t stride = n_pad * segments;
+    const auto kern = width == 16             ? merge_part_thresholds_kernel<16, PARTS>
+                      : segments == PARTS     ? merge_part_thresholds_kernel<32, PARTS>
+                      : segments == 2 * PARTS ? merge_part_thresholds_kernel<32, 2 * PARTS>
+                                              : merge_part_thresholds_kernel<32, 4 * PARTS>;
+    kern<<<blocks, 256, 0, s>>>(topk, stride, n, k, counts, bA, bdelta, beps2, theta);
     return cudaGetLastError();
 }
 

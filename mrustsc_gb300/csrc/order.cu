@@ -875,6 +875,26 @@ __global__ void gather_rows_kernel(const float* __restrict__ x, const uint32_t* 
     xs[i] = (r == 0xffffffffu || t >= d) ? 0.f : x[(int64_t)r * d + t];
 }
 
+// One thread per (list, segment, tile of the segment).
+__global__ void deal_tiles_kernel(const uint32_t* __restrict__ src, const uint32_t* __restrict__ cnt,
+                                  const uint32_t* __restrict__ order, int items, int stride, int parts,
+                                  uint32_t* __restrict__ dst, uint32_t* __restrict__ dst_cnt,
+                                  uint32_t* __restrict__ dst_order) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int share = (stride + parts - 1) / parts;
+    const int64_t list = t / share;
+    const int p = (int)(t % share);
+    if (list >= (int64_t)parts * items) return;
+    const int64_t i = list / parts;
+    const int s = (int)(list % parts);
+    const int c = (int)min(cnt[i], (uint32_t)stride);
+    if (parts * p + s < c) dst[list * stride + p] = src[i * stride + parts * p + s];
+    if (p == 0) {
+        dst_cnt[list] = (uint32_t)((c + parts - 1 - s) / parts);
+        dst_order[list] = (uint32_t)parts * order[i] + (uint32_t)s;
+    }
+}
+
 // The operand type and width pick the instantiation.
 void launch_tile_balls(bool bf16, const void* ops, int64_t n, int d, int tiles, const uint32_t* cell_of_pos,
                        const float* theta, const float* bA, const float* bdelta, const TileBalls& b, cudaStream_t s) {
@@ -934,6 +954,14 @@ cudaError_t sort_by_work(scrust_context* ctx, const uint32_t* counts, int items,
         return e;
     narrow_kernel<<<(items + 255) / 256, 256, 0, ctx->stream>>>(vs, items, order);
     ctx->launches += 2;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_deal_tiles(const uint32_t* src, const uint32_t* cnt, const uint32_t* order, int items, int stride,
+                              int parts, uint32_t* dst, uint32_t* dst_cnt, uint32_t* dst_order, cudaStream_t s) {
+    const int64_t threads = (int64_t)parts * items * ((stride + parts - 1) / parts);
+    deal_tiles_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(src, cnt, order, items, stride, parts, dst,
+                                                                        dst_cnt, dst_order);
     return cudaGetLastError();
 }
 

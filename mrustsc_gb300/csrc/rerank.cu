@@ -60,6 +60,9 @@ struct RerankArgs {
     uint32_t* big_rows;   // rows with many survivors, for the second sorted pass
     uint32_t* big_count;
     uint32_t* big_next;
+    uint32_t* wide_rows;  // rows for the eight-a-lane pass of a solve of many neighbours
+    uint32_t* wide_count;
+    uint32_t* wide_next;
     float* fb_scratch;
     int* err;
 };
@@ -568,6 +571,250 @@ __device__ int sorted_row_regs(const RerankArgs& a, int64_t slot, unsigned long 
     return 0;
 }
 
+// Ascending bitonic sort across the warp of 32 R keys, position lane + 32 r in
+// key[r]; fully unrolled.
+template <int R>
+__device__ __forceinline__ void warp_sort_wide(unsigned long long (&key)[R]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * R; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= 32) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int o = r ^ (stride / 32);
+                    if (o > r) {
+                        const unsigned long long lo = min_u64(key[r], key[o]), hi = max_u64(key[r], key[o]);
+                        const bool up = ((32 * r) & size) == 0;
+                        key[r] = up ? lo : hi;
+                        key[o] = up ? hi : lo;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int i = lane + 32 * r;
+                    const unsigned long long o = __shfl_xor_sync(0xffffffffu, key[r], stride);
+                    const bool take_min = ((i & stride) == 0) == ((i & size) == 0);
+                    key[r] = ((key[r] < o) == take_min) ? key[r] : o;
+                }
+            }
+        }
+    }
+}
+
+// sorted_row_regs for collected lists (ids below their thresholds) of up to
+// 32 R entries in all: R entries a lane, the same result.  Solves of more than
+// 32 neighbours keep 1.2 to 1.5 k candidates a row, past the 64 that
+// sorted_row_regs holds (its shared-memory form, with the queue of rows above
+// 128 entries, took 3.1 ms for 50,021 rows at k = 50 and 4.3 ms at k = 100).
+// Returns 0 when done, 2 for the fallback, 3 for more entries than that.
+template <int R>
+__device__ int sorted_row_wide(const RerankArgs& a, int64_t slot, unsigned long long* keys_s, double* dbl) {
+    constexpr uint32_t FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int segs = a.lists.segments;
+    if (segs > 32) return 3;
+    const uint32_t ovf = a.lists.overflow[slot];
+    const int cl = lane < segs ? (int)min(a.lists.cnt[slot * segs + lane], (uint32_t)a.lists.ctot) : 0;
+    if (ovf) return 2;
+    // Entry e of the row's lists (in list order) -> list and position.
+    int list[R], pos[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) list[r] = -1;
+    int m = 0;
+    for (int l = 0; l < segs; ++l) {
+        const int c = __shfl_sync(FULL, cl, l);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int e = lane + 32 * r;
+            if (list[r] < 0 && e < m + c) {
+                list[r] = l;
+                pos[r] = e - m;
+            }
+        }
+        m += c;
+    }
+    if (m > 32 * R) return 3;
+    if (m < a.k) return 2;
+    const float* xq = a.xs + slot * a.xs_stride;
+    uint32_t id[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        id[r] = list[r] >= 0 ? a.lists.ids[(slot * segs + list[r]) * (int64_t)a.lists.ctot + pos[r]] : 0xffffffffu;
+    unsigned long long key[R];
+    bool bad = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        key[r] = ~0ull;
+        if (list[r] < 0) continue;
+        if ((int64_t)id[r] >= a.nr) {  // never written by a candidate kernel: refuse to read it
+            bad = true;
+            continue;
+        }
+        const float* xr = a.xr_list + (int64_t)id[r] * a.xs_stride;
+        const float d2 = a.xs_v8 ? dist2_f32_v8(xq, xr, a.xs_stride / 8) : dist2_f32(xq, xr, a.d);
+        key[r] = ((unsigned long long)float_key(d2) << 32) | (uint32_t)input_row(a, id[r]);
+    }
+    if (__any_sync(FULL, bad)) {
+        if (lane == 0) atomicExch(a.err + DERR_CANDIDATES, 1);
+        return 2;
+    }
+    warp_sort_wide<R>(key);
+    // Positions that start a tie group (runs of consecutive tied values).
+    uint32_t S[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = lane + 32 * r;
+        const unsigned long long up = __shfl_up_sync(FULL, key[r], 1);
+        const unsigned long long last = __shfl_sync(FULL, key[r > 0 ? r - 1 : 0], 31);
+        const unsigned long long prev = lane == 0 ? last : up;
+        S[r] = __ballot_sync(FULL, p == 0 || p >= m || !tied(a, key_r(prev), key_r(key[r])));
+    }
+    const int k = a.k;
+    const bool cosine = a.metric == SCRUST_METRIC_COSINE;
+    const int64_t q = query_row(a, slot);
+    // The common case: positions 0..k all start a group.
+    bool plain = !cosine && k < 32 * R;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int bits = k + 1 - 32 * r;  // of this word that must be set
+        const uint32_t want = bits >= 32 ? FULL : bits > 0 ? (1u << bits) - 1u : 0u;
+        plain &= (S[r] & want) == want;
+    }
+    if (plain) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int p = lane + 32 * r;
+            if (p < k) {
+                const uint32_t c = key_id(key[r]);
+                a.out_idx[q * k + p] = a.row_lo ? c - a.row_lo[q] : c;
+                a.out_dist[q * k + p] = sqrtf(key_r(key[r]));
+            }
+        }
+        return 0;
+    }
+    int gs[R], ge[R];
+    bool grouped[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = lane + 32 * r;
+        // The last start at or before p, and the one before the next start.
+        gs[r] = 0;
+        ge[r] = 32 * R - 1;
+#pragma unroll
+        for (int w = 0; w < R; ++w) {
+            const uint32_t upto = w < r ? FULL : w == r ? FULL >> (31 - lane) : 0u;
+            if (S[w] & upto) gs[r] = 32 * w + 31 - __clz(S[w] & upto);
+        }
+#pragma unroll
+        for (int w = R - 1; w >= 0; --w) {
+            const uint32_t after = w > r ? FULL : w == r ? ~(FULL >> (31 - lane)) : 0u;
+            if (S[w] & after) ge[r] = 32 * w + __ffs(S[w] & after) - 2;
+        }
+        ge[r] = min(ge[r], m - 1);
+        grouped[r] = p < m && gs[r] < k && ge[r] > gs[r];
+        keys_s[p] = key[r];
+    }
+    __syncwarp();
+    // Members whose row differs from their group's first member's row.
+    uint32_t D[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = lane + 32 * r;
+        const bool differs = !cosine && grouped[r] && p != gs[r] &&
+                             !rows_equal(a.rraw + (int64_t)key_id(keys_s[gs[r]]) * a.d,
+                                         a.rraw + (int64_t)key_id(key[r]) * a.d, a.d);
+        D[r] = __ballot_sync(FULL, differs);
+    }
+    bool need[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = lane + 32 * r;
+        bool any = false;  // a differing member in positions gs..ge
+#pragma unroll
+        for (int w = 0; w < R; ++w) {
+            const int lo = max(gs[r] - 32 * w, 0), hi = min(ge[r] - 32 * w, 31);
+            if (lo <= hi) any |= (D[w] & (FULL >> (31 - hi)) & (FULL << lo)) != 0u;
+        }
+        need[r] = p < m && gs[r] < k && (cosine || (grouped[r] && any));
+        if (need[r]) dbl[p] = adjudicate(a, q, key_id(key[r]));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = lane + 32 * r;
+        if (p >= m || gs[r] >= k) continue;
+        const uint32_t c = key_id(key[r]);
+        int at = p;
+        if (need[r] && ge[r] > gs[r]) {
+            const double dv = dbl[p];
+            int rank = 0;
+            for (int o = gs[r]; o <= ge[r]; ++o) {
+                const double dq = dbl[o];
+                const uint32_t io = key_id(keys_s[o]);
+                rank += (dq < dv) || (dq == dv && io < c);
+            }
+            at = gs[r] + rank;
+        }
+        if (at < k) {
+            const float dist = need[r] ? __double2float_rn(dbl[p]) : sqrtf(key_r(key[r]));
+            a.out_idx[q * k + at] = a.row_lo ? c - a.row_lo[q] : c;
+            a.out_dist[q * k + at] = dist;
+        }
+    }
+    __syncwarp();
+    return 0;
+}
+
+// rerank_sorted_kernel's rows by sorted_row_wide, four entries a lane: 0.27 ms
+// for 50,021 rows at k = 50 (eight a lane takes twice as long for the same
+// rows: twice the network, half the warps).
+__global__ void __launch_bounds__(RS_WARPS * 32, 4) rerank_wide_kernel(RerankArgs a, int64_t span) {
+    __shared__ unsigned long long keys[RS_WARPS][128];
+    __shared__ double dbl[RS_WARPS][128];
+    const int warp = threadIdx.x >> 5;
+    const int64_t lo = (int64_t)blockIdx.x * span, hi = min(a.nq, lo + span);
+    for (int64_t slot = lo + warp; slot < hi; slot += RS_WARPS) {
+        if (a.qperm && a.qperm[slot] == 0xffffffffu) continue;  // padding of a batch layout
+        const int r = sorted_row_wide<4>(a, slot, keys[warp], dbl[warp]);
+        if (r && (threadIdx.x & 31) == 0) {
+            if (r == 3) {
+                a.wide_rows[atomicAdd(a.wide_count, 1u)] = (uint32_t)slot;
+            } else {
+                push_fallback(a, slot);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The rows with 129 to 256 entries, eight a lane: warps take them from a queue
+// (at k = 100 half of the rows are among them).
+__global__ void __launch_bounds__(RS_WARPS * 32, 2) rerank_wide_queue_kernel(RerankArgs a) {
+    __shared__ unsigned long long keys[RS_WARPS][256];
+    __shared__ double dbl[RS_WARPS][256];
+    const int warp = threadIdx.x >> 5;
+    const uint32_t count = *a.wide_count;
+    for (;;) {
+        uint32_t i = 0;
+        if ((threadIdx.x & 31) == 0) i = atomicAdd(a.wide_next, 1u);
+        i = __shfl_sync(0xffffffffu, i, 0);
+        if (i >= count) break;
+        const int64_t slot = a.wide_rows[i];
+        const int r = sorted_row_wide<8>(a, slot, keys[warp], dbl[warp]);
+        if (r && (threadIdx.x & 31) == 0) {
+            if (r == 3) {
+                a.big_rows[atomicAdd(a.big_count, 1u)] = (uint32_t)slot;
+            } else {
+                push_fallback(a, slot);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // Each block walks its own contiguous range of list rows, its warps on
 // consecutive rows: the rows an SM holds at once come from a few ranges, and
 // neighbouring rows' candidate rows (mostly the same cells) stay in its L1.
@@ -778,13 +1025,17 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     a.big_count = ctx->d_counter + 2;
     a.big_next = ctx->d_counter + 3;
     a.big_rows = nullptr;
+    a.wide_rows = nullptr;
+    a.wide_count = ctx->d_counter + 4;
+    a.wide_next = ctx->d_counter + 5;
     if (xs && theta) {
-        a.big_rows = (uint32_t*)ws_get(ctx, SLOT_RERANK_BIG, sizeof(uint32_t) * (size_t)plan.nq, &e);
+        a.big_rows = (uint32_t*)ws_get(ctx, SLOT_RERANK_BIG, sizeof(uint32_t) * 2 * (size_t)plan.nq, &e);
         if (!a.big_rows) return e;
+        a.wide_rows = a.big_rows + plan.nq;
     }
     a.fb_scratch = fb_scratch;
     a.err = ctx->d_err;
-    e = cudaMemsetAsync(ctx->d_counter, 0, 4 * sizeof(uint32_t), ctx->stream);
+    e = cudaMemsetAsync(ctx->d_counter, 0, 6 * sizeof(uint32_t), ctx->stream);
     if (e != cudaSuccess) return e;
     if (xs && theta) {
         const size_t smem_s = (size_t)RS_WARPS * (2 * RS_KEYS * sizeof(unsigned long long) + RS_KEYS);
@@ -797,8 +1048,16 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
         // of the SM's unified memory to L1, which caches the candidate rows
         // that neighbouring rows share.
         static_assert(RS_WARPS * (2 * RS_KEYS * 8 + RS_KEYS) <= 24 * 1024, "rerank block smem");
-        if ((e = set_smem_carveout(ctx, (const void*)rerank_sorted_kernel, 50)) != cudaSuccess) return e;
-        rerank_sorted_kernel<<<(unsigned)((plan.nq + span - 1) / span), RS_WARPS * 32, smem_s, ctx->stream>>>(a, span);
+        const unsigned grid = (unsigned)((plan.nq + span - 1) / span);
+        if (ids_only && plan.k > 32) {  // most rows hold more than 64 entries
+            rerank_wide_kernel<<<grid, RS_WARPS * 32, 0, ctx->stream>>>(a, span);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            rerank_wide_queue_kernel<<<2 * ctx->sm_count, RS_WARPS * 32, 0, ctx->stream>>>(a);
+            ctx->launches += 1;
+        } else {
+            if ((e = set_smem_carveout(ctx, (const void*)rerank_sorted_kernel, 50)) != cudaSuccess) return e;
+            rerank_sorted_kernel<<<grid, RS_WARPS * 32, smem_s, ctx->stream>>>(a, span);
+        }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         const size_t smem_b = (size_t)RS_BIG_WARPS * (2 * RS_BIG_KEYS * sizeof(unsigned long long) + RS_BIG_KEYS);
         if ((e = set_smem_limit(ctx, (const void*)rerank_sorted_big_kernel, (int)smem_b)) != cudaSuccess) return e;

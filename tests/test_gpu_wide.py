@@ -1,6 +1,6 @@
 """The tensor form with two operand blocks per row (62 to 125 dimensions,
-ordered solves of 2048 cells or more, up to 32 neighbours): the edges of the
-range, top-k widths on both sides of 1 and 16, both operand types and metrics, sizes on and off
+ordered solves of 2048 cells or more): the edges of the range, top-k widths on
+both sides of 1, 16, 32 and 40, both operand types and metrics, sizes on and off
 the tiles, against the FP64 oracle; and where it ends, the plain form."""
 
 from __future__ import annotations
@@ -51,7 +51,8 @@ def check(oracle, x, k, idx, dist, metric):
 
 
 @pytest.mark.parametrize("n,d,k", [(2048, 62, 15), (2049, 64, 16), (2303, 100, 17), (3000, 125, 32), (2500, 100, 1),
-                                   (2500, 90, 2)])
+                                   (2500, 90, 2), (2600, 65, 33), (2700, 125, 41), (2048, 70, 64), (2400, 80, 65),
+                                   (2100, 125, 128)])
 @pytest.mark.parametrize("precision", ["fp16", "bf16"])
 def test_wide_rows_match_fp64(lib, oracle, n, d, k, precision):
     x = synthetic.mixture(n, d, clusters=6, dup_frac=0.01, near_dup_frac=0.01, seed=n + d + k)
@@ -86,9 +87,3 @@ def test_outside_its_range_the_plain_form_runs(lib, n, d, kw):
     assert tiles == 0 and "ran the plain form" in message
     _, _, tiles, message = solve(lib, x, 15, **kw)
     assert tiles == 0 and message == ""
-
-
-def test_more_than_32_neighbours_take_the_plain_form(lib):
-    x = synthetic.mixture(2300, 100, clusters=4, dup_frac=0.01, seed=6)
-    _, _, tiles, message = solve(lib, x, 33, form="tensor")
-    assert tiles == 0 and "ran the plain form" in message
