@@ -378,6 +378,12 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
 cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
                                          const uint32_t* counts, const float* bA, const float* bdelta,
                                          const float* beps2, float* theta, cudaStream_t s);
+// The same for rows of up to 32 lists that share row_theta (a query solve's
+// column segments): row_theta falls to the bound of the k-th of a row's lists
+// together.
+cudaError_t launch_merge_segment_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
+                                            const uint32_t* counts, const float* bA, const float* bdelta,
+                                            const float* beps2, uint32_t* row_theta, cudaStream_t s);
 // The tiles of `items` explicit lists (`stride` apart, in work order) dealt out
 // in turn to `parts` column segments: segment s of list i at
 // dst + (parts i + s) stride (order.cu).

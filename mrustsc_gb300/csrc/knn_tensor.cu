@@ -869,25 +869,37 @@ __global__ void __launch_bounds__(THREADS, 1)
                         // At the final thresholds every column that passes is a
                         // candidate: only its id is kept (the rerank measures it
                         // again), and each lane loops over its own passes.
+                        auto take = [&](int c) {
+                            uint32_t mask = below_mask(va, th);
+                            const int64_t cb = col0 + 32 * c;
+                            while (mask) {
+                                const int64_t col = cb + below_col(__ffs(mask) - 1);
+                                mask &= mask - 1;
+                                // Not past the reference rows, not the row itself.
+                                if (col < a.nr && !(a.self && col == row + a.self_offset))
+                                    ids[cnt++] = (uint32_t)col;  // ids only: no values
+                            }
+                        };
+                        // The priority tiles of a self solve hold its rows' own
+                        // cells, nearly every chunk some row's candidate: the
+                        // mask is formed at once.  The tiles that the balls
+                        // kept beside them, and a query's, have many chunks
+                        // with none: a minimum tree and a vote skip those
+                        // (300,000 x 20 in 60 clusters, three quarters of its
+                        // tiles such: 3.5 -> 2.7 ms).
+                        if (PASS == 2 && it < order.count1) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            tmem_ld32(tbase + 32 * c, va);
-                            tmem_ld_wait(va);
-                            // A self solve's rows collect among their own
-                            // cells, nearly every chunk holding some row's
-                            // candidate: the mask is formed at once (PASS 2).
-                            // Query rows meet many chunks with none: a
-                            // minimum tree and a vote skip those (PASS 4).
-                            if (PASS == 2 || __any_sync(0xffffffffu, min32(va) < th)) {
-                                uint32_t mask = below_mask(va, th);
-                                const int64_t cb = col0 + 32 * c;
-                                while (mask) {
-                                    const int64_t col = cb + below_col(__ffs(mask) - 1);
-                                    mask &= mask - 1;
-                                    // Not past the reference rows, not the row itself.
-                                    if (col < a.nr && !(a.self && col == row + a.self_offset))
-                                        ids[cnt++] = (uint32_t)col;  // ids only: no values
-                                }
+                            for (int c = 0; c < 4; ++c) {
+                                tmem_ld32(tbase + 32 * c, va);
+                                tmem_ld_wait(va);
+                                take(c);
+                            }
+                        } else {
+#pragma unroll 1
+                            for (int c = 0; c < 4; ++c) {
+                                tmem_ld32(tbase + 32 * c, va);
+                                tmem_ld_wait(va);
+                                if (__any_sync(0xffffffffu, min32(va) < th)) take(c);
                             }
                         }
                     } else if constexpr (PASS == 3) {
@@ -914,10 +926,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                         // costs a sort of its group minima and a merge instead
                         // of an insertion per entrant.  Groups of 8 on an
                         // item's first tile (16 minima per lane: the K-th is
-                        // finite after one tile), of 16 after it.
+                        // finite after one tile), of 16 after it -- and of 8
+                        // throughout for queries, whose nearest rows often
+                        // sit in one small cell: 128 of its rows in a row are
+                        // eight groups of 16, fewer than k.
                         const float kth0 = top.kth();
                         uint32_t vb[32];
-                        if (it == 0) {
+                        if (it == 0 || !a.self) {
 #pragma unroll 1
                             for (int c = 0; c < 4; ++c) {
                                 float q[4];
@@ -989,7 +1004,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 }
                             }
                             if (a.k <= TOPK) th = fminf(th, bnd.theta_f32(top.kth()));
-                        } else if (a.k > kGroup16MaxK) {
+                        } else if (a.k > kGroup16MaxK || !a.self) {
                             // Many neighbours share 16-column groups: groups
                             // of 8, merged chunk by chunk (at k = 100 the
                             // rows keep 133 candidates instead of 198; at
@@ -1001,11 +1016,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 tmem_ld_wait(va);
                                 quarter_mins(va, col0 + 32 * c, row, a, q);
                                 cm[c] = fminf(fminf(q[0], q[1]), fminf(q[2], q[3]));
-                                if (__any_sync(0xffffffffu, cm[c] < top.kth())) {
+                                if (__any_sync(0xffffffffu, cm[c] < fminf(top.kth(), th))) {
                                     sort4(q);
                                     top.merge_few(q);
                                 }
                             }
+                            if (a.k <= TOPK && top.kth() < kth0) th = fminf(th, bnd.theta_f32(top.kth()));
                         } else {
                             float g[8];
 #pragma unroll
@@ -1442,7 +1458,8 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
     a.topk_out = topk_out;
     a.topk_stride = nq_pad * lists.segments;
     // (The top-K is written by the top-16 and top-32 threshold passes: k >= 2.)
-    if (topk_out && (!a.thr_only || (lists.segments != PARTS && !lists_apart) || plan.k < 2)) return cudaErrorInvalidValue;
+    if (topk_out && (!a.thr_only || (lists.segments != PARTS && !lists_apart && !a.row_theta) || plan.k < 2))
+        return cudaErrorInvalidValue;
     if (argmin_out && (plan.k != 1 || resume)) return cudaErrorInvalidValue;
     if (a.tl2 && !a.collect) return cudaErrorInvalidValue;  // a second list is read by collect passes only
     if (resume && !theta_io) return cudaErrorInvalidValue;
@@ -1549,6 +1566,49 @@ cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n
                       : segments == 2 * PARTS ? merge_part_thresholds_kernel<32, 2 * PARTS>
                                               : merge_part_thresholds_kernel<32, 4 * PARTS>;
     kern<<<blocks, 256, 0, s>>>(topk, stride, n, k, counts, bA, bdelta, beps2, theta);
+    return cudaGetLastError();
+}
+
+// A warp per row, a lane per list: the lists' top-K in shared memory, k rounds
+// of the smallest head.  A list of a row with a shared threshold holds every
+// value of its columns below that threshold (or its K smallest), so the k-th
+// of the lists together bounds the row wherever it exists.
+template <int K>
+__global__ void __launch_bounds__(256)
+    merge_segment_thresholds_kernel(const float* __restrict__ topk, int64_t stride, int64_t n, int k, int lists,
+                                    const uint32_t* __restrict__ counts, const float* __restrict__ bA,
+                                    const float* __restrict__ bdelta, const float* __restrict__ beps2,
+                                    uint32_t* __restrict__ row_theta) {
+    __shared__ float vals[8][32][K + 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 8 + w;
+    if (i >= n) return;
+    const float inf = __int_as_float(0x7f800000);
+    const bool written = lane < lists && counts[i / ROWS * (lists / PARTS) + lane / PARTS] != 0u;
+    // (The first K - k slots are -inf.)
+    for (int t = 0; t < k; ++t) vals[w][lane][t] = written ? topk[(int64_t)(K - k + t) * stride + i * lists + lane] : inf;
+    int at = 0;
+    uint32_t kth = 0;
+    for (int t = 0; t < k; ++t) {
+        const uint32_t head = float_key(at < k ? vals[w][lane][at] : inf);
+        kth = __reduce_min_sync(0xffffffffu, head);
+        const uint32_t who = __ballot_sync(0xffffffffu, head == kth);
+        if (lane == __ffs(who) - 1) ++at;
+    }
+    if (lane == 0) {
+        const float th = TensorBound{bA[i], bdelta[i], beps2[i]}.theta_f32(key_float(kth));
+        row_theta[i] = min(row_theta[i], float_key(th));
+    }
+}
+
+cudaError_t launch_merge_segment_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
+                                            const uint32_t* counts, const float* bA, const float* bdelta,
+                                            const float* beps2, uint32_t* row_theta, cudaStream_t s) {
+    if (k < 2 || k > width || (width != 16 && width != 32) || segments > 32 || segments % PARTS)
+        return cudaErrorInvalidValue;
+    const auto kern = width == 16 ? merge_segment_thresholds_kernel<16> : merge_segment_thresholds_kernel<32>;
+    kern<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(topk, n_pad * segments, n, k, segments, counts, bA, bdelta, beps2,
+                                                 row_theta);
     return cudaGetLastError();
 }
 

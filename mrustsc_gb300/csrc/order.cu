@@ -320,7 +320,10 @@ __global__ void unpack_perm_kernel(const uint32_t* __restrict__ skeys, const uns
 // cells, then those holding the cells of their nearest anchors, nearest
 // anchors first; distinct, at most kPrioMax.  In a self solve the item's own
 // tile always comes first, so no list is empty.
-constexpr int kHomeMax = 8;
+// (With the first 8 home cells only, a block of many small cells gave the rows
+// past them thresholds from other clusters: 40 rows of one million overflowed
+// their lists, and the exact fallback took 32 ms for them.)
+constexpr int kHomeMax = 32;
 __global__ void prio_tiles_kernel(const uint32_t* __restrict__ cell_of_pos, int64_t n,
                                   const uint32_t* __restrict__ cell_start, int m,
                                   const uint32_t* __restrict__ anchor_nb, int ka, int items, int col_tiles,
@@ -394,7 +397,10 @@ __device__ __forceinline__ float op_bits<__nv_bfloat16>(uint32_t w) {
 // rows of one cell; a cell lies in one region of the data, while a tile
 // may straddle two far-apart cells).  Segments past kSegMax merge into the
 // last.  Centres are stored dimension-major for coalesced pair tests.
-constexpr int kSegMax = 8;
+// Segments past kSegMax share one ball, which then reaches everywhere: with 8,
+// one block of a million cells kept all 3,900 tiles and its CTA took 6.4 ms of
+// a collect pass of 1.3 ms.
+constexpr int kSegMax = 32;
 struct TileBalls {
     float* centre;      // [d][tiles]
     float* radius;      // [tiles]
@@ -636,11 +642,11 @@ __global__ void __launch_bounds__(256) tile_lists_kernel(const uint32_t* __restr
     __shared__ int wsum[8];
     const int I = blockIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int pc = (int)min(prio_cnt[I], (uint32_t)min(prio_stride, (int)blockDim.x));
+    const int pc = (int)min(prio_cnt[I], (uint32_t)prio_stride);
     for (int i = threadIdx.x; i < words; i += blockDim.x) in_prio[i] = 0u;
     __syncthreads();
-    if (threadIdx.x < pc) {
-        const uint32_t t = prio[(int64_t)I * prio_stride + threadIdx.x];
+    for (int i = threadIdx.x; i < pc; i += blockDim.x) {
+        const uint32_t t = prio[(int64_t)I * prio_stride + i];
         if (t < (uint32_t)tiles) atomicOr(&in_prio[t >> 5], 1u << (t & 31));
     }
     __syncthreads();
@@ -734,93 +740,187 @@ __global__ void transpose_centres_kernel(const float* __restrict__ fc, int64_t s
     out[(i % 64) * segs + i / 64] = fc[i];
 }
 
-// Query blocks against atlas tiles: for every (query segment, atlas segment)
-// pair, the atlas tile may hold a candidate of the query block while
-// tile_needed holds (the same test as a self solve's, with the query
-// segment's reach).  One block per query segment at a time, its centre in
-// shared memory; threads over the atlas segments.
-__global__ void __launch_bounds__(256) cross_segment_pairs_kernel(
-    const float* __restrict__ qc, const float* __restrict__ qr, const float* __restrict__ qu,
-    const uint32_t* __restrict__ qo, const uint32_t* __restrict__ q_count, const float* __restrict__ act,
-    const float* __restrict__ ar, const uint32_t* __restrict__ ao, int64_t asegs, int d, int words,
-    uint32_t* __restrict__ bitmap) {
-    __shared__ float c[64];
-    const uint32_t sq = *q_count;
-    for (uint32_t a = blockIdx.x; a < sq; a += gridDim.x) {
-        __syncthreads();
-        if (threadIdx.x < 64) c[threadIdx.x] = qc[(int64_t)a * 64 + threadIdx.x];
-        __syncthreads();
-        const float ra = qr[a], ua = qu[a];
-        const uint32_t item = qo[a];
-        for (int64_t b = threadIdx.x; b < asegs; b += blockDim.x) {
-            float acc = 0.f;
-            for (int t = 0; t < d; ++t) {
-                const float df = c[t] - act[(int64_t)t * asegs + b];
-                acc = fmaf(df, df, acc);
-            }
-            if (tile_needed(acc, ra, ar[b], ua)) {
-                const uint32_t tb = ao[b];
-                atomicOr(bitmap + (int64_t)item * words + (tb >> 5), 1u << (tb & 31));
-            }
-        }
+// Query rows against atlas tiles: the atlas tile of a segment ball may hold a
+// candidate of a query while tile_needed holds for the query as a ball of
+// radius 0 and of its own reach sqrt(theta + A + delta); the row block takes
+// the tiles of all its queries.  64 queries x 64 atlas segments a block, 4 x 4
+// a thread, distances in f32 on the quantised rows.  Testing every query costs
+// 3 d operations a segment (5,000 x 8,000 segments: 200 us), and a block of
+// queries sorted by cell falls in a hundred cells or more: balls around runs
+// of its queries (eight at most, tested one by one in 276 us) covered so much
+// that nearly every tile was kept, three passes of 600 us and more.
+template <class T>
+__global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ ops, int64_t q,
+                                                          const uint32_t* __restrict__ row_theta,
+                                                          const float* __restrict__ bA,
+                                                          const float* __restrict__ bdelta,
+                                                          const float* __restrict__ act, const float* __restrict__ ar,
+                                                          const uint32_t* __restrict__ ao, int64_t asegs, int d,
+                                                          int words, uint32_t* __restrict__ bitmap) {
+    __shared__ __align__(16) float As[64][64 + 4];
+    __shared__ __align__(16) float Bs[64][64 + 4];
+    __shared__ float reach[64];
+    __shared__ uint32_t hit[64];
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+    const int64_t i0 = (int64_t)blockIdx.y * 64, j0 = (int64_t)blockIdx.x * 64;
+    for (int p = threadIdx.x; p < 64 * 64; p += blockDim.x) {
+        const int r = p / 64, t = p % 64;
+        As[t][r] = i0 + r < q && t < d ? op_float(ops[(i0 + r) * 64 + t]) : 0.f;
+        // (The centres come dimension by dimension.)
+        const int u = p / 64, c = p % 64;
+        Bs[u][c] = j0 + c < asegs && u < d ? act[(int64_t)u * asegs + j0 + c] : 0.f;
     }
+    if (threadIdx.x < 64) {
+        hit[threadIdx.x] = 0u;
+        const int64_t i = i0 + threadIdx.x;
+        float u = 0.f;
+        if (i < q) {
+            // Every step rounded up; a row without a threshold reaches all.
+            const uint32_t key = row_theta[i];
+            const float th = key == 0xffffffffu ? __int_as_float(0x7f800000) : key_float(key);
+            const float v = __fadd_ru(__fadd_ru(th, bA[i]), bdelta[i]);
+            u = isinf(th) && th > 0.f ? th : (v > 0.f ? __fsqrt_ru(v) : 0.f);
+        }
+        reach[threadIdx.x] = u;
+    }
+    __syncthreads();
+    float acc[4][4] = {};
+    for (int t = 0; t < d; ++t) {
+        const float4 a4 = *reinterpret_cast<const float4*>(&As[t][ty * 4]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&Bs[t][tx * 4]);
+        const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float df = av[p] - bv[c];
+                acc[p][c] = fmaf(df, df, acc[p][c]);
+            }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int64_t j = j0 + tx * 4 + c;
+        if (j >= asegs) continue;
+        const float rj = ar[j];
+        bool any = false;
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+            any |= i0 + ty * 4 + p < q && tile_needed(acc[p][c], 0.f, rj, reach[ty * 4 + p]);
+        if (any) hit[tx * 4 + c] = 1u;
+    }
+    __syncthreads();
+    if (threadIdx.x < 64 && hit[threadIdx.x]) {
+        const uint32_t tile = ao[j0 + threadIdx.x];
+        atomicOr(bitmap + i0 / 256 * words + (tile >> 5), 1u << (tile & 31));
+    }
+}
+
+// Exclusive prefix of `v` over the block's 256 threads, and the total.
+__device__ __forceinline__ int block_prefix(int v, int* wsum, int* total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    __syncthreads();
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int i = 0; i < 8; ++i) {
+        before += i < w ? wsum[i] : 0;
+        all += wsum[i];
+    }
+    *total = all;
+    return before + incl - v;
 }
 
 // Priority tiles of a block of routed queries.  A block of 256 queries sorted
 // by cell may span many cells (queries are few per cell), so every cell of
-// its rows counts: the tiles holding those cells, lowest first, then the
-// tiles of their eight nearest neighbouring cells, at most kQueryPrio in all.
-// One block of 256 threads per query block; two tile bitmaps in shared memory.
-constexpr int kQueryPrio = 256;
+// its rows counts: the tiles holding those cells, then, for small cells, the
+// nearest neighbouring cells until they hold `want` rows between them (16 k: the
+// threshold pass looks at groups of 8 columns, and k of them must come from
+// the query's own surroundings), up to kQueryPrio tiles; and while fewer than kQueryPrioNear have been taken,
+// the tiles of the cells' eight nearest neighbours, lowest first.  The tiles come
+// in ascending order, so that the chunks they are cut into hold whole
+// clusters.  (A query whose cell was small, or whose tiles were left out, kept
+// a threshold from another cluster, and its block then every tile of the
+// atlas: 11,691 second tiles of 20 blocks for 5,000 queries of a million
+// cells, 3,651 of one block for 100.)
+// One block of 256 threads per query block; three tile bitmaps in shared memory.
+constexpr int kQueryPrio = 512;
+constexpr int kQueryPrioNear = 256;
 constexpr int kQueryPrioNb = 8;
 __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restrict__ cell_of_pos, int64_t n,
                                                          const uint32_t* __restrict__ cell_start, int m,
                                                          const uint32_t* __restrict__ cell_nb, int col_tiles,
-                                                         uint32_t* __restrict__ prio, uint32_t* __restrict__ prio_cnt) {
+                                                         uint32_t want, uint32_t* __restrict__ prio,
+                                                         uint32_t* __restrict__ prio_cnt) {
     extern __shared__ uint32_t qp_bm[];
+    __shared__ int wsum[8];
     const int words = (col_tiles + 31) / 32;
     uint32_t* home = qp_bm;
-    uint32_t* near = qp_bm + words;
+    uint32_t* more = qp_bm + words;
+    uint32_t* near = qp_bm + 2 * words;
     const int I = blockIdx.x;
-    for (int i = threadIdx.x; i < 2 * words; i += blockDim.x) qp_bm[i] = 0u;
+    for (int i = threadIdx.x; i < 3 * words; i += blockDim.x) qp_bm[i] = 0u;
     __syncthreads();
     const int64_t p = (int64_t)I * 256 + threadIdx.x;
+    // Marks the tiles of cell c; its rows.
     auto mark = [&](uint32_t* bm, uint32_t c) {
-        if (c >= (uint32_t)m) return;
+        if (c >= (uint32_t)m) return 0u;
         const uint32_t a = cell_start[c], b = cell_start[c + 1];
-        if (b <= a) return;
+        if (b <= a) return 0u;
         for (uint32_t t = a / 256; t <= (b - 1) / 256 && t < (uint32_t)col_tiles; ++t)
             atomicOr(&bm[t >> 5], 1u << (t & 31));
+        return b - a;
     };
     if (p < n) {
         const uint32_t c = cell_of_pos[p];
         // Rows of one cell come together: the first of each run marks for all.
         if (p == (int64_t)I * 256 || cell_of_pos[p - 1] != c) {
-            mark(home, c);
-            if (c < (uint32_t)m)
-                for (int j = 0; j < kQueryPrioNb; ++j) mark(near, cell_nb[(int64_t)c * kAnchorNeighbours + j]);
+            uint32_t rows = mark(home, c);
+            if (c < (uint32_t)m) {
+                const uint32_t* nb = cell_nb + (int64_t)c * kAnchorNeighbours;
+                int j = 0;
+                for (; j < kAnchorNeighbours && rows < want; ++j) rows += mark(more, nb[j]);
+                for (const int j1 = min(j + kQueryPrioNb, kAnchorNeighbours); j < j1; ++j) mark(near, nb[j]);
+            }
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t* out = prio + (int64_t)I * kQueryPrio;
-        int cnt = 0;
-        for (int w = 0; w < words && cnt < kQueryPrio; ++w) {
-            uint32_t bits = home[w];
-            while (bits && cnt < kQueryPrio) {
-                out[cnt++] = (uint32_t)(w * 32 + __ffs(bits) - 1);
-                bits &= bits - 1;
-            }
+    // Each thread has a run of words; a bit stays while its place among the
+    // bits of its kind is within the budget.
+    const int per = (words + 255) / 256, w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
+    auto keep = [&](uint32_t* bm, int budget) {
+        int c = 0, total = 0;
+        for (int w = w0; w < w1; ++w) c += __popc(bm[w]);
+        int at = block_prefix(c, wsum, &total);
+        for (int w = w0; w < w1; ++w) {
+            uint32_t bits = bm[w];
+            const int here = __popc(bits);
+            for (int over = min(here, at + here - budget); over > 0; --over) bits &= ~(0x80000000u >> __clz(bits));
+            bm[w] = bits;
+            at += here;
         }
-        for (int w = 0; w < words && cnt < kQueryPrio; ++w) {
-            uint32_t bits = near[w] & ~home[w];
-            while (bits && cnt < kQueryPrio) {
-                out[cnt++] = (uint32_t)(w * 32 + __ffs(bits) - 1);
-                bits &= bits - 1;
-            }
-        }
-        prio_cnt[I] = (uint32_t)cnt;
+        return min(total, budget);
+    };
+    int taken = keep(home, kQueryPrio);
+    for (int w = w0; w < w1; ++w) more[w] &= ~home[w];
+    taken += keep(more, kQueryPrio - taken);
+    for (int w = w0; w < w1; ++w) near[w] &= ~(home[w] | more[w]);
+    keep(near, max(0, kQueryPrioNear - taken));
+    int c = 0, total = 0;
+    for (int w = w0; w < w1; ++w) {
+        home[w] |= more[w] | near[w];
+        c += __popc(home[w]);
     }
+    int at = block_prefix(c, wsum, &total);
+    uint32_t* out = prio + (int64_t)I * kQueryPrio;
+    for (int w = w0; w < w1; ++w)
+        for (uint32_t bits = home[w]; bits; bits &= bits - 1) out[at++] = (uint32_t)(w * 32 + __ffs(bits) - 1);
+    if (threadIdx.x == 0) prio_cnt[I] = (uint32_t)total;
 }
 
 // A row block's tile list cut into `segs` contiguous chunks of equal size,
@@ -841,17 +941,6 @@ __global__ void split_lists_kernel(const uint32_t* __restrict__ src, int src_str
         dst[((int64_t)I * segs + t / chunk) * dst_stride + t % chunk] = src[(int64_t)I * src_stride + t];
     if (threadIdx.x < segs)
         dst_cnt[(int64_t)I * segs + threadIdx.x] = (uint32_t)max(0, min(chunk, c - (int)threadIdx.x * chunk));
-}
-
-// Per row, its shared threshold as both part thresholds (the layout the
-// tile balls read).
-__global__ void row_theta_pairs_kernel(const uint32_t* __restrict__ row_theta, int64_t n, float* __restrict__ out) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t k = row_theta[i];
-    const float t = k == 0xffffffffu ? __int_as_float(0x7f800000) : key_float(k);  // none yet: reach everything
-    out[2 * i] = t;
-    out[2 * i + 1] = t;
 }
 
 __global__ void gather_rows_kernel(const float* __restrict__ x, const uint32_t* __restrict__ perm, int64_t n, int d,
@@ -1367,7 +1456,6 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     const int ps = (kQueryPrio + csegs - 1) / csegs, es = (col_tiles + csegs - 1) / csegs;
     const int P = padded_row_floats(d);
     const int nblocks = radix_blocks(q);
-    const int64_t smax = (int64_t)items * kSegMax;
     const size_t scan_elems =
         scan_scratch_elems(std::max<int64_t>((int64_t)256 * nblocks, std::max<int64_t>(items, at.anchors) + 1));
     size_t off = 0;
@@ -1385,17 +1473,11 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
                  o_pc = take(4 * (size_t)items), o_ps = take(4 * (size_t)work * ps), o_psc = take(4 * (size_t)work),
                  o_po = take(4 * (size_t)work), o_po2 = take(4 * (size_t)work), o_ws = take(work_order_scratch(work)),
                  o_rt = take(4 * (size_t)q_pad), o_th = take(4 * 2 * (size_t)csegs * q_pad),
-                 o_th2 = take(4 * 2 * (size_t)q_pad), o_so = take(4 * ((size_t)items + 1)),
-                 o_fc = take(4 * 64 * (size_t)smax), o_fr = take(4 * (size_t)smax), o_fu = take(4 * (size_t)smax),
-                 o_fo = take(4 * (size_t)smax), o_bm = take(4 * (size_t)items * words_t),
-                 o_cnt = take(4 * ((size_t)items + 1)), o_ent = take(4 * (size_t)items * col_tiles),
+                 o_bm = take(4 * (size_t)items * words_t), o_cnt = take(4 * ((size_t)items + 1)), o_ent = take(4 * (size_t)items * col_tiles),
                  o_es = take(4 * (size_t)work * es), o_esc = take(4 * (size_t)work),
                  o_hist = take(4 * ((size_t)256 * nblocks + 16)), o_scan = take(4 * scan_elems);
-    TileBalls qballs;
-    const size_t total = carve_balls(nullptr, off, items, d, &qballs);
-    char* base = (char*)ws_get(ctx, SLOT_XORDER, total, &e);
+    char* base = (char*)ws_get(ctx, SLOT_XORDER, off, &e);
     if (!base) return cuda_fail(st, e, "query routing: workspace");
-    carve_balls(base, off, items, d, &qballs);
     float* t0 = (float*)(base + o_t0);
     float *bA0 = t0, *eps0 = t0 + q_pad;
     float* ts = (float*)(base + o_ts);
@@ -1407,9 +1489,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     uint32_t* prio_cnt = (uint32_t*)(base + o_pc);
     uint32_t* row_theta = (uint32_t*)(base + o_rt);
     float* theta = (float*)(base + o_th);
-    float* theta2 = (float*)(base + o_th2);
     float* xs = (float*)(base + o_xs);
-    uint32_t* seg_off = (uint32_t*)(base + o_so);
     uint32_t* bitmap = (uint32_t*)(base + o_bm);
     uint32_t* counts = (uint32_t*)(base + o_cnt);
     uint32_t* entries = (uint32_t*)(base + o_ent);
@@ -1465,11 +1545,11 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
         (e = launch_gather_rows(dq, qperm, q, d, P, xs, s)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: gather");
     // Priority tiles per row block, dealt over its column segments.
-    const size_t prio_smem = 8 * (size_t)words_t;
+    const size_t prio_smem = 12 * (size_t)words_t;
     if ((e = set_smem_limit(ctx, (const void*)query_prio_kernel, (int)prio_smem)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: priority tiles");
     query_prio_kernel<<<items, 256, prio_smem, s>>>(cell_of_pos, q, at.cell_start, (int)at.anchors, at.cell_nb,
-                                                    col_tiles, prio, prio_cnt);
+                                                    col_tiles, 16u * (uint32_t)k, prio, prio_cnt);
     split_lists_kernel<<<items, 256, 0, s>>>(prio, kQueryPrio, prio_cnt, csegs, (uint32_t*)(base + o_ps), ps,
                                              (uint32_t*)(base + o_psc));
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: priority tiles");
@@ -1506,28 +1586,38 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     if ((e = cudaMemsetAsync(theta, 0x7f, 4 * 2 * (size_t)csegs * q_pad, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(row_theta, 0xff, 4 * (size_t)q_pad, s)) != cudaSuccess)
         return cuda_fail(st, e, "query knn: memset");
+    // Each row's threshold is then taken from its lists together: a list sees
+    // one column part of one segment's few tiles, so the best list's own k-th
+    // lies far beyond the row's (one query alone, 13 tiles over 16 segments,
+    // kept some 400 candidates).
+    const int width = k <= 16 ? 16 : 32;
+    float* topk = nullptr;
+    if (k >= 2) {
+        topk = (float*)ws_get(ctx, SLOT_TOPK, sizeof(float) * (size_t)lists.segments * width * q_pad, &e);
+        if (!topk) return cuda_fail(st, e, "query knn: workspace");
+    }
     if ((e = launch_tensor_candidates(ctx, plan, base + o_As, q_pad, at.B16, at.m_pad, bA, bdelta, beps2, lists, bf16,
-                                      &first, false, theta, nullptr, nullptr, nullptr, kPassThresholds)) != cudaSuccess)
+                                      &first, false, theta, nullptr, nullptr, nullptr, kPassThresholds, topk)) !=
+            cudaSuccess ||
+        (topk && (e = launch_merge_segment_thresholds(topk, width, q, q_pad, k, lists.segments, first.count, bA, bdelta,
+                                                      beps2, row_theta, s)) != cudaSuccess))
         return cuda_fail(st, e, "query knn: threshold pass");
-    // The atlas tiles each row block cannot rule out: its segment balls
-    // (reach from the rows' shared thresholds) against the atlas segment
-    // balls.
-    row_theta_pairs_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>(row_theta, q, theta2);
-    if ((e = cudaMemsetAsync(qballs.nseg + items, 0, sizeof(uint32_t), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)items * words_t, s)) != cudaSuccess)
+    ctx->launches += topk ? 1 : 0;
+    // The atlas tiles each row block cannot rule out: its queries, with the
+    // reach of their shared thresholds, against the atlas segment balls.
+    if ((e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)items * words_t, s)) != cudaSuccess)
         return cuda_fail(st, e, "query knn: memset");
-    launch_tile_balls(bf16, base + o_As, q, d, items, cell_of_pos, theta2, bA, bdelta, qballs, s);
-    if ((e = cudaGetLastError()) != cudaSuccess ||
-        (e = device_exclusive_scan(ctx, qballs.nseg, seg_off, (int64_t)items + 1, (uint32_t*)(base + o_scan),
-                                   scan_elems)) != cudaSuccess)
-        return cuda_fail(st, e, "query knn: query balls");
-    flatten_segments_kernel<<<items, 64, 0, s>>>(qballs, d, 64, items, seg_off, (float*)(base + o_fc),
-                                                 (float*)(base + o_fr), (float*)(base + o_fu),
-                                                 (uint32_t*)(base + o_fo));
-    cross_segment_pairs_kernel<<<(unsigned)std::min<int64_t>(smax, 8 * ctx->sm_count), 256, 0, s>>>(
-        (const float*)(base + o_fc), (const float*)(base + o_fr), (const float*)(base + o_fu),
-        (const uint32_t*)(base + o_fo), seg_off + items, at.seg_centre_t, at.seg_radius, at.seg_tile, at.segs, d,
-        words_t, bitmap);
+    if (at.segs) {
+        const dim3 grid((unsigned)((at.segs + 63) / 64), (unsigned)((q + 63) / 64));
+        if (bf16)
+            query_tiles_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)(base + o_As), q, row_theta, bA,
+                                                                   bdelta, at.seg_centre_t, at.seg_radius, at.seg_tile,
+                                                                   at.segs, d, words_t, bitmap);
+        else
+            query_tiles_kernel<__half><<<grid, 256, 0, s>>>((const __half*)(base + o_As), q, row_theta, bA, bdelta,
+                                                            at.seg_centre_t, at.seg_radius, at.seg_tile, at.segs, d,
+                                                            words_t, bitmap);
+    }
     const size_t lists_smem = 4 * (size_t)words_t;
     if ((e = cudaGetLastError()) != cudaSuccess ||
         (e = set_smem_limit(ctx, (const void*)tile_lists_kernel, (int)lists_smem)) != cudaSuccess)
