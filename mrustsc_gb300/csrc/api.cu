@@ -875,6 +875,7 @@ void scrust_cuda_context_destroy(scrust_context* ctx) {
         cudaFree(b.indices);
         cudaFree(b.values);
     }
+    for (auto& b : ctx->cluster_blocks) cudaFree(b.first);
     for (int i = 0; i < PH_COUNT; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     for (int i = 0; i < kCsrRanges; i++)

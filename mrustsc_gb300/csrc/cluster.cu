@@ -19,10 +19,12 @@
 //     (cluster.rs:425-455).  A node alone in its community joins another
 //     lone node's community only when that id is smaller, so two lone
 //     nodes never swap.  Rounds continue until two in a row move nothing.
-//   - A block of 32 threads per node sums the node's edge weight per
-//     neighbouring community in a shared-memory table, 32 neighbours at a
-//     time, each community's partial in lane order, so every sum is formed
-//     in one fixed order.
+//   - A node's edge weight per neighbouring community is summed in a
+//     shared-memory table.  Where every sum of a level's weights is exact in
+//     f64 (their lowest set bit against the largest row sum), the weights are
+//     taken as integers and added in any order; else a warp per node adds
+//     them 32 neighbours at a time, each community's partial in lane order,
+//     so every sum is formed in one fixed order.  Both give the same bits.
 //   - Community strengths are fixed-point (int64, scale 2^s with
 //     2m * 2^s <= 2^61) and change by integer atomics, whose result does not
 //     depend on their order.
@@ -34,7 +36,7 @@
 //     lone node may move in that round.  Cuts are recomputed each round.
 //   - Aggregation: entries keyed by (community, community) with two stable
 //     radix sorts and per-key sums in sorted order.
-// Nodes whose neighbours span more than 4096 communities do not move (the
+// Nodes whose neighbours span more than 2048 communities do not move (the
 // table's limit); on kNN graphs no node comes near it.
 #include <math.h>
 #include <string.h>
@@ -131,22 +133,59 @@ __global__ void cl_strength_kernel(const uint32_t* __restrict__ ptr, const doubl
     k[v] = s;
 }
 
-// Sum of `count` doubles in index order by one block, into out[0].
-__global__ void cl_sum_kernel(const double* __restrict__ x, int64_t count, double* __restrict__ out) {
+// Sum of `count` doubles: blocks of 256 by a tree each, then the blocks'
+// totals in order (one block doing both took 300 us for 60,000).
+__global__ void cl_sum_blocks_kernel(const double* __restrict__ x, int64_t count, double* __restrict__ totals) {
     __shared__ double part[256];
-    double total = 0.0;
-    for (int64_t base = 0; base < count; base += 256) {
-        const int64_t i = base + threadIdx.x;
-        part[threadIdx.x] = i < count ? x[i] : 0.0;
-        __syncthreads();
-        for (int o = 128; o > 0; o >>= 1) {
-            if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) total += part[0];
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    part[threadIdx.x] = i < count ? x[i] : 0.0;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[0] = total;
+    if (threadIdx.x == 0) totals[blockIdx.x] = part[0];
+}
+__global__ void cl_sum_totals_kernel(const double* __restrict__ totals, int64_t blocks, double* __restrict__ out) {
+    double total = 0.0;
+#pragma unroll 8
+    for (int64_t b = 0; b < blocks; ++b) total += totals[b];
+    out[0] = total;
+}
+
+// The lowest set bit of any positive weight as an exponent (min into
+// exps[0]) and the exponent above the largest strength (max into exps[1]).
+__global__ void cl_exponents_kernel(const double* __restrict__ w, int64_t m, const double* __restrict__ k, int64_t n,
+                                    int* __restrict__ exps) {
+    int low = 2000, high = -2000;
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = t0; i < m; i += step) {
+        const unsigned long long u = (unsigned long long)__double_as_longlong(w[i]) & 0x7fffffffffffffffull;
+        if (!u) continue;
+        const int e = (int)(u >> 52);
+        const unsigned long long mant = (u & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+        low = min(low, (e ? e : 1) - 1075 + __ffsll((long long)mant) - 1);
+    }
+    for (int64_t i = t0; i < n; i += step) {
+        const unsigned long long u = (unsigned long long)__double_as_longlong(k[i]) & 0x7fffffffffffffffull;
+        if (u) high = max(high, (int)(u >> 52) - 1022);
+    }
+    low = __reduce_min_sync(0xffffffffu, low);
+    high = __reduce_max_sync(0xffffffffu, high);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(exps, low);
+        atomicMax(exps + 1, high);
+    }
+}
+
+// Weights as integers: w[i] 2^shift, exact (and below 2^53); and those in f32.
+__global__ void cl_integers_kernel(const double* __restrict__ w, int64_t m, double scale, long long* __restrict__ out,
+                                   float* __restrict__ flt) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const double x = w[i] * scale;  // scale: a power of two
+    out[i] = (long long)x;
+    flt[i] = (float)x;
 }
 
 __global__ void cl_fix_kernel(const double* __restrict__ x, int64_t count, double scale, long long* __restrict__ fx) {
@@ -161,6 +200,11 @@ __global__ void cl_iota_kernel(int64_t n, uint32_t* __restrict__ out) {
     if (v < n) out[v] = (uint32_t)v;
 }
 
+__global__ void cl_ones_kernel(int64_t n, int* __restrict__ out) {
+    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < n) out[v] = 1;
+}
+
 __global__ void cl_comm_init_kernel(const uint32_t* __restrict__ labels, const long long* __restrict__ kfix, int64_t n,
                                     long long* __restrict__ K, int* __restrict__ size) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -169,24 +213,62 @@ __global__ void cl_comm_init_kernel(const uint32_t* __restrict__ labels, const l
     atomicAdd(size + labels[v], 1);
 }
 
+// Sum over the lanes in `peers`, at its lowest lane, in lane order (wbuf: 32
+// values of the warp's own), or for integers in any order, in log2 of the
+// largest group's size steps: each lane adds the next lane left in its group,
+// then every second lane leaves.  For all lanes of a warp.
+__device__ __forceinline__ double peer_sum(uint32_t peers, bool lead, double x, double* wbuf) {
+    wbuf[threadIdx.x & 31] = x;
+    __syncwarp();
+    double s = 0.0;
+    if (lead)
+        for (uint32_t b = peers; b; b &= b - 1) s += wbuf[__ffs(b) - 1];
+    __syncwarp();
+    return s;
+}
+template <class V>
+__device__ __forceinline__ V peer_tree(uint32_t peers, V x) {
+    const int lane = threadIdx.x & 31;
+    uint32_t above = peers & (0xfffffffeu << lane);
+    int rank = __popc(peers & ((1u << lane) - 1u));
+    while (__any_sync(0xffffffffu, above != 0u)) {
+        const int next = __ffs(above);
+        const V t = __shfl_sync(0xffffffffu, x, next ? next - 1 : lane);
+        if (next) x += t;
+        above &= ~__ballot_sync(0xffffffffu, rank & 1);
+        rank >>= 1;
+    }
+    return x;
+}
+__device__ __forceinline__ long long peer_sum(uint32_t peers, bool, long long x, long long*) {
+    return peer_tree(peers, x);
+}
+
 // The per-node table of edge weight to each neighbouring community (or
 // subcommunity), one warp per node: neighbours in chunks of 32; in a chunk
 // each community's partial is summed by its lowest lane in lane order, then
-// added to the table, so each entry is summed in one fixed order.  With
-// `group_of`, only neighbours in the node's own group count.  Returns false
-// when the table overflowed.
-template <int T>
-__device__ bool gather_table(const uint32_t* __restrict__ nb, const double* __restrict__ w, uint32_t p0, uint32_t p1,
-                             uint32_t self, const uint32_t* __restrict__ label, const uint32_t* __restrict__ group_of,
-                             uint32_t group, uint32_t* keys, double* vals, double* wbuf, int* overflow) {
+// added to the table, so each entry is summed in one fixed order.  V: double,
+// or long long for weights as integers.  With `group_of`, only neighbours in
+// the node's own group count.  slots receives the table's occupied places;
+// returns their count, or -1 when the table overflowed.  (The callers look at
+// the occupied places alone: testing all T, 32 at a time, cost a node up to 64
+// rounds of f64 divisions, 64 clocks an instruction.)
+template <int T, class V>
+__device__ int gather_table(const uint32_t* __restrict__ nb, const V* __restrict__ w, uint32_t p0, uint32_t p1,
+                            uint32_t self, const uint32_t* __restrict__ label, const uint32_t* __restrict__ group_of,
+                            uint32_t group, uint32_t* keys, V* vals, V* wbuf, uint16_t* slots, int* count,
+                            int* overflow) {
     const int lane = threadIdx.x & 31;
     for (int t = lane; t < T; t += 32) keys[t] = kEmpty;
-    if (lane == 0) *overflow = 0;
+    if (lane == 0) {
+        *overflow = 0;
+        *count = 0;
+    }
     __syncwarp();
     for (uint32_t base = p0; base < p1; base += 32) {
         const uint32_t p = base + lane;
         uint32_t c = kEmpty;
-        double wt = 0.0;
+        V wt = 0;
         if (p < p1) {
             const uint32_t u = nb[p];
             if (u != self && (!group_of || group_of[u] == group)) {
@@ -194,18 +276,19 @@ __device__ bool gather_table(const uint32_t* __restrict__ nb, const double* __re
                 wt = w[p];
             }
         }
-        wbuf[lane] = wt;
-        __syncwarp();
         const uint32_t peers = __match_any_sync(0xffffffffu, c);
-        if (c != kEmpty && (__ffs(peers) - 1) == lane) {
-            double s = 0.0;
-            for (uint32_t b = peers; b; b &= b - 1) s += wbuf[__ffs(b) - 1];
+        const bool lead = c != kEmpty && (__ffs(peers) - 1) == lane;
+        const V s = peer_sum(c == kEmpty ? 0u : peers, lead, wt, wbuf);
+        if (lead) {
             uint32_t slot = (uint32_t)(mix64(c) & (T - 1));
             bool placed = false;
             for (int probe = 0; probe < T; ++probe) {
                 const uint32_t prev = atomicCAS(keys + slot, kEmpty, c);
                 if (prev == kEmpty || prev == c) {
-                    if (prev == kEmpty) vals[slot] = 0.0;
+                    if (prev == kEmpty) {
+                        vals[slot] = 0;
+                        slots[atomicAdd(count, 1)] = (uint16_t)slot;
+                    }
                     vals[slot] += s;
                     placed = true;
                     break;
@@ -216,53 +299,446 @@ __device__ bool gather_table(const uint32_t* __restrict__ nb, const double* __re
         }
         __syncwarp();
     }
-    return *overflow == 0;
+    return *overflow ? -1 : *count;
 }
 
-// Local moving, one round, one warp per node: the nodes of this round's half
-// each take the neighbouring community of largest gain (ties to the smaller
-// id) when it beats staying (cluster.rs:420-455).  A node whose best gain,
-// staying included, is negative goes alone to its reserved id n + v, when
-// that community is empty.  Community ids are below 2n.
+// An f64 as an unsigned integer of the same order (both zeros alike, no NaN).
+__device__ __forceinline__ unsigned long long order_key(double x) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x + 0.0);
+    return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double key_order(unsigned long long k) {
+    return __longlong_as_double((long long)((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
+}
+
+// What a move decision reads besides the node's own table.
+struct MoveArgs {
+    const uint32_t* ptr;
+    const uint32_t* nb;
+    const long long* wint;   // weights as integers, w 2^wshift
+    const float* wflt;       // the same in f32
+    const double* w;
+    const long long* kfix;
+    const uint32_t* comm;
+    const long long* K;
+    const int* size;
+    int64_t n_level;
+    double unit;             // 2^-wshift
+    float gain_unit;         // res inv_scale^2 / total / unit 2^31, or a NaN when that has no safe f32
+    double inv_scale, res, total;
+    uint32_t* moved;         // the round's moves: node and community
+    uint32_t* to;
+    unsigned int* moves;
+};
+
+// The node's end of a round (cluster.rs:420-455): the neighbouring community
+// of largest gain when it beats staying; a node whose best gain, staying
+// included, is negative goes alone to its reserved id n + v, when that
+// community is empty.
+__device__ __forceinline__ uint32_t destination(const MoveArgs& a, uint32_t v, uint32_t own, double best,
+                                                uint32_t best_c, double stay) {
+    uint32_t to = own;
+    if (best_c != kEmpty && best > stay) to = best_c;
+    const double top = to == own ? stay : best;
+    const uint32_t fresh = (uint32_t)(a.n_level + v);
+    if (top < 0.0 && own != fresh && a.size[fresh] == 0) to = fresh;
+    return to;
+}
+__device__ __forceinline__ void record_move(const MoveArgs& a, uint32_t v, uint32_t own, uint32_t to) {
+    if (to == own) return;
+    const unsigned int i = atomicAdd(a.moves, 1u);
+    a.moved[i] = v;
+    a.to[i] = to;
+}
+
+// Gain of community strength k for a node of strength kv and weight e to it.
+__device__ __forceinline__ double move_gain(const MoveArgs& a, double e, long long k, double kv) {
+    return e - a.res * ((double)k * a.inv_scale) * kv / a.total;
+}
+
+// A non-negative integer in f32 by its halves, within 2 roundings of 2^-24 (the
+// conversion instruction for 64 bits is an f64-rate one: 64 clocks a warp).
+__device__ __forceinline__ float to_f32(long long x) {
+    return fmaf((float)(uint32_t)((unsigned long long)x >> 32), 4294967296.0f, (float)(uint32_t)x);
+}
+// The same gain in f32, in units of the integer weights, as bounds: e the
+// node's weight to the community, f its strength times gain_unit.  At most 9
+// roundings of 2^-24 on either product or their difference (the weight summed
+// in f32 in up to five steps, too), within 2^-20 of their sum; the constant
+// covers what underflows (k f below 2^62 2^-126).  A NaN bounds nothing.
+__device__ __forceinline__ void gain_bounds(float e, long long k, float f, float* low, float* high) {
+    const float q = to_f32(k) * f;
+    const float g = e - q, err = (e + fabsf(q)) * 9.5367431640625e-7f + 1e-18f;
+    *low = g - err;
+    *high = g + err;
+}
+__device__ __forceinline__ float gain_factor(const MoveArgs& a, long long kfix) {
+    return (to_f32(kfix) * 4.656612873077393e-10f) * a.gain_unit;
+}
+// f32 as an unsigned integer of the same order (no NaN); 0 stands for none and
+// reads back as a NaN, below which nothing is.
+__device__ __forceinline__ uint32_t order_key(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return (u >> 31) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float key_order(uint32_t k) { return __uint_as_float((k >> 31) ? (k & 0x7fffffffu) : ~k); }
+
+// Where a node of community `own` goes by the bounds of its gains, one warp:
+// each lane holds up to E neighbouring communities c (kEmpty: none) with the
+// node's weight s to them and their strength k; e_own is its weight to its own
+// and k_own that one's strength without it.  One community above all others
+// and above zero decides; kEmpty when the bounds leave it open.
+template <int E>
+__device__ __forceinline__ uint32_t bounded_move(uint32_t own, float f, const uint32_t (&c)[E], const float (&s)[E],
+                                                 const long long (&k)[E], float e_own, long long k_own) {
+    float own_low, own_high, high[E];
+    gain_bounds(e_own, k_own, f, &own_low, &own_high);
+    uint32_t key = own_low == own_low ? order_key(own_low) : 0u;
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+        float low;
+        gain_bounds(s[i], k[i], f, &low, &high[i]);
+        if (c[i] != kEmpty && low == low) key = max(key, order_key(low));
+    }
+    key = __reduce_max_sync(0xffffffffu, key);
+    const float least = key_order(key);
+    const bool stays = !(own_high < least);
+    int cands = stays ? 1 : 0;
+    uint32_t to = own;
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+        const uint32_t who = __ballot_sync(0xffffffffu, c[i] != kEmpty && !(high[i] < least));
+        cands += __popc(who);
+        if (who) to = __shfl_sync(0xffffffffu, c[i], __ffs(who) - 1);
+    }
+    return cands == 1 && least > 0.0f ? to : kEmpty;
+}
+
+// The same by the f64 gains (some 25 instructions of 64 clocks each), from the
+// warp's table of `found` places: the largest wins, ties to the smaller id.
+template <int T>
+__device__ uint32_t exact_move(const MoveArgs& a, uint32_t v, uint32_t own, bool alone, long long kf, long long k_own,
+                               const uint32_t* keys, const long long* vals, const uint16_t* slots, int found) {
+    const int lane = threadIdx.x & 31;
+    const double kv = (double)kf * a.inv_scale;
+    double best = -INFINITY;
+    long long e_own = 0;
+    uint32_t best_c = kEmpty;
+    for (int i0 = 0; i0 < found; i0 += 32) {
+        uint32_t c = kEmpty;
+        long long e = 0;
+        if (i0 + lane < found) {
+            c = keys[slots[i0 + lane]];
+            e = vals[slots[i0 + lane]];
+        }
+        const uint32_t home = __ballot_sync(0xffffffffu, c == own);
+        if (home) e_own = __shfl_sync(0xffffffffu, e, __ffs(home) - 1);
+        // Lone nodes only join smaller lone ids.
+        if (c == kEmpty || c == own || (alone && c > own && a.size[c] == 1)) continue;
+        const double g = move_gain(a, (double)e * a.unit, a.K[c], kv);
+        if (g > best || (g == best && c < best_c)) {
+            best = g;
+            best_c = c;
+        }
+    }
+    __syncwarp();
+    for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const uint32_t oc = __shfl_xor_sync(0xffffffffu, best_c, o);
+        if (ob > best || (ob == best && oc < best_c)) {
+            best = ob;
+            best_c = oc;
+        }
+    }
+    return destination(a, v, own, best, best_c, move_gain(a, (double)e_own * a.unit, k_own, kv));
+}
+
+// Local moving, one round, exact integer weights, nodes of at most
+// kSmallDegree entries, kMoveNodes nodes a warp: a node's weights are summed
+// per community in registers where its entries are one chunk of 32, else by
+// the warp's table.  Bound by the latency of node -> neighbours -> labels ->
+// strengths, so the warp's nodes are in flight together, and before by f64
+// units, so sums and gains are bounded in f32 first.  A late round of 60,000
+// nodes of 46 entries (23 merged): 112 us (a warp per node, f64 gains at 128
+// places), 32 us (f64 gains, one thread per occupied place of a block), 22 us
+// (bounds in f32, places of a block), 17 us (four nodes a warp), 16 us here.
+constexpr int kMoveWarps = 4;
+constexpr int kMoveNodes = 2;
+__global__ void __launch_bounds__(32 * kMoveWarps) cl_move_small_kernel(MoveArgs a, const uint32_t* __restrict__ nodes,
+                                                                        int64_t count) {
+    constexpr int T = kSmallTable, P = kMoveNodes;
+    __shared__ uint32_t keys[kMoveWarps][T];
+    __shared__ long long vals[kMoveWarps][T];
+    __shared__ uint16_t slots[kMoveWarps][T];
+    __shared__ int tab_count[kMoveWarps], tab_over[kMoveWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t i0 = ((int64_t)blockIdx.x * kMoveWarps + warp) * P;
+    if (i0 >= count) return;
+    const int here = (int)min((int64_t)P, count - i0);
+    // Lane j holds node j.
+    uint32_t my_v = 0, my_own = 0, my_p0 = 0, my_deg = 0;
+    long long my_kf = 0, my_kown = 0;
+    bool my_alone = false;
+    if (lane < here) {
+        my_v = nodes[i0 + lane];
+        my_own = a.comm[my_v];
+        my_p0 = a.ptr[my_v];
+        my_deg = a.ptr[my_v + 1] - my_p0;
+        my_kf = a.kfix[my_v];
+        my_kown = a.K[my_own] - my_kf;
+        my_alone = a.size[my_own] == 1;
+    }
+    const float my_f = gain_factor(a, my_kf);
+    uint32_t my_to = lane < here ? kEmpty : my_own;
+    uint32_t c[P];
+    float s[P], e_own[P];
+    long long k[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const uint32_t v = __shfl_sync(0xffffffffu, my_v, j), p = __shfl_sync(0xffffffffu, my_p0, j) + lane;
+        const uint32_t deg = __shfl_sync(0xffffffffu, my_deg, j);
+        c[j] = kEmpty;
+        s[j] = 0.0f;
+        if (deg <= 32u && (uint32_t)lane < deg) {
+            const uint32_t u = a.nb[p];
+            s[j] = a.wflt[p];
+            if (u != v) c[j] = u;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < P; ++j)
+        if (c[j] != kEmpty) c[j] = a.comm[c[j]];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const uint32_t own = __shfl_sync(0xffffffffu, my_own, j);
+        const bool alone = __shfl_sync(0xffffffffu, my_alone, j);
+        const uint32_t peers = __match_any_sync(0xffffffffu, c[j]);
+        s[j] = peer_tree(c[j] == kEmpty ? 0u : peers, s[j]);
+        if ((__ffs(peers) - 1) != lane) c[j] = kEmpty;
+        const uint32_t home = __ballot_sync(0xffffffffu, c[j] == own);
+        e_own[j] = __shfl_sync(0xffffffffu, s[j], home ? __ffs(home) - 1 : 0);
+        if (!home) e_own[j] = 0.0f;
+        if (c[j] == own) c[j] = kEmpty;
+        // Lone nodes only join smaller lone ids.
+        if (alone && c[j] != kEmpty && c[j] > own && a.size[c[j]] == 1) c[j] = kEmpty;
+        k[j] = c[j] != kEmpty ? a.K[c[j]] : 0ll;
+    }
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const uint32_t c1[1] = {c[j]};
+        const float s1[1] = {s[j]};
+        const long long k1[1] = {k[j]};
+        const uint32_t to = bounded_move<1>(__shfl_sync(0xffffffffu, my_own, j), __shfl_sync(0xffffffffu, my_f, j), c1,
+                                            s1, k1, e_own[j], __shfl_sync(0xffffffffu, my_kown, j));
+        if (lane == j && j < here && my_deg <= 32u) my_to = to;
+    }
+    // Nodes of more than one chunk, and those that the bounds leave open.  (At
+    // most kSmallDegree communities: the table never overflows.)
+    for (uint32_t rest = __ballot_sync(0xffffffffu, my_to == kEmpty); rest; rest &= rest - 1) {
+        const int j = __ffs(rest) - 1;
+        const uint32_t v = __shfl_sync(0xffffffffu, my_v, j), own = __shfl_sync(0xffffffffu, my_own, j);
+        const uint32_t p0 = __shfl_sync(0xffffffffu, my_p0, j), deg = __shfl_sync(0xffffffffu, my_deg, j);
+        const bool alone = __shfl_sync(0xffffffffu, my_alone, j);
+        const int found = gather_table<T>(a.nb, a.wint, p0, p0 + deg, v, a.comm, nullptr, 0u, keys[warp], vals[warp],
+                                          (long long*)nullptr, slots[warp], &tab_count[warp], &tab_over[warp]);
+        const long long k_own = __shfl_sync(0xffffffffu, my_kown, j);
+        uint32_t to = kEmpty;
+        if (deg > 32u) {
+            uint32_t c2[2];
+            float s2[2], e2 = 0.0f;
+            long long k2[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                c2[i] = kEmpty;
+                s2[i] = 0.0f;
+                k2[i] = 0;
+                if (lane + 32 * i < found) {
+                    const int t = slots[warp][lane + 32 * i];
+                    c2[i] = keys[warp][t];
+                    s2[i] = to_f32(vals[warp][t]);
+                }
+                const uint32_t home = __ballot_sync(0xffffffffu, c2[i] == own);
+                if (home) e2 = __shfl_sync(0xffffffffu, s2[i], __ffs(home) - 1);
+                if (c2[i] == own || (alone && c2[i] != kEmpty && c2[i] > own && a.size[c2[i]] == 1)) c2[i] = kEmpty;
+                if (c2[i] != kEmpty) k2[i] = a.K[c2[i]];
+            }
+            to = bounded_move<2>(own, __shfl_sync(0xffffffffu, my_f, j), c2, s2, k2, e2, k_own);
+        }
+        if (to == kEmpty)
+            to = exact_move<T>(a, v, own, alone, __shfl_sync(0xffffffffu, my_kf, j), k_own, keys[warp], vals[warp],
+                               slots[warp], found);
+        if (lane == j) my_to = to;
+        __syncwarp();
+    }
+    const uint32_t movers = __ballot_sync(0xffffffffu, my_to != my_own);
+    if (!movers) return;
+    unsigned int at = 0;
+    if (lane == 0) at = atomicAdd(a.moves, (unsigned int)__popc(movers));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(movers & ((1u << lane) - 1u));
+    if (my_to != my_own) {
+        a.moved[at] = my_v;
+        a.to[at] = my_to;
+    }
+}
+
+// The same for nodes of more entries, a block per node: the warps add their
+// chunks to one table by atomics, of twice the node's entries up to kBigTable
+// places (a warp per node, clearing and testing 2,048 places: 59 us a round).
+__global__ void __launch_bounds__(32 * kMoveWarps) cl_move_big_kernel(MoveArgs a, const uint32_t* __restrict__ nodes) {
+    constexpr int T = kBigTable, N = 32 * kMoveWarps;
+    __shared__ uint32_t keys[T];
+    __shared__ unsigned long long vals[T];
+    __shared__ float high[T];
+    __shared__ uint16_t slots[T], cand[T];
+    __shared__ int found_s, over_s, cand_s;
+    __shared__ uint32_t low;
+    __shared__ unsigned long long best, own_val;
+    __shared__ uint32_t best_c;
+    __shared__ double stay;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t v = nodes[blockIdx.x];
+    const uint32_t own = a.comm[v];
+    const uint32_t p0 = a.ptr[v], p1 = a.ptr[v + 1];
+    const long long kf = a.kfix[v];
+    const float factor = gain_factor(a, kf);
+    uint32_t mask = T - 1;
+    while (mask >= 255u && (mask >> 1) >= 2u * (p1 - p0)) mask >>= 1;
+    for (uint32_t t = tid; t <= mask; t += N) {
+        keys[t] = kEmpty;
+        vals[t] = 0ull;
+    }
+    if (tid == 0) {
+        found_s = 0;
+        over_s = 0;
+        cand_s = 0;
+        low = 0u;
+        best = 0ull;
+        own_val = 0ull;
+        best_c = kEmpty;
+        stay = -INFINITY;
+    }
+    __syncthreads();
+    for (uint32_t base = p0 + (uint32_t)(tid - lane); base < p1; base += N) {
+        const uint32_t p = base + lane;
+        uint32_t c = kEmpty;
+        long long wt = 0;
+        if (p < p1) {
+            const uint32_t u = a.nb[p];
+            if (u != v) {
+                c = a.comm[u];
+                wt = a.wint[p];
+            }
+        }
+        const uint32_t peers = __match_any_sync(0xffffffffu, c);
+        const long long s = peer_sum(c == kEmpty ? 0u : peers, false, wt, nullptr);
+        if (c != kEmpty && (__ffs(peers) - 1) == lane) {
+            uint32_t slot = (uint32_t)mix64(c) & mask;
+            bool placed = false;
+            for (uint32_t probe = 0; probe <= mask; ++probe) {
+                const uint32_t prev = atomicCAS(keys + slot, kEmpty, c);
+                if (prev == kEmpty || prev == c) {
+                    if (prev == kEmpty) slots[atomicAdd(&found_s, 1)] = (uint16_t)slot;
+                    atomicAdd(&vals[slot], (unsigned long long)s);
+                    placed = true;
+                    break;
+                }
+                slot = (slot + 1) & mask;
+            }
+            if (!placed) over_s = 1;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (over_s) return;
+    const int found = found_s;
+    const bool alone = a.size[own] == 1;
+    for (int i = tid; i < found; i += N) {
+        const int s = slots[i];
+        const uint32_t c = keys[s];
+        high[s] = -INFINITY;
+        if (c == own) {
+            own_val = vals[s];
+            keys[s] = kEmpty;
+        } else if (alone && c > own && a.size[c] == 1) {
+            keys[s] = kEmpty;
+        } else {
+            float lo;
+            gain_bounds(to_f32((long long)vals[s]), a.K[c], factor, &lo, &high[s]);
+            if (lo == lo) atomicMax(&low, order_key(lo));
+        }
+    }
+    __syncthreads();
+    // The node's own community, adjacent or not.
+    const long long k_own = a.K[own] - kf;
+    float own_low, own_high;
+    gain_bounds(to_f32((long long)own_val), k_own, factor, &own_low, &own_high);
+    if (tid == 0 && own_low == own_low) atomicMax(&low, order_key(own_low));
+    __syncthreads();
+    const float least = key_order(low);
+    for (int i = tid; i < found; i += N) {
+        const int s = slots[i];
+        if (keys[s] != kEmpty && !(high[s] < least)) cand[atomicAdd(&cand_s, 1)] = (uint16_t)s;
+    }
+    __syncthreads();
+    const int cands = cand_s;
+    const bool stays = !(own_high < least);
+    if (cands + (stays ? 1 : 0) == 1 && least > 0.0f) {
+        if (tid == 0 && !stays) record_move(a, v, own, keys[cand[0]]);
+        return;
+    }
+    const double kv = (double)kf * a.inv_scale;
+    for (int t = tid; t <= cands; t += N) {
+        if (!t && !stays) continue;
+        const int s = t ? cand[t - 1] : 0;
+        const double g = t ? move_gain(a, (double)(long long)vals[s] * a.unit, a.K[keys[s]], kv)
+                           : move_gain(a, (double)(long long)own_val * a.unit, k_own, kv);
+        if (!t) {
+            stay = g;
+        } else if (g == g) {
+            vals[s] = order_key(g);
+            atomicMax(&best, vals[s]);
+        } else {
+            keys[s] = kEmpty;
+        }
+    }
+    __syncthreads();
+    for (int t = tid; t < cands; t += N)
+        if (keys[cand[t]] != kEmpty && vals[cand[t]] == best) atomicMin(&best_c, keys[cand[t]]);
+    __syncthreads();
+    if (tid == 0) record_move(a, v, own, destination(a, v, own, key_order(best), best_c, stay));
+}
+
+// Local moving, one round, one warp per node, f64 weights whose sums round:
+// the fixed order of gather_table.
 template <int T, int W>
-__global__ void __launch_bounds__(32 * W) cl_move_kernel(const uint32_t* __restrict__ ptr,
-                                                         const uint32_t* __restrict__ nb,
-                                                         const double* __restrict__ w,
-                                                         const long long* __restrict__ kfix,
-                                                         const uint32_t* __restrict__ nodes, int64_t count,
-                                                         int64_t n_level, const uint32_t* __restrict__ comm,
-                                                         const long long* __restrict__ K,
-                                                         const int* __restrict__ size, double inv_scale, double res,
-                                                         double total, int round, uint64_t salt,
-                                                         uint32_t* __restrict__ next,
-                                                         unsigned int* __restrict__ moves) {
+__global__ void __launch_bounds__(32 * W) cl_move_kernel(MoveArgs a, const uint32_t* __restrict__ nodes, int64_t count) {
     __shared__ uint32_t keys[W][T];
     __shared__ double vals[W][T];
     __shared__ double wbuf[W][32];
-    __shared__ int overflow[W];
+    __shared__ uint16_t slots[W][T];
+    __shared__ int found_s[W], overflow[W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t idx = (int64_t)blockIdx.x * W + warp;
     if (idx >= count) return;
     const uint32_t v = nodes[idx];
-    if (!active_in(v, round, salt)) return;
-    const uint32_t own = comm[v];
-    if (!gather_table<T>(nb, w, ptr[v], ptr[v + 1], v, comm, nullptr, 0, keys[warp], vals[warp], wbuf[warp],
-                         &overflow[warp]))
-        return;
-    const double kv = (double)kfix[v] * inv_scale;
+    const uint32_t own = a.comm[v];
+    const int found = gather_table<T>(a.nb, a.w, a.ptr[v], a.ptr[v + 1], v, a.comm, nullptr, 0u, keys[warp], vals[warp],
+                                      wbuf[warp], slots[warp], &found_s[warp], &overflow[warp]);
+    if (found < 0) return;
+    const double kv = (double)a.kfix[v] * a.inv_scale;
     double e_own = 0.0;
     double best = -INFINITY;
     uint32_t best_c = kEmpty;
-    const bool alone = size[own] == 1;
-    for (int t = lane; t < T; t += 32) {
+    const bool alone = a.size[own] == 1;
+    for (int i = lane; i < found; i += 32) {
+        const int t = slots[warp][i];
         const uint32_t c = keys[warp][t];
-        if (c == kEmpty) continue;
         if (c == own) {
             e_own = vals[warp][t];
             continue;
         }
-        if (alone && size[c] == 1 && c > own) continue;  // lone nodes only join smaller lone ids
-        const double g = vals[warp][t] - res * ((double)K[c] * inv_scale) * kv / total;
+        if (alone && a.size[c] == 1 && c > own) continue;  // lone nodes only join smaller lone ids
+        const double g = move_gain(a, vals[warp][t], a.K[c], kv);
         if (g > best || (g == best && c < best_c)) {
             best = g;
             best_c = c;
@@ -277,30 +753,23 @@ __global__ void __launch_bounds__(32 * W) cl_move_kernel(const uint32_t* __restr
             best_c = oc;
         }
     }
-    if (lane != 0) return;
-    const double stay = e_own - res * ((double)(K[own] - kfix[v]) * inv_scale) * kv / total;
-    uint32_t to = own;
-    if (best_c != kEmpty && best > stay) to = best_c;
-    const double top = to == own ? stay : best;
-    const uint32_t fresh = (uint32_t)(n_level + v);
-    if (top < 0.0 && own != fresh && size[fresh] == 0) to = fresh;
-    if (to != own) {
-        next[v] = to;
-        atomicAdd(moves, 1u);
-    }
+    if (lane == 0)
+        record_move(a, v, own, destination(a, v, own, best, best_c, move_gain(a, e_own, a.K[own] - a.kfix[v], kv)));
 }
 
-__global__ void cl_apply_kernel(int64_t n, const long long* __restrict__ kfix, uint32_t* __restrict__ comm,
-                                const uint32_t* __restrict__ next, long long* __restrict__ K, int* __restrict__ size) {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const uint32_t a = comm[v], b = next[v];
-    if (a == b) return;
-    atomicAdd((unsigned long long*)(K + a), (unsigned long long)(-kfix[v]));
-    atomicAdd((unsigned long long*)(K + b), (unsigned long long)kfix[v]);
-    atomicSub(size + a, 1);
-    atomicAdd(size + b, 1);
-    comm[v] = b;
+// The round's moves applied (each node at most once).
+__global__ void cl_apply_kernel(const unsigned int* __restrict__ count, const uint32_t* __restrict__ moved,
+                                const uint32_t* __restrict__ to, const long long* __restrict__ kfix,
+                                uint32_t* __restrict__ comm, long long* __restrict__ K, int* __restrict__ size) {
+    const unsigned int moves = *count;
+    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < moves; i += gridDim.x * blockDim.x) {
+        const uint32_t v = moved[i], a = comm[v], b = to[i];
+        atomicAdd((unsigned long long*)(K + a), (unsigned long long)(-kfix[v]));
+        atomicAdd((unsigned long long*)(K + b), (unsigned long long)kfix[v]);
+        atomicSub(size + a, 1);
+        atomicAdd(size + b, 1);
+        comm[v] = b;
+    }
 }
 
 // ---- refinement -------------------------------------------------------------
@@ -340,6 +809,30 @@ __global__ void cl_cut_kernel(const uint32_t* __restrict__ ptr, const uint32_t* 
     }
     atomicAdd((unsigned long long*)(cut + s), (unsigned long long)llrint((to_subset[v] - inside) * scale));
 }
+// The same with weights as integers, eight lanes a node (latency of a row's
+// scattered reads: 23 us a round at 60,000 nodes with a thread a node).
+__global__ void cl_cut_int_kernel(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ nb,
+                                  const long long* __restrict__ w, double unit, int64_t n,
+                                  const uint32_t* __restrict__ sub, const double* __restrict__ to_subset, double scale,
+                                  long long* __restrict__ cut) {
+    const int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int lane = threadIdx.x & 7;
+    long long inside = 0;
+    uint32_t s = 0;
+    if (v < n) {
+        s = sub[v];
+        const uint32_t p1 = ptr[v + 1];
+#pragma unroll 4
+        for (uint32_t p = ptr[v] + lane; p < p1; p += 8) {
+            const uint32_t u = nb[p];
+            if (u != (uint32_t)v && sub[u] == s) inside += w[p];
+        }
+    }
+    for (int o = 4; o > 0; o >>= 1) inside += __shfl_xor_sync(0xffffffffu, inside, o);
+    if (v < n && lane == 0)
+        atomicAdd((unsigned long long*)(cut + s),
+                  (unsigned long long)llrint((to_subset[v] - (double)inside * unit) * scale));
+}
 
 // Refinement, one round, one warp per node (cluster.rs:560-641): a lone,
 // well-connected node of this round's half merges into a subcommunity of
@@ -349,11 +842,10 @@ __global__ void cl_cut_kernel(const uint32_t* __restrict__ ptr, const uint32_t* 
 // gain / 0.01 + G, G a Gumbel variate from a hash of seed, node,
 // subcommunity and round).  A lone node that may itself move in this round
 // is not a target.
-template <int T, int W>
+template <int T, int W, class V>
 __global__ void __launch_bounds__(32 * W) cl_refine_kernel(const uint32_t* __restrict__ ptr,
-                                                           const uint32_t* __restrict__ nb,
-                                                           const double* __restrict__ w,
-                                                           const long long* __restrict__ kfix,
+                                                           const uint32_t* __restrict__ nb, const V* __restrict__ w,
+                                                           double unit, const long long* __restrict__ kfix,
                                                            const uint32_t* __restrict__ nodes, int64_t count,
                                                            const uint32_t* __restrict__ part,
                                                            const uint32_t* __restrict__ sub,
@@ -363,30 +855,31 @@ __global__ void __launch_bounds__(32 * W) cl_refine_kernel(const uint32_t* __res
                                                            const long long* __restrict__ cut,
                                                            const unsigned char* __restrict__ well, double inv_scale,
                                                            double res, double total, int round, uint64_t salt,
-                                                           uint32_t* __restrict__ next,
+                                                           uint32_t* __restrict__ moved, uint32_t* __restrict__ to,
                                                            unsigned int* __restrict__ moves) {
     __shared__ uint32_t keys[W][T];
-    __shared__ double vals[W][T];
-    __shared__ double wbuf[W][32];
-    __shared__ int overflow[W];
+    __shared__ V vals[W][T];
+    __shared__ V wbuf[W][32];
+    __shared__ uint16_t slots[W][T];
+    __shared__ int found_s[W], overflow[W];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t idx = (int64_t)blockIdx.x * W + warp;
     if (idx >= count) return;
     const uint32_t v = nodes[idx];
-    if (sub[v] != v || subsize[v] != 1 || !well[v] || !active_in(v, round, salt)) return;
+    if (sub[v] != v || subsize[v] != 1 || !well[v]) return;
     const uint32_t c = part[v];
-    if (!gather_table<T>(nb, w, ptr[v], ptr[v + 1], v, sub, part, c, keys[warp], vals[warp], wbuf[warp],
-                         &overflow[warp]))
-        return;
+    const int found = gather_table<T>(nb, w, ptr[v], ptr[v + 1], v, sub, part, c, keys[warp], vals[warp], wbuf[warp],
+                                      slots[warp], &found_s[warp], &overflow[warp]);
+    if (found < 0) return;
     const double kv = (double)kfix[v] * inv_scale;
     const double kc = (double)K[c] * inv_scale;
     double best = -INFINITY;
     uint32_t best_s = kEmpty;
-    for (int t = lane; t < T; t += 32) {
+    for (int i = lane; i < found; i += 32) {
+        const int t = slots[warp][i];
         const uint32_t s = keys[warp][t];
-        if (s == kEmpty) continue;
         const double ks = (double)Ksub[s] * inv_scale;
-        const double gain = vals[warp][t] - res * ks * kv / total;
+        const double gain = (double)vals[warp][t] * unit - res * ks * kv / total;
         const bool frozen = !(subsize[s] == 1 && well[s] && active_in(s, round, salt));
         if (!(gain >= 0.0 && frozen && (double)cut[s] * inv_scale >= res * ks * (kc - ks) / total)) continue;
         const uint64_t h = mix64(salt ^ mix64(((uint64_t)v << 32 | s) ^ mix64((uint64_t)round + 0x51ed27ull)));
@@ -406,8 +899,9 @@ __global__ void __launch_bounds__(32 * W) cl_refine_kernel(const uint32_t* __res
         }
     }
     if (lane == 0 && best_s != kEmpty) {
-        next[v] = best_s;
-        atomicAdd(moves, 1u);
+        const unsigned int i = atomicAdd(moves, 1u);
+        moved[i] = v;
+        to[i] = best_s;
     }
 }
 
@@ -536,14 +1030,24 @@ __global__ void cl_rank_kernel(const unsigned long long* __restrict__ order, int
     if (i < nc) rank[order[i] & 0xffffffffull] = (uint32_t)i;
 }
 
-__global__ void cl_small_big_kernel(const uint32_t* __restrict__ ptr, int64_t n, uint32_t* __restrict__ small,
-                                    uint32_t* __restrict__ big, unsigned int* __restrict__ counts) {
+// The nodes by degree and by the half of the rounds they are active in
+// (active_in): small nodes of even and odd rounds from the two ends of
+// `small`, the rest from the two ends of `big`.
+__global__ void cl_node_lists_kernel(const uint32_t* __restrict__ ptr, int64_t n, uint64_t salt,
+                                     uint32_t* __restrict__ small, uint32_t* __restrict__ big,
+                                     unsigned int* __restrict__ counts) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    if (ptr[v + 1] - ptr[v] <= (uint32_t)kSmallDegree)
-        small[atomicAdd(counts, 1u)] = (uint32_t)v;
-    else
-        big[atomicAdd(counts + 1, 1u)] = (uint32_t)v;
+    const int lane = threadIdx.x & 31;
+    const int kind = v >= n ? 4
+                            : (ptr[v + 1] - ptr[v] <= (uint32_t)kSmallDegree ? 0 : 2) +
+                                  (active_in((uint32_t)v, 0, salt) ? 0 : 1);
+    const uint32_t peers = __match_any_sync(0xffffffffu, kind);
+    unsigned int at = 0;
+    if (kind < 4 && (__ffs(peers) - 1) == lane) at = atomicAdd(counts + kind, (unsigned int)__popc(peers));
+    at = __shfl_sync(0xffffffffu, at, __ffs(peers) - 1) + __popc(peers & ((1u << lane) - 1u));
+    if (kind >= 4) return;
+    uint32_t* list = kind < 2 ? small : big;
+    list[(kind & 1) ? n - 1 - (int64_t)at : (int64_t)at] = (uint32_t)v;
 }
 
 __global__ void cl_scatter_kernel(const uint32_t* __restrict__ collapse, const uint32_t* __restrict__ partition,
@@ -561,6 +1065,14 @@ struct Level {
     double* w = nullptr;
     double* k = nullptr;
     long long* kfix = nullptr;
+    // The graph that moves read: where every sum over a row is exact, entries
+    // of one neighbour merged and weights as integers (w 2^shift); else the
+    // graph itself and wint null.
+    const uint32_t* mptr = nullptr;
+    const uint32_t* mnb = nullptr;
+    long long* wint = nullptr;
+    float* wflt = nullptr;
+    int shift = 0;
 };
 
 unsigned grid_for(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 255) / 256); }
@@ -568,24 +1080,49 @@ unsigned grid_for(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 255) /
 }  // namespace
 
 // The whole algorithm on device buffers, under the context lock.  Buffers
-// are allocated per call and released when the object goes.
+// are cut from blocks of 32 MB or more, of which the context keeps at most
+// kKeepBytes from call to call (some hundred cudaMalloc and cudaFree pairs
+// took milliseconds).
 class Clusterer {
+    static constexpr size_t kKeepBytes = (size_t)1 << 30;
+
 public:
     Clusterer(scrust_context* ctx, scrust_status* st) : ctx_(ctx), st_(st), s_(ctx->stream) {}
     ~Clusterer() {
         cudaStreamSynchronize(s_);
-        for (void* p : owned_) cudaFree(p);
+        auto& blocks = ctx_->cluster_blocks;
+        size_t total = 0;
+        for (auto& b : blocks) total += b.second;
+        if (blocks.size() < 2 && total <= kKeepBytes) return;
+        // One block of the same size serves the next call without gaps.
+        for (auto& b : blocks) cudaFree(b.first);
+        blocks.clear();
+        void* p = nullptr;
+        if (total <= kKeepBytes && cudaMalloc(&p, total) == cudaSuccess) blocks.emplace_back(p, total);
+        cudaGetLastError();
     }
 
     template <class T>
     T* alloc(size_t count) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            ok_ = false;
-            return nullptr;
+        const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+        auto& blocks = ctx_->cluster_blocks;
+        while (block_ < blocks.size() && used_ + bytes > blocks[block_].second) {
+            ++block_;
+            used_ = 0;
         }
-        owned_.push_back(p);
+        if (block_ == blocks.size()) {
+            const size_t want = std::max(bytes, (size_t)32 << 20);
+            void* p = nullptr;
+            if (cudaMalloc(&p, want) != cudaSuccess) {
+                cudaGetLastError();
+                ok_ = false;
+                return nullptr;
+            }
+            blocks.emplace_back(p, want);
+            used_ = 0;
+        }
+        void* p = (char*)blocks[block_].first + used_;
+        used_ += bytes;
         return (T*)p;
     }
 
@@ -608,9 +1145,9 @@ private:
     cudaError_t sort_pairs(uint32_t* kA, unsigned long long* vA, uint32_t* kB, unsigned long long* vB, int64_t m,
                            int bits, uint32_t** kout, unsigned long long** vout);
     int64_t compact(const uint32_t* labels, int64_t n, int64_t width, uint32_t* out);
-    int32_t node_lists(const Level& L);
-    int32_t local_moving(const Level& L, uint32_t* comm, long long* K, int* size, double res, uint64_t salt,
-                         bool* moved_any);
+    int32_t node_lists(const Level& L, uint64_t salt);
+    int32_t integer_weights(Level* L, bool merged);
+    int32_t local_moving(const Level& L, uint32_t* comm, long long* K, int* size, double res, bool* moved_any);
     int32_t refine(const Level& L, const uint32_t* part, const long long* K, double res, uint64_t salt,
                    uint32_t* sub);
     int32_t aggregate(const Level& L, const uint32_t* lab, int64_t nc, Level* out);
@@ -622,15 +1159,30 @@ private:
     scrust_status* st_;
     cudaStream_t s_;
     bool ok_ = true;
-    std::vector<void*> owned_;
+    size_t block_ = 0, used_ = 0;  // the next free byte of the context's blocks
     Level g0_;
     double total_ = 0.0, scale_ = 1.0, inv_scale_ = 1.0;
-    unsigned int* counter_ = nullptr;
-    // node lists of the current level: small-degree nodes, then the rest
+    unsigned int* counter_ = nullptr;  // 4 list counts, 2 exponents, the moves of each round, labels changed
+    // Node lists of the current level (cl_node_lists_kernel) and their counts.
     uint32_t* small_ = nullptr;
     uint32_t* big_ = nullptr;
-    int64_t n_small_ = 0, n_big_ = 0;
+    unsigned int counts_[4] = {0, 0, 0, 0};
+    // The list of small (0) or other (1) nodes active in `round`, and its length.
+    const uint32_t* active(const Level& L, int kind, int round, int64_t* count) const {
+        const int odd = round & 1;
+        *count = counts_[2 * kind + odd];
+        const uint32_t* list = kind ? big_ : small_;
+        return odd ? list + (L.n - *count) : list;
+    }
 };
+
+// Rounds enqueued between two looks at their move counts.  Two rounds without
+// a move leave every later one without any (nothing they read has changed), so
+// the rounds past the last do nothing; a look after every round left the GPU
+// idle for as long as a round took.
+constexpr int kRoundBatch = 8;
+constexpr int kCounterMoves = 6;
+static_assert(kMaxRounds % kRoundBatch == 0, "whole batches");
 
 cudaError_t Clusterer::sort_pairs(uint32_t* kA, unsigned long long* vA, uint32_t* kB, unsigned long long* vB,
                                   int64_t m, int bits, uint32_t** kout, unsigned long long** vout) {
@@ -679,7 +1231,8 @@ int32_t Clusterer::build(const uint32_t* indptr, const uint32_t* indices, const 
     g0_.k = alloc<double>(n);
     g0_.kfix = alloc<long long>(n);
     double* tot = alloc<double>(1);
-    counter_ = alloc<unsigned int>(4);
+    double* tots = alloc<double>((size_t)(n / 256 + 1));
+    counter_ = alloc<unsigned int>(kCounterMoves + kMaxRounds + 1);
     if (!ok_) return oom();
     cudaMemsetAsync(bad, 0, sizeof(int), s_);
     cl_check_kernel<<<(unsigned)std::min<int64_t>(1024, nnz / 256 + 1), 256, 0, s_>>>(values, nnz, bad);
@@ -698,8 +1251,9 @@ int32_t Clusterer::build(const uint32_t* indptr, const uint32_t* indices, const 
     cl_starts_kernel<<<grid_for(m + 1), 256, 0, s_>>>(keys, m, n, g0_.ptr);
     cl_sym_fill_kernel<<<grid_for(m), 256, 0, s_>>>(order, m, nnz, erow, indices, values, g0_.nb, g0_.w);
     cl_strength_kernel<<<grid_for(n), 256, 0, s_>>>(g0_.ptr, g0_.w, n, g0_.k);
-    cl_sum_kernel<<<1, 256, 0, s_>>>(g0_.k, n, tot);
-    ctx_->launches += 7;
+    cl_sum_blocks_kernel<<<grid_for(n), 256, 0, s_>>>(g0_.k, n, tots);
+    cl_sum_totals_kernel<<<1, 1, 0, s_>>>(tots, (int64_t)grid_for(n), tot);
+    ctx_->launches += 8;
     if (!download(&total_, tot, 1)) return fail(st_, SCRUST_KERNEL, "clustering: graph");
     if (!(total_ > 0.0))
         return fail(st_, SCRUST_INVALID_PARAMETER, "the graph needs at least one edge of positive weight");
@@ -713,47 +1267,129 @@ int32_t Clusterer::build(const uint32_t* indptr, const uint32_t* indices, const 
     return ok(st_);
 }
 
-int32_t Clusterer::node_lists(const Level& L) {
+int32_t Clusterer::node_lists(const Level& L, uint64_t salt) {
     small_ = alloc<uint32_t>(L.n);
     big_ = alloc<uint32_t>(L.n);
     if (!ok_) return oom();
-    cudaMemsetAsync(counter_, 0, 2 * sizeof(unsigned int), s_);
-    cl_small_big_kernel<<<grid_for(L.n), 256, 0, s_>>>(L.ptr, L.n, small_, big_, counter_);
+    cudaMemsetAsync(counter_, 0, 4 * sizeof(unsigned int), s_);
+    cl_node_lists_kernel<<<grid_for(L.n), 256, 0, s_>>>(L.mptr, L.n, salt, small_, big_, counter_);
     ctx_->launches += 1;
-    unsigned int counts[2] = {0, 0};
-    if (!download(counts, counter_, 2)) return fail(st_, SCRUST_KERNEL, "clustering: node lists");
-    n_small_ = counts[0];
-    n_big_ = counts[1];
+    if (!download(counts_, counter_, 4)) return fail(st_, SCRUST_KERNEL, "clustering: node lists");
     return ok(st_);
 }
 
-int32_t Clusterer::local_moving(const Level& L, uint32_t* comm, long long* K, int* size, double res, uint64_t salt,
-                                bool* moved_any) {
-    uint32_t* next = alloc<uint32_t>(L.n);
+// The level's weights as integers, where every sum over a row is exact: a
+// multiple of their lowest set bit, below 2^53 of it.  Entries of one neighbour
+// are merged then (the symmetric graph holds most edges twice; half the
+// entries make most rows one chunk of 32), unless they already are.
+int32_t Clusterer::integer_weights(Level* L, bool merged) {
+    L->mptr = L->ptr;
+    L->mnb = L->nb;
+    L->wint = nullptr;
+    int exps[2] = {2000, -2000};
+    cudaMemcpyAsync(counter_ + 4, exps, sizeof(exps), cudaMemcpyHostToDevice, s_);
+    cl_exponents_kernel<<<(unsigned)std::min<int64_t>(4 * ctx_->sm_count, grid_for(L->m)), 256, 0, s_>>>(
+        L->w, L->m, L->k, L->n, (int*)(counter_ + 4));
+    ctx_->launches += 1;
+    if (!download(exps, (const int*)(counter_ + 4), 2)) return fail(st_, SCRUST_KERNEL, "clustering: weights");
+    // (|shift| <= 1000 keeps 2^-shift an f64; a strength rounds up to at most
+    // the next power of two.)
+    if (exps[0] >= 2000 || exps[1] + 1 - exps[0] > 53 || exps[0] < -1000 || exps[0] > 900) return ok(st_);
+    Level g = *L;
+    if (!merged) {
+        uint32_t* each = alloc<uint32_t>(L->n);
+        if (!ok_) return oom();
+        cl_iota_kernel<<<grid_for(L->n), 256, 0, s_>>>(L->n, each);
+        ctx_->launches += 1;
+        const int32_t rc = aggregate(*L, each, L->n, &g);
+        if (rc) return rc;
+    }
+    L->shift = -exps[0];
+    L->wint = alloc<long long>(g.m);
+    L->wflt = alloc<float>(g.m);
+    if (!ok_) return oom();
+    L->mptr = g.ptr;
+    L->mnb = g.nb;
+    cl_integers_kernel<<<grid_for(g.m), 256, 0, s_>>>(g.w, g.m, std::ldexp(1.0, L->shift), L->wint, L->wflt);
+    ctx_->launches += 1;
+    return ok(st_);
+}
+
+int32_t Clusterer::local_moving(const Level& L, uint32_t* comm, long long* K, int* size, double res, bool* moved_any) {
+    MoveArgs a;
+    a.ptr = L.mptr;
+    a.nb = L.mnb;
+    a.wint = L.wint;
+    a.wflt = L.wflt;
+    a.w = L.w;
+    a.kfix = L.kfix;
+    a.comm = comm;
+    a.K = K;
+    a.size = size;
+    a.n_level = L.n;
+    a.unit = std::ldexp(1.0, -L.shift);
+    a.inv_scale = inv_scale_;
+    a.res = res;
+    a.total = total_;
+    const double gu = res * inv_scale_ * inv_scale_ / total_ / a.unit * 2147483648.0;
+    a.gain_unit = gu > 1e-28 && gu < 1e28 ? (float)gu : NAN;
+    a.moved = alloc<uint32_t>(L.n);
+    a.to = alloc<uint32_t>(L.n);
+    if (!ok_) return oom();
+    uint32_t* seen = alloc<uint32_t>(L.n);
     if (!ok_) return oom();
     *moved_any = false;
-    int quiet = 0;
-    for (int round = 0; round < kMaxRounds && quiet < 2; ++round) {
-        cudaMemcpyAsync(next, comm, sizeof(uint32_t) * L.n, cudaMemcpyDeviceToDevice, s_);
-        cudaMemsetAsync(counter_ + 2, 0, sizeof(unsigned int), s_);
-        if (n_small_)
-            cl_move_kernel<kSmallTable, kSmallWarps>
-                <<<(unsigned)((n_small_ + kSmallWarps - 1) / kSmallWarps), 32 * kSmallWarps, 0, s_>>>(
-                    L.ptr, L.nb, L.w, L.kfix, small_, n_small_, L.n, comm, K, size, inv_scale_, res, total_, round,
-                    salt, next, counter_ + 2);
-        if (n_big_)
-            cl_move_kernel<kBigTable, 1><<<(unsigned)n_big_, 32, 0, s_>>>(L.ptr, L.nb, L.w, L.kfix, big_, n_big_,
-                                                                          L.n, comm, K, size, inv_scale_, res,
-                                                                          total_, round, salt, next, counter_ + 2);
-        cl_apply_kernel<<<grid_for(L.n), 256, 0, s_>>>(L.n, L.kfix, comm, next, K, size);
-        ctx_->launches += 3;
-        unsigned int moves = 0;
-        if (!download(&moves, counter_ + 2, 1)) return fail(st_, SCRUST_KERNEL, "clustering: local moving");
-        if (moves) {
-            *moved_any = true;
-            quiet = 0;
-        } else {
-            ++quiet;
+    const unsigned apply_blocks = std::min<unsigned>(grid_for(L.n), 2u * (unsigned)ctx_->sm_count);
+    cudaMemsetAsync(counter_ + kCounterMoves, 0, sizeof(unsigned int) * (kMaxRounds + 1), s_);
+    int quiet = 0, end = kMaxRounds, seen_batch = -1;
+    for (int r0 = 0; r0 < end && quiet < 2; r0 += kRoundBatch) {
+        for (int round = r0; round < r0 + kRoundBatch; ++round) {
+            a.moves = counter_ + kCounterMoves + round;
+            int64_t ns = 0, nb = 0;
+            const uint32_t* small = active(L, 0, round, &ns);
+            const uint32_t* big = active(L, 1, round, &nb);
+            if (ns && L.wint)
+                cl_move_small_kernel<<<(unsigned)((ns + kMoveNodes * kMoveWarps - 1) / (kMoveNodes * kMoveWarps)),
+                                       32 * kMoveWarps, 0, s_>>>(a, small, ns);
+            else if (ns)
+                cl_move_kernel<kSmallTable, kSmallWarps>
+                    <<<(unsigned)((ns + kSmallWarps - 1) / kSmallWarps), 32 * kSmallWarps, 0, s_>>>(a, small, ns);
+            if (nb && L.wint)
+                cl_move_big_kernel<<<(unsigned)nb, 32 * kMoveWarps, 0, s_>>>(a, big);
+            else if (nb)
+                cl_move_kernel<kBigTable, 1><<<(unsigned)nb, 32, 0, s_>>>(a, big, nb);
+            cl_apply_kernel<<<apply_blocks, 256, 0, s_>>>(a.moves, a.moved, a.to, L.kfix, comm, K, size);
+            ctx_->launches += 3;
+        }
+        // Rounds read the labels and the round's parity alone (strengths and
+        // sizes follow from the labels, in integers), so labels equal to those
+        // some whole batches ago repeat from there: only what is left over of
+        // the remaining batches after whole repeats has to run.  (On a graph of
+        // 60,000 cells ten nodes that swap for ever kept the first level going
+        // to kMaxRounds, the last 60 rounds of it such a repeat.)
+        // `seen` is taken at batches 1, 2, 4, 8 .. (Brent's rule).
+        const int batch = r0 / kRoundBatch;
+        unsigned int got[kRoundBatch], differ = 1;
+        unsigned int* d_differ = counter_ + kCounterMoves + kMaxRounds;
+        const bool look = end == kMaxRounds && seen_batch >= 0;
+        if (look) {
+            cudaMemsetAsync(d_differ, 0, sizeof(unsigned int), s_);
+            cl_differ_kernel<<<grid_for(L.n), 256, 0, s_>>>(seen, comm, L.n, d_differ);
+            cudaMemcpyAsync(&differ, d_differ, sizeof(differ), cudaMemcpyDeviceToHost, s_);
+            ctx_->launches += 1;
+        }
+        if (!download(got, counter_ + kCounterMoves + r0, kRoundBatch))
+            return fail(st_, SCRUST_KERNEL, "clustering: local moving");
+        for (int i = 0; i < kRoundBatch && quiet < 2; ++i) {
+            if (got[i]) *moved_any = true;
+            quiet = got[i] ? 0 : quiet + 1;
+        }
+        if (look && !differ) {
+            const int left = (kMaxRounds - r0) / kRoundBatch - 1;
+            end = r0 + kRoundBatch * (1 + left % (batch - seen_batch));
+        } else if (batch && !(batch & (batch - 1))) {
+            cudaMemcpyAsync(seen, comm, sizeof(uint32_t) * L.n, cudaMemcpyDeviceToDevice, s_);
+            seen_batch = batch;
         }
     }
     return ok(st_);
@@ -767,39 +1403,59 @@ int32_t Clusterer::refine(const Level& L, const uint32_t* part, const long long*
     long long* Ksub = alloc<long long>(n);
     int* subsize = alloc<int>(n);
     long long* cut = alloc<long long>(n);
-    uint32_t* next = alloc<uint32_t>(n);
+    uint32_t* moved = alloc<uint32_t>(n);
+    uint32_t* to = alloc<uint32_t>(n);
     if (!ok_) return oom();
+    int32_t rc = node_lists(L, salt);
+    if (rc) return rc;
     const unsigned nb = grid_for(n);
     cl_to_subset_kernel<<<nb, 256, 0, s_>>>(L.ptr, L.nb, L.w, L.k, n, part, K, inv_scale_, res, total_, to_subset,
                                            well);
     cl_iota_kernel<<<nb, 256, 0, s_>>>(n, sub);
+    cl_ones_kernel<<<nb, 256, 0, s_>>>(n, subsize);
     cudaMemcpyAsync(Ksub, L.kfix, sizeof(long long) * n, cudaMemcpyDeviceToDevice, s_);
-    ctx_->launches += 2;
-    {
-        std::vector<int> ones((size_t)n, 1);
-        cudaMemcpyAsync(subsize, ones.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s_);
-        cudaStreamSynchronize(s_);
-    }
+    ctx_->launches += 3;
+    const unsigned apply_blocks = std::min<unsigned>(nb, 2u * (unsigned)ctx_->sm_count);
+    const double unit = std::ldexp(1.0, -L.shift);
+    cudaMemsetAsync(counter_ + kCounterMoves, 0, sizeof(unsigned int) * kMaxRounds, s_);
     int quiet = 0;
-    for (int round = 0; round < kMaxRounds && quiet < 2; ++round) {
-        cudaMemsetAsync(cut, 0, sizeof(long long) * n, s_);
-        cl_cut_kernel<<<nb, 256, 0, s_>>>(L.ptr, L.nb, L.w, n, sub, to_subset, scale_, cut);
-        cudaMemcpyAsync(next, sub, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s_);
-        cudaMemsetAsync(counter_ + 2, 0, sizeof(unsigned int), s_);
-        if (n_small_)
-            cl_refine_kernel<kSmallTable, kSmallWarps>
-                <<<(unsigned)((n_small_ + kSmallWarps - 1) / kSmallWarps), 32 * kSmallWarps, 0, s_>>>(
-                    L.ptr, L.nb, L.w, L.kfix, small_, n_small_, part, sub, Ksub, subsize, K, cut, well, inv_scale_,
-                    res, total_, round, salt, next, counter_ + 2);
-        if (n_big_)
-            cl_refine_kernel<kBigTable, 1><<<(unsigned)n_big_, 32, 0, s_>>>(
-                L.ptr, L.nb, L.w, L.kfix, big_, n_big_, part, sub, Ksub, subsize, K, cut, well, inv_scale_, res,
-                total_, round, salt, next, counter_ + 2);
-        cl_apply_kernel<<<nb, 256, 0, s_>>>(n, L.kfix, sub, next, Ksub, subsize);
-        ctx_->launches += 4;
-        unsigned int moves = 0;
-        if (!download(&moves, counter_ + 2, 1)) return fail(st_, SCRUST_KERNEL, "clustering: refinement");
-        quiet = moves ? 0 : quiet + 1;
+    for (int r0 = 0; r0 < kMaxRounds && quiet < 2; r0 += kRoundBatch) {
+        for (int round = r0; round < r0 + kRoundBatch; ++round) {
+            unsigned int* moves = counter_ + kCounterMoves + round;
+            cudaMemsetAsync(cut, 0, sizeof(long long) * n, s_);
+            if (L.wint)
+                cl_cut_int_kernel<<<grid_for(8 * n), 256, 0, s_>>>(L.mptr, L.mnb, L.wint, unit, n, sub, to_subset,
+                                                                  scale_, cut);
+            else
+                cl_cut_kernel<<<nb, 256, 0, s_>>>(L.ptr, L.nb, L.w, n, sub, to_subset, scale_, cut);
+            for (int kind = 0; kind < 2; ++kind) {
+                int64_t count = 0;
+                const uint32_t* nodes = active(L, kind, round, &count);
+                if (!count) continue;
+                const unsigned grid = kind ? (unsigned)count : (unsigned)((count + kSmallWarps - 1) / kSmallWarps);
+                auto go = [&](auto kernel, auto* w, double u) {
+                    kernel<<<grid, kind ? 32 : 32 * kSmallWarps, 0, s_>>>(
+                        L.mptr, L.mnb, w, u, L.kfix, nodes, count, part, sub, Ksub, subsize, K, cut, well, inv_scale_, res,
+                        total_, round, salt, moved, to, moves);
+                };
+                if (L.wint) {
+                    if (kind)
+                        go(cl_refine_kernel<kBigTable, 1, long long>, (const long long*)L.wint, unit);
+                    else
+                        go(cl_refine_kernel<kSmallTable, kSmallWarps, long long>, (const long long*)L.wint, unit);
+                } else if (kind) {
+                    go(cl_refine_kernel<kBigTable, 1, double>, (const double*)L.w, 1.0);
+                } else {
+                    go(cl_refine_kernel<kSmallTable, kSmallWarps, double>, (const double*)L.w, 1.0);
+                }
+            }
+            cl_apply_kernel<<<apply_blocks, 256, 0, s_>>>(moves, moved, to, L.kfix, sub, Ksub, subsize);
+            ctx_->launches += 4;
+        }
+        unsigned int moves[kRoundBatch];
+        if (!download(moves, counter_ + kCounterMoves + r0, kRoundBatch))
+            return fail(st_, SCRUST_KERNEL, "clustering: refinement");
+        for (int i = 0; i < kRoundBatch && quiet < 2; ++i) quiet = moves[i] ? 0 : quiet + 1;
     }
     return ok(st_);
 }
@@ -901,10 +1557,11 @@ int32_t Clusterer::optimise(const uint32_t* initial, double res, bool leiden, ui
         cl_comm_init_kernel<<<grid_for(n), 256, 0, s_>>>(labels, level.kfix, n, K, size);
         ctx_->launches += 1;
         const uint64_t level_salt = mix_host(salt ^ ((uint64_t)depth * 0xD1B54A32D192ED03ull));
-        int32_t rc = node_lists(level);
-        if (rc) return rc;
+        int32_t rc = SCRUST_OK;
+        if (depth && (rc = integer_weights(&level, true))) return rc;
+        if ((rc = node_lists(level, level_salt))) return rc;
         bool moved = false;
-        if ((rc = local_moving(level, labels, K, size, res, level_salt, &moved))) return rc;
+        if ((rc = local_moving(level, labels, K, size, res, &moved))) return rc;
         const int64_t nc = compact(labels, n, 2 * n, partition);
         if (nc < 0) return fail(st_, SCRUST_KERNEL, "clustering: compact");
         if (!moved || nc == n) {
@@ -956,11 +1613,13 @@ int32_t Clusterer::run(bool leiden, double res, int n_iterations, uint64_t seed,
     if (!ok_) return oom();
     cl_iota_kernel<<<grid_for(n), 256, 0, s_>>>(n, cur);
     ctx_->launches += 1;
+    int32_t rc = integer_weights(&g0_, false);
+    if (rc) return rc;
     int64_t nc = n;
     const int passes = leiden ? n_iterations : 1;
     for (int pass = 0; pass < passes; ++pass) {
         int64_t fnc = 0;
-        int32_t rc = optimise(cur, res, leiden, mix_host(seed ^ ((uint64_t)pass << 40)), found, &fnc);
+        rc = optimise(cur, res, leiden, mix_host(seed ^ ((uint64_t)pass << 40)), found, &fnc);
         if (rc) return rc;
         if (leiden) {
             // A pass that returns its own input has converged (cluster.rs:104-118).

@@ -11,6 +11,7 @@
 
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "scrust_cuda.h"
@@ -129,6 +130,7 @@ struct scrust_context {
     int* d_err = nullptr;          // scrust::DERR_COUNT ints
     uint32_t* d_counter = nullptr; // small device counters (fallback rows, work queue)
     std::vector<scrust::CsrBuffers> csr_pool;
+    std::vector<std::pair<void*, size_t>> cluster_blocks;  // workspace of the clusterings, kept from call to call
     PFN_cuTensorMapEncodeTiled_v12000 encode_tiled = nullptr;
     uint64_t launches = 0;              // kernels enqueued so far
     // Kernel counters when statistics are on: 16 words per sweep launch of a
