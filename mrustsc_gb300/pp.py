@@ -15,6 +15,12 @@ from ._shared import _INDEX_DTYPE, _VALUE_DTYPE, _csr_from_parts, _extension, _r
 METRICS = ("euclidean", "cosine")
 
 
+def _one_pass(extension, embedding, k: int) -> bool:
+    """Whether the core builds both graphs in one call: where it has one, and
+    the union's entries fit (else `connectivities` refuses, after the kNN)."""
+    return hasattr(extension, "neighbors_graph") and 2 * embedding.shape[0] * k < 0xFFFFFFFF
+
+
 def neighbors(adata, *, n_neighbors: int = 15, use_rep: str = "X_pca", device: str = "auto",
               metric: str = "euclidean", form: str = "auto") -> None:
     """Build the k-nearest-neighbour graph and its UMAP connectivities."""
@@ -25,14 +31,24 @@ def neighbors(adata, *, n_neighbors: int = 15, use_rep: str = "X_pca", device: s
     extension = _extension()
     # scanpy counts the cell itself among its n_neighbors; the core does not.
     kwargs = {} if metric == "euclidean" and form == "auto" else {"metric": metric, "form": form}
-    indices, distances = extension.knn(_representation(adata, use_rep), n_neighbors - 1, device, **kwargs)
+    embedding, k = _representation(adata, use_rep), n_neighbors - 1
+    graph = None
+    if _one_pass(extension, embedding, k):
+        # Both graphs in one call: no download, check and upload of the
+        # neighbours between them (with the conversion below, 3.8 ms against
+        # 2.2 ms at 30,011 cells and 30 neighbours).
+        indices, distances, graph = extension.neighbors_graph(embedding, k, device, **kwargs)
+    else:
+        indices, distances = extension.knn(embedding, k, device, **kwargs)
     indices = np.asarray(indices)
     distances = np.asarray(distances, dtype=_VALUE_DTYPE)
 
     n_obs, k = indices.shape
     indptr = np.arange(0, n_obs * k + 1, k, dtype=_INDEX_DTYPE)
     adata.obsp["distances"] = _csr_from_parts((indptr, indices.ravel(), distances.ravel()), (n_obs, n_obs))
-    adata.obsp["connectivities"] = _csr_from_parts(extension.connectivities(indices, distances), (n_obs, n_obs))
+    if graph is None:
+        graph = extension.connectivities(indices, distances)
+    adata.obsp["connectivities"] = _csr_from_parts(graph, (n_obs, n_obs))
     params = {"n_neighbors": n_neighbors, "method": "umap", "use_rep": use_rep}
     if metric != "euclidean":
         params["metric"] = metric
