@@ -194,13 +194,6 @@ int32_t check_options(const scrust_knn_options* o, scrust_status* st) {
 }
 
 
-struct KnnBuffers {
-    const float* xr = nullptr;   // rows the rerank measures
-    float* xwork = nullptr;
-    double* norm64 = nullptr;
-    float* norm2 = nullptr;
-};
-
 // Candidate-list geometry: column segments per row block (so small inputs
 // still fill the GPU) and the list capacity that triggers a prune.
 int32_t plan_lists(scrust_context* ctx, const scrust_knn_options& o, int k, int row_blocks, int col_tiles,
@@ -306,14 +299,14 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
 
     const float* xwork = x;
     float* xcentred = nullptr;
-    double* norm64 = nullptr;
+    CosineRows cosine_rows;
     ctx->stats_launch = 0;
     mark(ctx, PH_START);
     if (cosine) {
         float* xn = (float*)ws_get(ctx, SLOT_XWORK, sizeof(float) * (size_t)n * d, &e);
-        norm64 = (double*)ws_get(ctx, SLOT_NORM64, sizeof(double) * (size_t)n, &e);
-        if (!xn || !norm64) return cuda_fail(st, e, "workspace");
-        if ((e = launch_normalise_rows(x, n, d, xn, norm64, ctx->d_err, s)) != cudaSuccess)
+        void* buf = ws_get(ctx, SLOT_NORM64, cosine_rows_bytes(n, d), &e);
+        if (!xn || !buf) return cuda_fail(st, e, "workspace");
+        if ((e = launch_normalise_rows(x, n, d, xn, buf, &cosine_rows, ctx->d_err, s)) != cudaSuccess)
             return cuda_fail(st, e, "normalise");
         ctx->launches += 1;
         xwork = xn;
@@ -534,7 +527,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
     }
 
     const float* xr = ref ? xcentred : xwork;
-    if ((e = launch_rerank(ctx, plan, xr, xr, norm2, norm2, norm64, norm64, x, x, bounds, lists, perm, rerank_xs,
+    if ((e = launch_rerank(ctx, plan, xr, xr, norm2, norm2, cosine_rows, x, x, bounds, lists, perm, rerank_xs,
                            rerank_theta, out_idx, out_dist, nullptr, nullptr, nullptr, rerank_stride,
                            rerank_ids_only)) != cudaSuccess)
         return cuda_fail(st, e, "knn_rerank");

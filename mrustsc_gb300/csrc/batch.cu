@@ -133,12 +133,12 @@ int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, ui
     const bool bf16 = o.precision == SCRUST_PRECISION_BF16;
     const bool cosine = o.metric == SCRUST_METRIC_COSINE;
     const float* xwork = x;
-    double* norm64 = nullptr;
+    CosineRows cosine_rows;
     if (cosine) {
         float* xn = (float*)ws_get(ctx, SLOT_XWORK, sizeof(float) * (size_t)n_total * d, &e);
-        norm64 = (double*)ws_get(ctx, SLOT_NORM64, sizeof(double) * (size_t)n_total, &e);
-        if (!xn || !norm64) return cuda_fail(st, e, "workspace");
-        if ((e = launch_normalise_rows(x, n_total, d, xn, norm64, ctx->d_err, s)) != cudaSuccess)
+        void* buf = ws_get(ctx, SLOT_NORM64, cosine_rows_bytes(n_total, d), &e);
+        if (!xn || !buf) return cuda_fail(st, e, "workspace");
+        if ((e = launch_normalise_rows(x, n_total, d, xn, buf, &cosine_rows, ctx->d_err, s)) != cudaSuccess)
             return cuda_fail(st, e, "normalise");
         ctx->launches += 1;
         xwork = xn;
@@ -235,7 +235,7 @@ int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, ui
     bounds.A = bA;
     bounds.delta = bdelta;
     bounds.eps2 = beps2;
-    if ((e = launch_rerank(ctx, plan, xwork, xwork, norm2, norm2, norm64, norm64, x, x, bounds, lists, row_map, xs, theta,
+    if ((e = launch_rerank(ctx, plan, xwork, xwork, norm2, norm2, cosine_rows, x, x, bounds, lists, row_map, xs, theta,
                            out_idx, out_dist, row_lo, row_hi, nullptr, padded_row_floats(d))) != cudaSuccess)
         return cuda_fail(st, e, "batch: knn_rerank");
     ctx->launches += 1;  // the row gather (the rerank counts its own)

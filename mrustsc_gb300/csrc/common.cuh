@@ -164,6 +164,11 @@ __device__ __forceinline__ double dist2_f64(const float* __restrict__ a, const f
     return s;
 }
 
+// Whether every value within err of h + l (h the sum rounded) rounds to h.
+__device__ __forceinline__ bool rounds_surely(float h, float l, float err) {
+    return __fadd_rn(h, __fadd_ru(l, err)) == h && __fadd_rn(h, __fadd_rd(l, -err)) == h;
+}
+
 // FP64 cosine distance 1 - a.b / (|a| |b|) with precomputed FP64 norms.
 __device__ __forceinline__ double cosine_f64(const float* __restrict__ a, const float* __restrict__ b,
                                              int d, double na, double nb) {

@@ -107,7 +107,7 @@ int32_t cross_knn_enqueue(scrust_context* ctx, const Reference& ref, const float
     bounds.A = bA;
     bounds.delta = bdelta;
     bounds.eps2 = beps2;
-    if ((e = launch_rerank(ctx, plan, dq, ref.rows, nullptr, nullptr, nullptr, nullptr, dq, ref.rows, bounds, lists,
+    if ((e = launch_rerank(ctx, plan, dq, ref.rows, nullptr, nullptr, CosineRows(), dq, ref.rows, bounds, lists,
                            nullptr, dq, theta, d_idx, d_dist, nullptr, nullptr, ref.rows)) != cudaSuccess)
         return cuda_fail(st, e, "cross: knn_rerank");
     return SCRUST_OK;

@@ -304,8 +304,19 @@ constexpr int64_t kOrderMaxRows = 8000000;
 // prep.cu
 cudaError_t launch_column_means(const float* x, int64_t n, int d, bool sequential, double* means,
                                 double* partial, cudaStream_t s);
-cudaError_t launch_normalise_rows(const float* x, int64_t n, int d, float* xn, double* norm64,
-                                  int* d_err, cudaStream_t s);
+// Cosine solves: what the exact distances of rows read besides their ids.
+struct CosineRows {
+    int64_t n = 0;
+    const double* norm64 = nullptr;  // FP64 norms
+    const float2* inverse = nullptr; // 1 / norm as a sum of two floats, or NaNs where products of such rows may leave f32's range
+    const float* raw = nullptr;      // the rows padded with zeros to padded_row_floats(d), 32-byte aligned
+};
+// Rows of up to kCosineMaxDims dimensions have `inverse` and `raw`.
+constexpr int kCosineMaxDims = 128;
+size_t cosine_rows_bytes(int64_t n, int d);
+// Normalised rows into xn; `buf` holds cosine_rows_bytes(n, d) bytes.
+cudaError_t launch_normalise_rows(const float* x, int64_t n, int d, float* xn, void* buf, CosineRows* out, int* d_err,
+                                  cudaStream_t s);
 // Tensor operands: 64-wide (128-byte) blocks per row that hold d coordinates
 // and the three norm columns: one up to 61 dimensions, two up to 125.
 constexpr int kTensorMaxDim = 61, kTensorWideMaxDim = 125;
@@ -419,7 +430,7 @@ struct RowBounds {
 // rows by list entry when they are not xs (a query-versus-reference solve).
 cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float* qx,
                           const float* rx, const float* qnorm2, const float* rnorm2,
-                          const double* qn64, const double* rn64, const float* qraw,
+                          const CosineRows& cosine, const float* qraw,
                           const float* rraw, const RowBounds& bounds, const Lists& lists,
                           const uint32_t* perm, const float* xs, const float* theta, uint32_t* out_idx,
                           float* out_dist, const uint32_t* row_lo = nullptr, const uint32_t* row_hi = nullptr,

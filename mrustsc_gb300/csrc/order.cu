@@ -1655,7 +1655,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     bounds.A = bA;
     bounds.delta = bdelta;
     bounds.eps2 = beps2;
-    if ((e = launch_rerank(ctx, plan, dq, atlas_rows, nullptr, nullptr, nullptr, nullptr, dq, atlas_rows, bounds,
+    if ((e = launch_rerank(ctx, plan, dq, atlas_rows, nullptr, nullptr, CosineRows(), dq, atlas_rows, bounds,
                            lists, at.perm, xs, theta, d_idx, d_dist, nullptr, nullptr, at.rows, P, true, qperm)) !=
         cudaSuccess)
         return cuda_fail(st, e, "query knn: rerank");

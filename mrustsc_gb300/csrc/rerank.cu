@@ -32,8 +32,9 @@ struct RerankArgs {
     const float* rx;
     const float* qn2;
     const float* rn2;
-    const double* qn64;
-    const double* rn64;
+    CosineRows cosine;
+    int raw_stride;  // floats per row of cosine.raw
+    int post;  // distances of cosine rows are written by a pass after this one
     const float* qraw;
     const float* rraw;
     RowBounds bounds;
@@ -84,7 +85,7 @@ __device__ __forceinline__ bool tied(const RerankArgs& a, float r1, float r2) {
 
 __device__ __forceinline__ double adjudicate(const RerankArgs& a, int64_t q, uint32_t j) {
     if (a.metric == SCRUST_METRIC_COSINE)
-        return cosine_f64(a.qraw + q * a.d, a.rraw + (int64_t)j * a.d, a.d, a.qn64[q], a.rn64[j]);
+        return cosine_f64(a.qraw + q * a.d, a.rraw + (int64_t)j * a.d, a.d, a.cosine.norm64[q], a.cosine.norm64[j]);
     return sqrt(dist2_f64(a.qraw + q * a.d, a.rraw + (int64_t)j * a.d, a.d));
 }
 
@@ -111,7 +112,9 @@ __device__ __forceinline__ bool rows_equal(const float* __restrict__ u, const fl
 // unless every member's row has the same bits as the first member's row
 // (duplicated cells): the FP32 values are then equal, the order by id that
 // the sort left is already the FP64 order, and the FP32 value is the
-// distance.  Cosine rows always take FP64 values.
+// distance.  Cosine rows always take FP64 values: in a pass of their own where
+// the solve has one (`post`; equal rows have equal FP64 distances, too), else
+// here.
 enum : uint8_t { TIE_NONE = 0, TIE_SAME = 1, TIE_DIFF = 2 };
 
 // Writes the first k of the sorted candidates keys[0..m), resolving tie
@@ -128,7 +131,7 @@ __device__ void finalize_row(const Team& team, const RerankArgs& a, int64_t q,
         int ge = p;
         while (ge + 1 < m && tied(a, key_r(keys[ge]), key_r(keys[ge + 1]))) ge++;
         uint8_t f = TIE_NONE;
-        if (ge > gs && !cosine)
+        if (ge > gs && (!cosine || a.post))
             f = (p == gs || rows_equal(a.rraw + (int64_t)key_id(keys[gs]) * a.d,
                                        a.rraw + (int64_t)key_id(keys[p]) * a.d, a.d))
                     ? TIE_SAME
@@ -142,8 +145,8 @@ __device__ void finalize_row(const Team& team, const RerankArgs& a, int64_t q,
         if (gs >= k) continue;
         int ge = p;
         while (ge + 1 < m && tied(a, key_r(keys[ge]), key_r(keys[ge + 1]))) ge++;
-        bool fp64 = cosine;
-        if (ge > gs && !cosine)
+        bool fp64 = cosine && !a.post;
+        if (ge > gs && !fp64)
             for (int o = gs; o <= ge; ++o) fp64 |= flags[o] == TIE_DIFF;
         if (fp64) dbl[p] = adjudicate(a, q, key_id(keys[p]));
     }
@@ -154,8 +157,8 @@ __device__ void finalize_row(const Team& team, const RerankArgs& a, int64_t q,
         if (gs >= k) continue;
         int ge = p;
         while (ge + 1 < m && tied(a, key_r(keys[ge]), key_r(keys[ge + 1]))) ge++;
-        bool fp64 = cosine;
-        if (ge > gs && !cosine)
+        bool fp64 = cosine && !a.post;
+        if (ge > gs && !fp64)
             for (int o = gs; o <= ge; ++o) fp64 |= flags[o] == TIE_DIFF;
         const uint32_t id = key_id(keys[p]);
         int pos = p;
@@ -260,6 +263,72 @@ __global__ void __launch_bounds__(RR_WARPS * 32) rerank_warp_kernel(RerankArgs a
     finalize_row(team, a, q, B, m, reinterpret_cast<double*>(A), flags);
 }
 
+// The cosine distance of rows q and j in f32 pairs (the Dot2 scheme of Ogita,
+// Rump and Oishi, SIAM J. Sci. Comput. 26 (2005), in eight chains, times the
+// norms' reciprocals): h + l, h rounded, within cosine_pair_error of the true
+// value and of cosine_f64's.  NaN for rows without reciprocals, whose products
+// may leave f32's range.
+//
+// With u = 2^-24, m terms a chain and S = sum |x y| <= |x| |y|: a chain's low
+// part sums 2 m terms that come to at most (m + 1) u of its share of S, so it
+// is off by 2 m (m + 1) u^2 of that; combining the chains adds 16 (m + 2)
+// u^2 S; the two products with reciprocals, themselves within u^2, and the
+// subtraction 32 u^2.  cosine_f64 is off by (d + 4) 2^-53.
+__device__ __forceinline__ float cosine_pair_error(int stride, int d) {
+    const float m = (float)(stride / 8);
+    return (2.f * m * (m + 1.f) + 16.f * (m + 2.f) + 32.f + 0.0625f * (d + 4)) * 4.44089210e-15f;  // 1.25 u^2
+}
+__device__ __forceinline__ void two_sum(float a, float b, float* sum, float* error) {
+    const float z = __fadd_rn(a, b), t = __fsub_rn(z, a);
+    *error = __fadd_rn(__fsub_rn(a, __fsub_rn(z, t)), __fsub_rn(b, t));
+    *sum = z;
+}
+__device__ __forceinline__ void cosine_pair(const CosineRows& rows, int stride, int64_t q, int64_t j, float* high,
+                                            float* low) {
+    const float* x = rows.raw + q * stride;
+    const float* y = rows.raw + j * stride;
+    float s[8], c[8];
+#pragma unroll
+    for (int h = 0; h < 8; ++h) s[h] = c[h] = 0.f;
+    for (int t = 0; t < stride; t += 8) {
+        float xv[8], yv[8];
+        ldg_v8(x + t, xv);
+        ldg_v8(y + t, yv);
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+            const float p = __fmul_rn(xv[h], yv[h]);
+            const float pe = __fmaf_rn(xv[h], yv[h], -p);
+            float ze;
+            two_sum(s[h], p, &s[h], &ze);
+            c[h] = __fadd_rn(c[h], __fadd_rn(pe, ze));
+        }
+    }
+#pragma unroll
+    for (int w = 4; w > 0; w >>= 1) {
+#pragma unroll
+        for (int h = 0; h < w; ++h) {
+            float ze;
+            two_sum(s[h], s[h + w], &s[h], &ze);
+            c[h] = __fadd_rn(__fadd_rn(c[h], c[h + w]), ze);
+        }
+    }
+    float th = s[0], tl = c[0];
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        const float2 inv = __ldg(rows.inverse + (side ? j : q));
+        const float p = __fmul_rn(th, inv.x);
+        float e = __fmaf_rn(th, inv.x, -p);
+        e = __fmaf_rn(th, inv.y, e);
+        e = __fmaf_rn(tl, inv.x, e);
+        th = __fadd_rn(p, e);
+        tl = __fsub_rn(e, __fsub_rn(th, p));
+    }
+    float z, ze;
+    two_sum(1.f, -th, &z, &ze);
+    const float rest = __fsub_rn(ze, tl);
+    *high = __fadd_rn(z, rest);
+    *low = __fsub_rn(rest, __fsub_rn(*high, z));
+}
 // Tensor-form solves: the candidate pass left every list with a threshold no
 // smaller than the final one, so the rerank needs no selection.  A warp per
 // list row keeps the entries below the smaller of its lists' thresholds,
@@ -487,7 +556,7 @@ __device__ int sorted_row_regs(const RerankArgs& a, int64_t slot, unsigned long 
     const int64_t q = query_row(a, slot);
     // The common case: positions 0..k all start a group, so the first k are
     // singletons and the sort's order and FP32 values are final.
-    if (!cosine && k < 63 && (S & ((2ull << k) - 1)) == ((2ull << k) - 1)) {
+    if ((!cosine || a.post) && k < 63 && (S & ((2ull << k) - 1)) == ((2ull << k) - 1)) {
         if (lane < k) {
             const uint32_t id = key_id(key[0]);
             a.out_idx[q * k + lane] = a.row_lo ? id - a.row_lo[q] : id;
@@ -513,7 +582,7 @@ __device__ int sorted_row_regs(const RerankArgs& a, int64_t slot, unsigned long 
     }
     // Members whose row differs from their group's first member's row.
     unsigned long long D = 0;
-    if (!cosine && __any_sync(0xffffffffu, grouped[0] || grouped[1])) {
+    if ((!cosine || a.post) && __any_sync(0xffffffffu, grouped[0] || grouped[1])) {
         bool differs[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -533,7 +602,7 @@ __device__ int sorted_row_regs(const RerankArgs& a, int64_t slot, unsigned long 
         const int p = lane + 32 * r;
         const unsigned long long span =
             (ge[r] == 63 ? ~0ull : (2ull << ge[r]) - 1) & ~((1ull << gs[r]) - 1);  // positions gs..ge
-        need[r] = p < m && gs[r] < k && (cosine || (grouped[r] && (D & span) != 0));
+        need[r] = p < m && gs[r] < k && ((cosine && !a.post) || (grouped[r] && (D & span) != 0));
     }
     const bool any_group = __any_sync(0xffffffffu, need[0] || need[1]);
     if (any_group) {
@@ -676,7 +745,7 @@ __device__ int sorted_row_wide(const RerankArgs& a, int64_t slot, unsigned long 
     const bool cosine = a.metric == SCRUST_METRIC_COSINE;
     const int64_t q = query_row(a, slot);
     // The common case: positions 0..k all start a group.
-    bool plain = !cosine && k < 32 * R;
+    bool plain = (!cosine || a.post) && k < 32 * R;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int bits = k + 1 - 32 * r;  // of this word that must be set
@@ -723,7 +792,7 @@ __device__ int sorted_row_wide(const RerankArgs& a, int64_t slot, unsigned long 
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int p = lane + 32 * r;
-        const bool differs = !cosine && grouped[r] && p != gs[r] &&
+        const bool differs = (!cosine || a.post) && grouped[r] && p != gs[r] &&
                              !rows_equal(a.rraw + (int64_t)key_id(keys_s[gs[r]]) * a.d,
                                          a.rraw + (int64_t)key_id(key[r]) * a.d, a.d);
         D[r] = __ballot_sync(FULL, differs);
@@ -738,7 +807,7 @@ __device__ int sorted_row_wide(const RerankArgs& a, int64_t slot, unsigned long 
             const int lo = max(gs[r] - 32 * w, 0), hi = min(ge[r] - 32 * w, 31);
             if (lo <= hi) any |= (D[w] & (FULL >> (31 - hi)) & (FULL << lo)) != 0u;
         }
-        need[r] = p < m && gs[r] < k && (cosine || (grouped[r] && any));
+        need[r] = p < m && gs[r] < k && ((cosine && !a.post) || (grouped[r] && any));
         if (need[r]) dbl[p] = adjudicate(a, q, key_id(key[r]));
     }
     __syncwarp();
@@ -975,11 +1044,31 @@ __global__ void __launch_bounds__(FB_THREADS) rerank_fallback_kernel(RerankArgs 
     }
 }
 
+// Distances of cosine rows' neighbours, one a thread: the f32 value that the
+// FP64 form (cosine_f64) rounds to, from f32 pairs wherever every value within
+// the two forms' error bounds rounds alike; else by cosine_f64 itself.  Bound
+// by the row gathers (30,011 rows of 50, k = 30: with f64 products, three
+// 64-clock instructions a coordinate, the rerank took 409 us; now it takes
+// 80 us and this pass 52).
+__global__ void __launch_bounds__(256) cosine_distances_kernel(RerankArgs a, int64_t total, int stride) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= total) return;
+    const int64_t q = i / a.k;
+    const uint32_t j = a.out_idx[i] + (a.row_lo ? a.row_lo[q] : 0u);
+    if ((int64_t)j >= a.cosine.n) return;  // a row that the rerank left open
+    float h, l;
+    cosine_pair(a.cosine, stride, q, (int64_t)j, &h, &l);
+    a.out_dist[i] = rounds_surely(h, l, cosine_pair_error(stride, a.d))
+                        ? h
+                        : __double2float_rn(cosine_f64(a.qraw + q * a.d, a.rraw + (int64_t)j * a.d, a.d,
+                                                       a.cosine.norm64[q], a.cosine.norm64[j]));
+}
+
 }  // namespace
 
 cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float* qx,
                           const float* rx, const float* qnorm2, const float* rnorm2,
-                          const double* qn64, const double* rn64, const float* qraw,
+                          const CosineRows& cosine, const float* qraw,
                           const float* rraw, const RowBounds& bounds, const Lists& lists,
                           const uint32_t* perm, const float* xs, const float* theta, uint32_t* out_idx,
                           float* out_dist, const uint32_t* row_lo, const uint32_t* row_hi, const float* xr_list,
@@ -995,8 +1084,9 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     a.rx = rx;
     a.qn2 = qnorm2;
     a.rn2 = rnorm2;
-    a.qn64 = qn64;
-    a.rn64 = rn64;
+    a.cosine = cosine;
+    a.raw_stride = padded_row_floats(plan.d);
+    a.post = plan.metric == SCRUST_METRIC_COSINE && plan.mode != SCRUST_MODE_REFERENCE_SNAP && cosine.raw ? 1 : 0;
     a.qraw = qraw;
     a.rraw = rraw;
     a.bounds = bounds;
@@ -1089,6 +1179,12 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     if (e != cudaSuccess) return e;
     rerank_fallback_kernel<<<FB_BLOCKS, FB_THREADS, smem_f, ctx->stream>>>(a);
     ctx->launches += 1;
+    if (a.post) {
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const int64_t total = cosine.n * plan.k;
+        cosine_distances_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(a, total, a.raw_stride);
+        ctx->launches += 1;
+    }
     return cudaGetLastError();
 }
 
