@@ -263,8 +263,8 @@ SCRUST_API int32_t scrust_cuda_knn_batch_device(scrust_context* context, const f
                                                 uint32_t* out_indices, float* out_distances, scrust_status* status);
 /* A plan fixes the layout and the device buffers, autotunes the candidate
  * over-provisioning (the list capacity, when options->list_capacity is 0),
- * the sweep's register top-k width and the operand precision on this batch,
- * and captures the whole solve in a CUDA graph.  Each launch is one graph
+ * the sweep's form (its register top-k width, or one pass for thresholds and
+ * one that collects) and the operand precision on this batch, and captures the whole solve in a CUDA graph.  Each launch is one graph
  * launch on the context stream. */
 SCRUST_API scrust_batch_plan* scrust_cuda_batch_plan_create(scrust_context* context, const uint64_t* row_offsets,
                                                             uint32_t n_samples, uint64_t d, uint32_t k,

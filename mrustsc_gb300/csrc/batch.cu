@@ -45,7 +45,7 @@ struct scrust_batch_plan {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     float tuned_ms = 0.f;
-    int32_t topk_width = 0;            // the autotuner's register top-k width (0: by k, -1: lists)
+    int32_t topk_width = 0;            // the autotuner's choice: a register top-k width (0: by k, -1: lists) or kTwoPasses
     bool graphs = false;               // the launch also builds the connectivities
     scrust::CsrBuffers csr;            // the batch's connectivities (sample-local columns)
 };
@@ -53,6 +53,19 @@ struct scrust_batch_plan {
 namespace scrust {
 
 namespace {
+
+// A solve's sweep (batch_enqueue's `topk_width`): 0, 16, 32 and -1 are one pass
+// that keeps lists (KnnPlan::topk_width); kTwoPasses is a pass for thresholds,
+// as in ordered solves, then one that collects the ids below them.
+constexpr int kTwoPasses = -2;
+// 2 to 32 neighbours and no capacity asked for: two passes.  Neither inserts
+// entrants one by one, and lists hold a third of the candidates (16 samples of
+// 200 to 20,000 cells, 53,000 in all, k = 15: one pass at the best capacity
+// 638 us and 78 candidates a row, which the rerank takes 197 us for; two
+// passes @@ and @@ us).
+int default_sweep(const scrust_knn_options& o, uint32_t k) {
+    return o.list_capacity == 0 && k >= 2 && k <= 32 ? kTwoPasses : 0;
+}
 
 struct SampleRow {
     uint32_t start;  // first 256-row block position of the sample (P_s * 256)
@@ -123,10 +136,10 @@ __global__ void batch_local_cols_kernel(const uint32_t* __restrict__ indptr, con
 // so a second call with the same arguments can be captured in a graph.
 // With `csr` non-null the sequence ends with every sample's connectivities
 // in it (sample-local columns, rows in input order).  `topk_width` is the
-// sweep's register top-k width (KnnPlan::topk_width).
+// sweep: a register top-k width (KnnPlan::topk_width) or kTwoPasses.
 int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, uint32_t S, int64_t n_total,
                       int64_t n_pad, int d, int k, const scrust_knn_options& o, uint32_t* out_idx, float* out_dist,
-                      scrust_status* st, CsrBuffers* csr = nullptr, int topk_width = 0) {
+                      scrust_status* st, CsrBuffers* csr, int topk_width) {
     cudaStream_t s = ctx->stream;
     cudaError_t e = cudaSuccess;
     const int items = (int)(n_pad / 256);
@@ -202,9 +215,12 @@ int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, ui
     plan.metric = o.metric;
     plan.mode = SCRUST_MODE_EXACT;
     plan.precision = o.precision;
-    plan.topk_width = topk_width;
+    const bool two_passes = topk_width == kTwoPasses;
+    plan.topk_width = two_passes ? 0 : topk_width;
     Lists lists;
-    lists.cap = std::max<int>(o.list_capacity ? (int)o.list_capacity : 64, k + 32);
+    // (A collected list must hold a tile's 128 columns: a sample with fewer
+    // groups of columns than neighbours has no threshold.)
+    lists.cap = two_passes ? 256 : std::max<int>(o.list_capacity ? (int)o.list_capacity : 64, k + 32);
     lists.cap = (lists.cap + 3) / 4 * 4;
     lists.ctot = lists.cap + 128;
     lists.segments = 2;
@@ -219,10 +235,24 @@ int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, ui
     tl.row_map = row_map;
     tl.order = order;
     mark(ctx, PH_PREP);
-    if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16, &tl, false,
-                                      theta, nullptr, sweep_stats(ctx))) != cudaSuccess)
-        return cuda_fail(st, e, "batch: knn_candidates_tc");
-    ctx->launches += 1;
+    if (two_passes) {
+        const int width = k <= 16 ? 16 : 32;
+        float* topk = (float*)ws_get(ctx, SLOT_TOPK, sizeof(float) * 2 * (size_t)width * (size_t)n_pad, &e);
+        if (!topk) return cuda_fail(st, e, "batch: workspace");
+        if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16, &tl, false,
+                                          theta, nullptr, sweep_stats(ctx), nullptr, kPassThresholds, topk)) != cudaSuccess ||
+            (e = launch_merge_part_thresholds(topk, width, n_pad, n_pad, k, 2, counts, bA, bdelta, beps2, theta, s)) !=
+                cudaSuccess ||
+            (e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16, &tl, false,
+                                          theta, nullptr, sweep_stats(ctx), nullptr, kPassCollect)) != cudaSuccess)
+            return cuda_fail(st, e, "batch: knn_candidates_tc");
+        ctx->launches += 3;
+    } else {
+        if ((e = launch_tensor_candidates(ctx, plan, A16, n_pad, B16, n_pad, bA, bdelta, beps2, lists, bf16, &tl, false,
+                                          theta, nullptr, sweep_stats(ctx))) != cudaSuccess)
+            return cuda_fail(st, e, "batch: knn_candidates_tc");
+        ctx->launches += 1;
+    }
     mark(ctx, PH_CAND);
 
     // Exact rerank over the rows in the padded layout; ids relative to each
@@ -236,7 +266,7 @@ int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, ui
     bounds.delta = bdelta;
     bounds.eps2 = beps2;
     if ((e = launch_rerank(ctx, plan, xwork, xwork, norm2, norm2, cosine_rows, x, x, bounds, lists, row_map, xs, theta,
-                           out_idx, out_dist, row_lo, row_hi, nullptr, padded_row_floats(d))) != cudaSuccess)
+                           out_idx, out_dist, row_lo, row_hi, nullptr, padded_row_floats(d), two_passes)) != cudaSuccess)
         return cuda_fail(st, e, "batch: knn_rerank");
     ctx->launches += 1;  // the row gather (the rerank counts its own)
     mark(ctx, PH_RERANK);
@@ -316,7 +346,8 @@ int32_t scrust_cuda_knn_batch_device(scrust_context* ctx, const float* x, const 
         (e = cudaMemcpy(table, rows.data(), sizeof(SampleRow) * rows.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
         return cuda_fail(st, e, "batch: table upload");
     mark(ctx, PH_START);
-    return batch_enqueue(ctx, x, table, n_samples, n_total, n_pad, (int)d, (int)k, o, out_idx, out_dist, st);
+    return batch_enqueue(ctx, x, table, n_samples, n_total, n_pad, (int)d, (int)k, o, out_idx, out_dist, st, nullptr,
+                         default_sweep(o, k));
 }
 
 int32_t scrust_cuda_knn_batch(scrust_context* ctx, const float* x, const uint64_t* row_offsets, uint32_t n_samples,
@@ -386,7 +417,7 @@ int32_t scrust_cuda_neighbors_graph_batch(scrust_context* ctx, const float* x, c
     CsrBuffers b;
     if ((rc = csr_take(ctx, (uint64_t)n_total, 2 * (uint64_t)n_total * k, &b, st))) return rc;
     mark(ctx, PH_START);
-    rc = batch_enqueue(ctx, dx, table, n_samples, n_total, n_pad, (int)d, (int)k, o, di, dd, st, &b);
+    rc = batch_enqueue(ctx, dx, table, n_samples, n_total, n_pad, (int)d, (int)k, o, di, dd, st, &b, default_sweep(o, k));
     if (rc == SCRUST_OK &&
         ((e = cudaMemcpyAsync(out_idx, di, sizeof(uint32_t) * (size_t)n_total * k, cudaMemcpyDeviceToHost,
                               ctx->stream)) != cudaSuccess ||
@@ -484,6 +515,13 @@ scrust_batch_plan* plan_create(scrust_context* ctx, const uint64_t* row_offsets,
                 o.precision = prec;
                 cands.push_back(Cand{o, w});
             }
+    if (default_sweep(p->opts, k) == kTwoPasses)
+        for (int prec = 0; prec < 2; ++prec) {
+            scrust_knn_options o = p->opts;
+            o.list_capacity = 256;
+            o.precision = prec;
+            cands.push_back(Cand{o, kTwoPasses});
+        }
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
@@ -581,7 +619,7 @@ int32_t scrust_cuda_batch_plan_graph(const scrust_batch_plan* p, const uint32_t*
 int32_t scrust_cuda_batch_plan_topk_width(const scrust_batch_plan* p) {
     if (!p) return -1;
     const int w = p->topk_width;
-    if (w < 0 || p->k > 32) return 0;
+    if (w == -1 || p->k > 32) return 0;
     if (w == 32 || p->k > 16) return 32;
     return p->k == 1 ? 1 : 16;
 }
