@@ -1199,11 +1199,11 @@ __device__ __forceinline__ float f32_of(__nv_bfloat16 v) { return __bfloat162flo
 __device__ __forceinline__ uint32_t bits16(__half v) { return (uint32_t)__half_as_ushort(v); }
 __device__ __forceinline__ uint32_t bits16(__nv_bfloat16 v) { return (uint32_t)__bfloat16_as_ushort(v); }
 
-// One thread per padded row: writes A_i and B_i of input row perm[i] (a
-// padding row where perm[i] is 0xffffffff or i >= n) (64 BLOCKS 16-bit values each), the
-// quantised squared norm A = |a_hat|^2, the per-row error radius
-// eps = |a_hat - scale*c| + scale*u*|c| (+ scale*u for normalised rows), and
-// the running maxima of eps and |b_hat|.
+// Eight lanes a row and operand block, eight columns each: A_i and B_i of input
+// row perm[i] (a padding row where perm[i] is 0xffffffff or i >= n) (64 BLOCKS
+// 16-bit values each), the quantised squared norm A = |a_hat|^2, the per-row
+// error radius eps = |a_hat - scale*c| + scale*u*|c| (+ scale*u for normalised
+// rows), and the running maxima of eps and |b_hat|.
 //
 // All in f32.  Rows are centred on the f32-rounded column means (the same
 // centre for every row and query, so no distance depends on it).  A square
@@ -1211,114 +1211,118 @@ __device__ __forceinline__ uint32_t bits16(__nv_bfloat16 v) { return (uint32_t)_
 // unevaluated pair (two-sum), so its three-part split is as close as an f64
 // sum's.  Sums of rounded non-negative terms are scaled up past their
 // rounding and every step of a bound is rounded upwards.
+//
+// Bound by the bytes: a row's lanes read and write neighbouring words.  A
+// million rows of 50: a thread a row and a warp's atomics for the maxima, 209
+// us; 132 us so.  kOperandBlocks: eight blocks an SM; each ends with two atomics.
+constexpr int kOperandBlocks = 8 * 152;
+__device__ __forceinline__ void pair_add(float& h, float& l, float x, float xl) {
+    const float sum = __fadd_rn(h, x), bv = __fsub_rn(sum, h);
+    l = __fadd_rn(__fadd_rn(l, xl), __fadd_rn(__fsub_rn(h, __fsub_rn(sum, bv)), __fsub_rn(x, bv)));
+    h = sum;
+}
 template <class T, int BLOCKS>
-__global__ void __launch_bounds__(128) tensor_operands_kernel(const float* __restrict__ x, int64_t n, int64_t n_pad, int d,
+__global__ void __launch_bounds__(256) tensor_operands_kernel(const float* __restrict__ x, int64_t n, int64_t n_pad, int d,
                                        const double* __restrict__ means, const uint32_t* __restrict__ max_norm_bits,
                                        int cosine, const uint32_t* __restrict__ perm, T* __restrict__ A16,
                                        T* __restrict__ B16,
                                        float* __restrict__ bA, float* __restrict__ eps,
                                        uint32_t* __restrict__ max_eps_bits, uint32_t* __restrict__ max_bhat_bits) {
-    constexpr int W = TK * BLOCKS;  // halves per row
-    __shared__ float mean32[W];
-    for (int t = threadIdx.x; t < d; t += blockDim.x) mean32[t] = __double2float_rn(means[t]);
+    constexpr int L = 8 * BLOCKS;  // lanes a row
+    __shared__ uint32_t block_eps, block_bhat;
+    if (threadIdx.x == 0) block_eps = block_bhat = 0u;
     __syncthreads();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_pad) return;
+    const int lane = threadIdx.x & (L - 1), t0 = 8 * lane;
     const float M = __uint_as_float(*max_norm_bits);
     // Power-of-two scale so every |scale * c| <= 64 (and |b_hat|^2 < 65504).
     int sexp = M > 0.f ? (int)floorf(log2f(64.0f / M)) : 0;
     sexp = max(-100, min(100, sexp));
     const float scale = ldexpf(1.0f, sexp);
-    // Rows are built as packed 16-bit pairs in registers (static indices
-    // only): aw[w] holds columns 2w and 2w + 1.
-    uint32_t aw[W / 2], bw[W / 2];
-    const bool real = i < n && (!perm || perm[i] != 0xffffffffu);
     const uint32_t one = bits16(to16<T>(1.0f));
-    if (real) {
-        const int64_t src = perm ? (int64_t)perm[i] : i;
-        const float* xr = x + src * d;
+    float mean[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mean[e] = t0 + e < d ? __double2float_rn(means[t0 + e]) : 0.f;
+    uint32_t most_eps = 0u, most_bhat = 0u;  // as bits, where NaNs come out on top
+    // (n_pad is a multiple of a warp's rows: whole warps stay in the loop.)
+    for (int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) / L; i < n_pad; i += (int64_t)gridDim.x * 256 / L) {
+        const uint32_t src = i < n ? (perm ? perm[i] : (uint32_t)i) : 0xffffffffu;
+        const bool real = src != 0xffffffffu;
+        // The lane's columns as packed 16-bit pairs: w holds t0 + 2w and t0 + 2w + 1.
+        uint32_t aw[4] = {0u, 0u, 0u, 0u}, bw[4] = {0u, 0u, 0u, 0u};
         float hs = 0.f, hl = 0.f, e2 = 0.f, c2 = 0.f;
+        float v[8];
 #pragma unroll
-        for (int w = 0; w < W / 2; w++) {
-            uint32_t pa = 0u, pb = 0u;
+        for (int e = 0; e < 8; ++e) v[e] = real && t0 + e < d ? __ldg(x + (int64_t)src * d + t0 + e) : 0.f;
 #pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const int t = 2 * w + hh;
-                if (t < d) {
-                    const float c = __fsub_rn(__ldg(xr + t), mean32[t]);
-                    const float y = c * scale;
-                    const T q = to16<T>(y);
-                    const float qf = f32_of(q);
-                    pa |= bits16(q) << (16 * hh);
-                    pb |= bits16(to16<T>(-2.0f * qf)) << (16 * hh);
-                    const float sq = __fmul_rn(qf, qf);  // exact: at most 22 significant bits
-                    const float sum = __fadd_rn(hs, sq), bv = __fsub_rn(sum, hs);
-                    hl = __fadd_rn(hl, __fadd_rn(__fsub_rn(hs, __fsub_rn(sum, bv)), __fsub_rn(sq, bv)));
-                    hs = sum;
-                    const float err = __fsub_rn(qf, y);  // exact: q is y rounded
-                    e2 = __fmaf_rn(err, err, e2);
-                    c2 = __fmaf_rn(c, c, c2);
-                }
+        for (int e = 0; e < 8; ++e) {
+            if (real && t0 + e < d) {
+                const float c = __fsub_rn(v[e], mean[e]);
+                const float y = c * scale;
+                const T q = to16<T>(y);
+                const float qf = f32_of(q);
+                aw[e / 2] |= bits16(q) << (16 * (e & 1));
+                bw[e / 2] |= bits16(to16<T>(-2.0f * qf)) << (16 * (e & 1));
+                pair_add(hs, hl, __fmul_rn(qf, qf), 0.f);  // the square is exact: at most 22 significant bits
+                const float err = __fsub_rn(qf, y);        // exact: q is y rounded
+                e2 = __fmaf_rn(err, err, e2);
+                c2 = __fmaf_rn(c, c, c2);
             }
-            aw[w] = pa;
-            bw[w] = pb;
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
+            const float xh = __shfl_xor_sync(0xffffffffu, hs, o), xl = __shfl_xor_sync(0xffffffffu, hl, o);
+            // (The lane with the lower number adds first, so that a row's lanes agree.)
+            float h = (lane & o) ? xh : hs, l = (lane & o) ? xl : hl;
+            pair_add(h, l, (lane & o) ? hs : xh, (lane & o) ? hl : xl);
+            hs = h;
+            hl = l;
+            e2 = __fadd_rn(e2, __shfl_xor_sync(0xffffffffu, e2, o));
+            c2 = __fadd_rn(c2, __shfl_xor_sync(0xffffffffu, c2, o));
         }
         // |a_hat|^2 = h + hlo, then n1 + n2 + n3 (each difference below is
-        // exact: a value less its own 16-bit rounding).
+        // exact: a value less its own 16-bit rounding), in columns d .. d + 2 of B
+        // beside ones in A.  Padding: a reference row whose value against any
+        // query is +inf, so it can never become a candidate (and a query row with
+        // the same ones as a real row, so that no product is 0 * inf).
         const float h = __fadd_rn(hs, hl), hlo = __fsub_rn(hl, __fsub_rn(h, hs));
-        const T n1 = to16<T>(h);
+        const T n1 = to16<T>(real ? h : __int_as_float(0x7f800000));
         const float r1 = __fadd_rn(__fsub_rn(h, f32_of(n1)), hlo);
-        const T n2 = to16<T>(r1);
+        const T n2 = to16<T>(real ? r1 : 0.f);
         const float r2 = __fsub_rn(r1, f32_of(n2));
-        const T n3 = to16<T>(r2);
-        // Columns d .. d + 2: ones in A, the split norm in B.
+        const T n3 = to16<T>(real ? r2 : 0.f);
 #pragma unroll
-        for (int w = 0; w < W / 2; w++)
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const int t = 2 * w + hh;
-                const int k3 = t - d;
-                if (k3 >= 0 && k3 < 3) {
-                    const uint32_t nb = bits16(k3 == 0 ? n1 : (k3 == 1 ? n2 : n3));
-                    aw[w] |= one << (16 * hh);
-                    bw[w] |= nb << (16 * hh);
-                }
+        for (int e = 0; e < 8; ++e) {
+            const int k3 = t0 + e - d;
+            if (k3 >= 0 && k3 < 3) {
+                aw[e / 2] |= one << (16 * (e & 1));
+                bw[e / 2] |= bits16(k3 == 0 ? n1 : (k3 == 1 ? n2 : n3)) << (16 * (e & 1));
             }
-        bA[i] = h;
-        const float grow = 1.0f + (float)(d + 4) * 1.1920929e-07f;
-        const float ku = __fmul_ru(__fmul_ru(1.01f, scale), 5.9604645e-08f);
-        float ep = __fadd_ru(__fsqrt_ru(__fmul_ru(e2, grow)), __fmul_ru(ku, __fsqrt_ru(__fmul_ru(c2, grow))));
-        if (cosine) ep = __fadd_ru(ep, ku);
-        ep = __fadd_ru(ep, 1e-30f);
-        eps[i] = ep;
-        atomicMax(max_eps_bits, __float_as_uint(ep));
-        atomicMax(max_bhat_bits, __float_as_uint(__fmul_ru(__fsqrt_ru(__fadd_ru(hs, hl)), 1.0f + 1e-6f)));
-    } else {
-        // Padding: a reference row whose value against any query is +inf,
-        // so it can never become a candidate (and a query row with the same
-        // ones as a real row, so that no product is 0 * inf).
-        const uint32_t inf = bits16(to16<T>(__int_as_float(0x7f800000)));
-#pragma unroll
-        for (int w = 0; w < W / 2; w++) {
-            uint32_t pa = 0u, pb = 0u;
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const int k3 = 2 * w + hh - d;
-                if (k3 >= 0 && k3 < 3) pa |= one << (16 * hh);
-                if (k3 == 0) pb |= inf << (16 * hh);
-            }
-            aw[w] = pa;
-            bw[w] = pb;
         }
-        bA[i] = 0.f;
-        eps[i] = 0.f;
+        float ep = 0.f, bh = 0.f;
+        if (real) {
+            const float grow = 1.0f + (float)(d + 4) * 1.1920929e-07f;
+            const float ku = __fmul_ru(__fmul_ru(1.01f, scale), 5.9604645e-08f);
+            ep = __fadd_ru(__fsqrt_ru(__fmul_ru(e2, grow)), __fmul_ru(ku, __fsqrt_ru(__fmul_ru(c2, grow))));
+            if (cosine) ep = __fadd_ru(ep, ku);
+            ep = __fadd_ru(ep, 1e-30f);
+            bh = __fmul_ru(__fsqrt_ru(__fadd_ru(hs, hl)), 1.0f + 1e-6f);
+        }
+        if (lane == 0) {
+            bA[i] = real ? h : 0.f;
+            eps[i] = ep;
+        }
+        reinterpret_cast<uint4*>(A16)[i * L + lane] = make_uint4(aw[0], aw[1], aw[2], aw[3]);
+        reinterpret_cast<uint4*>(B16)[i * L + lane] = make_uint4(bw[0], bw[1], bw[2], bw[3]);
+        most_eps = max(most_eps, __float_as_uint(ep));
+        most_bhat = max(most_bhat, __float_as_uint(bh));
     }
-    uint4* ad = reinterpret_cast<uint4*>(A16 + i * W);
-    uint4* bd = reinterpret_cast<uint4*>(B16 + i * W);
-#pragma unroll
-    for (int q = 0; q < W / 8; q++) {
-        ad[q] = make_uint4(aw[4 * q], aw[4 * q + 1], aw[4 * q + 2], aw[4 * q + 3]);
-        bd[q] = make_uint4(bw[4 * q], bw[4 * q + 1], bw[4 * q + 2], bw[4 * q + 3]);
+    // One atomic a block: one a warp queues up at the two words.
+    atomicMax(&block_eps, most_eps);
+    atomicMax(&block_bhat, most_bhat);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(max_eps_bits, block_eps);
+        atomicMax(max_bhat_bits, block_bhat);
     }
 }
 
@@ -1352,15 +1356,16 @@ cudaError_t launch_tensor_operands(const float* x, int64_t n, int64_t n_pad, int
                                    const uint32_t* max_norm_bits, bool cosine, bool bf16, const uint32_t* perm,
                                    void* A16, void* B16, float* bA, float* eps, uint32_t* max_eps_bits,
                                    uint32_t* max_bhat_bits, cudaStream_t s) {
-    const unsigned blocks = (unsigned)((n_pad + 127) / 128);
-    const int one = operand_blocks(d) == 1;
+    const int wide = operand_blocks(d);
+    if (n_pad % 256) return cudaErrorInvalidValue;
+    const unsigned blocks = (unsigned)std::min<int64_t>((n_pad * 8 * wide + 255) / 256, kOperandBlocks);
     if (bf16) {
-        const auto kern = one ? tensor_operands_kernel<__nv_bfloat16, 1> : tensor_operands_kernel<__nv_bfloat16, 2>;
-        kern<<<blocks, 128, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__nv_bfloat16*)A16,
+        const auto kern = wide == 1 ? tensor_operands_kernel<__nv_bfloat16, 1> : tensor_operands_kernel<__nv_bfloat16, 2>;
+        kern<<<blocks, 256, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__nv_bfloat16*)A16,
                                     (__nv_bfloat16*)B16, bA, eps, max_eps_bits, max_bhat_bits);
     } else {
-        const auto kern = one ? tensor_operands_kernel<__half, 1> : tensor_operands_kernel<__half, 2>;
-        kern<<<blocks, 128, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__half*)A16,
+        const auto kern = wide == 1 ? tensor_operands_kernel<__half, 1> : tensor_operands_kernel<__half, 2>;
+        kern<<<blocks, 256, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__half*)A16,
                                     (__half*)B16, bA, eps, max_eps_bits, max_bhat_bits);
     }
     return cudaGetLastError();

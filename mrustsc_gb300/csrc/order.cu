@@ -306,14 +306,22 @@ __global__ void anchor_rank_kernel(uint32_t* __restrict__ keys, int64_t n, const
     if (i < n) keys[i] = rank[keys[i]];
 }
 
+// The sorted pairs taken apart, and (unless null) the m + 1 first places of the
+// cells, each written by the first row past the cells before it.  (Counting
+// rows by atomics took 22 us for 100,000 rows in 390 cells, 50 us for a
+// million, and a scan after it; 2 and 5 us so.)
 __global__ void unpack_perm_kernel(const uint32_t* __restrict__ skeys, const unsigned long long* __restrict__ svals,
-                                   int64_t n, uint32_t* __restrict__ perm, uint32_t* __restrict__ cell_of_pos,
-                                   uint32_t* __restrict__ cell_count) {
+                                   int64_t n, uint32_t m, uint32_t* __restrict__ perm,
+                                   uint32_t* __restrict__ cell_of_pos, uint32_t* __restrict__ cell_start) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
+    const uint32_t key = skeys[s];
     perm[s] = (uint32_t)svals[s];
-    cell_of_pos[s] = skeys[s];
-    atomicAdd(cell_count + skeys[s], 1u);
+    cell_of_pos[s] = key;
+    if (!cell_start) return;
+    for (uint32_t c = s ? skeys[s - 1] + 1u : 0u; c <= key && c <= m; ++c) cell_start[c] = (uint32_t)s;
+    if (s == n - 1)
+        for (uint32_t c = key + 1u; c <= m; ++c) cell_start[c] = (uint32_t)n;
 }
 
 // One warp per 256-row work item: the column tiles holding the item's own
@@ -327,20 +335,29 @@ constexpr int kHomeMax = 32;
 __global__ void prio_tiles_kernel(const uint32_t* __restrict__ cell_of_pos, int64_t n,
                                   const uint32_t* __restrict__ cell_start, int m,
                                   const uint32_t* __restrict__ anchor_nb, int ka, int items, int col_tiles,
-                                  uint32_t* __restrict__ prio, uint32_t* __restrict__ prio_cnt, int self_tile = 1) {
+                                  uint32_t* __restrict__ prio, uint32_t* __restrict__ prio_cnt) {
     __shared__ uint32_t outs[4][kPrioMax];
     __shared__ uint32_t homes[4][kHomeMax];
     __shared__ int nhome[4];
+    __shared__ uint32_t seen[4][(kMaxAnchors + 31) / 32];
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int item = blockIdx.x * 4 + wi;
     if (item >= items) return;
+    for (int w = lane; w < (m + 31) / 32; w += 32) seen[wi][w] = 0u;
     uint32_t* out = outs[wi];
     const int64_t s0 = (int64_t)item * 256, s1 = min(n, s0 + 256);
     if (lane == 0) nhome[wi] = 0;
     __syncwarp();
-    for (int64_t b = s0; b < s1; b += 32) {
-        const int64_t sp = b + lane;
-        const bool head = sp < s1 && (sp == s0 || cell_of_pos[sp] != cell_of_pos[sp - 1]);
+    bool heads[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int64_t sp = s0 + 32 * r + lane;
+        heads[r] = sp < s1 && (sp == s0 || cell_of_pos[sp] != cell_of_pos[sp - 1]);
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int64_t sp = s0 + 32 * r + lane;
+        const bool head = heads[r];
         const uint32_t bal = __ballot_sync(0xffffffffu, head);
         if (head) {
             const int pos = nhome[wi] + __popc(bal & lanemask_lt());
@@ -361,17 +378,38 @@ __global__ void prio_tiles_kernel(const uint32_t* __restrict__ cell_of_pos, int6
         cnt++;
         __syncwarp();
     };
-    if (self_tile) add((uint32_t)item);  // a self solve's own tile (query solves have none)
-    const int kk = min(ka, kAnchorNeighbours);
-    for (int j = -1; j < kk && cnt < kPrioMax; ++j) {
-        for (int hh = 0; hh < nh && cnt < kPrioMax; ++hh) {
-            const uint32_t h = homes[wi][hh];
-            const uint32_t c = j < 0 ? h : anchor_nb[(int64_t)h * ka + j];
-            if (c >= (uint32_t)m) continue;
-            const uint32_t a = cell_start[c], b = cell_start[c + 1];
-            if (b <= a) continue;
-            for (uint32_t t = a / 256; t <= (b - 1) / 256 && cnt < kPrioMax; ++t) add(t);
+    add((uint32_t)item);
+    // The cells in turn (each home, then each home's nearest neighbour, its
+    // second nearest ..), 32 at a time so that their loads are in flight
+    // together, and each cell once: homes share neighbours (adding the tiles
+    // of every repeat, 41 us for 100,000 rows, 21 us so; 54 and 25 us for a million).
+    const int cells = (min(ka, kAnchorNeighbours) + 1) * nh;
+    auto cell_at = [&](int i) {
+        if (i >= cells) return 0xffffffffu;
+        const int j = i / nh - 1;
+        const uint32_t h = homes[wi][i % nh];
+        return j < 0 ? h : anchor_nb[(int64_t)h * ka + j];
+    };
+    uint32_t ahead = cell_at(lane);
+    for (int i0 = 0; i0 < cells && cnt < kPrioMax; i0 += 32) {
+        const uint32_t c = ahead;
+        ahead = cell_at(i0 + 32 + lane);
+        const uint32_t peers = __match_any_sync(0xffffffffu, c);
+        bool first = c < (uint32_t)m && (__ffs(peers) - 1) == lane && !((seen[wi][c >> 5] >> (c & 31)) & 1u);
+        if (!__any_sync(0xffffffffu, first)) continue;
+        uint32_t a = 0u, b = 0u;
+        if (first) {
+            atomicOr(&seen[wi][c >> 5], 1u << (c & 31));
+            a = cell_start[c];
+            b = cell_start[c + 1];
+            first = b > a;
         }
+        for (uint32_t live = __ballot_sync(0xffffffffu, first); live && cnt < kPrioMax; live &= live - 1) {
+            const int l = __ffs(live) - 1;
+            const uint32_t t0 = __shfl_sync(0xffffffffu, a, l) / 256, t1 = (__shfl_sync(0xffffffffu, b, l) - 1) / 256;
+            for (uint32_t t = t0; t <= t1 && cnt < kPrioMax; ++t) add(t);
+        }
+        __syncwarp();
     }
     __syncwarp();
     for (int t = lane; t < cnt; t += 32) prio[(int64_t)item * kPrioMax + t] = out[t];
@@ -725,6 +763,58 @@ __global__ void work_keys_kernel(const uint32_t* __restrict__ counts, int items,
     vals[i] = (unsigned long long)i;
 }
 
+// The same order by one block, for up to kOrderOneBlock row blocks: bitonic
+// over (key, block) words, all distinct.  (Keys, two radix passes of three
+// launches and the ids taken out again: eight launches, 33 us of a solve of
+// any size below that, twice; this is one, of 5 us at 400 and 18 us at 4,000.)
+constexpr int kOrderOneBlock = 8192;
+// R words a thread: word r of thread t is element t + r blockDim.x.  Distances
+// below a warp go by shuffles, at or above a block between a thread's words.
+template <int R>
+__global__ void __launch_bounds__(1024) order_one_block_kernel(const uint32_t* __restrict__ counts, int items,
+                                                               uint32_t* __restrict__ order) {
+    __shared__ uint32_t swap[R * 1024];
+    const int tid = threadIdx.x, n = blockDim.x;
+    uint32_t key[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = tid + r * n;
+        key[r] = i < items ? (0xffffu - min(counts[i], 0xffffu)) << 16 | (uint32_t)i : 0xffffffffu;
+    }
+    for (int size = 2; size <= R * n; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= n) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+#pragma unroll
+                    for (int o = 1; o < R; o <<= 1) {
+                        if (stride != o * n || (r & o)) continue;
+                        const uint32_t lo = min(key[r], key[r ^ o]), hi = max(key[r], key[r ^ o]);
+                        const bool up = ((tid + r * n) & size) == 0;
+                        key[r] = up ? lo : hi;
+                        key[r ^ o] = up ? hi : lo;
+                    }
+                }
+                continue;
+            }
+            if (stride >= 32) {
+                __syncthreads();
+#pragma unroll
+                for (int r = 0; r < R; ++r) swap[tid + r * n] = key[r];
+                __syncthreads();
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int i = tid + r * n;
+                const uint32_t o = stride >= 32 ? swap[i ^ stride] : __shfl_xor_sync(0xffffffffu, key[r], stride);
+                key[r] = ((i & stride) == 0) == ((i & size) == 0) ? min(key[r], o) : max(key[r], o);
+            }
+        }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (tid + r * n < items) order[tid + r * n] = key[r] & 0xffffu;
+}
+
 __global__ void narrow_kernel(const unsigned long long* __restrict__ vals, int items, uint32_t* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < items) out[i] = (uint32_t)vals[i];
@@ -1020,6 +1110,18 @@ size_t work_order_scratch(int items) {
 }
 
 cudaError_t sort_by_work(scrust_context* ctx, const uint32_t* counts, int items, char* scratch, uint32_t* order) {
+    if (items <= kOrderOneBlock) {
+        int width = 32;
+        while (width < items) width *= 2;
+        const int threads = std::min(1024, width);
+        const auto kern = width <= 1024   ? order_one_block_kernel<1>
+                          : width == 2048 ? order_one_block_kernel<2>
+                          : width == 4096 ? order_one_block_kernel<4>
+                                          : order_one_block_kernel<8>;
+        kern<<<1, threads, 0, ctx->stream>>>(counts, items, order);
+        ctx->launches += 1;
+        return cudaGetLastError();
+    }
     const int nb = radix_blocks(items);
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -1086,8 +1188,7 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     const size_t o_src = take(4 * (size_t)m), o_anc = take(4 * (size_t)m * d), o_aA = take(row_bytes * (size_t)m_pad),
                  o_aB = take(row_bytes * (size_t)m_pad), o_arb = take(8 * (size_t)m_pad), o_kA = take(4 * (size_t)n),
                  o_kB = take(4 * (size_t)n), o_vA = take(8 * (size_t)n), o_vB = take(8 * (size_t)n),
-                 o_perm = take(4 * (size_t)n), o_cell = take(4 * (size_t)n), o_ccnt = take(4 * (size_t)(m + 1)),
-                 o_cst = take(4 * (size_t)(m + 1)), o_nb = take(4 * (size_t)m * kAnchorNeighbours),
+                 o_perm = take(4 * (size_t)n), o_cell = take(4 * (size_t)n), o_cst = take(4 * (size_t)(m + 1)), o_nb = take(4 * (size_t)m * kAnchorNeighbours),
                  o_nb2 = take(4 * (size_t)m * kAnchorNeighbours), o_rank = take(4 * (size_t)m),
                  o_adist = take(4 * (size_t)m * (size_t)m),
                  o_prio = take(4 * (size_t)items * kPrioMax), o_pc = take(4 * (size_t)items),
@@ -1104,7 +1205,6 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     unsigned long long *valsA = (unsigned long long*)(base + o_vA), *valsB = (unsigned long long*)(base + o_vB);
     uint32_t* perm = (uint32_t*)(base + o_perm);
     uint32_t* cell_of_pos = (uint32_t*)(base + o_cell);
-    uint32_t* cell_count = (uint32_t*)(base + o_ccnt);
     uint32_t* cell_start = (uint32_t*)(base + o_cst);
     uint32_t* anchor_nb = (uint32_t*)(base + o_nb);
     uint32_t* cell_nb = (uint32_t*)(base + o_nb2);
@@ -1191,13 +1291,9 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     if ((e = radix_sort_pairs(ctx, keysA, valsA, keysB, valsB, n, bits, (uint32_t*)(base + o_hist),
                               (uint32_t*)(base + o_scan), scan_elems, &skeys, &svals)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: sort");
-    if ((e = cudaMemsetAsync(cell_count, 0, 4 * (size_t)(m + 1), s)) != cudaSuccess)
-        return cuda_fail(st, e, "ordering: memset");
-    unpack_perm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(skeys, svals, n, perm, cell_of_pos, cell_count);
+    unpack_perm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(skeys, svals, n, (uint32_t)m, perm, cell_of_pos,
+                                                                   cell_start);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: permutation");
-    if ((e = device_exclusive_scan(ctx, cell_count, cell_start, m + 1, (uint32_t*)(base + o_scan), scan_elems)) !=
-        cudaSuccess)
-        return cuda_fail(st, e, "ordering: cell scan");
 
     // The priority tiles of every work item.
     prio_tiles_kernel<<<(unsigned)((items + 3) / 4), 128, 0, s>>>(cell_of_pos, n, cell_start, (int)m, cell_nb,
@@ -1468,7 +1564,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
                  o_As = take(128 * (size_t)q_pad), o_Bs = take(128 * (size_t)q_pad), o_ts = take(4 * 4 * (size_t)q_pad),
                  o_w = take(64), o_best = take(16 * (size_t)q_pad), o_kA = take(4 * (size_t)q), o_kB = take(4 * (size_t)q),
                  o_vA = take(8 * (size_t)q), o_vB = take(8 * (size_t)q), o_qp = take(4 * (size_t)q),
-                 o_cell = take(4 * (size_t)q), o_cc = take(4 * ((size_t)at.anchors + 1)),
+                 o_cell = take(4 * (size_t)q),
                  o_xs = take(4 * (size_t)q * P), o_prio = take(4 * (size_t)items * kQueryPrio),
                  o_pc = take(4 * (size_t)items), o_ps = take(4 * (size_t)work * ps), o_psc = take(4 * (size_t)work),
                  o_po = take(4 * (size_t)work), o_po2 = take(4 * (size_t)work), o_ws = take(work_order_scratch(work)),
@@ -1532,11 +1628,9 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     if ((e = radix_sort_pairs(ctx, (uint32_t*)(base + o_kA), (unsigned long long*)(base + o_vA),
                               (uint32_t*)(base + o_kB), (unsigned long long*)(base + o_vB), q, bits,
                               (uint32_t*)(base + o_hist), (uint32_t*)(base + o_scan), scan_elems, &skeys, &svals)) !=
-            cudaSuccess ||
-        (e = cudaMemsetAsync(base + o_cc, 0, 4 * ((size_t)at.anchors + 1), s)) != cudaSuccess)
+            cudaSuccess)
         return cuda_fail(st, e, "query routing: sort");
-    unpack_perm_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>(skeys, svals, q, qperm, cell_of_pos,
-                                                                  (uint32_t*)(base + o_cc));
+    unpack_perm_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>(skeys, svals, q, 0u, qperm, cell_of_pos, nullptr);
     gather_operands_kernel<1><<<(unsigned)((q_pad * 8 + 255) / 256), 256, 0, s>>>(
         (const uint4*)(base + o_A0), (const uint4*)(base + o_B0), bA0, eps0, qperm, q, q_pad, (uint4*)(base + o_As),
         (uint4*)(base + o_Bs), bA, beps);

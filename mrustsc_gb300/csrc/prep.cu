@@ -379,7 +379,13 @@ __global__ void __launch_bounds__(256) max_centred_norm_kernel(const float* __re
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         best = fmaxf(best, acc);
     }
-    if (lane == 0 && best > 0.f) {
+    // One atomic a block (with one a warp, half of the 16 us of 100,000 rows was
+    // their queue at the one word; 8 us so).
+    __shared__ float most[8];
+    if (lane == 0) most[threadIdx.x >> 5] = best;
+    __syncthreads();
+    for (int w = 0; w < 8; ++w) best = fmaxf(best, most[w]);
+    if (threadIdx.x == 0 && best > 0.f) {
         // A sum of d rounded non-negative terms, scaled past its rounding.
         const float grow = 1.0f + (float)(d + 4) * 1.1920929e-07f;
         atomicMax(max_norm_bits, __float_as_uint(__fmul_ru(__fsqrt_ru(__fmul_ru(best, grow)), 1.0f + 9.5367431640625e-07f)));
@@ -389,7 +395,7 @@ __global__ void __launch_bounds__(256) max_centred_norm_kernel(const float* __re
 cudaError_t launch_max_centred_norm(const float* x, int64_t n, int d, const double* means, uint32_t* max_norm_bits,
                                     int sm_count, cudaStream_t s) {
     const int64_t want = (n + 7) / 8;
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count * 16));
+    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sm_count * 8));
     const auto kern = operand_blocks(d) == 1 ? max_centred_norm_kernel<1> : max_centred_norm_kernel<2>;
     kern<<<blocks, 256, 0, s>>>(x, n, d, means, max_norm_bits);
     return cudaGetLastError();
