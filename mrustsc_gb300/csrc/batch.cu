@@ -62,7 +62,7 @@ constexpr int kTwoPasses = -2;
 // entrants one by one, and lists hold a third of the candidates (16 samples of
 // 200 to 20,000 cells, 53,000 in all, k = 15: one pass at the best capacity
 // 638 us and 78 candidates a row, which the rerank takes 197 us for; two
-// passes @@ and @@ us).
+// passes 287 and 75 us).
 int default_sweep(const scrust_knn_options& o, uint32_t k) {
     return o.list_capacity == 0 && k >= 2 && k <= 32 ? kTwoPasses : 0;
 }

@@ -431,22 +431,31 @@ __device__ void warp_sort_bucket(unsigned long long* v, uint32_t len) {
 // per row, k <= 32 and n < 2^31.  The row's directed entries (nf, sorted by
 // column) and its bucket of incoming edges (nb, sources unique, any order)
 // are keyed column << 1 | direction and sorted together across the warp
-// (32 or 64 positions, position lane + 32 r in register r), so an edge
+// (32, 64 or 128 positions, position lane + 32 r in register r), so an edge
 // present in both directions becomes a directed entry followed by its
 // incoming twin: the pair merges into (w + r) - (w * r), every other entry
 // keeps its weight.  The merged row goes, compacted, to the row's scratch run
 // at i * k + start[i] (room for k + nb entries) and its length to rowcnt[i];
-// merge_place_kernel then copies the runs into the CSR.  Rows with more than
-// 64 entries in all sort their bucket in place and place every entry by
+// merge_place_kernel then copies the runs into the CSR.  Rows with more
+// entries in all sort their bucket in place and place every entry by
 // binary search.  Rows [r0, r1) only.
+//
+// Bound by instruction issue, of which the sort is the most.  PACKED, for n <
+// kPackedMaxRows: the key's low bits hold the entry's position, so that the
+// sort moves and compares one word an entry and the weights are fetched once
+// after it (a million rows of 15: 530 us with the weights moved along, 420 us
+// so; 100,000 rows of 30, a third of which have more than 64 entries: 143, 124,
+// and with rows of up to 128 sorted so as well, instead of in memory, 93 us).
+constexpr int64_t kPackedMaxRows = (int64_t)1 << 24;  // column, direction and 7 bits of position in a word
 __device__ __forceinline__ uint32_t mask_below(int c) { return c >= 32 ? 0xffffffffu : ((1u << c) - 1u); }
 
-template <int P>
+template <int P, bool PACKED>
 __device__ __forceinline__ int union_sorted_row(const uint32_t* __restrict__ dcol, const float* __restrict__ dw,
                                                 const unsigned long long* __restrict__ tval, int64_t i, int k,
                                                 int nf, uint32_t b0, int nb, uint32_t* __restrict__ scol,
                                                 float* __restrict__ sval) {
     constexpr int R = P / 32;
+    static_assert(PACKED || R <= 2, "pairs are sorted in at most two registers");
     const int lane = threadIdx.x & 31;
     uint32_t key[R];
     float w[R];
@@ -463,6 +472,7 @@ __device__ __forceinline__ int union_sorted_row(const uint32_t* __restrict__ dco
             key[r] = ((uint32_t)(e >> 32) << 1) | 1u;
             w[r] = __uint_as_float((uint32_t)e);
         }
+        if (PACKED && p < nf + nb) key[r] = key[r] << 7 | (uint32_t)p;
     }
     // Ascending bitonic sort over the P positions (keys of valid entries are
     // unique; the padding keys are equal and carry nothing).
@@ -470,7 +480,25 @@ __device__ __forceinline__ int union_sorted_row(const uint32_t* __restrict__ dco
     for (int size = 2; size <= P; size <<= 1) {
 #pragma unroll
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride == 32) {
+            if (PACKED && stride >= 32) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int o = r ^ (stride / 32);
+                    if (o > r) {
+                        const uint32_t lo = min(key[r], key[o]), hi = max(key[r], key[o]);
+                        const bool up = ((32 * r) & size) == 0;
+                        key[r] = up ? lo : hi;
+                        key[o] = up ? hi : lo;
+                    }
+                }
+            } else if (PACKED) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int p = lane + 32 * r;
+                    const uint32_t o = __shfl_xor_sync(0xffffffffu, key[r], stride);
+                    key[r] = ((p & stride) == 0) == ((p & size) == 0) ? min(key[r], o) : max(key[r], o);
+                }
+            } else if (stride == 32) {
                 if (key[R - 1] < key[0]) {
                     const uint32_t tk = key[0];
                     const float tw = w[0];
@@ -492,6 +520,24 @@ __device__ __forceinline__ int union_sorted_row(const uint32_t* __restrict__ dco
                     }
                 }
             }
+        }
+    }
+    if (PACKED) {
+        float sorted[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int at = (int)(key[r] & 127u);
+            sorted[r] = 0.f;
+#pragma unroll
+            for (int o = 0; o < R; ++o) {
+                const float v = __shfl_sync(0xffffffffu, w[o], at & 31);
+                if (at >> 5 == o) sorted[r] = v;
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            w[r] = sorted[r];
+            if (key[r] != 0xffffffffu) key[r] >>= 7;
         }
     }
     // Neighbouring positions: p - 1 and p + 1.
@@ -537,6 +583,7 @@ __device__ __forceinline__ int union_sorted_row(const uint32_t* __restrict__ dco
     return total;
 }
 
+template <bool PACKED>
 __global__ void __launch_bounds__(256) merge_union_kernel(const uint32_t* __restrict__ dcol,
                                                           const float* __restrict__ dw,
                                                           const uint32_t* __restrict__ dcnt,
@@ -555,9 +602,11 @@ __global__ void __launch_bounds__(256) merge_union_kernel(const uint32_t* __rest
     float* rv = sval + run;
     int total;
     if (nf + nb <= 32) {
-        total = union_sorted_row<32>(dcol, dw, tval, i, k, nf, b0, nb, rc, rv);
+        total = union_sorted_row<32, PACKED>(dcol, dw, tval, i, k, nf, b0, nb, rc, rv);
     } else if (nf + nb <= 64) {
-        total = union_sorted_row<64>(dcol, dw, tval, i, k, nf, b0, nb, rc, rv);
+        total = union_sorted_row<64, PACKED>(dcol, dw, tval, i, k, nf, b0, nb, rc, rv);
+    } else if (PACKED && nf + nb <= 128) {
+        total = union_sorted_row<PACKED ? 128 : 64, PACKED>(dcol, dw, tval, i, k, nf, b0, nb, rc, rv);
     } else {
         // Many incoming edges: the bucket sorted in place, every directed
         // entry placed by binary search among the sources and every incoming
@@ -1093,7 +1142,8 @@ int32_t run_connectivities_distinct(scrust_context* ctx, const uint32_t* idx, co
         const int64_t r0 = n * r / R, r1 = n * (r + 1) / R;
         if (r1 > r0) {
             const unsigned blocks = (unsigned)(((r1 - r0) * 32 + 255) / 256);
-            merge_union_kernel<<<blocks, 256, 0, s>>>(dcol, dw, dcnt, tval, indeg, r0, r1, k, scol, sval, rowcnt);
+            const auto merge = n < kPackedMaxRows ? merge_union_kernel<true> : merge_union_kernel<false>;
+            merge<<<blocks, 256, 0, s>>>(dcol, dw, dcnt, tval, indeg, r0, r1, k, scol, sval, rowcnt);
             // rowcnt[r1] is the next range's first row (or the zero past the
             // last): it only receives the range's total.
             if ((e = cudaGetLastError()) != cudaSuccess ||
