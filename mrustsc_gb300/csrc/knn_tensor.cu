@@ -859,6 +859,16 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * TBN + part * kPartCols);
                 const uint32_t before = cnt;
                 const float th_before = th;
+                // Gives the accumulator back: the specialised passes do so as
+                // soon as their last chunk is in registers, so that the tensor
+                // core refills it while they work on that chunk and on the
+                // tile's merge; a general pass may read chunks again and does
+                // so after its work, before any prune.
+                auto release = [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[h]);
+                };
                 if constexpr (TOPK > 0) {
                     // First look: the tile's columns update the top-K and the
                     // threshold.  Second look: chunks holding columns below
@@ -892,6 +902,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                             for (int c = 0; c < 4; ++c) {
                                 tmem_ld32(tbase + 32 * c, va);
                                 tmem_ld_wait(va);
+                                if (PASS != 0 && c == 3) release();
                                 take(c);
                             }
                         } else {
@@ -899,6 +910,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                             for (int c = 0; c < 4; ++c) {
                                 tmem_ld32(tbase + 32 * c, va);
                                 tmem_ld_wait(va);
+                                if (PASS != 0 && c == 3) release();
                                 if (__any_sync(0xffffffffu, min32(va) < th)) take(c);
                             }
                         }
@@ -916,6 +928,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                         tmem_ld32(tbase + 96, vb);
                         group_argmin_chunk(va, col0 + 64, row, a, clean, top.v[0], best);
                         tmem_ld_wait(vb);
+                        release();
                         group_argmin_chunk(vb, col0 + 96, row, a, clean, top.v[0], best);
                     } else if constexpr (TOPK == 16 && PASS == 1) {
                         // Threshold pass: each group of columns offers only
@@ -938,6 +951,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 float q[4];
                                 tmem_ld32(tbase + 32 * c, va);
                                 tmem_ld_wait(va);
+                                if (c == 3) release();
                                 quarter_mins(va, col0 + 32 * c, row, a, q);
                                 cm[c] = fminf(fminf(q[0], q[1]), fminf(q[2], q[3]));
                                 if (__any_sync(0xffffffffu, cm[c] < fminf(top.kth(), th))) {
@@ -959,6 +973,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                             tmem_ld32(tbase + 96, vb);
                             half_mins(va, col0 + 64, row, a, g[4], g[5]);
                             tmem_ld_wait(vb);
+                            release();
                             half_mins(vb, col0 + 96, row, a, g[6], g[7]);
 #pragma unroll
                             for (int c = 0; c < 4; ++c) cm[c] = fminf(g[2 * c], g[2 * c + 1]);
@@ -995,6 +1010,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 float q[8];
                                 tmem_ld32(tbase + 32 * c, va);
                                 tmem_ld_wait(va);
+                                if (c == 3) release();
                                 eighth_mins(va, col0 + 32 * c, row, a, q);
                                 cm[c] = fminf(fminf(fminf(q[0], q[1]), fminf(q[2], q[3])),
                                               fminf(fminf(q[4], q[5]), fminf(q[6], q[7])));
@@ -1014,6 +1030,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 float q[4];
                                 tmem_ld32(tbase + 32 * c, va);
                                 tmem_ld_wait(va);
+                                if (c == 3) release();
                                 quarter_mins(va, col0 + 32 * c, row, a, q);
                                 cm[c] = fminf(fminf(q[0], q[1]), fminf(q[2], q[3]));
                                 if (__any_sync(0xffffffffu, cm[c] < fminf(top.kth(), th))) {
@@ -1028,6 +1045,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                             for (int c = 0; c < 4; ++c) {
                                 tmem_ld32(tbase + 32 * c, va);
                                 tmem_ld_wait(va);
+                                if (c == 3) release();
                                 half_mins(va, col0 + 32 * c, row, a, g[2 * c], g[2 * c + 1]);
                                 cm[c] = fminf(g[2 * c], g[2 * c + 1]);
                             }
@@ -1093,11 +1111,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     tmem_ld_wait(vb);
                     test_chunk(vb, col0 + 96, th, row, a, ids, vals, cnt);
                 }
-                // Release the accumulator before any prune, so the tensor
-                // core refills it while this warp prunes.
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tempty[h]);
+                if (PASS == 0) release();
                 n_app += cnt - before;
                 const uint32_t need = __ballot_sync(0xffffffffu, cnt >= (uint32_t)cap);
                 if (need) {
