@@ -582,6 +582,17 @@ __device__ __forceinline__ bool tile_needed(float dc2, float rI, float rT, float
     return !(lhs >= reach * reach * (1.0f + 1e-6f));
 }
 
+// No more than the squared distance of two centres, from their squared norms and
+// product, all f32 sums of d terms: each is off by at most (d + 1) u of itself
+// (u = 2^-24; twice the product is at most the norms' sum), and adding them up
+// by 6 u of the sum.  Half the instructions of summing squared differences,
+// and its error lies well below that of the thresholds (a few 1e-2 against
+// 0.4, in the operands' scale).  0 for anything not finite, which keeps the tile.
+__device__ __forceinline__ float centres_apart(float a2, float b2, float product, int d) {
+    const float sum = a2 + b2;
+    return fmaxf(0.f, fmaf(-2.f, product, sum) - (2.f * d + 16.f) * 5.9604645e-8f * sum);
+}
+
 // The cell-segment balls of all tiles, one row each (centres padded to `width`
 // = 64 or 128 dimensions with zeros), in tile order.
 __global__ void flatten_segments_kernel(TileBalls b, int d, int width, int tiles, const uint32_t* __restrict__ seg_off,
@@ -601,7 +612,9 @@ __global__ void flatten_segments_kernel(TileBalls b, int d, int width, int tiles
     }
 }
 
-// All pairs of segment balls, 64 x 64 per block step, 4 x 4 per thread:
+// All pairs of segment balls, 64 x 64 per block step, 4 x 4 per thread (7,800
+// segments of 50 dimensions: 211 us with squared differences and 4-way bank
+// conflicts in the staging, 194 us so; 1,300 of 100: 18 and 11 us):
 // when segment i (of row block owner[i]) may reach segment j (of tile
 // owner[j]), bit (owner[i], owner[j]) of the reach bitmap is set.  The
 // segment count S is read on the device; blocks stride over the block pairs
@@ -613,10 +626,9 @@ __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restr
                                                             const uint32_t* __restrict__ fo,
                                                             const uint32_t* __restrict__ S_ptr, int d, int words,
                                                             uint32_t* __restrict__ bitmap) {
-    // Rows padded by 4 floats: the transposing stores (consecutive t, same
-    // r) then spread over 8 banks instead of one; float4 reads stay aligned.
     __shared__ __align__(16) float As[64][SP + 4];
     __shared__ __align__(16) float Bs[64][SP + 4];
+    __shared__ float norms[2][4][SP];
     const int S = (int)*S_ptr;
     const int nb = (S + SP - 1) / SP;
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
@@ -625,13 +637,27 @@ __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restr
         if (bi > bj) continue;
         const int i0 = bi * SP, j0 = bj * SP;
         float acc[4][4] = {};
+        // Thread t stages four dimensions of segment t % 64 at a time (conflict
+        // free) and sums their squares.
+        const int r = threadIdx.x % SP, part = threadIdx.x / SP;
+        float a2 = 0.f, b2 = 0.f;
 #pragma unroll
         for (int blk = 0; blk < BLOCKS; ++blk) {  // 64 dimensions at a time
             __syncthreads();
-            for (int p = threadIdx.x; p < SP * 64; p += blockDim.x) {
-                const int r = p / 64, t = p % 64;
-                As[t][r] = i0 + r < S ? fc[((int64_t)(i0 + r) * BLOCKS + blk) * 64 + t] : 0.f;
-                Bs[t][r] = j0 + r < S ? fc[((int64_t)(j0 + r) * BLOCKS + blk) * 64 + t] : 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int t = 4 * (part + 4 * c);
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 x = i0 + r < S ? __ldg(reinterpret_cast<const float4*>(fc + ((int64_t)(i0 + r) * BLOCKS + blk) * 64 + t)) : zero;
+                const float4 y = j0 + r < S ? __ldg(reinterpret_cast<const float4*>(fc + ((int64_t)(j0 + r) * BLOCKS + blk) * 64 + t)) : zero;
+                As[t][r] = x.x, As[t + 1][r] = x.y, As[t + 2][r] = x.z, As[t + 3][r] = x.w;
+                Bs[t][r] = y.x, Bs[t + 1][r] = y.y, Bs[t + 2][r] = y.z, Bs[t + 3][r] = y.w;
+                a2 += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+                b2 += y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w;
+            }
+            if (blk == BLOCKS - 1) {
+                norms[0][part][r] = a2;
+                norms[1][part][r] = b2;
             }
             __syncthreads();
             const int dims = min(64, d - 64 * blk);
@@ -642,16 +668,20 @@ __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restr
 #pragma unroll
                 for (int p = 0; p < 4; ++p)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float df = av[p] - bv[q];
-                        acc[p][q] = fmaf(df, df, acc[p][q]);
-                    }
+                    for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(av[p], bv[q], acc[p][q]);
             }
         }
+        auto norm = [&](int side, int row) {
+            return norms[side][0][row] + norms[side][1][row] + norms[side][2][row] + norms[side][3][row];
+        };
+        float nb2[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) nb2[q] = norm(1, tx * 4 + q);
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
             const int i = i0 + ty * 4 + p;
             if (i >= S) continue;
+            const float na2 = norm(0, ty * 4 + p);
             const float ri = fr[i], ui = fu[i];
             const uint32_t oi = fo[i];
 #pragma unroll
@@ -660,10 +690,11 @@ __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restr
                 if (j >= S) continue;
                 const float rj = fr[j];
                 const uint32_t oj = fo[j];
-                if (tile_needed(acc[p][q], ri, rj, ui))
+                const float apart = centres_apart(na2, nb2[q], acc[p][q], d);
+                if (tile_needed(apart, ri, rj, ui))
                     atomicOr(bitmap + (int64_t)oi * words + (oj >> 5), 1u << (oj & 31));
                 // Off the diagonal block, the same distance for j reaching i.
-                if (bi != bj && tile_needed(acc[p][q], rj, ri, fu[j]))
+                if (bi != bj && tile_needed(apart, rj, ri, fu[j]))
                     atomicOr(bitmap + (int64_t)oj * words + (oi >> 5), 1u << (oi & 31));
             }
         }
@@ -836,7 +867,8 @@ __global__ void transpose_centres_kernel(const float* __restrict__ fc, int64_t s
 // radius 0 and of its own reach sqrt(theta + A + delta); the row block takes
 // the tiles of all its queries.  64 queries x 64 atlas segments a block, 4 x 4
 // a thread, distances in f32 on the quantised rows.  Testing every query costs
-// 3 d operations a segment (5,000 x 8,000 segments: 200 us), and a block of
+// 2 d operations a segment (5,000 x 8,000 segments: 200 us with squared
+// differences and bank conflicts in the staging, 141 us so), and a block of
 // queries sorted by cell falls in a hundred cells or more: balls around runs
 // of its queries (eight at most, tested one by one in 276 us) covered so much
 // that nearly every tile was kept, three passes of 600 us and more.
@@ -850,21 +882,34 @@ __global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ 
                                                           int words, uint32_t* __restrict__ bitmap) {
     __shared__ __align__(16) float As[64][64 + 4];
     __shared__ __align__(16) float Bs[64][64 + 4];
-    __shared__ float reach[64];
+    __shared__ float reach[64], query2[64], centre2[4][64];
     __shared__ uint32_t hit[64];
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
     const int64_t i0 = (int64_t)blockIdx.y * 64, j0 = (int64_t)blockIdx.x * 64;
-    for (int p = threadIdx.x; p < 64 * 64; p += blockDim.x) {
-        const int r = p / 64, t = p % 64;
-        As[t][r] = i0 + r < q && t < d ? op_float(ops[(i0 + r) * 64 + t]) : 0.f;
-        // (The centres come dimension by dimension.)
-        const int u = p / 64, c = p % 64;
-        Bs[u][c] = j0 + c < asegs && u < d ? act[(int64_t)u * asegs + j0 + c] : 0.f;
+    const int r = threadIdx.x % 64, part = threadIdx.x / 64;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int t = 8 * (part + 4 * c);
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (i0 + r < q) w = __ldg(reinterpret_cast<const uint4*>(ops + (i0 + r) * 64 + t));
+        const T* v = reinterpret_cast<const T*>(&w);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) As[t + e][r] = t + e < d ? op_float(v[e]) : 0.f;
     }
+    float c2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {  // (the centres come dimension by dimension)
+        const int t = part + 4 * c;
+        const float v = j0 + r < asegs && t < d ? __ldg(act + (int64_t)t * asegs + j0 + r) : 0.f;
+        Bs[t][r] = v;
+        c2 += v * v;
+    }
+    centre2[part][r] = c2;
     if (threadIdx.x < 64) {
         hit[threadIdx.x] = 0u;
         const int64_t i = i0 + threadIdx.x;
         float u = 0.f;
+        query2[threadIdx.x] = i < q ? bA[i] : 0.f;
         if (i < q) {
             // Every step rounded up; a row without a threshold reaches all.
             const uint32_t key = row_theta[i];
@@ -883,20 +928,20 @@ __global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ 
 #pragma unroll
         for (int p = 0; p < 4; ++p)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float df = av[p] - bv[c];
-                acc[p][c] = fmaf(df, df, acc[p][c]);
-            }
+            for (int c = 0; c < 4; ++c) acc[p][c] = fmaf(av[p], bv[c], acc[p][c]);
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const int64_t j = j0 + tx * 4 + c;
         if (j >= asegs) continue;
         const float rj = ar[j];
+        const int cj = tx * 4 + c;
+        const float b2 = centre2[0][cj] + centre2[1][cj] + centre2[2][cj] + centre2[3][cj];
         bool any = false;
 #pragma unroll
         for (int p = 0; p < 4; ++p)
-            any |= i0 + ty * 4 + p < q && tile_needed(acc[p][c], 0.f, rj, reach[ty * 4 + p]);
+            any |= i0 + ty * 4 + p < q &&
+                   tile_needed(centres_apart(query2[ty * 4 + p], b2, acc[p][c], d), 0.f, rj, reach[ty * 4 + p]);
         if (any) hit[tx * 4 + c] = 1u;
     }
     __syncthreads();
