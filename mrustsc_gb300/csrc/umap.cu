@@ -163,7 +163,10 @@ __global__ void umap_rescale_kernel(int64_t n, int dim, const uint32_t* __restri
 // left it to the latency of ~60 moves in a row (613 us an epoch for 30,000
 // cells of 23 edges, 2 components); eight lanes a cell took 131 us, a sixth of
 // its instructions stepping streams in lockstep and its last fifth waiting
-// for cells of five times the mean degree.  DIM: components (0: `dim`, up to
+// for cells of five times the mean degree; 74 us so with five blocks an SM, 67
+// with six (42 registers: 30,000 cells are 938 blocks, then all but 26 of them
+// resident; seven spill, 70 us, and so do other splits of the block, 69 to 90).
+// DIM: components (0: `dim`, up to
 // kUmapMaxDim).
 template <int DIM>
 struct UmapShape {
@@ -186,7 +189,7 @@ __device__ __forceinline__ int umap_owner(const uint32_t* at, uint32_t x) {
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(kUmapRowThreads)
+__global__ void __launch_bounds__(kUmapRowThreads, DIM == 2 ? 6 : 1)
     umap_rows_kernel(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices, int64_t n, int dim_,
                      double now, float alpha, float a, float b, int neg_rate, const float* __restrict__ y,
                      const double* __restrict__ eps, const double* __restrict__ eps_neg, double* __restrict__ next,
