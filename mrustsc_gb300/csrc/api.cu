@@ -229,11 +229,10 @@ int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_
     const size_t slots = (size_t)rows_pad * lists->segments;
     lists->ids = (uint32_t*)ws_get(ctx, SLOT_LIST_IDS, sizeof(uint32_t) * slots * lists->ctot, &e);
     lists->vals = (float*)ws_get(ctx, SLOT_LIST_VALS, sizeof(float) * slots * lists->ctot, &e);
-    lists->cnt = (uint32_t*)ws_get(ctx, SLOT_LIST_CNT, sizeof(uint32_t) * slots, &e);
-    lists->overflow = (uint32_t*)ws_get(ctx, SLOT_OVERFLOW, sizeof(uint32_t) * (size_t)rows_pad, &e);
-    if (!lists->ids || !lists->vals || !lists->cnt || !lists->overflow) return cuda_fail(st, e, "workspace");
-    if ((e = cudaMemsetAsync(lists->overflow, 0, sizeof(uint32_t) * (size_t)rows_pad, ctx->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(lists->cnt, 0, sizeof(uint32_t) * slots, ctx->stream)) != cudaSuccess)
+    lists->cnt = (uint32_t*)ws_get(ctx, SLOT_LIST_CNT, sizeof(uint32_t) * (slots + (size_t)rows_pad), &e);
+    if (!lists->ids || !lists->vals || !lists->cnt) return cuda_fail(st, e, "workspace");
+    lists->overflow = lists->cnt + slots;
+    if ((e = cudaMemsetAsync(lists->cnt, 0, sizeof(uint32_t) * (slots + (size_t)rows_pad), ctx->stream)) != cudaSuccess)
         return cuda_fail(st, e, "memset");
     return SCRUST_OK;
 }
@@ -363,16 +362,15 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
                                          beps2, &order, st);
             if (rc) return rc;
         }
-        // An ordered solve has its operands in list order already.
+        // An ordered solve has its operands in list order already, and their bounds.
         if (!order_rows) {
             if ((e = launch_tensor_operands(xwork, n, n_pad, d, means, max_bits, cosine, bf16, nullptr, A16, B16, bA,
                                             beps, max_bits + 1, max_bits + 2, s)) != cudaSuccess)
                 return cuda_fail(st, e, "tensor operands");
-            ctx->launches += 1;
+            if ((e = launch_tensor_bounds(n, d, bA, beps, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess)
+                return cuda_fail(st, e, "tensor bounds");
+            ctx->launches += 2;
         }
-        if ((e = launch_tensor_bounds(n, d, bA, beps, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess)
-            return cuda_fail(st, e, "tensor bounds");
-        ctx->launches += 1;
         // Headroom of 128: a tensor-form list is checked once per tile, after
         // its warp has appended up to 128 columns.
         // Ordered solves keep long lists (256): a row block's first tiles

@@ -164,6 +164,25 @@ __device__ __forceinline__ double dist2_f64(const float* __restrict__ a, const f
     return s;
 }
 
+// A row's bound terms of the tensor form from its squared norm A, its
+// quantisation error eps, and the largest eps (E) and |b_hat| (Mb).  delta: bound
+// on the FP32 accumulation error of the MMA chain over a row's
+// `terms` = 64 or 128 halves, 8 * terms * 2^-24 * (2 |a_hat| Mb + Mb^2 + 3), plus the rounding of A to f32
+// and the residual of the three-part 16-bit split of |b_hat|^2 (at most
+// 2^-24 |b_hat|^2 for bf16 parts, far less for fp16); eps2 = 2 (eps_i + E).
+// Every step rounded upwards.
+__device__ __forceinline__ void tensor_row_bounds(float A, float eps, float E, float Mb, int terms, float* delta_out,
+                                                  float* eps2_out) {
+    const float a = __fsqrt_ru(A);
+    const float mb2 = __fmul_ru(Mb, Mb);
+    const float chain = __fadd_ru(__fadd_ru(__fmul_ru(__fmul_ru(2.0f, a), Mb), mb2), 3.0f);
+    float delta = __fmul_ru(4.76837158203125e-07f * (float)terms, chain);  // 8 * terms * 2^-24, exact
+    delta = __fadd_ru(delta, __fmul_ru(1.1920928955078125e-07f, A));  // 2 * 2^-24
+    delta = __fadd_ru(delta, __fmul_ru(2.384185791015625e-07f, mb2)); // 4 * 2^-24
+    *delta_out = __fadd_ru(delta, 1e-7f);
+    *eps2_out = __fmul_ru(2.0f, __fadd_ru(eps, E));
+}
+
 // Whether every value within err of h + l (h the sum rounded) rounds to h.
 __device__ __forceinline__ bool rounds_surely(float h, float l, float err) {
     return __fadd_rn(h, __fadd_ru(l, err)) == h && __fadd_rn(h, __fadd_rd(l, -err)) == h;

@@ -1103,13 +1103,12 @@ int32_t run_connectivities_distinct(scrust_context* ctx, const uint32_t* idx, co
     uint32_t* carry = dcnt + (n + 1);        // kCsrRanges + 1 offsets, in the 256 spare bytes
     static_assert(sizeof(uint32_t) * (kCsrRanges + 2) <= 256, "range offsets fit the spare bytes");
     const int R = ranges ? kCsrRanges : 1;
-    if ((e = cudaMemsetAsync(indeg, 0, sizeof(uint32_t) * (size_t)(n + 1), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(carry, 0, sizeof(uint32_t), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(rowcnt + n, 0, sizeof(uint32_t), s)) != cudaSuccess)
+    // The in-degrees, the last row count, the first carry and the flags, in one
+    // with what lies between them (a few us at a million rows; a launch each, else).
+    uint32_t* flags = carry + kCsrRanges + 1;
+    if ((e = cudaMemsetAsync(indeg, 0, sizeof(uint32_t) * (size_t)(flags + 1 - indeg), s)) != cudaSuccess)
         return cuda_fail(st, e, "memset");
     if (guard) {
-        uint32_t* flags = carry + kCsrRanges + 1;
-        if ((e = cudaMemsetAsync(flags, 0, sizeof(uint32_t), s)) != cudaSuccess) return cuda_fail(st, e, "memset");
         check_graph_kernel<<<(unsigned)std::min<int64_t>(8 * ctx->sm_count, (E + 255) / 256), 256, 0, s>>>(idx, dist, E, n,
                                                                                                        flags);
         if ((e = cudaGetLastError()) != cudaSuccess ||

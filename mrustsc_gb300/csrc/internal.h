@@ -27,8 +27,7 @@ enum Slot : int {
     SLOT_CNORM,         // per-row centred norm (for bounds)
     SLOT_LIST_IDS,
     SLOT_LIST_VALS,
-    SLOT_LIST_CNT,
-    SLOT_OVERFLOW,
+    SLOT_LIST_CNT,      // list counts, then the rows' overflow flags
     SLOT_FALLBACK_ROWS,
     SLOT_FALLBACK_SCRATCH,
     SLOT_XWORK,         // normalised (cosine) or centred (reference-snap) rows

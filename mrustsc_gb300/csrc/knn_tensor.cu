@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             float th = valid ? __int_as_float(0x7f800000) : __int_as_float(0xff800000);
             uint32_t cnt = 0;
             TensorBound bnd{0.f, 0.f, 0.f};
-            if (valid) bnd = TensorBound{a.bA[row], a.bdelta[row], a.beps2[row]};
+            if (valid && PASS != 3) bnd = TensorBound{a.bA[row], a.bdelta[row], a.beps2[row]};
             const int64_t lslot = (row * col_segs + seg) * PARTS + part;
             if (valid && collect) {
                 // The row's lists in this column segment are lslot and
@@ -1340,28 +1340,14 @@ __global__ void __launch_bounds__(256) tensor_operands_kernel(const float* __res
     }
 }
 
-// delta: bound on the FP32 accumulation error of the MMA chain over a row's
-// `terms` = 64 or 128 halves, 8 * terms * 2^-24 * (2 |a_hat| Mb + Mb^2 + 3), plus the rounding of A to f32
-// and the residual of the three-part 16-bit split of |b_hat|^2 (at most
-// 2^-24 |b_hat|^2 for bf16 parts, far less for fp16); eps2 = 2 (eps_i + E).
-// Every step rounded upwards.
 __global__ void tensor_bounds_kernel(int64_t n, int terms, const float* __restrict__ bA, const float* __restrict__ eps,
                                      const uint32_t* __restrict__ max_eps_bits,
                                      const uint32_t* __restrict__ max_bhat_bits, float* __restrict__ bdelta,
                                      float* __restrict__ beps2) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float Mb = __uint_as_float(*max_bhat_bits);
-    const float E = __uint_as_float(*max_eps_bits);
-    const float A = bA[i];
-    const float a = __fsqrt_ru(A);
-    const float mb2 = __fmul_ru(Mb, Mb);
-    const float chain = __fadd_ru(__fadd_ru(__fmul_ru(__fmul_ru(2.0f, a), Mb), mb2), 3.0f);
-    float delta = __fmul_ru(4.76837158203125e-07f * (float)terms, chain);  // 8 * terms * 2^-24, exact
-    delta = __fadd_ru(delta, __fmul_ru(1.1920928955078125e-07f, A));  // 2 * 2^-24
-    delta = __fadd_ru(delta, __fmul_ru(2.384185791015625e-07f, mb2)); // 4 * 2^-24
-    bdelta[i] = __fadd_ru(delta, 1e-7f);
-    beps2[i] = __fmul_ru(2.0f, __fadd_ru(eps[i], E));
+    tensor_row_bounds(bA[i], eps[i], __uint_as_float(*max_eps_bits), __uint_as_float(*max_bhat_bits), terms, bdelta + i,
+                      beps2 + i);
 }
 
 }  // namespace

@@ -447,7 +447,7 @@ struct TileBalls {
     float* seg_centre;  // [kSegMax][d][tiles]
     float* seg_radius;  // [kSegMax][tiles]
     float* seg_reach;   // [kSegMax][tiles]
-    uint32_t* nseg;     // [tiles]
+    uint32_t* nseg;     // [tiles + 1], the last 0
 };
 
 // One block of 256 threads per column tile (= row block, the solve being a
@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
         b.radius[tile] = __fmul_ru(__fsqrt_ru(__uint_as_float(rmax_all)), 1.0f + 1e-6f);
         b.reach[tile] = __uint_as_float(umax_all);
         b.nseg[tile] = (uint32_t)nseg;
+        if (tile == 0) b.nseg[tiles] = 0u;  // for the scan
     }
     if (threadIdx.x < nseg) {
         const int sg = threadIdx.x;
@@ -760,7 +761,9 @@ __global__ void gather_operands_kernel(const uint4* __restrict__ A0, const uint4
                                        const float* __restrict__ bA0, const float* __restrict__ eps0,
                                        const uint32_t* __restrict__ perm, int64_t n, int64_t n_pad,
                                        uint4* __restrict__ A16, uint4* __restrict__ B16, float* __restrict__ bA,
-                                       float* __restrict__ eps) {
+                                       float* __restrict__ eps, const uint32_t* __restrict__ max_eps_bits,
+                                       const uint32_t* __restrict__ max_bhat_bits, float* __restrict__ bdelta,
+                                       float* __restrict__ beps2) {
     constexpr int WORDS = 8 * BLOCKS;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t s = t / WORDS;
@@ -771,8 +774,11 @@ __global__ void gather_operands_kernel(const uint4* __restrict__ A0, const uint4
         A16[s * WORDS + q] = A0[r * WORDS + q];
         B16[s * WORDS + q] = B0[r * WORDS + q];
         if (q == 0) {
-            bA[s] = bA0[r];
-            eps[s] = eps0[r];
+            const float A = bA0[r], ep = eps0[r];
+            bA[s] = A;
+            eps[s] = ep;
+            tensor_row_bounds(A, ep, __uint_as_float(*max_eps_bits), __uint_as_float(*max_bhat_bits), 64 * BLOCKS,
+                              bdelta + s, beps2 + s);
         }
     } else {
         const uint4 z = make_uint4(0u, 0u, 0u, 0u);
@@ -1293,11 +1299,10 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     float* eps0 = (float*)(base + o_eps0);
     if ((e = launch_tensor_operands(x, n, n_pad, d, means, max_bits, cosine, bf16, nullptr, A0, B0, bA0, eps0,
                                     max_bits + 1, max_bits + 2, s)) != cudaSuccess ||
-        (e = launch_tensor_bounds(n, d, bA0, eps0, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess ||
         (e = launch_tensor_operands(x, m, m_pad, d, means, max_bits, cosine, bf16, src, base + o_aA, base + o_aB, arb,
                                     arb + m_pad, max_bits + 1, max_bits + 2, s)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: operands");
-    ctx->launches += 4;
+    ctx->launches += 3;
 
     // Rows x anchors with k = 1 on the tensor cores, keeping only each row's
     // nearest anchor.
@@ -1348,10 +1353,11 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     ctx->launches += 2;
     if ((e = sort_by_work(ctx, prio_cnt, items, base + o_ws, (uint32_t*)(base + o_po))) != cudaSuccess)
         return cuda_fail(st, e, "ordering: work order");
-    // The operands in list order (bounds follow in the caller).
+    // The operands and bounds in list order.
     const auto gather = blocks == 1 ? gather_operands_kernel<1> : gather_operands_kernel<2>;
     gather<<<(unsigned)((n_pad * 8 * blocks + 255) / 256), 256, 0, s>>>(
-        (const uint4*)A0, (const uint4*)B0, bA0, eps0, perm, n, n_pad, (uint4*)A16, (uint4*)B16, bA, beps);
+        (const uint4*)A0, (const uint4*)B0, bA0, eps0, perm, n, n_pad, (uint4*)A16, (uint4*)B16, bA, beps, max_bits + 1,
+        max_bits + 2, bdelta, beps2);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: operands");
     ctx->launches += 1;
     out->perm = perm;
@@ -1410,8 +1416,7 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
     uint32_t* bitmap = (uint32_t*)(base + o_bm);
     uint32_t* counts = (uint32_t*)(base + o_cnt);
     uint32_t* entries = (uint32_t*)(base + o_ent);
-    if ((e = cudaMemsetAsync(balls.nseg + tiles, 0, sizeof(uint32_t), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)tiles * words, s)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)tiles * words, s)) != cudaSuccess)
         return cuda_fail(st, e, "pruning: memset");
     launch_tile_balls(bf16, A16, n, d, tiles, order.cell_of_pos, order.theta, bA, bdelta, balls, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: tile balls");
@@ -1539,9 +1544,7 @@ int32_t atlas_order_build(scrust_context* ctx, const float* atlas, int64_t m, in
         (e = cudaMemcpyAsync(o.cell_nb, ord.cell_nb, 4 * na * kAnchorNeighbours, cudaMemcpyDeviceToDevice, s)) !=
             cudaSuccess ||
         (e = launch_gather_rows(atlas, ord.perm, m, d, P, o.rows, s)) != cudaSuccess ||
-        (e = launch_tensor_bounds(m, d, bA, beps, words + 1, words + 2, bdelta, beps2, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(base + o_th, 0, 4 * 2 * (size_t)o.m_pad, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(balls.nseg + tiles, 0, sizeof(uint32_t), s)) != cudaSuccess)
+        (e = cudaMemsetAsync(base + o_th, 0, 4 * 2 * (size_t)o.m_pad, s)) != cudaSuccess)
         return bail(cuda_fail(st, e, "atlas ordering"));
     // The cell-segment balls of the atlas tiles (their reach is not used).
     uint32_t* seg_off = (uint32_t*)(base + o_so);
@@ -1679,9 +1682,8 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     unpack_perm_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>(skeys, svals, q, 0u, qperm, cell_of_pos, nullptr);
     gather_operands_kernel<1><<<(unsigned)((q_pad * 8 + 255) / 256), 256, 0, s>>>(
         (const uint4*)(base + o_A0), (const uint4*)(base + o_B0), bA0, eps0, qperm, q, q_pad, (uint4*)(base + o_As),
-        (uint4*)(base + o_Bs), bA, beps);
+        (uint4*)(base + o_Bs), bA, beps, words + 1, words + 2, bdelta, beps2);
     if ((e = cudaGetLastError()) != cudaSuccess ||
-        (e = launch_tensor_bounds(q, d, bA, beps, words + 1, words + 2, bdelta, beps2, s)) != cudaSuccess ||
         (e = launch_gather_rows(dq, qperm, q, d, P, xs, s)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: gather");
     // Priority tiles per row block, dealt over its column segments.
