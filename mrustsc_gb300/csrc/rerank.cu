@@ -13,6 +13,8 @@
 // One warp per row in the common case; rows whose lists overflowed, or whose
 // union exceeds the warp's capacity, go to a block-per-row fallback that
 // re-measures the whole row.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "internal.h"
 #include "lists.cuh"
@@ -25,7 +27,8 @@ constexpr int RR_WARPS = 4;
 constexpr int RC = kRerankUnion;  // keys per warp
 constexpr int FB_CAP = 4096;  // keys per fallback block
 constexpr int FB_THREADS = 256;
-constexpr int FB_BLOCKS = 32;
+constexpr int FB_ROWS = 32;      // rows at a time, a cluster each
+constexpr int FB_CLUSTER = 8;
 
 struct RerankArgs {
     const float* qx;
@@ -938,110 +941,142 @@ __global__ void __launch_bounds__(RS_BIG_WARPS * 32) rerank_sorted_big_kernel(Re
     }
 }
 
-// One block per row, over every reference row: used for rows whose
-// candidate lists overflowed (many cells within the margin, e.g. duplicates).
-__global__ void __launch_bounds__(FB_THREADS) rerank_fallback_kernel(RerankArgs a) {
+// A cluster per row, over every reference row of its solve: used for rows whose
+// candidate lists overflowed (many cells within the margin, e.g. duplicates, or
+// data of few dimensions).  Bound by the latency of one SM's row reads: each
+// block measures and counts its share of the columns, and the first one
+// gathers the candidates in its shared memory, sorts and finishes them
+// (300,000 rows of 10 dimensions, k = 20, some 350 rows here: 10.6 ms with a
+// block a row, 1.6 ms so; a launch without rows returns at once).
+__global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
+    rerank_fallback_kernel(RerankArgs a) {
+    if (*a.fb_count == 0u) return;
+    namespace cg = cooperative_groups;
     extern __shared__ unsigned long long fb_smem[];
-    unsigned long long* keys = fb_smem;
+    unsigned long long* keys = fb_smem;  // the first block's: the row's candidates
     double* dbl = reinterpret_cast<double*>(fb_smem + FB_CAP);
     uint8_t* flags = reinterpret_cast<uint8_t*>(fb_smem + 2 * FB_CAP);
     __shared__ int scratch;
-    __shared__ uint32_t row_s;
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t sel_prefix;
-    __shared__ int sel_rank;
-    __shared__ int cnt_s;
+    __shared__ uint32_t hist[256], all[256];
+    __shared__ uint32_t row_s, sel_prefix;
+    __shared__ int sel_rank, cnt_s, outside_s;
+    __shared__ float limit_s, next_s;
+    __shared__ int again_s;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
+    const bool first = rank == 0;
+    auto of_first = [&](auto* p) { return cluster.map_shared_rank(p, 0); };
     BlockTeam team(&scratch);
-    const int tid = threadIdx.x;
-    float* sc = a.fb_scratch + (int64_t)blockIdx.x * a.nr;
+    float* sc = a.fb_scratch + (int64_t)(blockIdx.x / FB_CLUSTER) * a.nr;
     for (;;) {
-        if (tid == 0) {
+        if (first && tid == 0) {
             const uint32_t i = atomicAdd(a.fb_next, 1u);
             row_s = i < *a.fb_count ? a.fb_rows[i] : 0xffffffffu;
-        }
-        __syncthreads();
-        const uint32_t row = row_s;
-        __syncthreads();
-        if (row == 0xffffffffu) break;
-        const int64_t q = query_row(a, row);
-        // The columns of the row's own solve: [lo, hi) of the input rows.
-        const int64_t lo = a.row_lo ? (int64_t)a.row_lo[q] : 0, hi = a.row_lo ? (int64_t)a.row_hi[q] : a.nr;
-        for (int64_t j = tid; j < a.nr; j += blockDim.x)
-            sc[j] = (a.self && j == q + a.self_offset) || j < lo || j >= hi ? __int_as_float(0x7f800000) : compute_r(a, q, (uint32_t)j);
-        __syncthreads();
-        // k-th smallest of the row: four 8-bit radix passes.
-        if (tid == 0) {
             sel_prefix = 0;
             sel_rank = a.k;
         }
+        cluster.sync();
+        const uint32_t row = *of_first(&row_s);
+        if (row == 0xffffffffu) break;
+        const int64_t q = query_row(a, row);
+        // The columns of the row's own solve, [lo, hi) of the input rows, and
+        // the block's share of them.
+        const int64_t lo = a.row_lo ? (int64_t)a.row_lo[q] : 0, hi = a.row_lo ? (int64_t)a.row_hi[q] : a.nr;
+        const int64_t j0 = lo + (hi - lo) * rank / FB_CLUSTER, j1 = lo + (hi - lo) * (rank + 1) / FB_CLUSTER;
+        for (int64_t j = j0 + tid; j < j1; j += FB_THREADS)
+            sc[j] = a.self && j == q + a.self_offset ? __int_as_float(0x7f800000) : compute_r(a, q, (uint32_t)j);
+        // k-th smallest of the row: four 8-bit radix passes.
         uint32_t mask = 0;
         for (int pass = 0; pass < 4; ++pass) {
             const int shift = 24 - 8 * pass;
             hist[tid] = 0;
+            const uint32_t prefix = *of_first(&sel_prefix);
             __syncthreads();
-            const uint32_t prefix = sel_prefix;
-            for (int64_t j = tid; j < a.nr; j += blockDim.x) {
+            for (int64_t j = j0 + tid; j < j1; j += FB_THREADS) {
                 const uint32_t key = float_key(sc[j]);
                 if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
             }
-            __syncthreads();
-            if (tid == 0) {
-                int rank = sel_rank;
-                uint32_t b = 0;
-                for (; b < 256; ++b) {
-                    if ((int)hist[b] >= rank) break;
-                    rank -= (int)hist[b];
+            cluster.sync();
+            if (first) {
+                uint32_t sum = 0;
+                for (int b = 0; b < FB_CLUSTER; ++b) sum += *cluster.map_shared_rank(&hist[tid], b);
+                all[tid] = sum;
+                __syncthreads();
+                if (tid == 0) {
+                    int left = sel_rank;
+                    uint32_t b = 0;
+                    for (; b < 256; ++b) {
+                        if ((int)all[b] >= left) break;
+                        left -= (int)all[b];
+                    }
+                    sel_rank = left;
+                    sel_prefix = prefix | (b << shift);
                 }
-                sel_rank = rank;
-                sel_prefix = prefix | (b << shift);
             }
             mask |= 255u << shift;
-            __syncthreads();
+            cluster.sync();
         }
-        const float vk = key_float(sel_prefix);
-        float T = vk;
-        if (a.mode != SCRUST_MODE_REFERENCE_SNAP) T = vk + 4.0f * (a.gamma * 2.0f * vk + kTieAbs) +
-                                                      (a.metric == SCRUST_METRIC_COSINE ? 1e-6f : 0.0f);
+        if (first && tid == 0) {
+            const float vk = key_float(sel_prefix);
+            limit_s = vk;
+            if (a.mode != SCRUST_MODE_REFERENCE_SNAP)
+                limit_s = vk + 4.0f * (a.gamma * 2.0f * vk + kTieAbs) + (a.metric == SCRUST_METRIC_COSINE ? 1e-6f : 0.0f);
+        }
         int m = 0;
         for (int attempt = 0; attempt < 8; ++attempt) {
-            if (tid == 0) cnt_s = 0;
-            __syncthreads();
-            for (int64_t j = tid; j < a.nr; j += blockDim.x) {
+            if (first && tid == 0) cnt_s = outside_s = again_s = 0;
+            cluster.sync();
+            const float T = *of_first(&limit_s);
+            int* cnt = of_first(&cnt_s);
+            unsigned long long* out = of_first(keys);
+            for (int64_t j = j0 + tid; j < j1; j += FB_THREADS) {
                 const float r = sc[j];
                 if (r <= T) {
-                    const int pos = atomicAdd(&cnt_s, 1);
-                    if (pos < FB_CAP) keys[pos] = ((unsigned long long)float_key(r) << 32) | (uint32_t)j;
+                    const int pos = atomicAdd(cnt, 1);
+                    if (pos < FB_CAP) out[pos] = ((unsigned long long)float_key(r) << 32) | (uint32_t)j;
                 }
             }
-            __syncthreads();
-            m = cnt_s;
+            cluster.sync();
+            m = *cnt;
             if (m > FB_CAP) break;
-            const int P = next_pow2(m);
-            for (int p = m + tid; p < P; p += blockDim.x) keys[p] = ~0ull;
-            __syncthreads();
-            team_bitonic_sort(team, keys, P);
-            if (a.mode == SCRUST_MODE_REFERENCE_SNAP) break;
-            // If the tie group holding the last collected candidate reaches
-            // position k-1, make sure nothing just outside T could join it.
-            const float rl = key_r(keys[m - 1]);
-            int gs = m - 1;
-            while (gs > 0 && tied(a, key_r(keys[gs - 1]), key_r(keys[gs]))) gs--;
-            if (gs >= a.k) break;
-            const float T2 = rl + 2.0f * (a.gamma * 2.0f * rl + kTieAbs) +
+            if (first) {
+                const int P = next_pow2(m);
+                for (int p = m + tid; p < P; p += FB_THREADS) keys[p] = ~0ull;
+                __syncthreads();
+                team_bitonic_sort(team, keys, P);
+                // If the tie group holding the last collected candidate reaches
+                // position k-1, make sure nothing just outside T could join it.
+                if (tid == 0 && a.mode != SCRUST_MODE_REFERENCE_SNAP && m > 0) {
+                    const float rl = key_r(keys[m - 1]);
+                    int gs = m - 1;
+                    while (gs > 0 && tied(a, key_r(keys[gs - 1]), key_r(keys[gs]))) gs--;
+                    again_s = gs < a.k;
+                    next_s = rl + 2.0f * (a.gamma * 2.0f * rl + kTieAbs) +
                              (a.metric == SCRUST_METRIC_COSINE ? 1e-6f : 0.0f);
+                }
+            }
+            cluster.sync();
+            if (!*of_first(&again_s)) break;
+            const float T2 = *of_first(&next_s);
             int outside = 0;
-            for (int64_t j = tid; j < a.nr; j += blockDim.x) outside += (sc[j] > T && sc[j] <= T2);
-            if (team.sum(outside) == 0) break;
-            T = T2;
+            for (int64_t j = j0 + tid; j < j1; j += FB_THREADS) outside += (sc[j] > T && sc[j] <= T2);
+            outside = team.sum(outside);
+            if (tid == 0 && outside) atomicAdd(of_first(&outside_s), outside);
+            cluster.sync();
+            if (*of_first(&outside_s) == 0) break;
+            cluster.sync();  // all have read it before it is cleared
+            if (first && tid == 0) limit_s = T2;
         }
-        if (m > FB_CAP || m < a.k) {
-            if (tid == 0) atomicExch(a.err + (m > FB_CAP ? DERR_TIE_OVERFLOW : DERR_CANDIDATES), 1);
-            __syncthreads();
-            continue;
+        if (first) {
+            if (m > FB_CAP || m < a.k) {
+                if (tid == 0) atomicExch(a.err + (m > FB_CAP ? DERR_TIE_OVERFLOW : DERR_CANDIDATES), 1);
+            } else {
+                finalize_row(team, a, q, keys, m, dbl, flags);
+            }
         }
-        finalize_row(team, a, q, keys, m, dbl, flags);
-        __syncthreads();
+        cluster.sync();  // the first block's shared memory is free for the next row
     }
+    cluster.sync();  // it stays until all have read the last row
 }
 
 // Distances of cosine rows' neighbours, one a thread: the f32 value that the
@@ -1077,7 +1112,7 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     uint32_t* fb_rows = (uint32_t*)ws_get(ctx, SLOT_FALLBACK_ROWS, sizeof(uint32_t) * (size_t)plan.nq, &e);
     if (!fb_rows) return e;
     float* fb_scratch =
-        (float*)ws_get(ctx, SLOT_FALLBACK_SCRATCH, sizeof(float) * (size_t)plan.nr * FB_BLOCKS, &e);
+        (float*)ws_get(ctx, SLOT_FALLBACK_SCRATCH, sizeof(float) * (size_t)plan.nr * FB_ROWS, &e);
     if (!fb_scratch) return e;
     RerankArgs a;
     a.qx = qx;
@@ -1177,7 +1212,7 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     const size_t smem_f = (size_t)FB_CAP * (sizeof(unsigned long long) + sizeof(double) + 1);
     e = set_smem_limit(ctx, (const void*)rerank_fallback_kernel, (int)smem_f);
     if (e != cudaSuccess) return e;
-    rerank_fallback_kernel<<<FB_BLOCKS, FB_THREADS, smem_f, ctx->stream>>>(a);
+    rerank_fallback_kernel<<<FB_ROWS * FB_CLUSTER, FB_THREADS, smem_f, ctx->stream>>>(a);
     ctx->launches += 1;
     if (a.post) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
