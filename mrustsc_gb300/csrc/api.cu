@@ -834,7 +834,11 @@ scrust_context* scrust_cuda_context_create(int32_t device, scrust_status* st) {
     ctx->sm_count = p.multiProcessorCount;
     ctx->smem_optin = p.sharedMemPerBlockOptin;
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
+    // (Above the main stream: what an ordered solve runs beside its nearest-anchor
+    // pass must not wait for that pass's persistent blocks.)
+    int least = 0, greatest = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&ctx->copy_stream, cudaStreamNonBlocking, greatest);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->copy_ev, cudaEventDisableTiming);
     for (int i = 0; i < kCsrRanges && e == cudaSuccess; i++)
         e = cudaEventCreateWithFlags(&ctx->csr_stream.merged[i], cudaEventDisableTiming);

@@ -90,19 +90,81 @@ __global__ void __launch_bounds__(256) anchor_dist_kernel(const float* __restric
 }
 
 // One warp per anchor: its kAnchorNeighbours nearest other anchors, nearest
-// first, ties to the smaller id; 0xffffffff past the last.  Each lane keeps a
-// sorted top-k of its columns, then the lanes' heads are merged.
+// first, ties to the smaller id; 0xffffffff past the last.  The largest of the
+// lanes' smallest distances has kAnchorNeighbours <= 32 at or below it, one of
+// each lane: the candidates, some hundred and thirty of 3,906, are collected
+// and sorted (a sorted top-32 in every lane, which some lane entered at almost
+// every step, took 150 us for 3,906 anchors; @@ us so).  More of them than
+// kTopCap (many anchors at one distance) go through such lists.
+constexpr int kTopCap = 256;
+static_assert(kAnchorNeighbours <= 32, "a bound from one distance a lane");
 __global__ void __launch_bounds__(128) anchor_top_kernel(const float* __restrict__ dist, int m,
                                                          uint32_t* __restrict__ nb) {
+    __shared__ unsigned long long found_s[4][kTopCap];
     const int lane = threadIdx.x & 31;
     const int64_t c = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (c >= m) return;
     constexpr int K = kAnchorNeighbours;
+    const uint32_t none = float_key(__int_as_float(0x7f800000));
+    const float* row = dist + c * m;
+    uint32_t least = 0xffffffffu;
+#pragma unroll 8
+    for (int j = lane; j < m; j += 32) least = min(least, float_key(row[j]));
+    const uint32_t bound = __reduce_max_sync(0xffffffffu, least);
+    unsigned long long* found = found_s[threadIdx.x >> 5];
+    int count = 0;
+#pragma unroll 4
+    for (int j0 = 0; j0 < m; j0 += 32) {
+        const uint32_t key = j0 + lane < m ? float_key(row[j0 + lane]) : 0xffffffffu;
+        const bool in = j0 + lane < m && key <= bound;
+        const uint32_t who = __ballot_sync(0xffffffffu, in);
+        const int at = count + __popc(who & lanemask_lt());
+        if (in && at < kTopCap) found[at] = ((unsigned long long)key << 32) | (uint32_t)(j0 + lane);
+        count += __popc(who);
+    }
+    __syncwarp();
+    if (count <= kTopCap) {
+        constexpr int R = kTopCap / 32;
+        unsigned long long key[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) key[r] = lane + 32 * r < count ? found[lane + 32 * r] : ~0ull;
+        // (Ascending bitonic sort, position lane + 32 r in key[r]; the halves
+        // past `count` hold nothing and are left out.)
+#pragma unroll
+        for (int size = 2; size <= kTopCap; size <<= 1) {
+            if (size > 32 && size / 2 >= count) break;
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                if (stride >= 32) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const int o = r ^ (stride / 32);
+                        if (o > r) {
+                            const bool up = ((32 * r) & size) == 0;
+                            const unsigned long long a = key[r], b = key[o];
+                            key[r] = (a < b) == up ? a : b;
+                            key[o] = (a < b) == up ? b : a;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const int i = lane + 32 * r;
+                        const unsigned long long o = __shfl_xor_sync(0xffffffffu, key[r], stride);
+                        const bool take_min = ((i & stride) == 0) == ((i & size) == 0);
+                        key[r] = (key[r] < o) == take_min ? key[r] : o;
+                    }
+                }
+            }
+        }
+        if (lane < K) nb[c * K + lane] = (uint32_t)(key[0] >> 32) < none ? (uint32_t)key[0] : 0xffffffffu;
+        return;
+    }
     unsigned long long top[K];
 #pragma unroll
     for (int r = 0; r < K; ++r) top[r] = ~0ull;
     for (int j = lane; j < m; j += 32) {
-        unsigned long long key = ((unsigned long long)float_key(dist[c * m + j]) << 32) | (uint32_t)j;
+        unsigned long long key = ((unsigned long long)float_key(row[j]) << 32) | (uint32_t)j;
         if (key < top[K - 1]) {
 #pragma unroll
             for (int r = 0; r < K; ++r) {
@@ -123,10 +185,7 @@ __global__ void __launch_bounds__(128) anchor_top_kernel(const float* __restrict
             for (int q = 0; q < K - 1; ++q) top[q] = top[q + 1];
             top[K - 1] = ~0ull;
         }
-        if (lane == 0) {
-            const bool found = (uint32_t)(best >> 32) < float_key(__int_as_float(0x7f800000));
-            nb[c * K + r] = found ? (uint32_t)best : 0xffffffffu;
-        }
+        if (lane == 0) nb[c * K + r] = (uint32_t)(best >> 32) < none ? (uint32_t)best : 0xffffffffu;
     }
 }
 
