@@ -461,26 +461,35 @@ __device__ uint32_t exact_move(const MoveArgs& a, uint32_t v, uint32_t own, bool
 // units, so sums and gains are bounded in f32 first.  A late round of 60,000
 // nodes of 46 entries (23 merged): 112 us (a warp per node, f64 gains at 128
 // places), 32 us (f64 gains, one thread per occupied place of a block), 22 us
-// (bounds in f32, places of a block), 17 us (four nodes a warp), 16 us here.
+// (bounds in f32, places of a block), 16 us (two nodes a warp), 11 us with
+// nodes of more than one chunk a warp each and first, and the larger ones of
+// up to kFusedTable / 2 entries in the same launch (5 us of their own before).
 constexpr int kMoveWarps = 4;
 constexpr int kMoveNodes = 2;
-__global__ void __launch_bounds__(32 * kMoveWarps) cl_move_small_kernel(MoveArgs a, const uint32_t* __restrict__ nodes,
-                                                                        int64_t count) {
+struct SmallTables {
+    uint32_t keys[kMoveWarps][kSmallTable];
+    long long vals[kMoveWarps][kSmallTable];
+    uint16_t slots[kMoveWarps][kSmallTable];
+    int count[kMoveWarps], over[kMoveWarps];
+};
+__device__ __forceinline__ void move_small_nodes(const MoveArgs& a, const uint32_t* __restrict__ nodes, int64_t count,
+                                                 const uint32_t* __restrict__ mids, int64_t mid_count, int64_t block,
+                                                 SmallTables& tab) {
     constexpr int T = kSmallTable, P = kMoveNodes;
-    __shared__ uint32_t keys[kMoveWarps][T];
-    __shared__ long long vals[kMoveWarps][T];
-    __shared__ uint16_t slots[kMoveWarps][T];
-    __shared__ int tab_count[kMoveWarps], tab_over[kMoveWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t i0 = ((int64_t)blockIdx.x * kMoveWarps + warp) * P;
-    if (i0 >= count) return;
-    const int here = (int)min((int64_t)P, count - i0);
+    // The first warps take a node of more than one chunk each, being the longest.
+    const int64_t g = block * kMoveWarps + warp;
+    const bool mid = g < mid_count;
+    const uint32_t* list = mid ? mids : nodes;
+    const int64_t i0 = mid ? g : (g - mid_count) * P;
+    if (!mid && i0 >= count) return;
+    const int here = mid ? 1 : (int)min((int64_t)P, count - i0);
     // Lane j holds node j.
     uint32_t my_v = 0, my_own = 0, my_p0 = 0, my_deg = 0;
     long long my_kf = 0, my_kown = 0;
     bool my_alone = false;
     if (lane < here) {
-        my_v = nodes[i0 + lane];
+        my_v = list[i0 + lane];
         my_own = a.comm[my_v];
         my_p0 = a.ptr[my_v];
         my_deg = a.ptr[my_v + 1] - my_p0;
@@ -539,8 +548,9 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_small_kernel(MoveArgs
         const uint32_t v = __shfl_sync(0xffffffffu, my_v, j), own = __shfl_sync(0xffffffffu, my_own, j);
         const uint32_t p0 = __shfl_sync(0xffffffffu, my_p0, j), deg = __shfl_sync(0xffffffffu, my_deg, j);
         const bool alone = __shfl_sync(0xffffffffu, my_alone, j);
-        const int found = gather_table<T>(a.nb, a.wint, p0, p0 + deg, v, a.comm, nullptr, 0u, keys[warp], vals[warp],
-                                          (long long*)nullptr, slots[warp], &tab_count[warp], &tab_over[warp]);
+        const int found = gather_table<T>(a.nb, a.wint, p0, p0 + deg, v, a.comm, nullptr, 0u, tab.keys[warp],
+                                          tab.vals[warp], (long long*)nullptr, tab.slots[warp], &tab.count[warp],
+                                          &tab.over[warp]);
         const long long k_own = __shfl_sync(0xffffffffu, my_kown, j);
         uint32_t to = kEmpty;
         if (deg > 32u) {
@@ -553,9 +563,9 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_small_kernel(MoveArgs
                 s2[i] = 0.0f;
                 k2[i] = 0;
                 if (lane + 32 * i < found) {
-                    const int t = slots[warp][lane + 32 * i];
-                    c2[i] = keys[warp][t];
-                    s2[i] = to_f32(vals[warp][t]);
+                    const int t = tab.slots[warp][lane + 32 * i];
+                    c2[i] = tab.keys[warp][t];
+                    s2[i] = to_f32(tab.vals[warp][t]);
                 }
                 const uint32_t home = __ballot_sync(0xffffffffu, c2[i] == own);
                 if (home) e2 = __shfl_sync(0xffffffffu, s2[i], __ffs(home) - 1);
@@ -565,8 +575,8 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_small_kernel(MoveArgs
             to = bounded_move<2>(own, __shfl_sync(0xffffffffu, my_f, j), c2, s2, k2, e2, k_own);
         }
         if (to == kEmpty)
-            to = exact_move<T>(a, v, own, alone, __shfl_sync(0xffffffffu, my_kf, j), k_own, keys[warp], vals[warp],
-                               slots[warp], found);
+            to = exact_move<T>(a, v, own, alone, __shfl_sync(0xffffffffu, my_kf, j), k_own, tab.keys[warp], tab.vals[warp],
+                               tab.slots[warp], found);
         if (lane == j) my_to = to;
         __syncwarp();
     }
@@ -584,19 +594,25 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_small_kernel(MoveArgs
 // The same for nodes of more entries, a block per node: the warps add their
 // chunks to one table by atomics, of twice the node's entries up to kBigTable
 // places (a warp per node, clearing and testing 2,048 places: 59 us a round).
-__global__ void __launch_bounds__(32 * kMoveWarps) cl_move_big_kernel(MoveArgs a, const uint32_t* __restrict__ nodes) {
-    constexpr int T = kBigTable, N = 32 * kMoveWarps;
-    __shared__ uint32_t keys[T];
-    __shared__ unsigned long long vals[T];
-    __shared__ float high[T];
-    __shared__ uint16_t slots[T], cand[T];
-    __shared__ int found_s, over_s, cand_s;
-    __shared__ uint32_t low;
-    __shared__ unsigned long long best, own_val;
-    __shared__ uint32_t best_c;
-    __shared__ double stay;
+template <int T>
+struct BigTable {
+    uint32_t keys[T];
+    unsigned long long vals[T];
+    float high[T];
+    uint16_t slots[T], cand[T];
+    int found, over, cands;
+    uint32_t low, best_c;
+    unsigned long long best, own_val;
+    double stay;
+};
+template <int T>
+__device__ __forceinline__ void move_big_node(const MoveArgs& a, uint32_t v, BigTable<T>& tab) {
+    constexpr int N = 32 * kMoveWarps;
+    uint32_t* keys = tab.keys;
+    unsigned long long* vals = tab.vals;
+    float* high = tab.high;
+    uint16_t *slots = tab.slots, *cand = tab.cand;
     const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t v = nodes[blockIdx.x];
     const uint32_t own = a.comm[v];
     const uint32_t p0 = a.ptr[v], p1 = a.ptr[v + 1];
     const long long kf = a.kfix[v];
@@ -608,14 +624,14 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_big_kernel(MoveArgs a
         vals[t] = 0ull;
     }
     if (tid == 0) {
-        found_s = 0;
-        over_s = 0;
-        cand_s = 0;
-        low = 0u;
-        best = 0ull;
-        own_val = 0ull;
-        best_c = kEmpty;
-        stay = -INFINITY;
+        tab.found = 0;
+        tab.over = 0;
+        tab.cands = 0;
+        tab.low = 0u;
+        tab.best = 0ull;
+        tab.own_val = 0ull;
+        tab.best_c = kEmpty;
+        tab.stay = -INFINITY;
     }
     __syncthreads();
     for (uint32_t base = p0 + (uint32_t)(tid - lane); base < p1; base += N) {
@@ -637,50 +653,50 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_big_kernel(MoveArgs a
             for (uint32_t probe = 0; probe <= mask; ++probe) {
                 const uint32_t prev = atomicCAS(keys + slot, kEmpty, c);
                 if (prev == kEmpty || prev == c) {
-                    if (prev == kEmpty) slots[atomicAdd(&found_s, 1)] = (uint16_t)slot;
+                    if (prev == kEmpty) slots[atomicAdd(&tab.found, 1)] = (uint16_t)slot;
                     atomicAdd(&vals[slot], (unsigned long long)s);
                     placed = true;
                     break;
                 }
                 slot = (slot + 1) & mask;
             }
-            if (!placed) over_s = 1;
+            if (!placed) tab.over = 1;
         }
         __syncwarp();
     }
     __syncthreads();
-    if (over_s) return;
-    const int found = found_s;
+    if (tab.over) return;
+    const int found = tab.found;
     const bool alone = a.size[own] == 1;
     for (int i = tid; i < found; i += N) {
         const int s = slots[i];
         const uint32_t c = keys[s];
         high[s] = -INFINITY;
         if (c == own) {
-            own_val = vals[s];
+            tab.own_val = vals[s];
             keys[s] = kEmpty;
         } else if (alone && c > own && a.size[c] == 1) {
             keys[s] = kEmpty;
         } else {
             float lo;
             gain_bounds(to_f32((long long)vals[s]), a.K[c], factor, &lo, &high[s]);
-            if (lo == lo) atomicMax(&low, order_key(lo));
+            if (lo == lo) atomicMax(&tab.low, order_key(lo));
         }
     }
     __syncthreads();
     // The node's own community, adjacent or not.
     const long long k_own = a.K[own] - kf;
     float own_low, own_high;
-    gain_bounds(to_f32((long long)own_val), k_own, factor, &own_low, &own_high);
-    if (tid == 0 && own_low == own_low) atomicMax(&low, order_key(own_low));
+    gain_bounds(to_f32((long long)tab.own_val), k_own, factor, &own_low, &own_high);
+    if (tid == 0 && own_low == own_low) atomicMax(&tab.low, order_key(own_low));
     __syncthreads();
-    const float least = key_order(low);
+    const float least = key_order(tab.low);
     for (int i = tid; i < found; i += N) {
         const int s = slots[i];
-        if (keys[s] != kEmpty && !(high[s] < least)) cand[atomicAdd(&cand_s, 1)] = (uint16_t)s;
+        if (keys[s] != kEmpty && !(high[s] < least)) cand[atomicAdd(&tab.cands, 1)] = (uint16_t)s;
     }
     __syncthreads();
-    const int cands = cand_s;
+    const int cands = tab.cands;
     const bool stays = !(own_high < least);
     if (cands + (stays ? 1 : 0) == 1 && least > 0.0f) {
         if (tid == 0 && !stays) record_move(a, v, own, keys[cand[0]]);
@@ -691,21 +707,41 @@ __global__ void __launch_bounds__(32 * kMoveWarps) cl_move_big_kernel(MoveArgs a
         if (!t && !stays) continue;
         const int s = t ? cand[t - 1] : 0;
         const double g = t ? move_gain(a, (double)(long long)vals[s] * a.unit, a.K[keys[s]], kv)
-                           : move_gain(a, (double)(long long)own_val * a.unit, k_own, kv);
+                           : move_gain(a, (double)(long long)tab.own_val * a.unit, k_own, kv);
         if (!t) {
-            stay = g;
+            tab.stay = g;
         } else if (g == g) {
             vals[s] = order_key(g);
-            atomicMax(&best, vals[s]);
+            atomicMax(&tab.best, vals[s]);
         } else {
             keys[s] = kEmpty;
         }
     }
     __syncthreads();
     for (int t = tid; t < cands; t += N)
-        if (keys[cand[t]] != kEmpty && vals[cand[t]] == best) atomicMin(&best_c, keys[cand[t]]);
+        if (keys[cand[t]] != kEmpty && vals[cand[t]] == tab.best) atomicMin(&tab.best_c, keys[cand[t]]);
     __syncthreads();
-    if (tid == 0) record_move(a, v, own, destination(a, v, own, key_order(best), best_c, stay));
+    if (tid == 0) record_move(a, v, own, destination(a, v, own, key_order(tab.best), tab.best_c, tab.stay));
+}
+
+constexpr int kFusedTable = 512;  // nodes of at most half as many entries share a launch with the small ones
+__global__ void __launch_bounds__(32 * kMoveWarps) cl_move_kernel_all(MoveArgs a, const uint32_t* __restrict__ bigs,
+                                                                      int64_t big_count,
+                                                                      const uint32_t* __restrict__ nodes, int64_t count,
+                                                                      const uint32_t* __restrict__ mids,
+                                                                      int64_t mid_count) {
+    __shared__ union {
+        SmallTables small;
+        BigTable<kFusedTable> big;
+    } tab;
+    if ((int64_t)blockIdx.x < big_count)
+        move_big_node(a, bigs[blockIdx.x], tab.big);
+    else
+        move_small_nodes(a, nodes, count, mids, mid_count, (int64_t)blockIdx.x - big_count, tab.small);
+}
+__global__ void __launch_bounds__(32 * kMoveWarps) cl_move_big_kernel(MoveArgs a, const uint32_t* __restrict__ nodes) {
+    __shared__ BigTable<kBigTable> tab;
+    move_big_node(a, nodes[blockIdx.x], tab);
 }
 
 // Local moving, one round, one warp per node, f64 weights whose sums round:
@@ -1031,22 +1067,25 @@ __global__ void cl_rank_kernel(const unsigned long long* __restrict__ order, int
 }
 
 // The nodes by degree and by the half of the rounds they are active in
-// (active_in): small nodes of even and odd rounds from the two ends of
-// `small`, the rest from the two ends of `big`.
-__global__ void cl_node_lists_kernel(const uint32_t* __restrict__ ptr, int64_t n, uint64_t salt,
-                                     uint32_t* __restrict__ small, uint32_t* __restrict__ big,
-                                     unsigned int* __restrict__ counts) {
+// (active_in): nodes of at most `chunk` entries of even and odd rounds from
+// the two ends of `small`, those of up to kSmallDegree from the ends of `mid`,
+// the rest from the ends of `big`.
+__global__ void cl_node_lists_kernel(const uint32_t* __restrict__ ptr, int64_t n, uint64_t salt, uint32_t chunk,
+                                     uint32_t* __restrict__ small, uint32_t* __restrict__ mid,
+                                     uint32_t* __restrict__ big, unsigned int* __restrict__ counts) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const int kind = v >= n ? 4
-                            : (ptr[v + 1] - ptr[v] <= (uint32_t)kSmallDegree ? 0 : 2) +
+    const uint32_t degree = v < n ? ptr[v + 1] - ptr[v] : 0u;
+    const int kind = v >= n ? 6
+                            : (degree <= chunk ? 0 : degree <= (uint32_t)kSmallDegree ? 2 : 4) +
                                   (active_in((uint32_t)v, 0, salt) ? 0 : 1);
     const uint32_t peers = __match_any_sync(0xffffffffu, kind);
     unsigned int at = 0;
-    if (kind < 4 && (__ffs(peers) - 1) == lane) at = atomicAdd(counts + kind, (unsigned int)__popc(peers));
+    if (kind < 6 && (__ffs(peers) - 1) == lane) at = atomicAdd(counts + kind, (unsigned int)__popc(peers));
     at = __shfl_sync(0xffffffffu, at, __ffs(peers) - 1) + __popc(peers & ((1u << lane) - 1u));
-    if (kind >= 4) return;
-    uint32_t* list = kind < 2 ? small : big;
+    if (kind >= 6) return;
+    if (kind >= 4) atomicMax(counts + 8, degree);
+    uint32_t* list = kind < 2 ? small : kind < 4 ? mid : big;
     list[(kind & 1) ? n - 1 - (int64_t)at : (int64_t)at] = (uint32_t)v;
 }
 
@@ -1145,7 +1184,7 @@ private:
     cudaError_t sort_pairs(uint32_t* kA, unsigned long long* vA, uint32_t* kB, unsigned long long* vB, int64_t m,
                            int bits, uint32_t** kout, unsigned long long** vout);
     int64_t compact(const uint32_t* labels, int64_t n, int64_t width, uint32_t* out);
-    int32_t node_lists(const Level& L, uint64_t salt);
+    int32_t node_lists(const Level& L, uint64_t salt, uint32_t chunk);
     int32_t integer_weights(Level* L, bool merged);
     int32_t local_moving(const Level& L, uint32_t* comm, long long* K, int* size, double res, bool* moved_any);
     int32_t refine(const Level& L, const uint32_t* part, const long long* K, double res, uint64_t salt,
@@ -1162,16 +1201,17 @@ private:
     size_t block_ = 0, used_ = 0;  // the next free byte of the context's blocks
     Level g0_;
     double total_ = 0.0, scale_ = 1.0, inv_scale_ = 1.0;
-    unsigned int* counter_ = nullptr;  // 4 list counts, 2 exponents, the moves of each round, labels changed
+    unsigned int* counter_ = nullptr;  // 6 list counts, 2 exponents, the largest degree of a big node, the moves of each round, labels changed
     // Node lists of the current level (cl_node_lists_kernel) and their counts.
     uint32_t* small_ = nullptr;
+    uint32_t* mid_ = nullptr;
     uint32_t* big_ = nullptr;
-    unsigned int counts_[4] = {0, 0, 0, 0};
-    // The list of small (0) or other (1) nodes active in `round`, and its length.
+    unsigned int counts_[9] = {};
+    // The list of small (0), mid (1) or big (2) nodes active in `round`, and its length.
     const uint32_t* active(const Level& L, int kind, int round, int64_t* count) const {
         const int odd = round & 1;
         *count = counts_[2 * kind + odd];
-        const uint32_t* list = kind ? big_ : small_;
+        const uint32_t* list = kind == 2 ? big_ : kind ? mid_ : small_;
         return odd ? list + (L.n - *count) : list;
     }
 };
@@ -1181,7 +1221,7 @@ private:
 // the rounds past the last do nothing; a look after every round left the GPU
 // idle for as long as a round took.
 constexpr int kRoundBatch = 8;
-constexpr int kCounterMoves = 6;
+constexpr int kCounterMoves = 9;
 static_assert(kMaxRounds % kRoundBatch == 0, "whole batches");
 
 cudaError_t Clusterer::sort_pairs(uint32_t* kA, unsigned long long* vA, uint32_t* kB, unsigned long long* vB,
@@ -1267,14 +1307,15 @@ int32_t Clusterer::build(const uint32_t* indptr, const uint32_t* indices, const 
     return ok(st_);
 }
 
-int32_t Clusterer::node_lists(const Level& L, uint64_t salt) {
+int32_t Clusterer::node_lists(const Level& L, uint64_t salt, uint32_t chunk) {
     small_ = alloc<uint32_t>(L.n);
+    mid_ = alloc<uint32_t>(L.n);
     big_ = alloc<uint32_t>(L.n);
     if (!ok_) return oom();
-    cudaMemsetAsync(counter_, 0, 4 * sizeof(unsigned int), s_);
-    cl_node_lists_kernel<<<grid_for(L.n), 256, 0, s_>>>(L.mptr, L.n, salt, small_, big_, counter_);
+    cudaMemsetAsync(counter_, 0, 9 * sizeof(unsigned int), s_);
+    cl_node_lists_kernel<<<grid_for(L.n), 256, 0, s_>>>(L.mptr, L.n, salt, chunk, small_, mid_, big_, counter_);
     ctx_->launches += 1;
-    if (!download(counts_, counter_, 4)) return fail(st_, SCRUST_KERNEL, "clustering: node lists");
+    if (!download(counts_, counter_, 9)) return fail(st_, SCRUST_KERNEL, "clustering: node lists");
     return ok(st_);
 }
 
@@ -1287,11 +1328,11 @@ int32_t Clusterer::integer_weights(Level* L, bool merged) {
     L->mnb = L->nb;
     L->wint = nullptr;
     int exps[2] = {2000, -2000};
-    cudaMemcpyAsync(counter_ + 4, exps, sizeof(exps), cudaMemcpyHostToDevice, s_);
+    cudaMemcpyAsync(counter_ + 6, exps, sizeof(exps), cudaMemcpyHostToDevice, s_);
     cl_exponents_kernel<<<(unsigned)std::min<int64_t>(4 * ctx_->sm_count, grid_for(L->m)), 256, 0, s_>>>(
-        L->w, L->m, L->k, L->n, (int*)(counter_ + 4));
+        L->w, L->m, L->k, L->n, (int*)(counter_ + 6));
     ctx_->launches += 1;
-    if (!download(exps, (const int*)(counter_ + 4), 2)) return fail(st_, SCRUST_KERNEL, "clustering: weights");
+    if (!download(exps, (const int*)(counter_ + 6), 2)) return fail(st_, SCRUST_KERNEL, "clustering: weights");
     // (|shift| <= 1000 keeps 2^-shift an f64; a strength rounds up to at most
     // the next power of two.)
     if (exps[0] >= 2000 || exps[1] + 1 - exps[0] > 53 || exps[0] < -1000 || exps[0] > 900) return ok(st_);
@@ -1345,13 +1386,19 @@ int32_t Clusterer::local_moving(const Level& L, uint32_t* comm, long long* K, in
     for (int r0 = 0; r0 < end && quiet < 2; r0 += kRoundBatch) {
         for (int round = r0; round < r0 + kRoundBatch; ++round) {
             a.moves = counter_ + kCounterMoves + round;
-            int64_t ns = 0, nb = 0;
+            int64_t ns = 0, nm = 0, nb = 0;
             const uint32_t* small = active(L, 0, round, &ns);
-            const uint32_t* big = active(L, 1, round, &nb);
-            if (ns && L.wint)
-                cl_move_small_kernel<<<(unsigned)((ns + kMoveNodes * kMoveWarps - 1) / (kMoveNodes * kMoveWarps)),
-                                       32 * kMoveWarps, 0, s_>>>(a, small, ns);
-            else if (ns)
+            const uint32_t* mid = active(L, 1, round, &nm);
+            const uint32_t* big = active(L, 2, round, &nb);
+            if (L.wint && ns + nm + nb) {
+                const bool fused = counts_[8] <= kFusedTable / 2;
+                const int64_t warps = nm + (ns + kMoveNodes - 1) / kMoveNodes, with = fused ? nb : 0;
+                const int64_t blocks = with + (warps + kMoveWarps - 1) / kMoveWarps;
+                if (blocks)
+                    cl_move_kernel_all<<<(unsigned)blocks, 32 * kMoveWarps, 0, s_>>>(a, big, with, small, ns, mid, nm);
+                nb -= with;
+            }
+            if (ns && !L.wint)
                 cl_move_kernel<kSmallTable, kSmallWarps>
                     <<<(unsigned)((ns + kSmallWarps - 1) / kSmallWarps), 32 * kSmallWarps, 0, s_>>>(a, small, ns);
             if (nb && L.wint)
@@ -1406,7 +1453,7 @@ int32_t Clusterer::refine(const Level& L, const uint32_t* part, const long long*
     uint32_t* moved = alloc<uint32_t>(n);
     uint32_t* to = alloc<uint32_t>(n);
     if (!ok_) return oom();
-    int32_t rc = node_lists(L, salt);
+    int32_t rc = node_lists(L, salt, kSmallDegree);
     if (rc) return rc;
     const unsigned nb = grid_for(n);
     cl_to_subset_kernel<<<nb, 256, 0, s_>>>(L.ptr, L.nb, L.w, L.k, n, part, K, inv_scale_, res, total_, to_subset,
@@ -1430,7 +1477,7 @@ int32_t Clusterer::refine(const Level& L, const uint32_t* part, const long long*
                 cl_cut_kernel<<<nb, 256, 0, s_>>>(L.ptr, L.nb, L.w, n, sub, to_subset, scale_, cut);
             for (int kind = 0; kind < 2; ++kind) {
                 int64_t count = 0;
-                const uint32_t* nodes = active(L, kind, round, &count);
+                const uint32_t* nodes = active(L, 2 * kind, round, &count);
                 if (!count) continue;
                 const unsigned grid = kind ? (unsigned)count : (unsigned)((count + kSmallWarps - 1) / kSmallWarps);
                 auto go = [&](auto kernel, auto* w, double u) {
@@ -1559,7 +1606,7 @@ int32_t Clusterer::optimise(const uint32_t* initial, double res, bool leiden, ui
         const uint64_t level_salt = mix_host(salt ^ ((uint64_t)depth * 0xD1B54A32D192ED03ull));
         int32_t rc = SCRUST_OK;
         if (depth && (rc = integer_weights(&level, true))) return rc;
-        if ((rc = node_lists(level, level_salt))) return rc;
+        if ((rc = node_lists(level, level_salt, level.wint ? 32 : kSmallDegree))) return rc;
         bool moved = false;
         if ((rc = local_moving(level, labels, K, size, res, &moved))) return rc;
         const int64_t nc = compact(labels, n, 2 * n, partition);
