@@ -1159,8 +1159,8 @@ int32_t scrust_cuda_phase_times(scrust_context* ctx, float* ms, int32_t max_phas
         ms[written++] = t;
     }
     // Inside the candidates phase of an ordered solve: the first sweep pass,
-    // the building of the second pass's tile lists, the second pass, and the
-    // first collect pass (k <= 32).
+    // the building of the collect pass's second tile lists, a place where no
+    // pass is run, and the collect pass.
     const int sub[4][2] = {{PH_PREP, PH_PASS1}, {PH_PASS1, PH_LISTS}, {PH_LISTS, PH_PASS2}, {PH_PASS2, PH_COLLECT1}};
     for (int i = 0; i < 4 && written < max_phases; ++i) {
         float t = 0.f;

@@ -917,8 +917,6 @@ __global__ void narrow_kernel(const unsigned long long* __restrict__ vals, int i
     if (i < items) out[i] = (uint32_t)vals[i];
 }
 
-// One thread per 4-float group of an output row (stride is a multiple of 4
-// for the padded layout; otherwise one float per thread).
 // Segment centres transposed to [64][segs], so that threads reading one
 // dimension of consecutive segments read consecutive words.
 __global__ void transpose_centres_kernel(const float* __restrict__ fc, int64_t segs, float* __restrict__ out) {
