@@ -384,6 +384,88 @@ __global__ void unpack_perm_kernel(const uint32_t* __restrict__ skeys, const uns
         for (uint32_t c = key + 1u; c <= m; ++c) cell_start[c] = (uint32_t)n;
 }
 
+// anchor_rank_kernel, the stable sort by rank and unpack_perm_kernel by one
+// block, for up to kRowsOneBlock rows: rank and row in one word, 7-bit radix
+// passes in shared memory, a warp on R groups of 32 consecutive rows.  (Five
+// launches for ranks below 256, eight above, of 1.3 to 6 us and as many gaps
+// of 2: 27 us at 2,638 rows, 35 at one query; the chain of dependent steps,
+// not the data, is the time here.)
+constexpr int kRowsOneBlock = 8192;
+constexpr int kRowBits = 13;
+static_assert(kRowsOneBlock <= 1 << kRowBits && kMaxAnchors <= 1 << kRowBits, "rank and row in one word");
+template <int R>
+__global__ void __launch_bounds__(1024) order_rows_kernel(const uint32_t* __restrict__ anchor, int n,
+                                                          const uint32_t* __restrict__ rank, int bits, uint32_t m,
+                                                          uint32_t* __restrict__ perm,
+                                                          uint32_t* __restrict__ cell_of_pos,
+                                                          uint32_t* __restrict__ cell_start) {
+    __shared__ uint32_t words[R * 1024];
+    __shared__ uint16_t cnt[32][130];  // per warp and digit; the odd number of words spreads a digit's warps over the banks
+    __shared__ uint32_t wsum[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, base = warp * R * 32 + lane;
+    uint32_t key[R], at[R];
+    // Places past the rows hold the largest word and come last in every pass.
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = base + r * 32;
+        key[r] = i < n ? rank[anchor[i]] << kRowBits | (uint32_t)i : 0xffffffffu;
+    }
+    for (int shift = kRowBits; shift < kRowBits + bits; shift += 7) {
+        for (int d = lane; d < 128; d += 32) cnt[warp][d] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint32_t d = key[r] >> shift & 127u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d), before = cnt[warp][d];
+            at[r] = before + __popc(peers & lanemask_lt());
+            __syncwarp();
+            if (__ffs(peers) - 1 == lane) cnt[warp][d] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        // First places by digit, then warp: four warps' counts of a digit a thread.
+        const int d = threadIdx.x >> 3, w0 = (threadIdx.x & 7) * 4;
+        uint32_t c[4], sum = 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            c[j] = cnt[w0 + j][d];
+            sum += c[j];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        uint32_t first = incl - sum + __reduce_add_sync(0xffffffffu, lane < warp ? wsum[lane] : 0u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            cnt[w0 + j][d] = (uint16_t)first;
+            first += c[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) words[cnt[warp][key[r] >> shift & 127u] + at[r]] = key[r];
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) key[r] = words[base + r * 32];
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int s = base + r * 32;
+        if (s >= n) continue;
+        const uint32_t cell = key[r] >> kRowBits;
+        perm[s] = key[r] & ((1u << kRowBits) - 1u);
+        cell_of_pos[s] = cell;
+        if (!cell_start) continue;
+        for (uint32_t c = s ? (words[s - 1] >> kRowBits) + 1u : 0u; c <= cell && c <= m; ++c) cell_start[c] = (uint32_t)s;
+        if (s == n - 1)
+            for (uint32_t c = cell + 1u; c <= m; ++c) cell_start[c] = (uint32_t)n;
+    }
+}
+
 // One warp per 256-row work item: the column tiles holding the item's own
 // cells, then those holding the cells of their nearest anchors, nearest
 // anchors first; distinct, at most kPrioMax.  In a self solve the item's own
@@ -1208,6 +1290,37 @@ void launch_nearest_anchor(bool bf16, const unsigned long long* best, int64_t n,
     }
 }
 
+// The rows in the order of their anchors' walk ranks (stable): kA holds the
+// anchors and vA the rows, both overwritten; hist and scan as the radix sort
+// wants them.  cell_start (m + 1 places) may be null.
+cudaError_t order_rows(scrust_context* ctx, uint32_t* kA, unsigned long long* vA, uint32_t* kB, unsigned long long* vB,
+                       int64_t n, const uint32_t* rank, int64_t m, uint32_t* hist, uint32_t* scan, size_t scan_elems,
+                       uint32_t* perm, uint32_t* cell_of_pos, uint32_t* cell_start) {
+    cudaStream_t s = ctx->stream;
+    int bits = 1;
+    while (((int64_t)1 << bits) < m) bits++;
+    if (n <= kRowsOneBlock) {
+        const auto kern = n <= 1024   ? order_rows_kernel<1>
+                          : n <= 2048 ? order_rows_kernel<2>
+                          : n <= 4096 ? order_rows_kernel<4>
+                                      : order_rows_kernel<8>;
+        kern<<<1, 1024, 0, s>>>(kA, (int)n, rank, bits, (uint32_t)m, perm, cell_of_pos, cell_start);
+        ctx->launches += 1;
+        return cudaGetLastError();
+    }
+    anchor_rank_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(kA, n, rank);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    uint32_t* skeys = nullptr;
+    unsigned long long* svals = nullptr;
+    if ((e = radix_sort_pairs(ctx, kA, vA, kB, vB, n, bits, hist, scan, scan_elems, &skeys, &svals)) != cudaSuccess)
+        return e;
+    unpack_perm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(skeys, svals, n, (uint32_t)m, perm, cell_of_pos,
+                                                                   cell_start);
+    ctx->launches += 2;
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 // Row blocks sorted by decreasing count into `order`; scratch holds
@@ -1387,27 +1500,18 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     // The walk ranks (copy stream) are needed from here on.
     if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamWaitEvent(s, ctx->copy_ev, 0)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: nearest anchor");
-    anchor_rank_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(keysA, n, rank);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: nearest anchor");
-    ctx->launches += 3;
+    ctx->launches += 2;
 
     // Stable sort of the rows by anchor: the permutation and the cells.
-    int bits = 1;
-    while (((int64_t)1 << bits) < m) bits++;
-    uint32_t* skeys = nullptr;
-    unsigned long long* svals = nullptr;
-    if ((e = radix_sort_pairs(ctx, keysA, valsA, keysB, valsB, n, bits, (uint32_t*)(base + o_hist),
-                              (uint32_t*)(base + o_scan), scan_elems, &skeys, &svals)) != cudaSuccess)
+    if ((e = order_rows(ctx, keysA, valsA, keysB, valsB, n, rank, m, (uint32_t*)(base + o_hist),
+                        (uint32_t*)(base + o_scan), scan_elems, perm, cell_of_pos, cell_start)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: sort");
-    unpack_perm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(skeys, svals, n, (uint32_t)m, perm, cell_of_pos,
-                                                                   cell_start);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: permutation");
 
     // The priority tiles of every work item.
     prio_tiles_kernel<<<(unsigned)((items + 3) / 4), 128, 0, s>>>(cell_of_pos, n, cell_start, (int)m, cell_nb,
                                                                   kAnchorNeighbours, items, items, prio, prio_cnt);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "ordering: priority tiles");
-    ctx->launches += 2;
+    ctx->launches += 1;
     if ((e = sort_by_work(ctx, prio_cnt, items, base + o_ws, (uint32_t*)(base + o_po))) != cudaSuccess)
         return cuda_fail(st, e, "ordering: work order");
     // The operands and bounds in list order.
@@ -1722,21 +1826,14 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     const int op_words = (d + 3 + 7) / 8;  // 16-byte words of an operand row holding values
     launch_nearest_anchor(bf16, best, q, at.anchors, base + o_A0, at.anchor_B16, 1, op_words, (uint32_t*)(base + o_kA),
                           (unsigned long long*)(base + o_vA), s);
-    anchor_rank_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>((uint32_t*)(base + o_kA), q, at.anchor_rank);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: nearest anchor");
-    ctx->launches += 4;
+    ctx->launches += 3;
     // The queries sorted by the walk place of their cell; their operands,
     // bounds and rows in that order.
-    int bits = 1;
-    while (((int64_t)1 << bits) < at.anchors) bits++;
-    uint32_t* skeys = nullptr;
-    unsigned long long* svals = nullptr;
-    if ((e = radix_sort_pairs(ctx, (uint32_t*)(base + o_kA), (unsigned long long*)(base + o_vA),
-                              (uint32_t*)(base + o_kB), (unsigned long long*)(base + o_vB), q, bits,
-                              (uint32_t*)(base + o_hist), (uint32_t*)(base + o_scan), scan_elems, &skeys, &svals)) !=
-            cudaSuccess)
+    if ((e = order_rows(ctx, (uint32_t*)(base + o_kA), (unsigned long long*)(base + o_vA), (uint32_t*)(base + o_kB),
+                        (unsigned long long*)(base + o_vB), q, at.anchor_rank, at.anchors, (uint32_t*)(base + o_hist),
+                        (uint32_t*)(base + o_scan), scan_elems, qperm, cell_of_pos, nullptr)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: sort");
-    unpack_perm_kernel<<<(unsigned)((q + 255) / 256), 256, 0, s>>>(skeys, svals, q, 0u, qperm, cell_of_pos, nullptr);
     gather_operands_kernel<1><<<(unsigned)((q_pad * 8 + 255) / 256), 256, 0, s>>>(
         (const uint4*)(base + o_A0), (const uint4*)(base + o_B0), bA0, eps0, qperm, q, q_pad, (uint4*)(base + o_As),
         (uint4*)(base + o_Bs), bA, beps, words + 1, words + 2, bdelta, beps2);
@@ -1754,7 +1851,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: priority tiles");
     if ((e = sort_by_work(ctx, (uint32_t*)(base + o_psc), work, base + o_ws, (uint32_t*)(base + o_po))) != cudaSuccess)
         return cuda_fail(st, e, "query routing: work order");
-    ctx->launches += 7;
+    ctx->launches += 5;
 
     // The threshold pass over the priority tiles.
     KnnPlan plan;
