@@ -1578,31 +1578,49 @@ cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n
     return cudaGetLastError();
 }
 
-// A warp per row, a lane per list: the lists' top-K in shared memory, k rounds
-// of the smallest head.  A list of a row with a shared threshold holds every
+// A warp per row, a lane on L lists (rows with more than 32 lists take 4): the
+// lists' top-K in shared memory, k rounds of the smallest head.  A list of a row with a shared threshold holds every
 // value of its columns below that threshold (or its K smallest), so the k-th
 // of the lists together bounds the row wherever it exists.
-template <int K>
-__global__ void __launch_bounds__(256)
+template <int K, int L>
+__global__ void __launch_bounds__(256 / L)
     merge_segment_thresholds_kernel(const float* __restrict__ topk, int64_t stride, int64_t n, int k, int lists,
                                     const uint32_t* __restrict__ counts, const float* __restrict__ bA,
                                     const float* __restrict__ bdelta, const float* __restrict__ beps2,
                                     uint32_t* __restrict__ row_theta) {
-    __shared__ float vals[8][32][K + 1];
+    constexpr int W = 8 / L;
+    __shared__ float vals[W][32 * L][K + 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t i = (int64_t)blockIdx.x * 8 + w;
+    const int64_t i = (int64_t)blockIdx.x * W + w;
     if (i >= n) return;
     const float inf = __int_as_float(0x7f800000);
-    const bool written = lane < lists && counts[i / ROWS * (lists / PARTS) + lane / PARTS] != 0u;
-    // (The first K - k slots are -inf.)
-    for (int t = 0; t < k; ++t) vals[w][lane][t] = written ? topk[(int64_t)(K - k + t) * stride + i * lists + lane] : inf;
-    int at = 0;
+    int at[L];
+#pragma unroll
+    for (int j = 0; j < L; ++j) {
+        const int l = lane + 32 * j;
+        const bool written = l < lists && counts[i / ROWS * (lists / PARTS) + l / PARTS] != 0u;
+        // (The first K - k slots are -inf.)
+        for (int t = 0; t < k; ++t) vals[w][l][t] = written ? topk[(int64_t)(K - k + t) * stride + i * lists + l] : inf;
+        vals[w][l][k] = inf;
+        at[j] = 0;
+    }
     uint32_t kth = 0;
     for (int t = 0; t < k; ++t) {
-        const uint32_t head = float_key(at < k ? vals[w][lane][at] : inf);
+        float own = vals[w][lane][at[0]];
+        int mine = 0;
+#pragma unroll
+        for (int j = 1; j < L; ++j) {
+            const float v = vals[w][lane + 32 * j][at[j]];
+            mine = v < own ? j : mine;
+            own = fminf(own, v);
+        }
+        const uint32_t head = float_key(own);
         kth = __reduce_min_sync(0xffffffffu, head);
         const uint32_t who = __ballot_sync(0xffffffffu, head == kth);
-        if (lane == __ffs(who) - 1) ++at;
+        if (lane == __ffs(who) - 1) {
+#pragma unroll
+            for (int j = 0; j < L; ++j) at[j] += j == mine && at[j] < k ? 1 : 0;
+        }
     }
     if (lane == 0) {
         const float th = TensorBound{bA[i], bdelta[i], beps2[i]}.theta_f32(key_float(kth));
@@ -1613,10 +1631,13 @@ __global__ void __launch_bounds__(256)
 cudaError_t launch_merge_segment_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
                                             const uint32_t* counts, const float* bA, const float* bdelta,
                                             const float* beps2, uint32_t* row_theta, cudaStream_t s) {
-    if (k < 2 || k > width || (width != 16 && width != 32) || segments > 32 || segments % PARTS)
+    if (k < 2 || k > width || (width != 16 && width != 32) || segments > 128 || segments % PARTS)
         return cudaErrorInvalidValue;
-    const auto kern = width == 16 ? merge_segment_thresholds_kernel<16> : merge_segment_thresholds_kernel<32>;
-    kern<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(topk, n_pad * segments, n, k, segments, counts, bA, bdelta, beps2,
+    const int lanes = segments > 32 ? 4 : 1;
+    const auto kern = width == 16 ? (lanes == 1 ? merge_segment_thresholds_kernel<16, 1> : merge_segment_thresholds_kernel<16, 4>)
+                                  : (lanes == 1 ? merge_segment_thresholds_kernel<32, 1> : merge_segment_thresholds_kernel<32, 4>);
+    const int rows = 8 / lanes;
+    kern<<<(unsigned)((n + rows - 1) / rows), 32 * rows, 0, s>>>(topk, n_pad * segments, n, k, segments, counts, bA, bdelta, beps2,
                                                  row_theta);
     return cudaGetLastError();
 }

@@ -1133,6 +1133,10 @@ __device__ __forceinline__ int block_prefix(int v, int* wsum, int* total) {
 constexpr int kQueryPrio = 512;
 constexpr int kQueryPrioNear = 256;
 constexpr int kQueryPrioNb = 8;
+// Column segments of a row block at most, so 128 lists of a row.  (With 16, few
+// queries left most of the chip idle: 30, 300 and 1,000 of a million cells took
+// 427, 1,220 and 855 us, and 334, 609 and 634 us with 64.)
+constexpr int kQuerySegments = 64;
 __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restrict__ cell_of_pos, int64_t n,
                                                          const uint32_t* __restrict__ cell_start, int m,
                                                          const uint32_t* __restrict__ cell_nb, int col_tiles,
@@ -1753,9 +1757,9 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     // Column segments per row block, so that a small batch still fills the
     // GPU: each segment of a block is its own work item, and the segments of
     // a row share its threshold through HBM.
-    // (At most 16: the rerank reads up to 32 lists of a row in registers;
-    // and a count the sweep's segment split reproduces.)
-    int csegs = std::max(1, std::min({16, col_tiles, (2 * ctx->sm_count + items - 1) / items}));
+    // (At most 64, 128 lists of a row, and a count the sweep's segment split
+    // reproduces.)
+    int csegs = std::max(1, std::min({kQuerySegments, col_tiles, (2 * ctx->sm_count + items - 1) / items}));
     while (csegs > 1 && (col_tiles + (col_tiles + csegs - 1) / csegs - 1) / ((col_tiles + csegs - 1) / csegs) != csegs)
         csegs--;
     const int work = items * csegs;

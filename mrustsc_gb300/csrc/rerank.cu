@@ -437,7 +437,7 @@ __device__ __forceinline__ void warp_sort_keys(unsigned long long (&key)[2]) {
 __device__ int sorted_row_regs(const RerankArgs& a, int64_t slot, unsigned long long* keys_s, double* dbl) {
     const int lane = threadIdx.x & 31;
     const int segs = a.lists.segments;
-    if (segs > 32) return 3;
+    if (segs > 32 && !a.ids_only) return 3;  // the threshold below is that of the first 32 lists
     // The row's header, its own coordinates and -- with two lists, the
     // common case -- the first 32 slots of both lists are read at once (the
     // lists hold at least 64 slots each); only then is anything tested.
@@ -490,17 +490,25 @@ __device__ int sorted_row_regs(const RerankArgs& a, int64_t slot, unsigned long 
     } else {
         // Entry e of the row's lists (in list order) -> list and position.
         int list[2] = {-1, -1}, pos[2] = {0, 0};
-        for (int l = 0; l < segs; ++l) {
-            const int c = __shfl_sync(0xffffffffu, cl, l);
+        for (int l0 = 0; l0 < segs; l0 += 32) {
+            const int own = l0 == 0 ? cl
+                            : l0 + lane < segs
+                                ? (int)min(a.lists.cnt[slot * segs + l0 + lane], (uint32_t)a.lists.ctot)
+                                : 0;
+            // Only lists that hold something are looked at.
+            for (uint32_t some = __ballot_sync(0xffffffffu, own != 0); some; some &= some - 1) {
+                const int l = __ffs(some) - 1;
+                const int c = __shfl_sync(0xffffffffu, own, l);
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int e = lane + 32 * r;
-                if (list[r] < 0 && e < m0 + c) {
-                    list[r] = l;
-                    pos[r] = e - m0;
+                for (int r = 0; r < 2; ++r) {
+                    const int e = lane + 32 * r;
+                    if (list[r] < 0 && e < m0 + c) {
+                        list[r] = l0 + l;
+                        pos[r] = e - m0;
+                    }
                 }
+                m0 += c;
             }
-            m0 += c;
         }
         if (m0 > 64) return 3;
 #pragma unroll
@@ -687,26 +695,28 @@ __device__ int sorted_row_wide(const RerankArgs& a, int64_t slot, unsigned long 
     constexpr uint32_t FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int segs = a.lists.segments;
-    if (segs > 32) return 3;
-    const uint32_t ovf = a.lists.overflow[slot];
-    const int cl = lane < segs ? (int)min(a.lists.cnt[slot * segs + lane], (uint32_t)a.lists.ctot) : 0;
-    if (ovf) return 2;
+    if (a.lists.overflow[slot]) return 2;
     // Entry e of the row's lists (in list order) -> list and position.
     int list[R], pos[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) list[r] = -1;
     int m = 0;
-    for (int l = 0; l < segs; ++l) {
-        const int c = __shfl_sync(FULL, cl, l);
+    for (int l0 = 0; l0 < segs; l0 += 32) {
+        const int own =
+            l0 + lane < segs ? (int)min(a.lists.cnt[slot * segs + l0 + lane], (uint32_t)a.lists.ctot) : 0;
+        for (uint32_t some = __ballot_sync(FULL, own != 0); some; some &= some - 1) {
+            const int l = __ffs(some) - 1;
+            const int c = __shfl_sync(FULL, own, l);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int e = lane + 32 * r;
-            if (list[r] < 0 && e < m + c) {
-                list[r] = l;
-                pos[r] = e - m;
+            for (int r = 0; r < R; ++r) {
+                const int e = lane + 32 * r;
+                if (list[r] < 0 && e < m + c) {
+                    list[r] = l0 + l;
+                    pos[r] = e - m;
+                }
             }
+            m += c;
         }
-        m += c;
     }
     if (m > 32 * R) return 3;
     if (m < a.k) return 2;
