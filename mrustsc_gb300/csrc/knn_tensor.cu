@@ -109,7 +109,7 @@ struct TensorArgs {
     uint32_t* row_theta;        // per query row the smallest threshold any of its lists reached
                                 // (float_key; 0xffffffff = none), shared across column segments; or null
     const uint32_t* row_map;    // per query row its input row, 0xffffffff for padding; null: all rows real
-    // k = 1 without lists: per (row, part) the smallest MMA value and its
+    // k = 1 without lists: per (row, segment, part) the smallest MMA value and its
     // column, packed as float_key << 32 | column; null otherwise.  (The
     // nearest-column pass carries the column in the value's low five bits, so
     // its choice is exact up to values within 32 ulp of each other.)
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             if (argmin) {
                 if (valid && ok)
-                    a.argmin_out[row * PARTS + part] =
+                    a.argmin_out[lslot] =
                         ((unsigned long long)float_key(top.v[0]) << 32) | (unsigned long long)best;
                 continue;
             }

@@ -286,8 +286,8 @@ __global__ void relabel_neighbours_kernel(const uint32_t* __restrict__ nb, const
     out[(int64_t)rank[a] * kAnchorNeighbours + j] = c < (uint32_t)m ? rank[c] : 0xffffffffu;
 }
 
-// Each row's nearest anchor from the nearest-group pass: the better of its
-// two parts' groups, then the group's eight anchors measured on the same
+// Each row's nearest anchor from the nearest-group pass: the best of its
+// `parts` groups (one of each column part and segment), then the group's eight anchors measured on the same
 // 16-bit operands (a row's [a, 1, 1, 1] times an anchor's [-2b, three norm
 // parts], summed in f32 over the `words` 16-byte words that hold them) and
 // the smallest taken (ties to the lower anchor): an approximately nearest
@@ -318,14 +318,22 @@ __device__ __forceinline__ float dot_word(uint4 x, uint4 y) {
 }
 
 template <class T, int BLOCKS>
-__global__ void nearest_anchor_kernel(const unsigned long long* __restrict__ best, int64_t n, int64_t m,
+__global__ void nearest_anchor_kernel(const unsigned long long* __restrict__ best, int parts, int64_t n, int64_t m,
                                       const T* __restrict__ A, const T* __restrict__ B, int words,
                                       uint32_t* __restrict__ keys, unsigned long long* __restrict__ vals) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t i = t >> 3;
     const int l = (int)(t & 7);
     const bool row_ok = i < n;
-    const uint32_t g = row_ok ? (uint32_t)min(best[2 * i], best[2 * i + 1]) : 0u;
+    unsigned long long near = ~0ull;
+    if (parts == 2) {
+        if (row_ok) near = min(best[2 * i], best[2 * i + 1]);
+    } else {
+        for (int p = l; p < parts && row_ok; p += 8) near = min(near, best[i * parts + p]);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) near = min(near, __shfl_xor_sync(0xffffffffu, near, o));
+    }
+    const uint32_t g = row_ok ? (uint32_t)near : 0u;
     const int64_t c0 = (int64_t)g * 8;
     float part[8];
 #pragma unroll
@@ -1137,6 +1145,14 @@ constexpr int kQueryPrioNb = 8;
 // queries left most of the chip idle: 30, 300 and 1,000 of a million cells took
 // 427, 1,220 and 855 us, and 334, 609 and 634 us with 64.)
 constexpr int kQuerySegments = 64;
+
+// Column segments that give two work items an SM where `tiles` tiles and `most`
+// allow it, and that cutting the tiles into equal runs reproduces.
+int column_segments(int most, int tiles, int items, int sms) {
+    int c = std::max(1, std::min({most, tiles, (2 * sms + items - 1) / items}));
+    while (c > 1 && (tiles + (tiles + c - 1) / c - 1) / ((tiles + c - 1) / c) != c) c--;
+    return c;
+}
 __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restrict__ cell_of_pos, int64_t n,
                                                          const uint32_t* __restrict__ cell_start, int m,
                                                          const uint32_t* __restrict__ cell_nb, int col_tiles,
@@ -1282,15 +1298,15 @@ void launch_tile_balls(bool bf16, const void* ops, int64_t n, int d, int tiles, 
     }
 }
 
-void launch_nearest_anchor(bool bf16, const unsigned long long* best, int64_t n, int64_t m, const void* A, const void* B,
+void launch_nearest_anchor(bool bf16, const unsigned long long* best, int parts, int64_t n, int64_t m, const void* A, const void* B,
                            int blocks, int words, uint32_t* keys, unsigned long long* vals, cudaStream_t s) {
     const unsigned grid = (unsigned)((n * 8 + 255) / 256);
     if (bf16) {
         const auto kern = blocks == 1 ? nearest_anchor_kernel<__nv_bfloat16, 1> : nearest_anchor_kernel<__nv_bfloat16, 2>;
-        kern<<<grid, 256, 0, s>>>(best, n, m, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, words, keys, vals);
+        kern<<<grid, 256, 0, s>>>(best, parts, n, m, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, words, keys, vals);
     } else {
         const auto kern = blocks == 1 ? nearest_anchor_kernel<__half, 1> : nearest_anchor_kernel<__half, 2>;
-        kern<<<grid, 256, 0, s>>>(best, n, m, (const __half*)A, (const __half*)B, words, keys, vals);
+        kern<<<grid, 256, 0, s>>>(best, parts, n, m, (const __half*)A, (const __half*)B, words, keys, vals);
     }
 }
 
@@ -1500,7 +1516,7 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
                                       false, nullptr, nullptr, nullptr, best)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: anchor candidates");
     const int op_words = (d + 3 + 7) / 8;  // 16-byte words of an operand row holding values
-    launch_nearest_anchor(bf16, best, n, m, A0, base + o_aB, blocks, op_words, keysA, valsA, s);
+    launch_nearest_anchor(bf16, best, 2, n, m, A0, base + o_aB, blocks, op_words, keysA, valsA, s);
     // The walk ranks (copy stream) are needed from here on.
     if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamWaitEvent(s, ctx->copy_ev, 0)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: nearest anchor");
@@ -1757,11 +1773,11 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     // Column segments per row block, so that a small batch still fills the
     // GPU: each segment of a block is its own work item, and the segments of
     // a row share its threshold through HBM.
-    // (At most 64, 128 lists of a row, and a count the sweep's segment split
-    // reproduces.)
-    int csegs = std::max(1, std::min({kQuerySegments, col_tiles, (2 * ctx->sm_count + items - 1) / items}));
-    while (csegs > 1 && (col_tiles + (col_tiles + csegs - 1) / csegs - 1) / ((col_tiles + csegs - 1) / csegs) != csegs)
-        csegs--;
+    const int csegs = column_segments(kQuerySegments, col_tiles, items, ctx->sm_count);
+    // The anchors likewise: one query had one CTA pass over all 16 tiles of
+    // 3,906 anchors (23 us of its 320; 8 in 16 segments).
+    const int anchor_tiles = (int)(at.anchors_pad / 256);
+    const int anchor_segs = column_segments(anchor_tiles, anchor_tiles, items, ctx->sm_count);
     const int work = items * csegs;
     const int ps = (kQueryPrio + csegs - 1) / csegs, es = (col_tiles + csegs - 1) / csegs;
     const int P = padded_row_floats(d);
@@ -1776,7 +1792,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     };
     const size_t o_A0 = take(128 * (size_t)q_pad), o_B0 = take(128 * (size_t)q_pad), o_t0 = take(4 * 2 * (size_t)q_pad),
                  o_As = take(128 * (size_t)q_pad), o_Bs = take(128 * (size_t)q_pad), o_ts = take(4 * 4 * (size_t)q_pad),
-                 o_w = take(64), o_best = take(16 * (size_t)q_pad), o_kA = take(4 * (size_t)q), o_kB = take(4 * (size_t)q),
+                 o_w = take(64), o_best = take(16 * (size_t)anchor_segs * q_pad), o_kA = take(4 * (size_t)q), o_kB = take(4 * (size_t)q),
                  o_vA = take(8 * (size_t)q), o_vB = take(8 * (size_t)q), o_qp = take(4 * (size_t)q),
                  o_cell = take(4 * (size_t)q),
                  o_xs = take(4 * (size_t)q * P), o_prio = take(4 * (size_t)items * kQueryPrio),
@@ -1820,7 +1836,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     Lists lx;  // no storage: the pass keeps no lists
     lx.cap = 64;
     lx.ctot = 64 + 128;
-    lx.segments = 2;
+    lx.segments = 2 * anchor_segs;
     px.cap = lx.cap;
     px.ctot = lx.ctot;
     px.segments = lx.segments;
@@ -1828,7 +1844,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
                                       bf16, nullptr, false, nullptr, nullptr, nullptr, best)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: nearest anchor");
     const int op_words = (d + 3 + 7) / 8;  // 16-byte words of an operand row holding values
-    launch_nearest_anchor(bf16, best, q, at.anchors, base + o_A0, at.anchor_B16, 1, op_words, (uint32_t*)(base + o_kA),
+    launch_nearest_anchor(bf16, best, lx.segments, q, at.anchors, base + o_A0, at.anchor_B16, 1, op_words, (uint32_t*)(base + o_kA),
                           (unsigned long long*)(base + o_vA), s);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: nearest anchor");
     ctx->launches += 3;
