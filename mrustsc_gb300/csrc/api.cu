@@ -224,7 +224,8 @@ int32_t plan_lists(scrust_context* ctx, const scrust_knn_options& o, int k, int 
 
 }  // namespace
 
-int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_status* st) {
+// (Unless `clear`, the caller sets the counts and overflow marks to 0.)
+int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_status* st, bool clear) {
     cudaError_t e = cudaSuccess;
     const size_t slots = (size_t)rows_pad * lists->segments;
     lists->ids = (uint32_t*)ws_get(ctx, SLOT_LIST_IDS, sizeof(uint32_t) * slots * lists->ctot, &e);
@@ -232,7 +233,8 @@ int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_
     lists->cnt = (uint32_t*)ws_get(ctx, SLOT_LIST_CNT, sizeof(uint32_t) * (slots + (size_t)rows_pad), &e);
     if (!lists->ids || !lists->vals || !lists->cnt) return cuda_fail(st, e, "workspace");
     lists->overflow = lists->cnt + slots;
-    if ((e = cudaMemsetAsync(lists->cnt, 0, sizeof(uint32_t) * (slots + (size_t)rows_pad), ctx->stream)) != cudaSuccess)
+    if (clear &&
+        (e = cudaMemsetAsync(lists->cnt, 0, sizeof(uint32_t) * (slots + (size_t)rows_pad), ctx->stream)) != cudaSuccess)
         return cuda_fail(st, e, "memset");
     return SCRUST_OK;
 }

@@ -226,7 +226,7 @@ struct Lists {
     int cap = 0, ctot = 0, segments = 1;
 };
 
-int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_status* st);
+int32_t alloc_lists(scrust_context* ctx, int64_t rows_pad, Lists* lists, scrust_status* st, bool clear = true);
 
 // A spatial ordering of the rows of a self-kNN solve (order.cu): rows are
 // grouped into cells around anchors and each 256-row work item of the tensor

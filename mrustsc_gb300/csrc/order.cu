@@ -1224,6 +1224,20 @@ __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restr
     if (threadIdx.x == 0) prio_cnt[I] = (uint32_t)total;
 }
 
+// Up to five runs of words set, each to its value: one launch where every run
+// had its own: a request of one query 320 -> 312 us, 300 queries 667 -> 655.
+struct WordRuns {
+    uint32_t* p[5];
+    int64_t n[5];
+    uint32_t value[5];
+};
+__global__ void __launch_bounds__(256) set_words_kernel(WordRuns r) {
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+#pragma unroll
+    for (int j = 0; j < 5; ++j)
+        for (int64_t i = first; i < r.n[j]; i += step) r.p[j][i] = r.value[j];
+}
+
 // A row block's tile list cut into `segs` contiguous chunks of equal size,
 // one per column segment, so that each segment of a row block is its own
 // work item: dst row (block * segs + segment), `dst_stride` entries apart.
@@ -1821,8 +1835,23 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     uint32_t* entries = (uint32_t*)(base + o_ent);
     unsigned long long* best = (unsigned long long*)(base + o_best);
 
+    Lists lists;
+    lists.cap = 256;
+    lists.ctot = 256 + 128;
+    lists.segments = 2 * csegs;
+    int32_t rc = alloc_lists(ctx, q_pad, &lists, st, false);
+    if (rc) return rc;
     // The queries' operands, in input order; every query's nearest anchor.
-    if ((e = cudaMemsetAsync(qwords, 0, 64, s)) != cudaSuccess ||
+    // Everything that starts from a set value.  A list the threshold pass leaves
+    // without a threshold (a segment with no tile) keeps a huge one; a row
+    // without any keeps reach everywhere.
+    const size_t slots = (size_t)q_pad * lists.segments;
+    const WordRuns runs = {{qwords, lists.cnt, (uint32_t*)theta, row_theta, bitmap},
+                           {16, (int64_t)slots + q_pad, 2 * (int64_t)csegs * q_pad, q_pad, (int64_t)items * words_t},
+                           {0u, 0u, 0x7f7f7f7fu, 0xffffffffu, 0u}};
+    const int64_t longest = std::max((int64_t)slots + q_pad, (int64_t)items * words_t);
+    set_words_kernel<<<(unsigned)std::min<int64_t>((longest + 255) / 256, 4 * ctx->sm_count), 256, 0, s>>>(runs);
+    if ((e = cudaGetLastError()) != cudaSuccess ||
         (e = launch_tensor_operands(dq, q, q_pad, d, means, words, false, bf16, nullptr, base + o_A0, base + o_B0, bA0,
                                     eps0, qwords, qwords + 1, s)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: operands");
@@ -1847,7 +1876,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     launch_nearest_anchor(bf16, best, lx.segments, q, at.anchors, base + o_A0, at.anchor_B16, 1, op_words, (uint32_t*)(base + o_kA),
                           (unsigned long long*)(base + o_vA), s);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: nearest anchor");
-    ctx->launches += 3;
+    ctx->launches += 4;
     // The queries sorted by the walk place of their cell; their operands,
     // bounds and rows in that order.
     if ((e = order_rows(ctx, (uint32_t*)(base + o_kA), (unsigned long long*)(base + o_vA), (uint32_t*)(base + o_kB),
@@ -1882,12 +1911,6 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     plan.self = false;
     plan.form = SCRUST_FORM_TENSOR;
     plan.precision = bf16 ? SCRUST_PRECISION_BF16 : SCRUST_PRECISION_FP16;
-    Lists lists;
-    lists.cap = 256;
-    lists.ctot = 256 + 128;
-    lists.segments = 2 * csegs;
-    int32_t rc = alloc_lists(ctx, q_pad, &lists, st);
-    if (rc) return rc;
     plan.cap = lists.cap;
     plan.ctot = lists.ctot;
     plan.segments = lists.segments;
@@ -1897,11 +1920,6 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     first.stride = ps;
     first.order = (const uint32_t*)(base + o_po);
     first.row_theta = row_theta;
-    // A list the pass leaves without a threshold (a segment with no tile)
-    // keeps a huge one; a row without any keeps reach everywhere.
-    if ((e = cudaMemsetAsync(theta, 0x7f, 4 * 2 * (size_t)csegs * q_pad, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(row_theta, 0xff, 4 * (size_t)q_pad, s)) != cudaSuccess)
-        return cuda_fail(st, e, "query knn: memset");
     // Each row's threshold is then taken from its lists together: a list sees
     // one column part of one segment's few tiles, so the best list's own k-th
     // lies far beyond the row's (one query alone, 13 tiles over 16 segments,
@@ -1921,8 +1939,6 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     ctx->launches += topk ? 1 : 0;
     // The atlas tiles each row block cannot rule out: its queries, with the
     // reach of their shared thresholds, against the atlas segment balls.
-    if ((e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)items * words_t, s)) != cudaSuccess)
-        return cuda_fail(st, e, "query knn: memset");
     if (at.segs) {
         const dim3 grid((unsigned)((at.segs + 63) / 64), (unsigned)((q + 63) / 64));
         if (bf16)
