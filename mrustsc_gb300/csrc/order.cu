@@ -851,8 +851,9 @@ __global__ void __launch_bounds__(256) segment_pairs_kernel(const float* __restr
     }
 }
 
-// One block per row block I: the tiles of its reach bitmap row that are not
-// in its priority list, ascending, at entries[I * tiles ...].
+// One block per row block I: the tiles of its reach bitmap row (all tiles where
+// there is no bitmap) that are not in its priority list, ascending, at
+// entries[I * tiles ...].
 __global__ void __launch_bounds__(256) tile_lists_kernel(const uint32_t* __restrict__ bitmap, int words, int tiles,
                                                          const uint32_t* __restrict__ prio,
                                                          const uint32_t* __restrict__ prio_cnt,
@@ -870,12 +871,13 @@ __global__ void __launch_bounds__(256) tile_lists_kernel(const uint32_t* __restr
         if (t < (uint32_t)tiles) atomicOr(&in_prio[t >> 5], 1u << (t & 31));
     }
     __syncthreads();
-    const uint32_t* row = bitmap + (int64_t)I * words;
+    const uint32_t* row = bitmap ? bitmap + (int64_t)I * words : nullptr;
     uint32_t* out = entries + (int64_t)I * tiles;
     int base = 0;
     for (int w0 = 0; w0 < words; w0 += 256) {
         const int wd = w0 + threadIdx.x;
-        uint32_t bits = wd < words ? row[wd] & ~in_prio[wd] : 0u;
+        const uint32_t all = tiles - wd * 32 >= 32 ? 0xffffffffu : (1u << (tiles & 31)) - 1u;
+        uint32_t bits = wd < words ? (row ? row[wd] : all) & ~in_prio[wd] : 0u;
         int c = __popc(bits);
         int incl = c;
         for (int o = 1; o < 32; o <<= 1) {
@@ -1591,7 +1593,6 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
                  o_so = take(4 * ((size_t)tiles + 1)), o_fc = take(4 * 64 * blocks * (size_t)smax), o_fr = take(4 * (size_t)smax),
                  o_fu = take(4 * (size_t)smax), o_fo = take(4 * (size_t)smax), o_scan = take(4 * scan_elems),
                  o_bm = take(4 * (size_t)tiles * words), o_cnt = take(4 * ((size_t)tiles + 1)),
-                 o_wo = take(4 * (size_t)tiles), o_ws = take(work_order_scratch(tiles)),
                  o_ent = take(4 * (size_t)tiles * (size_t)tiles);
     char* base = (char*)ws_get(ctx, SLOT_PRUNE, off, &e);
     if (!base) return cuda_fail(st, e, "pruning: workspace");
@@ -1611,32 +1612,39 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
     uint32_t* bitmap = (uint32_t*)(base + o_bm);
     uint32_t* counts = (uint32_t*)(base + o_cnt);
     uint32_t* entries = (uint32_t*)(base + o_ent);
-    if ((e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)tiles * words, s)) != cudaSuccess)
-        return cuda_fail(st, e, "pruning: memset");
-    launch_tile_balls(bf16, A16, n, d, tiles, order.cell_of_pos, order.theta, bA, bdelta, balls, s);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: tile balls");
-    if ((e = device_exclusive_scan(ctx, balls.nseg, seg_off, (int64_t)tiles + 1, (uint32_t*)(base + o_scan),
-                                   scan_elems)) != cudaSuccess)
-        return cuda_fail(st, e, "pruning: segment scan");
-    flatten_segments_kernel<<<tiles, 64, 0, s>>>(balls, d, 64 * blocks, tiles, seg_off, fc, fr, fu, fo);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: segments");
-    const auto pairs = blocks == 1 ? segment_pairs_kernel<1> : segment_pairs_kernel<2>;
-    pairs<<<8 * ctx->sm_count, 256, 0, s>>>(fc, fr, fu, fo, seg_off + tiles, d, words, bitmap);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: segment pairs");
+    // Up to 17 anchors are all among each other's 16 nearest, so the priority
+    // lists hold every tile and there is nothing to test: the lists are what is
+    // left of all tiles, by one launch instead of six (2,638 rows, with the
+    // unused work order of these lists gone: 501 -> 482 us; from 18 anchors, 4,608
+    // rows, the balls rule tiles out).
+    const bool few = order.anchors <= kAnchorNeighbours + 1;
+    if (!few) {
+        if ((e = cudaMemsetAsync(bitmap, 0, 4 * (size_t)tiles * words, s)) != cudaSuccess)
+            return cuda_fail(st, e, "pruning: memset");
+        launch_tile_balls(bf16, A16, n, d, tiles, order.cell_of_pos, order.theta, bA, bdelta, balls, s);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: tile balls");
+        if ((e = device_exclusive_scan(ctx, balls.nseg, seg_off, (int64_t)tiles + 1, (uint32_t*)(base + o_scan),
+                                       scan_elems)) != cudaSuccess)
+            return cuda_fail(st, e, "pruning: segment scan");
+        flatten_segments_kernel<<<tiles, 64, 0, s>>>(balls, d, 64 * blocks, tiles, seg_off, fc, fr, fu, fo);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: segments");
+        const auto pairs = blocks == 1 ? segment_pairs_kernel<1> : segment_pairs_kernel<2>;
+        pairs<<<8 * ctx->sm_count, 256, 0, s>>>(fc, fr, fu, fo, seg_off + tiles, d, words, bitmap);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: segment pairs");
+        ctx->launches += 3;
+    }
     const size_t lists_smem = 4 * (size_t)words;
-    if ((e = set_smem_limit(ctx, (const void*)tile_lists_kernel, (int)lists_smem)) !=
-        cudaSuccess)
+    if ((e = set_smem_limit(ctx, (const void*)tile_lists_kernel, (int)lists_smem)) != cudaSuccess)
         return cuda_fail(st, e, "pruning: tile lists");
-    tile_lists_kernel<<<tiles, 256, lists_smem, s>>>(bitmap, words, tiles, order.prio, order.prio_cnt, counts, entries);
+    tile_lists_kernel<<<tiles, 256, lists_smem, s>>>(few ? nullptr : bitmap, words, tiles, order.prio, order.prio_cnt,
+                                                     counts, entries);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "pruning: tile lists");
-    ctx->launches += 3;
-    if ((e = sort_by_work(ctx, counts, tiles, base + o_ws, (uint32_t*)(base + o_wo))) != cudaSuccess)
-        return cuda_fail(st, e, "pruning: work order");
+    ctx->launches += 1;
     out->tiles = entries;
     out->offset = nullptr;
     out->count = counts;
     out->stride = tiles;
-    out->order = (const uint32_t*)(base + o_wo);
+    out->order = nullptr;  // the collect pass keeps the priority lists' order
     return SCRUST_OK;
 }
 
