@@ -596,21 +596,26 @@ __global__ void __launch_bounds__(kMulThreads)
     }
 }
 
-// Eigenpairs of the symmetric positive semi-definite H (w x w, f64) by
-// one-sided Jacobi rotations of its columns: at the end column j of the
-// rotated H is lambda_j times the j-th eigenvector (pca.rs:388-447 rotates H
-// from both sides; the eigenpairs are the same).  A round rotates w / 2
+// Eigenpairs of the symmetric H (w x w, f64) by one-sided Jacobi rotations of
+// its columns, the same rotations applied to the columns of V, the identity at
+// first: at the end column j of V is the j-th eigenvector and its product with
+// column j of the rotated H, H V, the eigenvalue (pca.rs:388-447 rotates H from
+// both sides; the eigenpairs are the same).  A round rotates w / 2
 // disjoint pairs, a warp each, over a cluster of kJacobiBlocks blocks; the
 // columns pass through L2 between rounds.  A sweep of rounds meets every pair
 // once.  A pair is done when its columns are orthogonal to f64 rounding, or
-// when one of them is zero to rounding (a rank-deficient H).
+// when one of them is zero.
+// (V stays orthonormal whatever H's columns are, and the sign of an eigenvalue
+// is kept, which a column's norm loses.  With eigenvectors from the columns
+// alone, and columns below 1e-13 of the trace left as they were, those past the
+// rank lay along the leading ones: their loadings had norms of 1e6 and more.)
 // Bound by the latency of a round, most of it f64 issue (64 clocks a warp
 // instruction): so the squared norms are kept beside the columns and followed
 // through the rotations (measured anew each sweep), the angle is taken in f32
 // (a pair comes out orthogonal to 1e-7 instead of 1e-16, and the next sweep
 // meets it again), and only the rotation's length is exact to f64.  One block
 // rotating one pair after another took 55 ms at w = 74; this form with norms,
-// angle and roots in f64 4.3 ms; so, 2.2 ms.
+// angle and roots in f64 4.3 ms; with the angle in f32 2.2 ms; V adds 0.3 ms.
 constexpr int kJacobiBlocks = 8;
 constexpr int kJacobiThreads = 256;  // kJacobiBlocks * 8 warps: kPcaMaxWidth / 2 pairs
 static_assert(kJacobiBlocks * kJacobiThreads / 32 * 2 >= kPcaMaxWidth, "a warp for every pair");
@@ -625,11 +630,11 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // H: w x w, symmetric, so its rows serve as its columns; overwritten with the
-// rotated columns (column j at H + j w), scaled by a power of two.  lambda:
-// w eigenvalues (between sweeps: squared norms).  rotated: kJacobiSweeps
-// flags, zero on entry.
+// rotated columns (column j at H + j w), scaled by a power of two.  V: w x w,
+// column j at V + j w.  lambda: w eigenvalues (between sweeps: squared norms).
+// rotated: kJacobiSweeps flags, zero on entry.
 __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiThreads)
-    pca_jacobi_kernel(double* H, int w, double* lambda, int* rotated, int* __restrict__ err) {
+    pca_jacobi_kernel(double* H, double* V, int w, double* lambda, int* rotated, int* __restrict__ err) {
     constexpr int SLOTS = kPcaMaxWidth / 32;
     constexpr int WARPS = kJacobiBlocks * kJacobiThreads / 32;
     constexpr double EPS = 2.220446049250313e-16;
@@ -646,11 +651,14 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
     const double scale = ldexp(1.0, -ex);
     cluster_barrier();  // everyone has read the diagonal
     for (int c = slot; c < w; c += WARPS)
-        for (int i = lane; i < w; i += 32) __stcg(H + (int64_t)c * w + i, __ldcg(H + (int64_t)c * w + i) * scale);
-    // Orthogonal: to 16 roundings.  Zero: a column whose squared norm is below
-    // 1e-26 of the trace's, under the f32 rounding of the basis H came from;
-    // above it the f32 angle of two small columns is in range.
-    constexpr double ORTHO2 = (16 * EPS) * (16 * EPS), TINY2 = 1e-26;
+        for (int i = lane; i < w; i += 32) {
+            __stcg(H + (int64_t)c * w + i, __ldcg(H + (int64_t)c * w + i) * scale);
+            __stcg(V + (int64_t)c * w + i, i == c ? 1.0 : 0.0);
+        }
+    // Orthogonal: to 16 roundings, whatever the columns' sizes (the Gram of a
+    // graded basis holds its small eigenvalues to as many digits as the large
+    // ones).  Zero: a column whose squared norm leaves f64's range.
+    constexpr double ORTHO2 = (16 * EPS) * (16 * EPS), TINY2 = 1e-280;
     int sweep = 0;
     bool done = w < 2;
     auto norms = [&]() {  // each column's squared norm, by the warp that owns it
@@ -673,13 +681,15 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
                 const int b = (round - slot + players - 1) % (players - 1);
                 const int p = min(a, b), q = max(a, b);
                 if (q < w) {
-                    double x[SLOTS], y[SLOTS];
+                    double x[SLOTS], y[SLOTS], vx[SLOTS], vy[SLOTS];
                     const double pp = __ldcg(lambda + p), qq = __ldcg(lambda + q);
 #pragma unroll
                     for (int t = 0; t < SLOTS; ++t) {
                         const int i = t * 32 + lane;
                         x[t] = i < w ? __ldcg(H + (int64_t)p * w + i) : 0.0;
                         y[t] = i < w ? __ldcg(H + (int64_t)q * w + i) : 0.0;
+                        vx[t] = i < w ? __ldcg(V + (int64_t)p * w + i) : 0.0;
+                        vy[t] = i < w ? __ldcg(V + (int64_t)q * w + i) : 0.0;
                     }
                     double pq = 0.0;
 #pragma unroll
@@ -689,11 +699,19 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
                     // (A NaN fails every comparison and keeps rotating, so it
                     // ends as not converged.)
                     if (!(pq * pq <= ORTHO2 * pp * qq) && !(fmin(pp, qq) <= TINY2)) {
-                        const float theta = (float)(qq - pp) / (float)(2.0 * pq);
+                        // By the power of two that brings the larger norm near
+                        // one (its exponent negated), so that the f32 quotient
+                        // of two small columns is in range.
+                        const int top = __double2hiint(fmax(pp, qq)) & 0x7ff00000;
+                        const double near_one = __hiloint2double(0x7fe00000 - top, 0);
+                        const float theta = (float)((qq - pp) * near_one) / (float)(2.0 * pq * near_one);
                         // (Past 1e6 the root is theta itself to f32, and theta^2
-                        // may be out of range.)
+                        // may be out of range; past 1e30 the product of the
+                        // columns may be, and the tangent is 1 / (2 theta).)
                         const float root = fabsf(theta) > 1e6f ? fabsf(theta) : sqrtf(fmaf(theta, theta, 1.f));
-                        const double tangent = (double)((theta < 0.f ? -1.f : 1.f) / (fabsf(theta) + root));
+                        const double tangent = fabsf(theta) > 1e30f
+                                                   ? pq / (qq - pp)
+                                                   : (double)((theta < 0.f ? -1.f : 1.f) / (fabsf(theta) + root));
                         const double cs = rsqrt64(fma(tangent, tangent, 1.0)), sn = tangent * cs;
 #pragma unroll
                         for (int t = 0; t < SLOTS; ++t) {
@@ -701,6 +719,8 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
                             if (i < w) {
                                 __stcg(H + (int64_t)p * w + i, cs * x[t] - sn * y[t]);
                                 __stcg(H + (int64_t)q * w + i, sn * x[t] + cs * y[t]);
+                                __stcg(V + (int64_t)p * w + i, cs * vx[t] - sn * vy[t]);
+                                __stcg(V + (int64_t)q * w + i, sn * vx[t] + cs * vy[t]);
                             }
                         }
                         if (lane == 0) {
@@ -716,16 +736,12 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
         done = __ldcg(rotated + sweep) == 0;
     }
     if (!done && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(err, 2);
-    cluster_barrier();
-    norms();
-    cluster_barrier();
-    // Column c is scale * lambda_c times the eigenvector.
     const double back = ldexp(1.0, ex);
     for (int c = slot; c < w; c += WARPS) {
-        const double l = sqrt(__ldcg(lambda + c));
+        double l = 0.0;
+        for (int i = lane; i < w; i += 32) l += __ldcg(V + (int64_t)c * w + i) * __ldcg(H + (int64_t)c * w + i);
+        l = warp_sum(l);
         if (lane == 0) __stcg(lambda + c, l * back);
-        for (int i = lane; i < w; i += 32)
-            __stcg(H + (int64_t)c * w + i, l > 0.0 ? __ldcg(H + (int64_t)c * w + i) / l : 0.0);
     }
 }
 
@@ -744,7 +760,7 @@ __global__ void pca_select_kernel(const double* __restrict__ lambda, const doubl
     for (int i = lane; i < w; i += 32) before += lambda[i] > l || (lambda[i] == l && i < idx);
     const int c = __reduce_add_sync(0xffffffffu, before);
     if (c >= nc) return;
-    const double s = sqrt(l);
+    const double s = sqrt(fmax(l, 0.0));  // (below zero: rounding past the rank)
     if (lane == 0) sing[c] = s;
     const double inv = s > 0.0 ? 1.0 / s : 0.0;
     for (int r = lane; r < w; r += 32) {
@@ -834,7 +850,7 @@ size_t al(size_t v) { return (v + 255) & ~(size_t)255; }
 
 struct PcaWork {
     float *omega, *Y, *Z, *mvec, *colsum, *mean, *T, *basis, *scaled, *ct;
-    double *var_term, *total, *gram_part, *G, *lambda, *sing, *colpart;
+    double *var_term, *total, *gram_part, *G, *V, *lambda, *sing, *colpart;
     uint32_t *kA, *kB, *cstart;
     unsigned long long *vA, *vB;
     uint32_t *hist, *scan;
@@ -873,7 +889,7 @@ int32_t pca_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint3
                  o_t = take(4 * (size_t)w * w), o_basis = take(4 * (size_t)w * nc), o_sc = take(4 * (size_t)w * nc),
                  o_ct = take(4 * (size_t)g * nc), o_vt = take(8 * (size_t)g), o_tot = take(8),
                  o_gp = take(8 * (size_t)gram_blocks * entries), o_g = take(8 * (size_t)w * w),
-                 o_lam = take(8 * (size_t)w), o_sing = take(8 * (size_t)nc),
+                 o_v = take(8 * (size_t)w * w), o_lam = take(8 * (size_t)w), o_sing = take(8 * (size_t)nc),
                  o_cp = take(8 * (size_t)col_blocks * w), o_ka = take(4 * (size_t)nnz), o_kb = take(4 * (size_t)nnz),
                  o_cst = take(4 * (size_t)(g + 1)), o_va = take(8 * (size_t)nnz), o_vb = take(8 * (size_t)nnz),
                  o_hist = take(4 * ((size_t)256 * nb + 16)), o_scan = take(4 * wk.scan_elems),
@@ -894,6 +910,7 @@ int32_t pca_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint3
     wk.total = (double*)(base + o_tot);
     wk.gram_part = (double*)(base + o_gp);
     wk.G = (double*)(base + o_g);
+    wk.V = (double*)(base + o_v);
     wk.lambda = (double*)(base + o_lam);
     wk.sing = (double*)(base + o_sing);
     wk.colpart = (double*)(base + o_cp);
@@ -991,8 +1008,8 @@ int32_t pca_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint3
     // B^T = X_c^T Q (g x w), its Gram, the eigenpairs, the outputs.
     if ((e = transpose_times(wk.Y, wk.Z)) != cudaSuccess || (e = gram(wk.Z, g)) != cudaSuccess)
         return cuda_fail(st, e, "pca: projection");
-    pca_jacobi_kernel<<<kJacobiBlocks, kJacobiThreads, 0, s>>>(wk.G, w, wk.lambda, rotated, err);
-    pca_select_kernel<<<(w + 7) / 8, 256, 0, s>>>(wk.lambda, wk.G, w, nc, wk.basis, wk.scaled, wk.sing);
+    pca_jacobi_kernel<<<kJacobiBlocks, kJacobiThreads, 0, s>>>(wk.G, wk.V, w, wk.lambda, rotated, err);
+    pca_select_kernel<<<(w + 7) / 8, 256, 0, s>>>(wk.lambda, wk.V, w, nc, wk.basis, wk.scaled, wk.sing);
     rows_mul(wk.Y, n, wk.basis, nc, emb, nc);
     rows_mul(wk.Z, g, wk.scaled, nc, wk.ct, nc);
     pca_signs_kernel<<<nc, kSumThreads, 0, s>>>(wk.ct, g, nc, wk.flip);
