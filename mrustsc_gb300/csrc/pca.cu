@@ -430,16 +430,6 @@ __global__ void __launch_bounds__(32 * kGramFinalLanes)
     G[j * w + i] = s;
 }
 
-// 1 / sqrt(x) in f64 for x well inside the f32 range: the f32 estimate y and
-// the third-order step y (1 + e / 2 + 3 e^2 / 8), e = 1 - x y^2, which triples
-// its 22 bits.  Four f64 operations deep, where sqrt and a division are some
-// thirty.
-__device__ __forceinline__ double rsqrt64(double x) {
-    const double y = (double)rsqrtf((float)x);
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // T = L^-T of the shifted Cholesky factor of G (w x w, f64), as f32.  Every
 // block factors G in its shared memory (right-looking: each entry still loses
 // its products in the order of the columns), then a warp solves each of the
@@ -491,7 +481,7 @@ __global__ void __launch_bounds__(kCholeskyThreads)
             d = shift;
             if (lane == 0) atomicExch(err, 1);
         }
-        const double y = rsqrt64(d);
+        const double y = rsqrt(d);
         if (lane == 0) inv[k] = y;
     };
     if (warp == 0) pivot(0, A[0]);
@@ -712,7 +702,7 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
                         const double tangent = fabsf(theta) > 1e30f
                                                    ? pq / (qq - pp)
                                                    : (double)((theta < 0.f ? -1.f : 1.f) / (fabsf(theta) + root));
-                        const double cs = rsqrt64(fma(tangent, tangent, 1.0)), sn = tangent * cs;
+                        const double cs = rsqrt(fma(tangent, tangent, 1.0)), sn = tangent * cs;
 #pragma unroll
                         for (int t = 0; t < SLOTS; ++t) {
                             const int i = t * 32 + lane;
