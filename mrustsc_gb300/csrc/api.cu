@@ -148,6 +148,23 @@ int32_t collect_device_errors(scrust_context* ctx, scrust_status* st) {
     return fail(st, SCRUST_KERNEL, "CUDA kernel knn_rerank: inconsistent candidate set");
 }
 
+// The end of a call on host arrays that failed with `rc`: both streams idle
+// and the device's error words read and cleared, which otherwise the next call
+// would report.  What they say came first and takes the place of `rc` (rows
+// that the kNN left open make its graph look malformed), unless the stream
+// itself failed and nothing could be read.
+int32_t host_call_failed(scrust_context* ctx, int32_t rc, scrust_status* st) {
+    cudaStreamSynchronize(ctx->copy_stream);
+    scrust_status found{};
+    const int32_t device = collect_device_errors(ctx, &found);
+    if (device && cudaStreamQuery(ctx->stream) == cudaSuccess) {
+        if (st) *st = found;
+        rc = device;
+    }
+    cudaGetLastError();
+    return rc;
+}
+
 namespace {
 
 constexpr uint32_t kMaxK = 128;
@@ -930,12 +947,12 @@ int32_t scrust_cuda_knn(scrust_context* ctx, const float* x, uint64_t n, uint64_
     if (!dx || !di || !dd) return cuda_fail(st, e, "workspace");
     if ((e = cudaMemcpyAsync(dx, x, sizeof(float) * n * d, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cuda_fail(st, e, "upload");
-    if ((rc = knn_device_impl(ctx, dx, n, d, k, opt, di, dd, st))) return rc;
+    if ((rc = knn_device_impl(ctx, dx, n, d, k, opt, di, dd, st))) return host_call_failed(ctx, rc, st);
     if ((e = cudaMemcpyAsync(out_idx, di, sizeof(uint32_t) * n * k, cudaMemcpyDeviceToHost, ctx->stream)) !=
             cudaSuccess ||
         (e = cudaMemcpyAsync(out_dist, dd, sizeof(float) * n * k, cudaMemcpyDeviceToHost, ctx->stream)) !=
             cudaSuccess)
-        return cuda_fail(st, e, "download");
+        return host_call_failed(ctx, cuda_fail(st, e, "download"), st);
     if ((rc = collect_device_errors(ctx, st))) return rc;
     return ok_form(st, opt, n, (int)d);
 }
@@ -1041,7 +1058,7 @@ int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_
     if (!dx || !di || !dd) return cuda_fail(st, e, "workspace");
     if ((e = cudaMemcpyAsync(dx, x, sizeof(float) * n * d, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cuda_fail(st, e, "upload");
-    if ((rc = knn_device_impl(ctx, dx, n, d, k, opt, di, dd, st))) return rc;
+    if ((rc = knn_device_impl(ctx, dx, n, d, k, opt, di, dd, st))) return host_call_failed(ctx, rc, st);
     // The neighbour lists download on the copy stream while the
     // connectivities run on the main one.  A copy to pageable memory holds the
     // host, so it is queued behind the connectivities' launches.
@@ -1056,10 +1073,8 @@ int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_
     cudaPointerAttributes attr;
     const bool pageable = cudaPointerGetAttributes(&attr, out_idx) != cudaSuccess || attr.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if ((e = cudaEventRecord(ctx->copy_ev, ctx->stream)) != cudaSuccess || (!pageable && (e = download()) != cudaSuccess)) {
-        cudaStreamSynchronize(ctx->copy_stream);
-        return cuda_fail(st, e, "download");
-    }
+    if ((e = cudaEventRecord(ctx->copy_ev, ctx->stream)) != cudaSuccess || (!pageable && (e = download()) != cudaSuccess))
+        return host_call_failed(ctx, cuda_fail(st, e, "download"), st);
     scrust_csr* dev = nullptr;
     bool streamed = false;
     rc = conn_device_impl(ctx, di, dd, n, k, true, &dev, st, true, n * (uint64_t)k >= kStreamEntries, &streamed);
@@ -1068,10 +1083,7 @@ int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_
         delete dev;
         rc = cuda_fail(st, e, "download");
     }
-    if (rc) {
-        cudaStreamSynchronize(ctx->copy_stream);
-        return rc;
-    }
+    if (rc) return host_call_failed(ctx, rc, st);
     rc = streamed ? csr_to_host_streamed(ctx, dev, conn, st) : csr_to_host(ctx, dev, conn, st);
     ctx->csr_pool.push_back(dev->buf);
     delete dev;
@@ -1080,9 +1092,9 @@ int32_t scrust_cuda_neighbors_graph(scrust_context* ctx, const float* x, uint64_
             scrust_csr_free(*conn);
             *conn = nullptr;
         }
-        return cuda_fail(st, e, "download");
+        return host_call_failed(ctx, cuda_fail(st, e, "download"), st);
     }
-    if (rc) return rc;
+    if (rc) return host_call_failed(ctx, rc, st);
     if ((rc = collect_device_errors(ctx, st))) return rc;
     return ok_form(st, opt, n, (int)d);
 }

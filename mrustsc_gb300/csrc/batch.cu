@@ -374,15 +374,16 @@ int32_t scrust_cuda_knn_batch(scrust_context* ctx, const float* x, const uint64_
             cudaSuccess)
             return cuda_fail(st, e, "upload");
     }
-    if ((rc = scrust_cuda_knn_batch_device(ctx, dx, row_offsets, n_samples, d, k, opt, di, dd, st))) return rc;
+    rc = scrust_cuda_knn_batch_device(ctx, dx, row_offsets, n_samples, d, k, opt, di, dd, st);
     std::lock_guard<std::mutex> lock(ctx->mu);
     DeviceGuard device_guard(ctx->device);
+    if (rc) return host_call_failed(ctx, rc, st);
     cudaError_t e;
     if ((e = cudaMemcpyAsync(out_idx, di, sizeof(uint32_t) * (size_t)n_total * k, cudaMemcpyDeviceToHost,
                              ctx->stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(out_dist, dd, sizeof(float) * (size_t)n_total * k, cudaMemcpyDeviceToHost, ctx->stream)) !=
             cudaSuccess)
-        return cuda_fail(st, e, "download");
+        return host_call_failed(ctx, cuda_fail(st, e, "download"), st);
     return collect_device_errors(ctx, st);
 }
 
@@ -426,7 +427,7 @@ int32_t scrust_cuda_neighbors_graph_batch(scrust_context* ctx, const float* x, c
         rc = cuda_fail(st, e, "download");
     if (rc == SCRUST_OK) rc = csr_download(ctx, b, (uint64_t)n_total, (uint64_t)n_total, conn, st);
     csr_give(ctx, b);
-    if (rc) return rc;
+    if (rc) return host_call_failed(ctx, rc, st);
     if ((rc = collect_device_errors(ctx, st))) {
         scrust_csr_free(*conn);
         *conn = nullptr;

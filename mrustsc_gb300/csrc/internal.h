@@ -173,6 +173,9 @@ unsigned long long* sweep_stats(scrust_context* ctx);
 
 // Maps the device error block to a status, then clears it (synchronises).
 int32_t collect_device_errors(scrust_context* ctx, scrust_status* st);
+// The same at the end of a call on host arrays that failed with `rc`: the
+// device's error, if there is one, else rc.
+int32_t host_call_failed(scrust_context* ctx, int32_t rc, scrust_status* st);
 
 // Status helpers.
 int32_t fail(scrust_status* st, int32_t code, const char* fmt, ...);
