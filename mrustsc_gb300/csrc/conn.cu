@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(256) directed_bucket_kernel(const uint32_t* __
     bool kept = false;
     if (row_ok && j < k) {
         nb = idx[i * k + j];
-        if ((int64_t)nb != i) {
+        if ((int64_t)nb != i && (int64_t)nb < n) {
             const float sigma = sigmas[i], rho = rhos[i];
             const float offset = __fsub_rn(dist[i * k + j], rho);
             wt = (offset <= 0.f || sigma == 0.f) ? 1.0f : expf(__fdiv_rn(-offset, sigma));

@@ -184,6 +184,19 @@ __device__ void finalize_row(const Team& team, const RerankArgs& a, int64_t q,
     team.sync();
 }
 
+// A row without k columns that can be ranked (NaN coordinates, more ties than
+// the fallback holds): the first k columns of its solve other than itself, at
+// distance NaN, so that no later kernel meets an id that was never written.
+template <class Team>
+__device__ void write_open_row(const Team& team, const RerankArgs& a, int64_t q) {
+    const int64_t lo = a.row_lo ? (int64_t)a.row_lo[q] : 0, own = a.self ? q + a.self_offset : -1;
+    for (int t = team.rank; t < a.k; t += team.size()) {
+        const int64_t j = lo + t + (own >= 0 && lo + t >= own ? 1 : 0);
+        a.out_idx[q * a.k + t] = (uint32_t)(j - lo);
+        a.out_dist[q * a.k + t] = __int_as_float(0x7fc00000);
+    }
+}
+
 __device__ void push_fallback(const RerankArgs& a, int64_t slot) {
     uint32_t pos = atomicAdd(a.fb_count, 1u);
     a.fb_rows[pos] = (uint32_t)slot;
@@ -257,6 +270,10 @@ __global__ void __launch_bounds__(RR_WARPS * 32) rerank_warp_kernel(RerankArgs a
             B[m + __popc(ballot & lanemask_lt())] = ((unsigned long long)float_key(r) << 32) | id;
         }
         m += __popc(ballot);
+    }
+    if (m < a.k) {  // no threshold: bounds of NaN
+        write_open_row(team, a, q);
+        return;
     }
     __syncwarp();
     const int P = next_pow2(m);
@@ -1080,6 +1097,7 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
         if (first) {
             if (m > FB_CAP || m < a.k) {
                 if (tid == 0) atomicExch(a.err + (m > FB_CAP ? DERR_TIE_OVERFLOW : DERR_CANDIDATES), 1);
+                write_open_row(team, a, q);
             } else {
                 finalize_row(team, a, q, keys, m, dbl, flags);
             }
@@ -1100,7 +1118,7 @@ __global__ void __launch_bounds__(256) cosine_distances_kernel(RerankArgs a, int
     if (i >= total) return;
     const int64_t q = i / a.k;
     const uint32_t j = a.out_idx[i] + (a.row_lo ? a.row_lo[q] : 0u);
-    if ((int64_t)j >= a.cosine.n) return;  // a row that the rerank left open
+    if ((int64_t)j >= a.cosine.n) return;
     float h, l;
     cosine_pair(a.cosine, stride, q, (int64_t)j, &h, &l);
     a.out_dist[i] = rounds_surely(h, l, cosine_pair_error(stride, a.d))
