@@ -264,8 +264,11 @@ SCRUST_API int32_t scrust_cuda_knn_batch_device(scrust_context* context, const f
 /* A plan fixes the layout and the device buffers, autotunes the candidate
  * over-provisioning (the list capacity, when options->list_capacity is 0),
  * the sweep's form (its register top-k width, or one pass for thresholds and
- * one that collects) and the operand precision on this batch, and captures the whole solve in a CUDA graph.  Each launch is one graph
- * launch on the context stream. */
+ * one that collects) and the operand precision on this batch, and captures
+ * the whole solve in a CUDA graph.  Each launch is one graph launch on the
+ * context stream.  Other calls on the context may come between launches: the
+ * first launch after one that has grown the context's workspace runs the solve
+ * once more and captures it anew (and so may allocate and synchronise). */
 SCRUST_API scrust_batch_plan* scrust_cuda_batch_plan_create(scrust_context* context, const uint64_t* row_offsets,
                                                             uint32_t n_samples, uint64_t d, uint32_t k,
                                                             const scrust_knn_options* options,

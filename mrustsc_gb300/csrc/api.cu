@@ -44,7 +44,10 @@ int32_t cuda_fail(scrust_status* st, cudaError_t e, const char* what) {
 void* ws_get(scrust_context* ctx, Slot slot, size_t bytes, cudaError_t* err) {
     Workspace& ws = ctx->ws;
     if (bytes == 0) bytes = 16;
-    if (ws.ptr[slot] && ws.bytes[slot] >= bytes) return ws.ptr[slot];
+    if (ws.ptr[slot] && ws.bytes[slot] >= bytes) {
+        if (ctx->ws_log) ctx->ws_log->push_back(WorkspaceUse{slot, ws.ptr[slot], bytes});
+        return ws.ptr[slot];
+    }
     // Queued work may still read the old buffer.
     cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e == cudaSuccess && ws.ptr[slot]) e = cudaFree(ws.ptr[slot]);

@@ -20,13 +20,17 @@
 // A plan fixes the layout, the buffers and the options, autotunes the
 // candidate over-provisioning (list capacity), the register top-k width and
 // the operand precision on the actual batch, and captures the whole sequence
-// in a CUDA graph; each run is one graph launch.  The tile shape (two 128-row
+// in a CUDA graph; each run is one graph launch.  The graph holds addresses of
+// the context's workspace, which other calls on the context may move by growing
+// it: a launch that finds one moved runs the sequence once, which grows what it
+// needs, and captures it anew.  The tile shape (two 128-row
 // MMA halves against 256-column tiles, K = 64) is the sweep kernel's fixed
 // design and is not a tuning choice.
 #include <string.h>
 
 #include <algorithm>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -36,6 +40,7 @@ struct scrust_batch_plan {
     scrust_context* ctx = nullptr;
     uint32_t n_samples = 0;
     uint64_t n_total = 0, d = 0;
+    int64_t n_pad = 0;
     uint32_t k = 0;
     scrust_knn_options opts{};
     const float* x = nullptr;
@@ -44,6 +49,8 @@ struct scrust_batch_plan {
     void* table = nullptr;  // device copy of the sample table
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    std::vector<scrust::WorkspaceUse> uses;       // what the graph was given of the workspace
+    const unsigned long long* stats = nullptr;    // the kernel counters it writes, if any
     float tuned_ms = 0.f;
     int32_t topk_width = 0;            // the autotuner's choice: a register top-k width (0: by k, -1: lists) or kTwoPasses
     bool graphs = false;               // the launch also builds the connectivities
@@ -439,6 +446,66 @@ int32_t scrust_cuda_neighbors_graph_batch(scrust_context* ctx, const float* x, c
 
 namespace {
 
+// Whether the plan's graph may run: the workspace it was captured with is in
+// place, and so are the kernel counters.
+bool plan_current(const scrust_batch_plan* p) {
+    const Workspace& ws = p->ctx->ws;
+    for (const WorkspaceUse& u : p->uses)
+        if (ws.ptr[u.slot] != u.ptr || ws.bytes[u.slot] < u.bytes) return false;
+    return !p->stats || p->stats == p->ctx->d_stats;
+}
+
+// Runs the plan's sequence once, which sizes the workspace, then captures it
+// as the plan's graph (in place of an earlier one).
+int32_t plan_capture(scrust_batch_plan* p, scrust_status* st) {
+    scrust_context* ctx = p->ctx;
+    cudaError_t e = cudaSuccess;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if ((e = cudaStreamIsCapturing(ctx->stream, &capturing)) != cudaSuccess)
+        return cuda_fail(st, e, "batch plan: capture");
+    if (capturing != cudaStreamCaptureStatusNone)
+        return fail(st, SCRUST_KERNEL, "CUDA kernel batch plan: its workspace has moved since the last launch; launch "
+                                       "the plan once before it is captured");
+    auto enqueue = [&]() {
+        return batch_enqueue(ctx, p->x, p->table, p->n_samples, (int64_t)p->n_total, p->n_pad, (int)p->d, (int)p->k,
+                             p->opts, p->out_idx, p->out_dist, st, p->graphs ? &p->csr : nullptr, p->topk_width);
+    };
+    int32_t rc = enqueue();
+    if (rc == SCRUST_OK && (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+        rc = cuda_fail(st, e, "batch plan: synchronise");
+    if (rc) return rc;
+    std::vector<WorkspaceUse> uses;
+    uses.reserve(2 * SLOT_COUNT);
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    const bool timing = ctx->timing;
+    ctx->timing = false;
+    if ((e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal)) == cudaSuccess) {
+        ctx->ws_log = &uses;
+        rc = enqueue();
+        ctx->ws_log = nullptr;
+        const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
+        if (rc == SCRUST_OK && e2 != cudaSuccess) rc = cuda_fail(st, e2, "batch plan: capture");
+    } else {
+        rc = cuda_fail(st, e, "batch plan: capture");
+    }
+    ctx->timing = timing;
+    if (rc == SCRUST_OK && (e = cudaGraphInstantiate(&exec, graph, 0)) != cudaSuccess)
+        rc = cuda_fail(st, e, "batch plan: instantiate");
+    if (rc != SCRUST_OK) {
+        cudaGetLastError();
+        if (graph) cudaGraphDestroy(graph);
+        return rc;
+    }
+    if (p->exec) cudaGraphExecDestroy(p->exec);
+    if (p->graph) cudaGraphDestroy(p->graph);
+    p->graph = graph;
+    p->exec = exec;
+    p->uses = std::move(uses);
+    p->stats = ctx->d_stats;
+    return ok(st);
+}
+
 scrust_batch_plan* plan_create(scrust_context* ctx, const uint64_t* row_offsets, uint32_t n_samples, uint64_t d,
                                uint32_t k, const scrust_knn_options* opt, const float* x, uint32_t* out_idx,
                                float* out_dist, bool graphs, scrust_status* st) {
@@ -461,6 +528,7 @@ scrust_batch_plan* plan_create(scrust_context* ctx, const uint64_t* row_offsets,
     p->ctx = ctx;
     p->n_samples = n_samples;
     p->n_total = (uint64_t)n_total;
+    p->n_pad = n_pad;
     p->d = d;
     p->k = k;
     scrust_knn_options_default(&p->opts);
@@ -549,39 +617,15 @@ scrust_batch_plan* plan_create(scrust_context* ctx, const uint64_t* row_offsets,
     }
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
-    if (rc == SCRUST_OK) {
-        // Size the workspace for the chosen options, then capture.
-        rc = batch_enqueue(ctx, x, p->table, n_samples, n_total, n_pad, (int)d, (int)k, chosen.o, out_idx, out_dist,
-                           st, csr, chosen.width);
-        if (rc == SCRUST_OK && (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
-            rc = cuda_fail(st, e, "batch plan: synchronise");
-    }
-    if (rc == SCRUST_OK) {
-        const bool timing = ctx->timing;
-        ctx->timing = false;
-        e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            rc = batch_enqueue(ctx, x, p->table, n_samples, n_total, n_pad, (int)d, (int)k, chosen.o, out_idx,
-                               out_dist, st, csr, chosen.width);
-            const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &p->graph);
-            if (rc == SCRUST_OK && e2 != cudaSuccess) rc = cuda_fail(st, e2, "batch plan: capture");
-        } else {
-            rc = cuda_fail(st, e, "batch plan: capture");
-        }
-        ctx->timing = timing;
-        if (rc == SCRUST_OK && (e = cudaGraphInstantiate(&p->exec, p->graph, 0)) != cudaSuccess)
-            rc = cuda_fail(st, e, "batch plan: instantiate");
-    }
-    if (rc != SCRUST_OK) {
-        cudaGetLastError();
-        if (p->exec) cudaGraphExecDestroy(p->exec);
-        if (p->graph) cudaGraphDestroy(p->graph);
-        release();
-        return nullptr;
-    }
     p->opts = chosen.o;
     p->topk_width = chosen.width;
     p->tuned_ms = best;
+    if (rc == SCRUST_OK) rc = plan_capture(p, st);
+    if (rc != SCRUST_OK) {
+        cudaGetLastError();
+        release();
+        return nullptr;
+    }
     ok(st);
     return p;
 }
@@ -629,6 +673,8 @@ int32_t scrust_cuda_batch_plan_launch(scrust_batch_plan* p, scrust_status* st) {
     if (!p) return fail(st, SCRUST_SHAPE, "expected a batch plan");
     std::lock_guard<std::mutex> lock(p->ctx->mu);
     DeviceGuard device_guard(p->ctx->device);
+    int32_t rc = SCRUST_OK;
+    if (!plan_current(p) && (rc = plan_capture(p, st))) return rc;
     const cudaError_t e = cudaGraphLaunch(p->exec, p->ctx->stream);
     if (e != cudaSuccess) return cuda_fail(st, e, "batch plan: launch");
     p->ctx->launches += 1;

@@ -72,6 +72,14 @@ struct Workspace {
     size_t bytes[SLOT_COUNT] = {};
 };
 
+// What a captured graph was given of the workspace.  A slot that grows later
+// moves: the graph is good for as long as every use still holds.
+struct WorkspaceUse {
+    Slot slot;
+    void* ptr;
+    size_t bytes;
+};
+
 // Makes `device` current for the scope of a public entry point and gives the
 // calling thread its previous device back on return, so a call on a context
 // never changes which device the caller's own CUDA work goes to.
@@ -126,6 +134,7 @@ struct scrust_context {
     scrust::CsrStream csr_stream;        // the streamed download of kNN-graph connectivities
     std::mutex mu;
     scrust::Workspace ws;
+    std::vector<scrust::WorkspaceUse>* ws_log = nullptr;  // while a graph is captured: what ws_get hands out
     int* d_err = nullptr;          // scrust::DERR_COUNT ints
     uint32_t* d_counter = nullptr; // small device counters (fallback rows, work queue)
     std::vector<scrust::CsrBuffers> csr_pool;
