@@ -1143,7 +1143,9 @@ __device__ __forceinline__ int block_prefix(int v, int* wsum, int* total) {
 // a threshold from another cluster, and its block then every tile of the
 // atlas: 11,691 second tiles of 20 blocks for 5,000 queries of a million
 // cells, 3,651 of one block for 100.)
-// One block of 256 threads per query block; three tile bitmaps in shared memory.
+// One block of 256 threads per query block; three tile bitmaps in shared memory,
+// or two and no tiles of nearest neighbours for an atlas whose third does not
+// fit (from some 155 million cells on).
 constexpr int kQueryPrio = 512;
 constexpr int kQueryPrioNear = 256;
 constexpr int kQueryPrioNb = 8;
@@ -1162,16 +1164,16 @@ int column_segments(int most, int tiles, int items, int sms) {
 __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restrict__ cell_of_pos, int64_t n,
                                                          const uint32_t* __restrict__ cell_start, int m,
                                                          const uint32_t* __restrict__ cell_nb, int col_tiles,
-                                                         uint32_t want, uint32_t* __restrict__ prio,
+                                                         uint32_t want, int maps, uint32_t* __restrict__ prio,
                                                          uint32_t* __restrict__ prio_cnt) {
     extern __shared__ uint32_t qp_bm[];
     __shared__ int wsum[8];
     const int words = (col_tiles + 31) / 32;
     uint32_t* home = qp_bm;
     uint32_t* more = qp_bm + words;
-    uint32_t* near = qp_bm + 2 * words;
+    uint32_t* near = maps == 3 ? qp_bm + 2 * words : nullptr;
     const int I = blockIdx.x;
-    for (int i = threadIdx.x; i < 3 * words; i += blockDim.x) qp_bm[i] = 0u;
+    for (int i = threadIdx.x; i < maps * words; i += blockDim.x) qp_bm[i] = 0u;
     __syncthreads();
     const int64_t p = (int64_t)I * 256 + threadIdx.x;
     // Marks the tiles of cell c; its rows.
@@ -1192,7 +1194,8 @@ __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restr
                 const uint32_t* nb = cell_nb + (int64_t)c * kAnchorNeighbours;
                 int j = 0;
                 for (; j < kAnchorNeighbours && rows < want; ++j) rows += mark(more, nb[j]);
-                for (const int j1 = min(j + kQueryPrioNb, kAnchorNeighbours); j < j1; ++j) mark(near, nb[j]);
+                if (near)
+                    for (const int j1 = min(j + kQueryPrioNb, kAnchorNeighbours); j < j1; ++j) mark(near, nb[j]);
             }
         }
     }
@@ -1216,11 +1219,13 @@ __global__ void __launch_bounds__(256) query_prio_kernel(const uint32_t* __restr
     int taken = keep(home, kQueryPrio);
     for (int w = w0; w < w1; ++w) more[w] &= ~home[w];
     taken += keep(more, kQueryPrio - taken);
-    for (int w = w0; w < w1; ++w) near[w] &= ~(home[w] | more[w]);
-    keep(near, max(0, kQueryPrioNear - taken));
+    if (near) {
+        for (int w = w0; w < w1; ++w) near[w] &= ~(home[w] | more[w]);
+        keep(near, max(0, kQueryPrioNear - taken));
+    }
     int c = 0, total = 0;
     for (int w = w0; w < w1; ++w) {
-        home[w] |= more[w] | near[w];
+        home[w] |= more[w] | (near ? near[w] : 0u);
         c += __popc(home[w]);
     }
     int at = block_prefix(c, wsum, &total);
@@ -1902,11 +1907,12 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
         (e = launch_gather_rows(dq, qperm, q, d, P, xs, s)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: gather");
     // Priority tiles per row block, dealt over its column segments.
-    const size_t prio_smem = 12 * (size_t)words_t;
+    const int maps = 12 * (size_t)words_t + 1024 <= ctx->smem_optin ? 3 : 2;
+    const size_t prio_smem = 4 * maps * (size_t)words_t;
     if ((e = set_smem_limit(ctx, (const void*)query_prio_kernel, (int)prio_smem)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: priority tiles");
     query_prio_kernel<<<items, 256, prio_smem, s>>>(cell_of_pos, q, at.cell_start, (int)at.anchors, at.cell_nb,
-                                                    col_tiles, 16u * (uint32_t)k, prio, prio_cnt);
+                                                    col_tiles, 16u * (uint32_t)k, maps, prio, prio_cnt);
     split_lists_kernel<<<items, 256, 0, s>>>(prio, kQueryPrio, prio_cnt, csegs, (uint32_t*)(base + o_ps), ps,
                                              (uint32_t*)(base + o_psc));
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(st, e, "query routing: priority tiles");
