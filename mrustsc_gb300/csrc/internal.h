@@ -303,7 +303,14 @@ void atlas_order_free(AtlasOrder* o);
 // pass over both, the sorted rerank.  `words` are the atlas's.
 int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const float* atlas_rows, const double* means,
                               const uint32_t* words, const float* dq, int64_t q, int k, uint32_t* d_idx,
-                              float* d_dist, scrust_status* st);
+                              float* d_dist, scrust_status* st, int most_segments);
+// Column segments of a row block of a routed batch at most, so 128 lists of a
+// row.  (With 16, few queries left most of the chip idle: 30, 300 and 1,000 of a
+// million cells took 427, 1,220 and 855 us, and 334, 609 and 634 us with 64.)
+constexpr int kQuerySegments = 64;
+// What the lists, thresholds and top-K values of a routed batch take of the
+// workspace when its row blocks have `most_segments` segments at most.
+size_t routed_list_bytes(const AtlasOrder& at, int64_t q, int k, int sm_count, int most_segments);
 // After the priority pass: the column tiles each row block still has to
 // visit, from tile bounding balls and the rows' thresholds (order.cu).
 int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64_t n, int d, const RowOrder& order,

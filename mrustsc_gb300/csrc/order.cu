@@ -1149,11 +1149,6 @@ __device__ __forceinline__ int block_prefix(int v, int* wsum, int* total) {
 constexpr int kQueryPrio = 512;
 constexpr int kQueryPrioNear = 256;
 constexpr int kQueryPrioNb = 8;
-// Column segments of a row block at most, so 128 lists of a row.  (With 16, few
-// queries left most of the chip idle: 30, 300 and 1,000 of a million cells took
-// 427, 1,220 and 855 us, and 334, 609 and 634 us with 64.)
-constexpr int kQuerySegments = 64;
-
 // Column segments that give two work items an SM where `tiles` tiles and `most`
 // allow it, and that cutting the tiles into equal runs reproduces.
 int column_segments(int most, int tiles, int items, int sms) {
@@ -1792,9 +1787,23 @@ int32_t atlas_order_build(scrust_context* ctx, const float* atlas, int64_t m, in
     return ok(st);
 }
 
+namespace {
+constexpr int kRoutedCap = 256, kRoutedTotal = 256 + 128;  // a routed batch's lists: capacity and storage
+}
+
+size_t routed_list_bytes(const AtlasOrder& at, int64_t q, int k, int sm_count, int most_segments) {
+    const int64_t q_pad = (q + 255) / 256 * 256;
+    const int col_tiles = (int)(at.m_pad / 256);
+    const size_t lists = 2 * (size_t)column_segments(std::min(most_segments, kQuerySegments), col_tiles,
+                                                     (int)(q_pad / 256), sm_count);
+    const size_t top = k < 2 ? 0 : k <= 16 ? 16 : 32;
+    const size_t row = lists * (kRoutedTotal * 8 + 4 + 4 + 4 * top) + 8;  // ids and values, count, threshold, top-K
+    return (size_t)q_pad * row * 9 / 8;                                   // the workspace grows by an eighth more
+}
+
 int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const float* atlas_rows, const double* means,
                               const uint32_t* words, const float* dq, int64_t q, int k, uint32_t* d_idx,
-                              float* d_dist, scrust_status* st) {
+                              float* d_dist, scrust_status* st, int most_segments) {
     cudaStream_t s = ctx->stream;
     cudaError_t e = cudaSuccess;
     const int d = at.d;
@@ -1804,7 +1813,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     // Column segments per row block, so that a small batch still fills the
     // GPU: each segment of a block is its own work item, and the segments of
     // a row share its threshold through HBM.
-    const int csegs = column_segments(kQuerySegments, col_tiles, items, ctx->sm_count);
+    const int csegs = column_segments(std::min(most_segments, kQuerySegments), col_tiles, items, ctx->sm_count);
     // The anchors likewise: one query had one CTA pass over all 16 tiles of
     // 3,906 anchors (23 us of its 320; 8 in 16 segments).
     const int anchor_tiles = (int)(at.anchors_pad / 256);
@@ -1853,8 +1862,8 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     unsigned long long* best = (unsigned long long*)(base + o_best);
 
     Lists lists;
-    lists.cap = 256;
-    lists.ctot = 256 + 128;
+    lists.cap = kRoutedCap;
+    lists.ctot = kRoutedTotal;
     lists.segments = 2 * csegs;
     int32_t rc = alloc_lists(ctx, q_pad, &lists, st, false);
     if (rc) return rc;

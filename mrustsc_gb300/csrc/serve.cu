@@ -124,6 +124,21 @@ size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 constexpr int64_t kRoutedMinQueries = 1;
 
+bool is_routed(const scrust_server* sv, int64_t q) { return sv->ordered && q >= sv->routed_min; }
+
+// Column segments that a routed batch of q cells may have: as many as help, in
+// a slot's share of what the budget leaves beside the atlas (a slot's workspace
+// keeps the most its batches took).  Admission counts cells, at 50 KB for k =
+// 15; more segments give few queries more of the chip and take up to 393 KB a
+// padded row at 64, one takes 6.
+int batch_segments(const scrust_server* sv, int64_t q) {
+    if (!is_routed(sv, q)) return kQuerySegments;
+    const uint64_t room = (sv->budget - sv->atlas_bytes) / sv->slots.size();
+    int most = kQuerySegments;
+    while (most > 1 && routed_list_bytes(sv->order, q, sv->k, sv->slots[0].ctx->sm_count, most) > room) most /= 2;
+    return most;
+}
+
 // Query rows of one batch against the atlas, on the slot's stream.
 int32_t cross_enqueue(scrust_server* sv, scrust_context* ctx, const float* dq, int64_t q, uint32_t* d_idx,
                       float* d_dist, CsrBuffers* csr, scrust_status* st) {
@@ -140,10 +155,10 @@ int32_t cross_enqueue(scrust_server* sv, scrust_context* ctx, const float* dq, i
     // at 500k atlas cells: 0.6 ms against 0.8 ms for one query, 1.3 against
     // 2.0 ms for 1000, 4.9 against 14.3 ms for 20,000); the sweep of every
     // tile stays for unordered atlases.
-    const bool routed = sv->ordered && q >= sv->routed_min;
-    int32_t rc = routed ? cross_ordered_enqueue(ctx, sv->order, sv->atlas, sv->means, sv->words, dq, q, sv->k, d_idx,
-                                                d_dist, st)
-                        : cross_knn_enqueue(ctx, ref, dq, q, sv->k, -1, d_idx, d_dist, st);
+    int32_t rc = is_routed(sv, q)
+                     ? cross_ordered_enqueue(ctx, sv->order, sv->atlas, sv->means, sv->words, dq, q, sv->k, d_idx, d_dist,
+                                             st, batch_segments(sv, q))
+                     : cross_knn_enqueue(ctx, ref, dq, q, sv->k, -1, d_idx, d_dist, st);
     if (rc) return rc;
     return run_query_connectivities(ctx, d_idx, d_dist, q, sv->k, csr, st);
 }
