@@ -1042,17 +1042,8 @@ __global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ 
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
     const int64_t j0 = (int64_t)blockIdx.x * 64;
     const int r = threadIdx.x % 64, part = threadIdx.x / 64;
-    float c2 = 0.f;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {  // (the centres come dimension by dimension)
-        const int t = part + 4 * c;
-        const float v = j0 + r < asegs && t < d ? __ldg(act + (int64_t)t * asegs + j0 + r) : 0.f;
-        Bs[t][r] = v;
-        c2 += v * v;
-    }
-    centre2[part][r] = c2;
     // (gridDim.y is 65,535 at most: more groups of queries take turns.)
-    for (int64_t i0 = (int64_t)blockIdx.y * 64; i0 < q; i0 += (int64_t)gridDim.y * 64) {
+    for (int64_t i0 = (int64_t)blockIdx.y * 64;;) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             const int t = 8 * (part + 4 * c);
@@ -1062,6 +1053,15 @@ __global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ 
 #pragma unroll
             for (int e = 0; e < 8; ++e) As[t + e][r] = t + e < d ? op_float(v[e]) : 0.f;
         }
+        float c2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {  // (the centres come dimension by dimension)
+            const int t = part + 4 * c;
+            const float v = j0 + r < asegs && t < d ? __ldg(act + (int64_t)t * asegs + j0 + r) : 0.f;
+            Bs[t][r] = v;
+            c2 += v * v;
+        }
+        centre2[part][r] = c2;
         if (threadIdx.x < 64) {
             hit[threadIdx.x] = 0u;
             const int64_t i = i0 + threadIdx.x;
@@ -1106,6 +1106,8 @@ __global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ 
             const uint32_t tile = ao[j0 + threadIdx.x];
             atomicOr(bitmap + i0 / 256 * words + (tile >> 5), 1u << (tile & 31));
         }
+        i0 += (int64_t)gridDim.y * 64;
+        if (i0 >= q) return;
         __syncthreads();
     }
 }
@@ -1149,6 +1151,7 @@ __device__ __forceinline__ int block_prefix(int v, int* wsum, int* total) {
 constexpr int kQueryPrio = 512;
 constexpr int kQueryPrioNear = 256;
 constexpr int kQueryPrioNb = 8;
+
 // Column segments that give two work items an SM where `tiles` tiles and `most`
 // allow it, and that cutting the tiles into equal runs reproduces.
 int column_segments(int most, int tiles, int items, int sms) {
