@@ -12,13 +12,15 @@
 // for an ordering); anchor neighbourhoods from an FP32 anchors x anchors kNN.
 //
 // The sweep then runs in two passes.  The first visits only the priority
-// tiles and leaves every list with a threshold.  Between the passes each
-// column tile gets a bounding ball of its quantised rows (centre c_T, radius
-// R_T) and each row block the largest distance U_I that can still matter:
-// the MMA value of a pair is at least |a_i - b_j|^2 - A_i - delta_i, so a
-// column j can join row i's list only while |a_i - b_j| < sqrt(theta_i + A_i
-// + delta_i).  A tile with |c_I - c_T| - R_I - R_T >= U_I cannot add to any
-// row of block I and is left out of the second pass, which visits the rest.
+// tiles and leaves every row with a threshold.  Between the passes the rows of
+// each cell within a 256-row block (a segment) get a bounding ball of their
+// quantised values (centre c, radius R) and the largest distance U that can
+// still matter to one of them: the MMA value of a pair is at least
+// |a_i - b_j|^2 - A_i - delta_i, so a column j can join row i's list only while
+// |a_i - b_j| < sqrt(theta_i + A_i + delta_i).  A tile all of whose segments t
+// have |c_s - c_t| - R_s - R_t >= U_s for every segment s of a row block cannot
+// add to any row of it and is left out of the collect pass, which visits the
+// rest.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -581,18 +583,14 @@ __device__ __forceinline__ float op_bits<__nv_bfloat16>(uint32_t w) {
     return __bfloat162float(__ushort_as_bfloat16((unsigned short)(w & 0xffffu)));
 }
 
-// Balls of one tile: the whole tile and each of its cell segments (runs of
-// rows of one cell; a cell lies in one region of the data, while a tile
-// may straddle two far-apart cells).  Segments past kSegMax merge into the
-// last.  Centres are stored dimension-major for coalesced pair tests.
-// Segments past kSegMax share one ball, which then reaches everywhere: with 8,
-// one block of a million cells kept all 3,900 tiles and its CTA took 6.4 ms of
-// a collect pass of 1.3 ms.
+// Balls of a tile's cell segments (runs of rows of one cell; a cell lies in one
+// region of the data, while a tile may straddle two far-apart cells).  Centres
+// are stored dimension-major for coalesced pair tests.
+// Segments past kSegMax share the last ball, which then reaches everywhere: with
+// 8, one block of a million cells kept all 3,900 tiles and its CTA took 6.4 ms
+// of a collect pass of 1.3 ms.
 constexpr int kSegMax = 32;
 struct TileBalls {
-    float* centre;      // [d][tiles]
-    float* radius;      // [tiles]
-    float* reach;       // [tiles]
     float* seg_centre;  // [kSegMax][d][tiles]
     float* seg_radius;  // [kSegMax][tiles]
     float* seg_reach;   // [kSegMax][tiles]
@@ -600,22 +598,19 @@ struct TileBalls {
 };
 
 // One block of 256 threads per column tile (= row block, the solve being a
-// self-kNN): centres (means) and radii of the tile's quantised rows, and the
-// reach U = max over the rows of sqrt(theta + A + delta), theta being the
-// smaller of the row's two list thresholds.
+// self-kNN): centres (means) and radii of the quantised rows of its segments,
+// and the reach U = max over the rows of sqrt(theta + A + delta), theta being
+// the smaller of the row's two list thresholds.
 template <class T, int BLOCKS>
 __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ ops, int64_t n, int d, int tiles,
                                                          const uint32_t* __restrict__ cell_of_pos,
                                                          const float* __restrict__ theta, const float* __restrict__ bA,
                                                          const float* __restrict__ bdelta, TileBalls b) {
     constexpr int W = 64 * BLOCKS;  // halves per operand row
-    __shared__ float part[8][W];
-    __shared__ float centre[W];
     __shared__ float scentre[kSegMax][W];
     __shared__ int sstart[kSegMax + 1];
     __shared__ int wheads[8];
-    __shared__ uint32_t rmax_all, rmax_seg[kSegMax];
-    __shared__ uint32_t umax_all, umax_seg[kSegMax];
+    __shared__ uint32_t rmax_seg[kSegMax], umax_seg[kSegMax];
     const int tile = blockIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t j = (int64_t)tile * 256 + threadIdx.x;
@@ -636,10 +631,6 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
     const bool head = valid && (threadIdx.x == 0 || cell_of_pos[j] != cell_of_pos[j - 1]);
     const uint32_t hb = __ballot_sync(0xffffffffu, head);
     if (lane == 0) wheads[w] = __popc(hb);
-    if (threadIdx.x == 0) {
-        rmax_all = 0u;
-        umax_all = 0u;
-    }
     if (threadIdx.x < kSegMax) {
         rmax_seg[threadIdx.x] = 0u;
         umax_seg[threadIdx.x] = 0u;
@@ -654,21 +645,7 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
     const int seg = min(before + __popc(hb & lanemask_lt()) + (head ? 1 : 0) - 1, kSegMax - 1);
     if (head && seg == before + __popc(hb & lanemask_lt())) sstart[seg] = threadIdx.x;
     if (threadIdx.x == 0) sstart[nseg] = rows;
-#pragma unroll
-    for (int t = 0; t < W; ++t) {
-        if (t < d) {
-            float v = valid ? op_bits<T>(rw[t >> 1] >> (16 * (t & 1))) : 0.f;
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) part[w][t] = v;
-        }
-    }
     __syncthreads();
-    if (threadIdx.x < d) {
-        float sum = 0.f;
-        for (int q = 0; q < 8; ++q) sum += part[q][threadIdx.x];
-        centre[threadIdx.x] = sum / (float)rows;
-        b.centre[(int64_t)threadIdx.x * tiles + tile] = centre[threadIdx.x];
-    }
     for (int p = threadIdx.x; p < nseg * d; p += blockDim.x) {
         const int sg = p / d, t = p % d;
         float sum = 0.f;
@@ -679,37 +656,30 @@ __global__ void __launch_bounds__(256) tile_balls_kernel(const T* __restrict__ o
     }
     __syncthreads();
     if (valid) {
-        // Squared distances to both centres in f32: a sum of d non-negative
+        // The squared distance to the centre in f32: a sum of d non-negative
         // rounded squares of rounded differences is at most (d + 2) units of
         // the last place below the exact value, so scaling by
         // 1 + (d + 4) 2^-23 (rounded up) bounds it from above.
-        float r2 = 0.f, s2 = 0.f;
+        float s2 = 0.f;
 #pragma unroll
         for (int t = 0; t < W; ++t) {
             if (t < d) {
-                const float v = op_bits<T>(rw[t >> 1] >> (16 * (t & 1)));
-                const float df = v - centre[t], ds = v - scentre[seg][t];
-                r2 = fmaf(df, df, r2);
+                const float ds = op_bits<T>(rw[t >> 1] >> (16 * (t & 1))) - scentre[seg][t];
                 s2 = fmaf(ds, ds, s2);
             }
         }
         const float grow = 1.0f + (float)(d + 4) * 1.1920929e-07f;
-        r2 = __fmul_ru(r2, grow);
         s2 = __fmul_ru(s2, grow);
         const float th = fminf(theta[2 * j], theta[2 * j + 1]);
         // The reach sqrt(theta + A + delta), every step rounded up.
         const float v = __fadd_ru(__fadd_ru(th, bA[j]), bdelta[j]);
         const float u = isinf(th) && th > 0.f ? th : (v > 0.f ? __fsqrt_ru(v) : 0.f);
         // Non-negative floats order like their bit patterns.
-        atomicMax(&rmax_all, __float_as_uint(r2));
         atomicMax(&rmax_seg[seg], __float_as_uint(s2));
-        atomicMax(&umax_all, __float_as_uint(u));
         atomicMax(&umax_seg[seg], __float_as_uint(u));
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        b.radius[tile] = __fmul_ru(__fsqrt_ru(__uint_as_float(rmax_all)), 1.0f + 1e-6f);
-        b.reach[tile] = __uint_as_float(umax_all);
         b.nseg[tile] = (uint32_t)nseg;
         if (tile == 0) b.nseg[tiles] = 0u;  // for the scan
     }
@@ -1594,8 +1564,7 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
     const int blocks = operand_blocks(d);
     const int64_t smax = (int64_t)tiles * kSegMax;
     const size_t scan_elems = scan_scratch_elems((int64_t)tiles + 1);
-    const size_t o_c = take(4 * (size_t)d * tiles), o_r = take(4 * (size_t)tiles), o_u = take(4 * (size_t)tiles),
-                 o_sc = take(4 * (size_t)kSegMax * d * tiles), o_sr = take(4 * (size_t)kSegMax * tiles),
+    const size_t o_sc = take(4 * (size_t)kSegMax * d * tiles), o_sr = take(4 * (size_t)kSegMax * tiles),
                  o_su = take(4 * (size_t)kSegMax * tiles), o_ns = take(4 * ((size_t)tiles + 1)),
                  o_so = take(4 * ((size_t)tiles + 1)), o_fc = take(4 * 64 * blocks * (size_t)smax), o_fr = take(4 * (size_t)smax),
                  o_fu = take(4 * (size_t)smax), o_fo = take(4 * (size_t)smax), o_scan = take(4 * scan_elems),
@@ -1604,9 +1573,6 @@ int32_t build_second_pass(scrust_context* ctx, const void* A16, bool bf16, int64
     char* base = (char*)ws_get(ctx, SLOT_PRUNE, off, &e);
     if (!base) return cuda_fail(st, e, "pruning: workspace");
     TileBalls balls;
-    balls.centre = (float*)(base + o_c);
-    balls.radius = (float*)(base + o_r);
-    balls.reach = (float*)(base + o_u);
     balls.seg_centre = (float*)(base + o_sc);
     balls.seg_radius = (float*)(base + o_sr);
     balls.seg_reach = (float*)(base + o_su);
@@ -1667,9 +1633,6 @@ size_t carve_balls(char* base, size_t at, int tiles, int d, TileBalls* b) {
         at = align_up(at + bytes);
         return base + a;
     };
-    b->centre = (float*)take(4 * (size_t)d * tiles);
-    b->radius = (float*)take(4 * (size_t)tiles);
-    b->reach = (float*)take(4 * (size_t)tiles);
     b->seg_centre = (float*)take(4 * (size_t)kSegMax * d * tiles);
     b->seg_radius = (float*)take(4 * (size_t)kSegMax * tiles);
     b->seg_reach = (float*)take(4 * (size_t)kSegMax * tiles);
