@@ -1496,7 +1496,7 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
         // Two operand blocks: the passes of an ordered self solve.
         smem = SweepShape<2>::SMEM_BYTES;
         kern = topk == 1 ? (argmin_out ? tensor_candidates_kernel<1, 3, 2> : tensor_candidates_kernel<1, 0, 2>)
-               : topk == 0 ? tensor_candidates_kernel<0, 0, 2>
+               : topk == 0 ? nullptr
                : a.thr_only ? (topk == 16 ? tensor_candidates_kernel<16, 1, 2> : tensor_candidates_kernel<32, 1, 2>)
                : a.collect && a.self
                    ? (topk == 16 ? tensor_candidates_kernel<16, 2, 2> : tensor_candidates_kernel<32, 2, 2>)
