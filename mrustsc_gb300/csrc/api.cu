@@ -475,7 +475,6 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
             TileLists second;
             if ((rc = build_second_pass(ctx, A16, bf16, n, d, order, bA, bdelta, &second, st))) return rc;
             mark(ctx, PH_LISTS);
-            mark(ctx, PH_PASS2);
             TileLists both = first;
             both.tiles2 = second.tiles;
             both.count2 = second.count;
@@ -484,7 +483,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
                                               false, order.theta, nullptr, sweep_stats(ctx), nullptr, kPassCollect)) !=
                 cudaSuccess)
                 return cuda_fail(st, e, "knn_candidates_tc");
-            mark(ctx, PH_COLLECT1);
+            mark(ctx, PH_COLLECT);
             ctx->launches += 1;
         } else {
             // Every list keeps its threshold, so the rerank needs no selection.
@@ -1176,9 +1175,9 @@ int32_t scrust_cuda_phase_times(scrust_context* ctx, float* ms, int32_t max_phas
         ms[written++] = t;
     }
     // Inside the candidates phase of an ordered solve: the first sweep pass,
-    // the building of the collect pass's second tile lists, a place where no
-    // pass is run, and the collect pass.
-    const int sub[4][2] = {{PH_PREP, PH_PASS1}, {PH_PASS1, PH_LISTS}, {PH_LISTS, PH_PASS2}, {PH_PASS2, PH_COLLECT1}};
+    // the building of the collect pass's second tile lists, nothing (the place
+    // of a second threshold pass, which no solve runs), and the collect pass.
+    const int sub[4][2] = {{PH_PREP, PH_PASS1}, {PH_PASS1, PH_LISTS}, {PH_LISTS, PH_LISTS}, {PH_LISTS, PH_COLLECT}};
     for (int i = 0; i < 4 && written < max_phases; ++i) {
         float t = 0.f;
         if (!(ctx->ev_recorded[sub[i][0]] && ctx->ev_recorded[sub[i][1]] &&

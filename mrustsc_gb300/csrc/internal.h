@@ -146,8 +146,8 @@ struct scrust_context {
     unsigned long long* d_stats = nullptr;
     int stats_launch = 0;               // sweep launches of the current solve so far
     bool timing = false;
-    cudaEvent_t ev[9] = {};             // phase boundaries: prep | candidates | rerank | connectivities, and
-    bool ev_recorded[9] = {};           // inside candidates: sweep pass 1 | tile lists | pass 2 | collect 1
+    cudaEvent_t ev[8] = {};             // phase boundaries: prep | candidates | rerank | connectivities, and
+    bool ev_recorded[8] = {};           // inside candidates: threshold pass | tile lists | collect pass
     std::vector<const void*> carveouts;  // kernels whose shared-memory carveout is set
 };
 
@@ -173,8 +173,8 @@ namespace scrust {
 
 // Phase boundary events (no-ops unless timing is enabled).
 enum Phase {
-    PH_START = 0, PH_PREP = 1, PH_CAND = 2, PH_RERANK = 3, PH_CONN = 4, PH_PASS1 = 5, PH_LISTS = 6, PH_PASS2 = 7,
-    PH_COLLECT1 = 8, PH_COUNT = 9
+    PH_START = 0, PH_PREP = 1, PH_CAND = 2, PH_RERANK = 3, PH_CONN = 4, PH_PASS1 = 5, PH_LISTS = 6, PH_COLLECT = 7,
+    PH_COUNT = 8
 };
 static_assert(sizeof(scrust_context::ev) / sizeof(cudaEvent_t) == PH_COUNT, "one event per phase boundary");
 void mark(scrust_context* ctx, Phase p);
