@@ -387,7 +387,7 @@ int32_t knn_device_impl(scrust_context* ctx, const float* x, uint64_t n64, uint6
         // An ordered solve has its operands in list order already, and their bounds.
         if (!order_rows) {
             if ((e = launch_tensor_operands(xwork, n, n_pad, d, means, max_bits, cosine, bf16, nullptr, A16, B16, bA,
-                                            beps, max_bits + 1, max_bits + 2, s)) != cudaSuccess)
+                                            beps, max_bits + 1, max_bits + 2, ctx->sm_count, s)) != cudaSuccess)
                 return cuda_fail(st, e, "tensor operands");
             if ((e = launch_tensor_bounds(n, d, bA, beps, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess)
                 return cuda_fail(st, e, "tensor bounds");

@@ -207,7 +207,7 @@ int32_t batch_enqueue(scrust_context* ctx, const float* x, const void* table, ui
         (e = launch_column_means_centre(xwork, n_total, d, means, means + d, s)) != cudaSuccess ||
         (e = launch_max_centred_norm(xwork, n_total, d, means, max_bits, ctx->sm_count, s)) != cudaSuccess ||
         (e = launch_tensor_operands(xwork, n_pad, n_pad, d, means, max_bits, cosine, bf16, row_map, A16, B16, bA, beps,
-                                    max_bits + 1, max_bits + 2, s)) != cudaSuccess ||
+                                    max_bits + 1, max_bits + 2, ctx->sm_count, s)) != cudaSuccess ||
         (e = launch_tensor_bounds(n_pad, d, bA, beps, max_bits + 1, max_bits + 2, bdelta, beps2, s)) != cudaSuccess)
         return cuda_fail(st, e, "batch: prep");
     ctx->launches += 5;

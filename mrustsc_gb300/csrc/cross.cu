@@ -38,7 +38,7 @@ int32_t reference_prepare(scrust_context* ctx, const float* x, int64_t n, int d,
         (e = launch_column_means_centre(x, n, d, means, means + d, s)) != cudaSuccess ||
         (e = launch_max_centred_norm(x, n, d, means, words, ctx->sm_count, s)) != cudaSuccess ||
         (e = launch_tensor_operands(x, n, n_pad, d, means, words, false, bf16, nullptr, A16, B16, terms + 2 * n_pad,
-                                    terms + 3 * n_pad, words + 1, words + 2, s)) != cudaSuccess)
+                                    terms + 3 * n_pad, words + 1, words + 2, ctx->sm_count, s)) != cudaSuccess)
         return cuda_fail(st, e, "reference: operands");
     ctx->launches += 4;
     out->rows = x;
@@ -67,7 +67,7 @@ int32_t cross_knn_enqueue(scrust_context* ctx, const Reference& ref, const float
     float *bA = rb, *eps = rb + q_pad, *bdelta = rb + 2 * q_pad, *beps2 = rb + 3 * q_pad;
     uint32_t* scratch_words = (uint32_t*)(rb + 4 * q_pad);
     if ((e = launch_tensor_operands(dq, q, q_pad, d, ref.means, ref.words, false, ref.bf16, nullptr, A16, B16, bA, eps,
-                                    scratch_words, scratch_words + 1, s)) != cudaSuccess ||
+                                    scratch_words, scratch_words + 1, ctx->sm_count, s)) != cudaSuccess ||
         (e = launch_tensor_bounds(q, d, bA, eps, ref.words + 1, ref.words + 2, bdelta, beps2, s)) != cudaSuccess)
         return cuda_fail(st, e, "cross: query operands");
     const int items = (int)(q_pad / 256), col_tiles = (int)(ref.n_pad / 256);

@@ -367,7 +367,7 @@ cudaError_t launch_plain_candidates(scrust_context* ctx, const KnnPlan& plan, co
 cudaError_t launch_tensor_operands(const float* x, int64_t n, int64_t n_pad, int d, const double* means,
                                    const uint32_t* max_norm_bits, bool cosine, bool bf16, const uint32_t* perm,
                                    void* A16, void* B16, float* bA, float* eps, uint32_t* max_eps_bits,
-                                   uint32_t* max_bhat_bits, cudaStream_t s);
+                                   uint32_t* max_bhat_bits, int sm_count, cudaStream_t s);
 cudaError_t launch_tensor_bounds(int64_t n, int d, const float* bA, const float* eps, const uint32_t* max_eps_bits,
                                  const uint32_t* max_bhat_bits, float* bdelta, float* beps2, cudaStream_t s);
 // Explicit column tiles per row block of the query rows.

@@ -1231,8 +1231,7 @@ __device__ __forceinline__ uint32_t bits16(__nv_bfloat16 v) { return (uint32_t)_
 //
 // Bound by the bytes: a row's lanes read and write neighbouring words.  A
 // million rows of 50: a thread a row and a warp's atomics for the maxima, 209
-// us; 132 us so.  kOperandBlocks: eight blocks an SM; each ends with two atomics.
-constexpr int kOperandBlocks = 8 * 152;
+// us; 132 us so, eight blocks an SM, each of which ends with two atomics.
 __device__ __forceinline__ void pair_add(float& h, float& l, float x, float xl) {
     const float sum = __fadd_rn(h, x), bv = __fsub_rn(sum, h);
     l = __fadd_rn(__fadd_rn(l, xl), __fadd_rn(__fsub_rn(h, __fsub_rn(sum, bv)), __fsub_rn(x, bv)));
@@ -1358,10 +1357,10 @@ __global__ void tensor_bounds_kernel(int64_t n, int terms, const float* __restri
 cudaError_t launch_tensor_operands(const float* x, int64_t n, int64_t n_pad, int d, const double* means,
                                    const uint32_t* max_norm_bits, bool cosine, bool bf16, const uint32_t* perm,
                                    void* A16, void* B16, float* bA, float* eps, uint32_t* max_eps_bits,
-                                   uint32_t* max_bhat_bits, cudaStream_t s) {
+                                   uint32_t* max_bhat_bits, int sm_count, cudaStream_t s) {
     const int wide = operand_blocks(d);
     if (n_pad % 256) return cudaErrorInvalidValue;
-    const unsigned blocks = (unsigned)std::min<int64_t>((n_pad * 8 * wide + 255) / 256, kOperandBlocks);
+    const unsigned blocks = (unsigned)std::min<int64_t>((n_pad * 8 * wide + 255) / 256, 8 * (int64_t)sm_count);
     if (bf16) {
         const auto kern = wide == 1 ? tensor_operands_kernel<__nv_bfloat16, 1> : tensor_operands_kernel<__nv_bfloat16, 2>;
         kern<<<blocks, 256, 0, s>>>(x, n, n_pad, d, means, max_norm_bits, cosine ? 1 : 0, perm, (__nv_bfloat16*)A16,

@@ -1481,9 +1481,9 @@ int32_t build_row_order(scrust_context* ctx, const float* x, int64_t n, int d, c
     float* bA0 = (float*)(base + o_bA0);
     float* eps0 = (float*)(base + o_eps0);
     if ((e = launch_tensor_operands(x, n, n_pad, d, means, max_bits, cosine, bf16, nullptr, A0, B0, bA0, eps0,
-                                    max_bits + 1, max_bits + 2, s)) != cudaSuccess ||
+                                    max_bits + 1, max_bits + 2, ctx->sm_count, s)) != cudaSuccess ||
         (e = launch_tensor_operands(x, m, m_pad, d, means, max_bits, cosine, bf16, src, base + o_aA, base + o_aB, arb,
-                                    arb + m_pad, max_bits + 1, max_bits + 2, s)) != cudaSuccess)
+                                    arb + m_pad, max_bits + 1, max_bits + 2, ctx->sm_count, s)) != cudaSuccess)
         return cuda_fail(st, e, "ordering: operands");
     ctx->launches += 3;
 
@@ -1845,7 +1845,7 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     set_words_kernel<<<(unsigned)std::min<int64_t>((longest + 255) / 256, 4 * ctx->sm_count), 256, 0, s>>>(runs);
     if ((e = cudaGetLastError()) != cudaSuccess ||
         (e = launch_tensor_operands(dq, q, q_pad, d, means, words, false, bf16, nullptr, base + o_A0, base + o_B0, bA0,
-                                    eps0, qwords, qwords + 1, s)) != cudaSuccess)
+                                    eps0, qwords, qwords + 1, ctx->sm_count, s)) != cudaSuccess)
         return cuda_fail(st, e, "query routing: operands");
     KnnPlan px;
     px.nq = q;

@@ -444,7 +444,7 @@ scrust_server* scrust_serve_create(int32_t device, const float* atlas, uint64_t 
         if (e == cudaSuccess)
             e = launch_tensor_operands(sv->atlas, (int64_t)m, sv->m_pad, (int)d, sv->means, sv->words, false, sv->bf16,
                                        nullptr, A16, sv->B16, tmp + 2 * sv->m_pad, tmp + 3 * sv->m_pad, sv->words + 1,
-                                       sv->words + 2, s);
+                                       sv->words + 2, c0->sm_count, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         cudaFree(A16);
         cudaFree(tmp);
