@@ -278,8 +278,10 @@ SCRUST_API int32_t scrust_cuda_batch_plan_launch(scrust_batch_plan* plan, scrust
 /* The autotuner's choice and its time for one batch; returns 0 for NULL. */
 SCRUST_API int32_t scrust_cuda_batch_plan_choice(const scrust_batch_plan* plan, uint32_t* list_capacity,
                                                  int32_t* precision, float* tuned_ms);
-/* The register top-k width the autotuner chose for the sweep: 16 or 32, or 0
- * for candidate lists alone (warp-cooperative prunes); -1 for NULL. */
+/* The register top-k width of the sweep the autotuner chose: 16 or 32 (of its
+ * threshold pass, where it runs a pass for thresholds and one that collects; 1
+ * for k = 1), or 0 for candidate lists alone (warp-cooperative prunes); -1 for
+ * NULL. */
 SCRUST_API int32_t scrust_cuda_batch_plan_topk_width(const scrust_batch_plan* plan);
 
 /* Graphs of many samples.  A plan made by scrust_cuda_batch_plan_create_graphs

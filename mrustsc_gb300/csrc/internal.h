@@ -305,8 +305,9 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
                               const uint32_t* words, const float* dq, int64_t q, int k, uint32_t* d_idx,
                               float* d_dist, scrust_status* st, int most_segments);
 // Column segments of a row block of a routed batch at most, so 128 lists of a
-// row.  (With 16, few queries left most of the chip idle: 30, 300 and 1,000 of a
-// million cells took 427, 1,220 and 855 us, and 334, 609 and 634 us with 64.)
+// row.  (With 16, few queries left most of the chip idle: requests of 30, 300 and
+// 1,000 on a million cells took 531, 1,164 and 1,000 us; 318-416, 643 and 683 us
+// with 64.)
 constexpr int kQuerySegments = 64;
 // What the lists, thresholds and top-K values of a routed batch take of the
 // workspace when its row blocks have `most_segments` segments at most.
@@ -409,7 +410,7 @@ cudaError_t launch_tensor_candidates(scrust_context* ctx, const KnnPlan& plan, c
 cudaError_t launch_merge_part_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,
                                          const uint32_t* counts, const float* bA, const float* bdelta,
                                          const float* beps2, float* theta, cudaStream_t s);
-// The same for rows of up to 32 lists that share row_theta (a query solve's
+// The same for rows of up to 128 lists that share row_theta (a query solve's
 // column segments): row_theta falls to the bound of the k-th of a row's lists
 // together.
 cudaError_t launch_merge_segment_thresholds(const float* topk, int width, int64_t n, int64_t n_pad, int k, int segments,

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) anchor_dist_kernel(const float* __restric
 // lanes' smallest distances has kAnchorNeighbours <= 32 at or below it, one of
 // each lane: the candidates, some hundred and thirty of 3,906, are collected
 // and sorted (a sorted top-32 in every lane, which some lane entered at almost
-// every step, took 150 us for 3,906 anchors; @@ us so).  More of them than
+// every step, took 150 us for 3,906 anchors; 87 us so).  More of them than
 // kTopCap (many anchors at one distance) go through such lists.
 constexpr int kTopCap = 256;
 static_assert(kAnchorNeighbours <= 32, "a bound from one distance a lane");

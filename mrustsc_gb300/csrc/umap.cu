@@ -9,16 +9,17 @@
 // layout is deterministic instead: within an epoch every update is computed
 // from the layout as it stood when the epoch began, and applied as one sum
 // per cell in a fixed order.
-//   - One thread per cell walks its CSR row in order, as the reference walks
-//     the edges whose head is that cell: the same firing schedule
+//   - A cell's CSR row counts in order, as the reference walks the edges whose
+//     head is that cell: the same firing schedule
 //     (epochs_per_sample from max / weight, umap.rs:113-170), the same
 //     per-cell Tausworthe stream for the negative samples (seeded from the
 //     seed and the cell id, umap.rs:407-412), so every cell draws exactly the
 //     reference's negative samples, and the same attraction, repulsion and
-//     +-4 clip (umap.rs:454-509).  It sums the cell's own moves in row order
-//     and keeps each attraction's move of the edge's tail.
-//   - One thread per cell then adds the moves its incoming edges gave it,
-//     in edge order (a stable transpose made once), and writes the cell's
+//     +-4 clip (umap.rs:454-509).  A block takes 32 cells, a thread per edge,
+//     per draw and per sum; the cell's own moves are summed in row order and
+//     each attraction's move of the edge's tail is kept.
+//   - Eight lanes per cell then add the moves its incoming edges gave it,
+//     in edge order (a stable transpose made once), and write the cell's
 //     next position.
 // Two runs with the same inputs give the same bits.  The layout differs from
 // the reference's sequential one by the usual Jacobi-versus-Gauss-Seidel
@@ -159,15 +160,18 @@ __global__ void umap_rescale_kernel(int64_t n, int dim, const uint32_t* __restri
 // draw computes a repulsion; (4) one thread per cell and component adds the
 // cell's moves in order, attraction then samples, edge by edge.  Draws beyond
 // kDraws go through in windows, the streams and sums carrying on.  What bounds
-// it is issue: two or three powf and divisions per move.  A thread per cell
+// it is latency inside a block and the end of the one wave of blocks, not a unit:
+// at 30,000 cells the SMs are busy for 66% of the launch, issue 28% of its
+// slots, the FP64 pipe (the schedule's) is the busiest at 22%, and 36% of a
+// warp's wait is for its block's barriers (while one warp steps the streams and
+// two warps of sums run through the moves, the others stand).  A thread per cell
 // left it to the latency of ~60 moves in a row (613 us an epoch for 30,000
 // cells of 23 edges, 2 components); eight lanes a cell took 131 us, a sixth of
 // its instructions stepping streams in lockstep and its last fifth waiting
 // for cells of five times the mean degree; 74 us so with five blocks an SM, 67
 // with six (42 registers: 30,000 cells are 938 blocks, then all but 26 of them
 // resident; seven spill, 70 us, and so do other splits of the block, 69 to 90).
-// DIM: components (0: `dim`, up to
-// kUmapMaxDim).
+// DIM: components (0: `dim`, up to kUmapMaxDim).
 template <int DIM>
 struct UmapShape {
     static constexpr int kDim = DIM ? DIM : kUmapMaxDim;
