@@ -29,6 +29,12 @@ constexpr int FB_CAP = 4096;  // keys per fallback block
 constexpr int FB_THREADS = 256;
 constexpr int FB_ROWS = 32;      // rows at a time, a cluster each
 constexpr int FB_CLUSTER = 8;
+// Solves of up to this many columns: a block a row, three an SM at a time.  (A
+// row is then short against the cluster's barriers: 700, 2,100, 4,000, 8,000 and
+// 16,000 rows of which every one comes here took 0.99, 2.2, 4.0, 8.6 and 21.5 ms
+// by clusters, 0.47, 0.53, 0.73, 1.5 and 3.9 ms so.  More columns would take
+// more scratch than the 32 rows of a million do.)
+constexpr int64_t FB_BLOCK_COLUMNS = 32768;
 
 struct RerankArgs {
     const float* qx;
@@ -968,15 +974,15 @@ __global__ void __launch_bounds__(RS_BIG_WARPS * 32) rerank_sorted_big_kernel(Re
     }
 }
 
-// A cluster per row, over every reference row of its solve: used for rows whose
+// A cluster (or block) per row, over every reference row of its solve: used for rows whose
 // candidate lists overflowed (many cells within the margin, e.g. duplicates, or
 // data of few dimensions).  Bound by the latency of one SM's row reads: each
 // block measures and counts its share of the columns, and the first one
 // gathers the candidates in its shared memory, sorts and finishes them
 // (300,000 rows of 10 dimensions, k = 20, some 350 rows here: 10.6 ms with a
 // block a row, 1.6 ms so; a launch without rows returns at once).
-__global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
-    rerank_fallback_kernel(RerankArgs a) {
+template <int CLUSTER>
+__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(FB_THREADS) rerank_fallback_kernel(RerankArgs a) {
     if (*a.fb_count == 0u) return;
     namespace cg = cooperative_groups;
     extern __shared__ unsigned long long fb_smem[];
@@ -990,11 +996,23 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
     __shared__ float limit_s, next_s;
     __shared__ int again_s;
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
+    const int rank = CLUSTER == 1 ? 0 : (int)cluster.block_rank(), tid = threadIdx.x;
     const bool first = rank == 0;
-    auto of_first = [&](auto* p) { return cluster.map_shared_rank(p, 0); };
+    auto of_block = [&](auto* p, int b) {
+        if constexpr (CLUSTER == 1)
+            return p;
+        else
+            return cluster.map_shared_rank(p, b);
+    };
+    auto of_first = [&](auto* p) { return of_block(p, 0); };
+    auto sync = [&]() {
+        if constexpr (CLUSTER == 1)
+            __syncthreads();
+        else
+            cluster.sync();
+    };
     BlockTeam team(&scratch);
-    float* sc = a.fb_scratch + (int64_t)(blockIdx.x / FB_CLUSTER) * a.nr;
+    float* sc = a.fb_scratch + (int64_t)(blockIdx.x / CLUSTER) * a.nr;
     for (;;) {
         if (first && tid == 0) {
             const uint32_t i = atomicAdd(a.fb_next, 1u);
@@ -1002,14 +1020,14 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
             sel_prefix = 0;
             sel_rank = a.k;
         }
-        cluster.sync();
+        sync();
         const uint32_t row = *of_first(&row_s);
         if (row == 0xffffffffu) break;
         const int64_t q = query_row(a, row);
         // The columns of the row's own solve, [lo, hi) of the input rows, and
         // the block's share of them.
         const int64_t lo = a.row_lo ? (int64_t)a.row_lo[q] : 0, hi = a.row_lo ? (int64_t)a.row_hi[q] : a.nr;
-        const int64_t j0 = lo + (hi - lo) * rank / FB_CLUSTER, j1 = lo + (hi - lo) * (rank + 1) / FB_CLUSTER;
+        const int64_t j0 = lo + (hi - lo) * rank / CLUSTER, j1 = lo + (hi - lo) * (rank + 1) / CLUSTER;
         for (int64_t j = j0 + tid; j < j1; j += FB_THREADS)
             sc[j] = a.self && j == q + a.self_offset ? __int_as_float(0x7f800000) : compute_r(a, q, (uint32_t)j);
         // k-th smallest of the row: four 8-bit radix passes.
@@ -1023,10 +1041,10 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
                 const uint32_t key = float_key(sc[j]);
                 if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
             }
-            cluster.sync();
+            sync();
             if (first) {
                 uint32_t sum = 0;
-                for (int b = 0; b < FB_CLUSTER; ++b) sum += *cluster.map_shared_rank(&hist[tid], b);
+                for (int b = 0; b < CLUSTER; ++b) sum += *of_block(&hist[tid], b);
                 all[tid] = sum;
                 __syncthreads();
                 if (tid == 0) {
@@ -1041,7 +1059,7 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
                 }
             }
             mask |= 255u << shift;
-            cluster.sync();
+            sync();
         }
         if (first && tid == 0) {
             const float vk = key_float(sel_prefix);
@@ -1052,7 +1070,7 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
         int m = 0;
         for (int attempt = 0; attempt < 8; ++attempt) {
             if (first && tid == 0) cnt_s = outside_s = again_s = 0;
-            cluster.sync();
+            sync();
             const float T = *of_first(&limit_s);
             int* cnt = of_first(&cnt_s);
             unsigned long long* out = of_first(keys);
@@ -1063,7 +1081,7 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
                     if (pos < FB_CAP) out[pos] = ((unsigned long long)float_key(r) << 32) | (uint32_t)j;
                 }
             }
-            cluster.sync();
+            sync();
             m = *cnt;
             if (m > FB_CAP) break;
             if (first) {
@@ -1082,16 +1100,16 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
                              (a.metric == SCRUST_METRIC_COSINE ? 1e-6f : 0.0f);
                 }
             }
-            cluster.sync();
+            sync();
             if (!*of_first(&again_s)) break;
             const float T2 = *of_first(&next_s);
             int outside = 0;
             for (int64_t j = j0 + tid; j < j1; j += FB_THREADS) outside += (sc[j] > T && sc[j] <= T2);
             outside = team.sum(outside);
             if (tid == 0 && outside) atomicAdd(of_first(&outside_s), outside);
-            cluster.sync();
+            sync();
             if (*of_first(&outside_s) == 0) break;
-            cluster.sync();  // all have read it before it is cleared
+            sync();  // all have read it before it is cleared
             if (first && tid == 0) limit_s = T2;
         }
         if (first) {
@@ -1102,9 +1120,9 @@ __global__ void __cluster_dims__(FB_CLUSTER, 1, 1) __launch_bounds__(FB_THREADS)
                 finalize_row(team, a, q, keys, m, dbl, flags);
             }
         }
-        cluster.sync();  // the first block's shared memory is free for the next row
+        sync();  // the first block's shared memory is free for the next row
     }
-    cluster.sync();  // it stays until all have read the last row
+    sync();  // it stays until all have read the last row
 }
 
 // Distances of cosine rows' neighbours, one a thread: the f32 value that the
@@ -1139,8 +1157,10 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     cudaError_t e;
     uint32_t* fb_rows = (uint32_t*)ws_get(ctx, SLOT_FALLBACK_ROWS, sizeof(uint32_t) * (size_t)plan.nq, &e);
     if (!fb_rows) return e;
+    const bool fb_blocks = plan.nr <= FB_BLOCK_COLUMNS;
+    const int fb_at_once = fb_blocks ? (int)std::min<int64_t>(plan.nq, 3 * ctx->sm_count) : FB_ROWS;
     float* fb_scratch =
-        (float*)ws_get(ctx, SLOT_FALLBACK_SCRATCH, sizeof(float) * (size_t)plan.nr * FB_ROWS, &e);
+        (float*)ws_get(ctx, SLOT_FALLBACK_SCRATCH, sizeof(float) * (size_t)plan.nr * fb_at_once, &e);
     if (!fb_scratch) return e;
     RerankArgs a;
     a.qx = qx;
@@ -1238,9 +1258,10 @@ cudaError_t launch_rerank(scrust_context* ctx, const KnnPlan& plan, const float*
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t smem_f = (size_t)FB_CAP * (sizeof(unsigned long long) + sizeof(double) + 1);
-    e = set_smem_limit(ctx, (const void*)rerank_fallback_kernel, (int)smem_f);
+    const auto fallback = fb_blocks ? rerank_fallback_kernel<1> : rerank_fallback_kernel<FB_CLUSTER>;
+    e = set_smem_limit(ctx, (const void*)fallback, (int)smem_f);
     if (e != cudaSuccess) return e;
-    rerank_fallback_kernel<<<FB_ROWS * FB_CLUSTER, FB_THREADS, smem_f, ctx->stream>>>(a);
+    fallback<<<fb_at_once * (fb_blocks ? 1 : FB_CLUSTER), FB_THREADS, smem_f, ctx->stream>>>(a);
     ctx->launches += 1;
     if (a.post) {
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
