@@ -1010,75 +1010,69 @@ __global__ void __launch_bounds__(256) query_tiles_kernel(const T* __restrict__ 
     __shared__ float reach[64], query2[64], centre2[4][64];
     __shared__ uint32_t hit[64];
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    const int64_t j0 = (int64_t)blockIdx.x * 64;
+    const int64_t i0 = (int64_t)blockIdx.y * 64, j0 = (int64_t)blockIdx.x * 64;
     const int r = threadIdx.x % 64, part = threadIdx.x / 64;
-    // (gridDim.y is 65,535 at most: more groups of queries take turns.)
-    for (int64_t i0 = (int64_t)blockIdx.y * 64;;) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int t = 8 * (part + 4 * c);
-            uint4 w = make_uint4(0u, 0u, 0u, 0u);
-            if (i0 + r < q) w = __ldg(reinterpret_cast<const uint4*>(ops + (i0 + r) * 64 + t));
-            const T* v = reinterpret_cast<const T*>(&w);
+    for (int c = 0; c < 2; ++c) {
+        const int t = 8 * (part + 4 * c);
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (i0 + r < q) w = __ldg(reinterpret_cast<const uint4*>(ops + (i0 + r) * 64 + t));
+        const T* v = reinterpret_cast<const T*>(&w);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) As[t + e][r] = t + e < d ? op_float(v[e]) : 0.f;
+        for (int e = 0; e < 8; ++e) As[t + e][r] = t + e < d ? op_float(v[e]) : 0.f;
+    }
+    float c2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {  // (the centres come dimension by dimension)
+        const int t = part + 4 * c;
+        const float v = j0 + r < asegs && t < d ? __ldg(act + (int64_t)t * asegs + j0 + r) : 0.f;
+        Bs[t][r] = v;
+        c2 += v * v;
+    }
+    centre2[part][r] = c2;
+    if (threadIdx.x < 64) {
+        hit[threadIdx.x] = 0u;
+        const int64_t i = i0 + threadIdx.x;
+        float u = 0.f;
+        query2[threadIdx.x] = i < q ? bA[i] : 0.f;
+        if (i < q) {
+            // Every step rounded up; a row without a threshold reaches all.
+            const uint32_t key = row_theta[i];
+            const float th = key == 0xffffffffu ? __int_as_float(0x7f800000) : key_float(key);
+            const float v = __fadd_ru(__fadd_ru(th, bA[i]), bdelta[i]);
+            u = isinf(th) && th > 0.f ? th : (v > 0.f ? __fsqrt_ru(v) : 0.f);
         }
-        float c2 = 0.f;
+        reach[threadIdx.x] = u;
+    }
+    __syncthreads();
+    float acc[4][4] = {};
+    for (int t = 0; t < d; ++t) {
+        const float4 a4 = *reinterpret_cast<const float4*>(&As[t][ty * 4]);
+        const float4 b4 = *reinterpret_cast<const float4*>(&Bs[t][tx * 4]);
+        const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {  // (the centres come dimension by dimension)
-            const int t = part + 4 * c;
-            const float v = j0 + r < asegs && t < d ? __ldg(act + (int64_t)t * asegs + j0 + r) : 0.f;
-            Bs[t][r] = v;
-            c2 += v * v;
-        }
-        centre2[part][r] = c2;
-        if (threadIdx.x < 64) {
-            hit[threadIdx.x] = 0u;
-            const int64_t i = i0 + threadIdx.x;
-            float u = 0.f;
-            query2[threadIdx.x] = i < q ? bA[i] : 0.f;
-            if (i < q) {
-                // Every step rounded up; a row without a threshold reaches all.
-                const uint32_t key = row_theta[i];
-                const float th = key == 0xffffffffu ? __int_as_float(0x7f800000) : key_float(key);
-                const float v = __fadd_ru(__fadd_ru(th, bA[i]), bdelta[i]);
-                u = isinf(th) && th > 0.f ? th : (v > 0.f ? __fsqrt_ru(v) : 0.f);
-            }
-            reach[threadIdx.x] = u;
-        }
-        __syncthreads();
-        float acc[4][4] = {};
-        for (int t = 0; t < d; ++t) {
-            const float4 a4 = *reinterpret_cast<const float4*>(&As[t][ty * 4]);
-            const float4 b4 = *reinterpret_cast<const float4*>(&Bs[t][tx * 4]);
-            const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
+        for (int p = 0; p < 4; ++p)
 #pragma unroll
-            for (int p = 0; p < 4; ++p)
+            for (int c = 0; c < 4; ++c) acc[p][c] = fmaf(av[p], bv[c], acc[p][c]);
+    }
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc[p][c] = fmaf(av[p], bv[c], acc[p][c]);
-        }
+    for (int c = 0; c < 4; ++c) {
+        const int64_t j = j0 + tx * 4 + c;
+        if (j >= asegs) continue;
+        const float rj = ar[j];
+        const int cj = tx * 4 + c;
+        const float b2 = centre2[0][cj] + centre2[1][cj] + centre2[2][cj] + centre2[3][cj];
+        bool any = false;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int64_t j = j0 + tx * 4 + c;
-            if (j >= asegs) continue;
-            const float rj = ar[j];
-            const int cj = tx * 4 + c;
-            const float b2 = centre2[0][cj] + centre2[1][cj] + centre2[2][cj] + centre2[3][cj];
-            bool any = false;
-#pragma unroll
-            for (int p = 0; p < 4; ++p)
-                any |= i0 + ty * 4 + p < q &&
-                       tile_needed(centres_apart(query2[ty * 4 + p], b2, acc[p][c], d), 0.f, rj, reach[ty * 4 + p]);
-            if (any) hit[tx * 4 + c] = 1u;
-        }
-        __syncthreads();
-        if (threadIdx.x < 64 && hit[threadIdx.x]) {
-            const uint32_t tile = ao[j0 + threadIdx.x];
-            atomicOr(bitmap + i0 / 256 * words + (tile >> 5), 1u << (tile & 31));
-        }
-        i0 += (int64_t)gridDim.y * 64;
-        if (i0 >= q) return;
-        __syncthreads();
+        for (int p = 0; p < 4; ++p)
+            any |= i0 + ty * 4 + p < q &&
+                   tile_needed(centres_apart(query2[ty * 4 + p], b2, acc[p][c], d), 0.f, rj, reach[ty * 4 + p]);
+        if (any) hit[tx * 4 + c] = 1u;
+    }
+    __syncthreads();
+    if (threadIdx.x < 64 && hit[threadIdx.x]) {
+        const uint32_t tile = ao[j0 + threadIdx.x];
+        atomicOr(bitmap + i0 / 256 * words + (tile >> 5), 1u << (tile & 31));
     }
 }
 
@@ -1932,16 +1926,23 @@ int32_t cross_ordered_enqueue(scrust_context* ctx, const AtlasOrder& at, const f
     ctx->launches += topk ? 1 : 0;
     // The atlas tiles each row block cannot rule out: its queries, with the
     // reach of their shared thresholds, against the atlas segment balls.
-    if (at.segs) {
-        const dim3 grid((unsigned)((at.segs + 63) / 64), (unsigned)std::min<int64_t>((q + 63) / 64, 65535));
+    // (A grid's second dimension ends at 65,535: more groups of 64 queries take
+    // more launches, whole row blocks each.)
+    constexpr int64_t kMostGroups = 65532;
+    static_assert(kMostGroups % 4 == 0 && kMostGroups <= 65535, "whole row blocks of 256 queries");
+    for (int64_t i0 = 0; at.segs && i0 < q; i0 += 64 * kMostGroups) {
+        const int64_t here = std::min<int64_t>(q - i0, 64 * kMostGroups);
+        const dim3 grid((unsigned)((at.segs + 63) / 64), (unsigned)((here + 63) / 64));
+        const char* ops = base + o_As + 128 * (size_t)i0;
+        uint32_t* bits = bitmap + i0 / 256 * words_t;
         if (bf16)
-            query_tiles_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)(base + o_As), q, row_theta, bA,
-                                                                   bdelta, at.seg_centre_t, at.seg_radius, at.seg_tile,
-                                                                   at.segs, d, words_t, bitmap);
+            query_tiles_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)ops, here, row_theta + i0, bA + i0,
+                                                                   bdelta + i0, at.seg_centre_t, at.seg_radius,
+                                                                   at.seg_tile, at.segs, d, words_t, bits);
         else
-            query_tiles_kernel<__half><<<grid, 256, 0, s>>>((const __half*)(base + o_As), q, row_theta, bA, bdelta,
+            query_tiles_kernel<__half><<<grid, 256, 0, s>>>((const __half*)ops, here, row_theta + i0, bA + i0, bdelta + i0,
                                                             at.seg_centre_t, at.seg_radius, at.seg_tile, at.segs, d,
-                                                            words_t, bitmap);
+                                                            words_t, bits);
     }
     const size_t lists_smem = 4 * (size_t)words_t;
     if ((e = cudaGetLastError()) != cudaSuccess ||
