@@ -622,9 +622,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 // H: w x w, symmetric, so its rows serve as its columns; overwritten with the
 // rotated columns (column j at H + j w), scaled by a power of two.  V: w x w,
 // column j at V + j w.  lambda: w eigenvalues (between sweeps: squared norms).
-// rotated: kJacobiSweeps flags, zero on entry.
+// rotated: kJacobiSweeps flags, zero on entry.  root: w values of scratch.
+// An eigenvalue below zero, or one that f32 cannot resolve, is 0 on return: the
+// loadings B^T v / sqrt(lambda) are f32 sums of terms of up to
+// |b_a| |v_a| / sqrt(lambda), b_a the rows of B, |b_a|^2 the diagonal of H, and
+// where those come to 2^24 and more nothing of the unit vector they stand for
+// is left (constant columns of 300 x 40: loadings of norm 2e5, and infinite ones).
 __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiThreads)
-    pca_jacobi_kernel(double* H, double* V, int w, double* lambda, int* rotated, int* __restrict__ err) {
+    pca_jacobi_kernel(double* H, double* V, int w, double* lambda, double* root, int* rotated, int* __restrict__ err) {
     constexpr int SLOTS = kPcaMaxWidth / 32;
     constexpr int WARPS = kJacobiBlocks * kJacobiThreads / 32;
     constexpr double EPS = 2.220446049250313e-16;
@@ -642,7 +647,9 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
     cluster_barrier();  // everyone has read the diagonal
     for (int c = slot; c < w; c += WARPS)
         for (int i = lane; i < w; i += 32) {
-            __stcg(H + (int64_t)c * w + i, __ldcg(H + (int64_t)c * w + i) * scale);
+            const double h = __ldcg(H + (int64_t)c * w + i);
+            if (i == c) __stcg(root + c, sqrt(fmax(h, 0.0)));
+            __stcg(H + (int64_t)c * w + i, h * scale);
             __stcg(V + (int64_t)c * w + i, i == c ? 1.0 : 0.0);
         }
     // Orthogonal: to 16 roundings, whatever the columns' sizes (the Gram of a
@@ -728,10 +735,15 @@ __global__ void __cluster_dims__(kJacobiBlocks, 1, 1) __launch_bounds__(kJacobiT
     if (!done && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(err, 2);
     const double back = ldexp(1.0, ex);
     for (int c = slot; c < w; c += WARPS) {
-        double l = 0.0;
-        for (int i = lane; i < w; i += 32) l += __ldcg(V + (int64_t)c * w + i) * __ldcg(H + (int64_t)c * w + i);
-        l = warp_sum(l);
-        if (lane == 0) __stcg(lambda + c, l * back);
+        double l = 0.0, terms = 0.0;
+        for (int i = lane; i < w; i += 32) {
+            const double v = __ldcg(V + (int64_t)c * w + i);
+            l += v * __ldcg(H + (int64_t)c * w + i);
+            terms += fabs(v) * __ldcg(root + i);
+        }
+        l = warp_sum(l) * back;
+        terms = warp_sum(terms) * 5.9604644775390625e-8;  // 2^-24
+        if (lane == 0) __stcg(lambda + c, l >= terms * terms && l >= 1.1754943508222875e-38 ? l : 0.0);  // f32's smallest
     }
 }
 
@@ -750,7 +762,7 @@ __global__ void pca_select_kernel(const double* __restrict__ lambda, const doubl
     for (int i = lane; i < w; i += 32) before += lambda[i] > l || (lambda[i] == l && i < idx);
     const int c = __reduce_add_sync(0xffffffffu, before);
     if (c >= nc) return;
-    const double s = sqrt(fmax(l, 0.0));  // (below zero: rounding past the rank)
+    const double s = sqrt(l);
     if (lane == 0) sing[c] = s;
     const double inv = s > 0.0 ? 1.0 / s : 0.0;
     for (int r = lane; r < w; r += 32) {
@@ -840,7 +852,7 @@ size_t al(size_t v) { return (v + 255) & ~(size_t)255; }
 
 struct PcaWork {
     float *omega, *Y, *Z, *mvec, *colsum, *mean, *T, *basis, *scaled, *ct;
-    double *var_term, *total, *gram_part, *G, *V, *lambda, *sing, *colpart;
+    double *var_term, *total, *gram_part, *G, *V, *lambda, *root, *sing, *colpart;
     uint32_t *kA, *kB, *cstart;
     unsigned long long *vA, *vB;
     uint32_t *hist, *scan;
@@ -879,7 +891,7 @@ int32_t pca_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint3
                  o_t = take(4 * (size_t)w * w), o_basis = take(4 * (size_t)w * nc), o_sc = take(4 * (size_t)w * nc),
                  o_ct = take(4 * (size_t)g * nc), o_vt = take(8 * (size_t)g), o_tot = take(8),
                  o_gp = take(8 * (size_t)gram_blocks * entries), o_g = take(8 * (size_t)w * w),
-                 o_v = take(8 * (size_t)w * w), o_lam = take(8 * (size_t)w), o_sing = take(8 * (size_t)nc),
+                 o_v = take(8 * (size_t)w * w), o_lam = take(8 * (size_t)w), o_root = take(8 * (size_t)w), o_sing = take(8 * (size_t)nc),
                  o_cp = take(8 * (size_t)col_blocks * w), o_ka = take(4 * (size_t)nnz), o_kb = take(4 * (size_t)nnz),
                  o_cst = take(4 * (size_t)(g + 1)), o_va = take(8 * (size_t)nnz), o_vb = take(8 * (size_t)nnz),
                  o_hist = take(4 * ((size_t)256 * nb + 16)), o_scan = take(4 * wk.scan_elems),
@@ -902,6 +914,7 @@ int32_t pca_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint3
     wk.G = (double*)(base + o_g);
     wk.V = (double*)(base + o_v);
     wk.lambda = (double*)(base + o_lam);
+    wk.root = (double*)(base + o_root);
     wk.sing = (double*)(base + o_sing);
     wk.colpart = (double*)(base + o_cp);
     wk.kA = (uint32_t*)(base + o_ka);
@@ -998,7 +1011,7 @@ int32_t pca_device_impl(scrust_context* ctx, const uint32_t* indptr, const uint3
     // B^T = X_c^T Q (g x w), its Gram, the eigenpairs, the outputs.
     if ((e = transpose_times(wk.Y, wk.Z)) != cudaSuccess || (e = gram(wk.Z, g)) != cudaSuccess)
         return cuda_fail(st, e, "pca: projection");
-    pca_jacobi_kernel<<<kJacobiBlocks, kJacobiThreads, 0, s>>>(wk.G, wk.V, w, wk.lambda, rotated, err);
+    pca_jacobi_kernel<<<kJacobiBlocks, kJacobiThreads, 0, s>>>(wk.G, wk.V, w, wk.lambda, wk.root, rotated, err);
     pca_select_kernel<<<(w + 7) / 8, 256, 0, s>>>(wk.lambda, wk.V, w, nc, wk.basis, wk.scaled, wk.sing);
     rows_mul(wk.Y, n, wk.basis, nc, emb, nc);
     rows_mul(wk.Z, g, wk.scaled, nc, wk.ct, nc);

@@ -37,3 +37,36 @@ def test_loadings_past_the_rank_are_orthonormal(built_library, rank, zero_center
     # The scores past the rank: what f32 products of 200 terms leave of the first.
     size = np.linalg.norm(res["embedding"].astype(np.float64), axis=0)
     assert np.all(size[rank:] <= 200 * 2.0 ** -24 * size[0])
+
+
+def with_constant_columns(n, g):
+    x = np.random.default_rng(n * g).random((n, g))
+    x[:, ::2] = 3.0
+    return x
+
+
+def two_kinds_of_rows(n, g):
+    x = np.zeros((n, g))
+    x[: n // 2] = 1.0
+    return x
+
+
+@pytest.mark.parametrize("make", [with_constant_columns, two_kinds_of_rows])
+@pytest.mark.parametrize("n,g", [(20, 50), (33, 33), (300, 40), (150, 300)])
+@pytest.mark.parametrize("zero_center", [True, False])
+def test_loadings_of_nothing_are_small(built_library, make, n, g, zero_center):
+    """All components of matrices of low rank: where f32 resolves nothing of a
+    component its loadings are zero; else their error is at most what it could
+    resolve, the component's own size 1, so that no norm passes 2."""
+    from mrustsc_gb300 import _lib, _scrust
+
+    m = sp.csr_matrix(make(n, g).astype(np.float32))
+    nc = min(n, g, 40)
+    try:
+        res = _scrust.pca(m.indptr.astype(np.uint32), m.indices.astype(np.uint32), m.data, g, nc, zero_center, 0, "auto")
+    except _lib.ScrustError as e:
+        assert "did not converge" in str(e) and make is two_kinds_of_rows  # refused, as it was
+        return
+    assert np.isfinite(res["components"]).all() and np.isfinite(res["embedding"]).all()
+    assert np.linalg.norm(res["components"].astype(np.float64), axis=1).max() <= 2.0
+    assert np.all(res["explained_variance"] >= 0)
